@@ -13,11 +13,10 @@ namespace {
 
 constexpr int kTile = 9;  // tile nodes per axis: [4b-2, 4b+6]
 constexpr int kTile3 = kTile * kTile * kTile;
-// A work item holds up to kItemMax particles binned to one home block b. A
+// A work item holds up to kItemMax particles (one per thread) binned to one home block b. A
 // particle whose base cell lies in [4b-1, 4b+4] (the home block plus one
 // cell of drift each way) has its whole stencil inside the tile; its base
 // cell has tile-local coordinates lc = base - (4b-2) - 1 in [0, 5]^3.
-constexpr int kItemMax = 256;
 // What a P2G tile pass accumulates: the grid mass alone (gMassCompute.glsl),
 // mass, momentum and stress force (p2gTransfer.glsl), or only a force-like
 // 3-vector per node (the semi-implicit solve's K u, into the force slots).
@@ -28,9 +27,15 @@ template <int KIND> struct P2gFields {
 };
 constexpr int kCellsPerAxis = kTile - 3;  // 6
 constexpr int kCells = kCellsPerAxis * kCellsPerAxis * kCellsPerAxis;
-constexpr int kPd = 11;  // float4 per particle of P2G data in shared memory: 10 used, the 11th pads
-                         // the stride to 44 words so the 8 threads of a 16-byte store phase hit 8
-                         // distinct groups of 4 banks
+// P2G data in shared memory: two particles share one record, their values
+// interleaved word by word (first particle's in the even word), so that a
+// 16-byte load fills two operand pairs of the packed FP32 instructions and one
+// instruction serves both particles. Order of the 38 pairs: A22, m, mv (3),
+// A00, A01, A02, A10, A11, A12, A20, A21, unused, wx[4], gx[4], (wy, gy)[4],
+// (wz, gz)[4].
+constexpr int kPdPairs = 38;
+constexpr int kPdStride = 2 * kPdPairs;  // words per record (304 bytes: 16-byte loads stay aligned)
+enum { kPdA22 = 0, kPdM = 1, kPdMv = 2, kPdA = 5, kPdWx = 14, kPdGx = 18, kPdY = 22, kPdZ = 30 };
 constexpr int kShColliders = 16;  // colliders cached in shared memory
 
 __device__ __forceinline__ int find_scene(const int* __restrict__ prefix, int nscenes, long long u) {
@@ -47,6 +52,39 @@ __device__ __forceinline__ int find_scene(const int* __restrict__ prefix, int ns
 
 __device__ __forceinline__ float sel4(int i, float a0, float a1, float a2, float a3) {
   return i == 0 ? a0 : (i == 1 ? a1 : (i == 2 ? a2 : a3));
+}
+
+// ---- packed FP32 pairs -----------------------------------------------------
+// Two floats in one 64-bit register pair; each half rounds as the scalar
+// instruction does.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, unsigned& lo, unsigned& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float lo2(f32x2 v) {
+  unsigned a, b;
+  unpack2(v, a, b);
+  return __uint_as_float(a);
+}
+__device__ __forceinline__ float hi2(f32x2 v) {
+  unsigned a, b;
+  unpack2(v, a, b);
+  return __uint_as_float(b);
 }
 
 // Axis weights of the 4 stencil nodes base-1 .. base+2 (cubic.include.glsl):
@@ -413,7 +451,7 @@ __device__ __forceinline__ int fix_force(float wxa, float gxa, const RowFactors&
 }
 
 // Scatter of one particle's 64 stencil nodes straight into acc (global
-// atomics), for a particle outside its work item's tile. FAST: the particle
+// atomics; loops not unrolled, the code's size counts), for a particle outside its work item's tile. FAST: the particle
 // fits the fast path's range and its contributions are rounded exactly as
 // the tile path rounds them; otherwise (wide) each contribution is rounded in
 // double precision to int64. ms, mvs, As: the scaled quantities.
@@ -421,13 +459,16 @@ template <int KIND, bool FAST>
 __device__ __forceinline__ void scatter_fix(const SceneDev& S, float ms, const float mvs[3], const float As[3][3],
                                             const AxisW& w, const int base[3]) {
   constexpr bool mo = KIND == kP2gMass;
+#pragma unroll 1
   for (int c = 0; c < 4; c++)
+#pragma unroll 1
     for (int b = 0; b < 4; b++) {
       const int g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
       if (g1 < 0 || g2 < 0 || g1 >= S.dim[1] || g2 >= S.dim[2]) continue;
       RowFactors f;
       row_factors(ms, mvs, As, sel4(b, w.wy[0], w.wy[1], w.wy[2], w.wy[3]), sel4(b, w.gy[0], w.gy[1], w.gy[2], w.gy[3]),
                   sel4(c, w.wz[0], w.wz[1], w.wz[2], w.wz[3]), sel4(c, w.gz[0], w.gz[1], w.gz[2], w.gz[3]), mo, f);
+#pragma unroll 1
       for (int a = 0; a < 4; a++) {
         const int g0 = base[0] - 1 + a;
         if (g0 < 0 || g0 >= S.dim[0]) continue;
@@ -466,8 +507,11 @@ __device__ __forceinline__ void scatter_fix(const SceneDev& S, float ms, const f
 // grid update and the next P2G; the solve's node passes read and clear them).
 __device__ __forceinline__ void scatter_force(const SceneDev& S, const P2GParticle& q, const AxisW& w, const int base[3]) {
   if (!q.force) return;
+#pragma unroll 1
   for (int c = 0; c < 4; c++)
+#pragma unroll 1
     for (int b = 0; b < 4; b++)
+#pragma unroll 1
       for (int a = 0; a < 4; a++) {
         const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
         if (!node_in_grid(S, g0, g1, g2)) continue;
@@ -489,19 +533,34 @@ __device__ __forceinline__ void scatter_force(const SceneDev& S, const P2GPartic
 }
 
 // ---- shared memory of one work item --------------------------------------
+// The staged grid values: the tile's 9 x 9 rows of nodes, each row copied from
+// the dense array in one piece that starts and ends on a 16-byte boundary.
+// gout: rows of 10 nodes from x = 4b - 2; u of the solve: 12 nodes from
+// 4b - 4. The planes' stride is padded so that a step in z and one in y lie in
+// different banks.
+template <int FIELDS> struct StageShape {
+  static constexpr int x0 = FIELDS == kOutFields ? 2 : 4;    // first node of a row is 4b - x0
+  static constexpr int row_nodes = FIELDS == kOutFields ? 10 : 12;
+  static constexpr int row = FIELDS * row_nodes;             // floats: 60 / 36
+  static constexpr int plane = kTile * row + (FIELDS == kOutFields ? 8 : 4);
+  static_assert(row * sizeof(float) % 16 == 0 && plane * sizeof(float) % 16 == 0, "rows of whole 16-byte words");
+};
+constexpr int kStageFloats = kTile * StageShape<kOutFields>::plane;
+static_assert(kTile * StageShape<kImpFields>::plane <= kStageFloats, "the solve's rows fit the same buffer");
+
 struct ItemShared {
-  float stage[27][kOutBlockFloats];  // G2P: the pool blocks around the home block
-  float4 pd[kItemMax][kPd];          // P2G: per-particle data, in tile-cell order
+  __align__(16) float stage[kStageFloats];             // G2P: the grid values of the tile's nodes
+  // the item's particles: its stretch of each stream (fc from an even particle on)
+  float4 pxm[kItemMax], pvv[kItemMax], pfa[kItemMax], pfb[kItemMax], pvq[kItemMax];
+  float2 pfc[kItemMax + 2];
+  __align__(16) float pd[kItemMax / 2 * kPdStride];  // P2G: particle data in tile-cell order, by pairs
   union {
     int tilei[kAccFields * kTile3];  // P2G sums of the tile's nodes (fixed point: mass, momentum, force) ...
     float tile[kAccFields * kTile3]; // ... or float (the semi-implicit solve's K u)
   };
   int cstart[kCells + 1];            // first pd slot of each tile cell
   int ccount[kCells];                // particles per tile cell (zero between items)
-  int wsum[kItemMax / 32];
-  int wocc[kItemMax / 32];
   short cells[kCells];               // occupied tile cells
-  int ncells;
   int4 item_q[2];                    // this and the next work item of the CTA
   int scene_q[2];                    // ... and their scenes
   int coll_scene;                    // scene whose colliders sit in coll
@@ -509,23 +568,16 @@ struct ItemShared {
   unsigned seen[3];                  // largest mass, |v|, force-term bound of coll_scene's particles (bits) ...
   unsigned pushed[3];                // ... and the part of them already recorded in FixState
   int next_same;                     // the CTA's next work item continues this item's home-block run
-  int next_issue;                    // ... or starts a run whose pool blocks the last warp copies
-  int next_slot[32];                 // the pool slots of those blocks (lane k: tile block k)
+  int next_issue;                    // ... or starts a run whose grid rows the last warp copies
   float run_bound;                   // sum of the contribution bounds of the particles in the tile's sums
   float item_bound;                  // ... and of this item's particles headed for the tile
-  int abort;                         // 1 + parity of a copy wait that ran out, else 0
-  uint64_t bar;
+  int abort;                         // 1 + parity of a wait for grid rows that ran out, else 0
+  int pabort;                        // ... for particles
+  uint64_t bar, pbar;                // completion of the grid rows' copies, of the particles'
   snow_collider coll[kShColliders];
   float4 chit[kShColliders];         // packed hit tests of the colliders
   int ctype[kShColliders];
 };
-
-// Tile block k (0..26) around home block (bx, by, bz), or -1 outside the grid.
-__device__ __forceinline__ int tile_block(const SceneDev& S, int bx, int by, int bz, int k) {
-  const int cx = bx - 1 + k % 3, cy = by - 1 + (k / 3) % 3, cz = bz - 1 + k / 9;
-  const bool in = cx >= 0 && cy >= 0 && cz >= 0 && cx < S.bdim[0] && cy < S.bdim[1] && cz < S.bdim[2];
-  return in ? block_id(S, cx, cy, cz) : -1;
-}
 
 __device__ __forceinline__ void home_coords(const SceneDev& S, int blk, int& bx, int& by, int& bz) {
   bx = blk % S.bdim[0];
@@ -533,45 +585,80 @@ __device__ __forceinline__ void home_coords(const SceneDev& S, int blk, int& bx,
   bz = blk / (S.bdim[0] * S.bdim[1]);
 }
 
-// Pool slot of tile block k of item `it`; -1: no block.
-__device__ __forceinline__ int tile_slot(const SceneDev& S, int4 it, int k) {
-  if (k >= 27) return -1;
-  int bx, by, bz;
-  home_coords(S, it.x, bx, by, bz);
-  const int b = tile_block(S, bx, by, bz, k);
-  return b < 0 ? -1 : __ldg(&S.blk_slot[b]);
+// Index of node (x, y, z) of the blocked grid in gout and cru.
+__device__ __forceinline__ size_t node_index(const SceneDev& S, int x, int y, int z) {
+  return ((size_t)z * (4 * S.bdim[1]) + y) * (4 * S.bdim[0]) + x;
 }
 
-// One full warp issues the bulk copies (TMA) of the tile's pool blocks into
-// `stage` (lane k < 27 copies block k, `block_floats` floats from pool slot
-// `slot` of `pool`; block_floats <= 384 and a multiple of 4) and zero-fills
-// the blocks without a slot; completion lands on sh.bar, which expects
+// Every thread of the CTA calls it: issues the bulk copies (TMA) of the rows,
+// one per thread, of the tile around home block `home` from the dense array `grid` into `stage` and zero-fills
+// what lies outside the grid; completion lands on sh.bar, which expects
 // `unsent` bytes more than are copied (0 except in tests of the timeout
-// path). The caller guarantees nobody reads `stage` until the barrier's
-// phase completes and that all earlier reads of `stage` are done.
-__device__ __forceinline__ void stage_issue(ItemShared& sh, const float* pool, int block_floats, int slot,
-                                            uint32_t unsent) {
-  const int k = threadIdx.x & 31;
-  const bool mine = k < 27 && slot >= 0;
-  const uint32_t bytes = (uint32_t)(block_floats * sizeof(float));
-  const uint32_t valid = __ballot_sync(0xffffffffu, mine);
-  if (k == 0) mbar_arrive_expect_tx(&sh.bar, __popc(valid) * bytes + unsent);
-  __syncwarp();
-  if (mine) {
+// path). The caller guarantees nobody reads `stage` until the barrier's phase
+// completes and that all earlier reads of `stage` are done. Rows instead of
+// the 27 whole blocks around the home block: 19 KB of shared memory instead
+// of 41 (the rest holds the next item's particles), and every stencil node at
+// a constant offset from the particle's first instead of through twelve
+// address registers.
+template <int FIELDS>
+__device__ __forceinline__ void stage_issue(ItemShared& sh, const SceneDev& S, const float* grid, int home) {
+  using T = StageShape<FIELDS>;
+  int bx, by, bz;
+  home_coords(S, home, bx, by, bz);
+  const int nx = 4 * S.bdim[0], ny = 4 * S.bdim[1], nz = 4 * S.bdim[2];
+  const int xs = 4 * bx - T::x0, xa = max(xs, 0), xe = min(xs + T::row_nodes, nx);  // multiples of 16 bytes: x0 and nx are
+  const uint32_t bytes = (uint32_t)((xe - xa) * FIELDS * (int)sizeof(float));
+  const int y0 = max(0, 2 - 4 * by), y1 = min(kTile, ny - (4 * by - 2));  // rows inside the grid
+  const int z0 = max(0, 2 - 4 * bz), z1 = min(kTile, nz - (4 * bz - 2));
+  if (threadIdx.x == 0) mbar_arrive_expect_tx(&sh.bar, (uint32_t)((y1 - y0) * (z1 - z0)) * bytes + S.tx_unsent);
+  static_assert(kTile * kTile <= kItemMax, "a row per thread");
+  if (threadIdx.x < kTile * kTile) {
     fence_proxy_async_smem();
-    bulk_g2s(sh.stage[k], pool + (size_t)slot * block_floats, bytes, &sh.bar);
-  }
-  uint32_t missing = __ballot_sync(0xffffffffu, k < 27 && slot < 0);
-  while (missing) {
-    const int m = __ffs(missing) - 1;
-    missing &= missing - 1;
-    float4* dst = reinterpret_cast<float4*>(sh.stage[m]);
-    for (int i = k; i < block_floats / 4; i += 32) dst[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int y = threadIdx.x % kTile, z = threadIdx.x / kTile;
+    float* dst = sh.stage + z * T::plane + y * T::row;
+    bool copied = false;
+    if (y >= y0 && y < y1 && z >= z0 && z < z1) {
+      bulk_g2s(dst + (xa - xs) * FIELDS, grid + node_index(S, xa, 4 * by - 2 + y, 4 * bz - 2 + z) * FIELDS, bytes, &sh.bar);
+      copied = true;
+      if (xe - xa == T::row_nodes) return;
+    }
+    for (int x = 0; x < T::row_nodes; x++)
+      if (!copied || x < xa - xs || x >= xe - xs)
+#pragma unroll
+        for (int f = 0; f < FIELDS; f++) dst[x * FIELDS + f] = 0.0f;
   }
 }
-// ... of the grid update's output (v*, d).
-__device__ __forceinline__ void stage_issue(ItemShared& sh, const SceneDev& S, int slot) {
-  stage_issue(sh, S.gout, kOutBlockFloats, slot, S.tx_unsent);
+
+// One full warp issues the bulk copies of the particles [first, first + count)
+// (a stretch of each stream, or of the binned copies) into the CTA's particle
+// buffer; completion lands on sh.pbar. The caller guarantees that all earlier
+// reads of the buffer are done. The loads of an item's particles are then
+// under way while the CTA sums the previous item, instead of being waited for
+// at the item's start and again before its advance.
+__device__ __forceinline__ void particles_issue(ItemShared& sh, const SceneDev& S, int first, int count, bool binned) {
+  const int lane = threadIdx.x & 31;
+  const int f0 = first & ~1, fn = (first + count - f0 + 1) & ~1;  // fc: whole 16-byte words (the streams' allocations are whole 256-byte units)
+  if (lane == 0) mbar_arrive_expect_tx(&sh.pbar, (uint32_t)(count * 5 * sizeof(float4) + fn * sizeof(float2)));
+  __syncwarp();
+  if (lane < 6) {
+    fence_proxy_async_smem();
+    const float4* src4[5] = {binned ? S.bxm : S.xm, binned ? S.bvv : S.vv, binned ? S.bfa : S.fa, binned ? S.bfb : S.fb,
+                             binned ? S.bvq : S.vq};
+    float4* dst4[5] = {sh.pxm, sh.pvv, sh.pfa, sh.pfb, sh.pvq};
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+      if (lane == k) bulk_g2s(dst4[k], src4[k] + first, (uint32_t)(count * sizeof(float4)), &sh.pbar);
+    if (lane == 5) bulk_g2s(sh.pfc, (binned ? S.bfc : S.fc) + f0, (uint32_t)(fn * sizeof(float2)), &sh.pbar);
+  }
+}
+// Waits for them, as stage_wait does for the grid rows.
+__device__ __forceinline__ bool particles_wait(ItemShared& sh, const SceneDev& S, uint32_t& phase) {
+  if (!mbar_wait(&sh.pbar, phase, S.wait_ns)) {
+    sh.pabort = 1 + (int)phase;
+    return false;
+  }
+  phase ^= 1u;
+  return true;
 }
 
 // Every thread waits for the stage copies of the current phase, at most
@@ -595,7 +682,8 @@ __device__ __forceinline__ bool stage_wait(ItemShared& sh, const SceneDev& S, ui
 __device__ __forceinline__ void stage_abort(ItemShared& sh, const SceneDev& S) {
   if (threadIdx.x == 0) {
     atomicAdd(&S.counters[CNT_TIMEOUT], 1);
-    mbar_wait(&sh.bar, (uint32_t)(sh.abort - 1), S.wait_ns);
+    if (sh.abort) mbar_wait(&sh.bar, (uint32_t)(sh.abort - 1), S.wait_ns);
+    if (sh.pabort) mbar_wait(&sh.pbar, (uint32_t)(sh.pabort - 1), S.wait_ns);
   }
 }
 
@@ -627,13 +715,18 @@ __device__ __forceinline__ void tile_zero(ItemShared& sh, int nf) {
   for (int i = 4 * n4 + threadIdx.x; i < nf * kTile3; i += blockDim.x) sh.tile[i] = 0.0f;
 }
 
-// Kernel start: cell counts, flags and the bulk-copy barrier. Ends with
-// __syncthreads.
+// Kernel start: cell counts, flags, the bulk-copy barrier and finite values in
+// the P2G records (the half of an item's last record that holds no particle
+// is multiplied by zero weights). Ends with __syncthreads.
 __device__ __forceinline__ void tile_init(ItemShared& sh) {
   for (int i = threadIdx.x; i < kCells; i += blockDim.x) sh.ccount[i] = 0;
+  static_assert(offsetof(ItemShared, pd) % 16 == 0 && sizeof(sh.pd) % 16 == 0, "records are cleared in 16-byte words");
+  float4* pd4 = reinterpret_cast<float4*>(sh.pd);
+  for (int i = threadIdx.x; i < (int)(sizeof(sh.pd) / 16); i += blockDim.x) pd4[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (threadIdx.x == 0) {
     mbar_init(&sh.bar, 1);
-    sh.abort = 0;
+    mbar_init(&sh.pbar, 1);
+    sh.abort = sh.pabort = 0;
     sh.run_bound = sh.item_bound = 0.0f;
   }
   __syncthreads();
@@ -642,80 +735,100 @@ __device__ __forceinline__ void tile_init(ItemShared& sh) {
 // G2P sums of one particle: dv = sum_i w_ip d_i (PIC/FLIP increment,
 // g2pTransfer.glsl:99-104) and L = sum_i v*_i (grad w_ip)^T (velocity
 // gradient, :121-129), contracted along x first for each (y, z) row.
-// node(a, b, c, v6) fills the 6 values (v*, d) of stencil node (a, b, c) or
-// returns false for a node that contributes nothing.
+// node(a, b, c, p) fills the 6 values (v*, d) of stencil node (a, b, c) as
+// three pairs (v0, v1), (v2, d0), (d1, d2) or returns false for a node that
+// contributes nothing. Bound by shared loads and instruction issue: the packed
+// instructions take 5 where the 9 sums along x take 9, and round each sum as
+// those do. The z loop is not unrolled: the code of the fused kernel does not
+// fit the instruction cache (0.234 against 0.237 ms, 1M particles, 256^3).
 template <class Node>
 __device__ __forceinline__ void g2p_sums(const AxisW& w, Node node, float dv[3], float L[3][3]) {
+  f32x2 dv12 = 0ull, L0[3] = {0ull, 0ull, 0ull};  // (dv1, dv2); (L0k, L1k)
+  float dv0 = 0.0f, L2[3] = {0.0f, 0.0f, 0.0f};
+  f32x2 wx[4], gx[4];
 #pragma unroll
-  for (int r = 0; r < 3; r++) {
-    dv[r] = 0.0f;
-    L[r][0] = L[r][1] = L[r][2] = 0.0f;
+  for (int a = 0; a < 4; a++) {
+    wx[a] = pack2(w.wx[a], w.wx[a]);
+    gx[a] = pack2(w.gx[a], w.gx[a]);
   }
-#pragma unroll
+  float wz = w.wz[0], gz = w.gz[0], wzn[3] = {w.wz[1], w.wz[2], w.wz[3]}, gzn[3] = {w.gz[1], w.gz[2], w.gz[3]};
+#pragma unroll 1
   for (int c = 0; c < 4; c++) {
 #pragma unroll
     for (int b = 0; b < 4; b++) {
-      float S1[3] = {0.0f, 0.0f, 0.0f}, S2[3] = {0.0f, 0.0f, 0.0f}, D[3] = {0.0f, 0.0f, 0.0f};
+      f32x2 S1 = 0ull, SD = 0ull, D = 0ull, S2 = 0ull;  // sum wx (v0, v1), wx (v2, d0), wx (d1, d2), gx (v0, v1)
+      float S22 = 0.0f;                                  // sum gx v2
 #pragma unroll
       for (int a = 0; a < 4; a++) {
-        float v6[6];
-        if (!node(a, b, c, v6)) continue;
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-          S1[r] += w.wx[a] * v6[r];
-          S2[r] += w.gx[a] * v6[r];
-          D[r] += w.wx[a] * v6[3 + r];
-        }
+        f32x2 p[3];
+        if (!node(a, b, c, p)) continue;
+        S1 = fma2(wx[a], p[0], S1);
+        SD = fma2(wx[a], p[1], SD);
+        D = fma2(wx[a], p[2], D);
+        S2 = fma2(gx[a], p[0], S2);
+        S22 += w.gx[a] * lo2(p[1]);
       }
-      const float t1 = w.wy[b] * w.wz[c], t2 = w.gy[b] * w.wz[c], t3 = w.wy[b] * w.gz[c];
-#pragma unroll
-      for (int r = 0; r < 3; r++) {
-        dv[r] += t1 * D[r];
-        L[r][0] += t1 * S2[r];
-        L[r][1] += t2 * S1[r];
-        L[r][2] += t3 * S1[r];
-      }
+      const float t1 = w.wy[b] * wz, t2 = w.gy[b] * wz, t3 = w.wy[b] * gz;
+      const float S12 = lo2(SD);
+      dv0 += t1 * hi2(SD);
+      dv12 = fma2(pack2(t1, t1), D, dv12);
+      L0[0] = fma2(pack2(t1, t1), S2, L0[0]);
+      L0[1] = fma2(pack2(t2, t2), S1, L0[1]);
+      L0[2] = fma2(pack2(t3, t3), S1, L0[2]);
+      L2[0] += t1 * S22;
+      L2[1] += t2 * S12;
+      L2[2] += t3 * S12;
     }
+    wz = wzn[0]; wzn[0] = wzn[1]; wzn[1] = wzn[2];
+    gz = gzn[0]; gzn[0] = gzn[1]; gzn[1] = gzn[2];
   }
+  dv[0] = dv0;
+  dv[1] = lo2(dv12);
+  dv[2] = hi2(dv12);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    L[0][k] = lo2(L0[k]);
+    L[1][k] = hi2(L0[k]);
+    L[2][k] = L2[k];
+  }
+}
+
+// Whether the stencil of base cell `base` lies in the tile of home block
+// (bx, by, bz); t = its first node in tile coordinates.
+__device__ __forceinline__ bool stencil_in_tile(int bx, int by, int bz, const int base[3], int t[3]) {
+  t[0] = base[0] - 1 - (4 * bx - 2);
+  t[1] = base[1] - 1 - (4 * by - 2);
+  t[2] = base[2] - 1 - (4 * bz - 2);
+  return t[0] >= 0 && t[1] >= 0 && t[2] >= 0 && t[0] <= kTile - 4 && t[1] <= kTile - 4 && t[2] <= kTile - 4;
 }
 
 // Gather for particle at base cell `base` of the item at home block
 // (bx, by, bz): from the staged tile when the stencil lies in it, else from
-// the pool in global memory. Pool nodes are 6-float records (v*, d).
+// global memory.
 __device__ __forceinline__ void g2p_gather(const ItemShared& sh, const SceneDev& S, int bx, int by, int bz,
                                            const int base[3], const AxisW& w, float dv[3], float L[3][3]) {
-  const int tx = base[0] - 1 - (4 * bx - 2), ty = base[1] - 1 - (4 * by - 2), tz = base[2] - 1 - (4 * bz - 2);
-  if (tx >= 0 && ty >= 0 && tz >= 0 && tx <= kTile - 4 && ty <= kTile - 4 && tz <= kTile - 4) {
-    // tile node t (0..8) lies in tile block floor((t + 2) / 4) at local (t + 2) & 3
-    int X[4], Y[4], Z[4];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int t = tx + a, q = ty + a, r = tz + a;
-      X[a] = ((t + 2) >> 2) * kOutBlockFloats + kOutFields * ((t + 2) & 3);
-      Y[a] = ((q + 2) >> 2) * 3 * kOutBlockFloats + kOutFields * 4 * ((q + 2) & 3);
-      Z[a] = ((r + 2) >> 2) * 9 * kOutBlockFloats + kOutFields * 16 * ((r + 2) & 3);
-    }
-    const float* st = &sh.stage[0][0];
+  using T = StageShape<kOutFields>;
+  int t[3];
+  if (stencil_in_tile(bx, by, bz, base, t)) {
+    const float* st = sh.stage + t[2] * T::plane + t[1] * T::row + t[0] * kOutFields;
     g2p_sums(w,
-             [&](int a, int b, int c, float v6[6]) {
-               const float2* o = reinterpret_cast<const float2*>(st + X[a] + Y[b] + Z[c]);
-               const float2 p0 = o[0], p1 = o[1], p2 = o[2];
-               v6[0] = p0.x; v6[1] = p0.y; v6[2] = p1.x;
-               v6[3] = p1.y; v6[4] = p2.x; v6[5] = p2.y;
+             [&](int a, int b, int c, f32x2 p[3]) {
+               const f32x2* o = reinterpret_cast<const f32x2*>(st + c * T::plane + b * T::row + a * kOutFields);
+               p[0] = o[0];
+               p[1] = o[1];
+               p[2] = o[2];
                return true;
              },
              dv, L);
   } else {
     g2p_sums(w,
-             [&](int a, int b, int c, float v6[6]) {
+             [&](int a, int b, int c, f32x2 p[3]) {
                const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
                if (!node_in_grid(S, g0, g1, g2)) return false;
-               const int sl = __ldg(&S.blk_slot[block_id(S, g0 >> 2, g1 >> 2, g2 >> 2)]);
-               if (sl < 0) return false;
-               const float* o = S.gout + (size_t)sl * kOutBlockFloats +
-                                kOutFields * ((g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3));
-#pragma unroll
-               for (int f = 0; f < 6; f++) v6[f] = __ldg(o + f);
+               const f32x2* o = reinterpret_cast<const f32x2*>(S.gout + node_index(S, g0, g1, g2) * kOutFields);
+               p[0] = __ldg(o);
+               p[1] = __ldg(o + 1);
+               p[2] = __ldg(o + 2);
                return true;
              },
              dv, L);
@@ -832,84 +945,103 @@ __device__ __forceinline__ void advance_particle(const SceneDev& S, int p, const
   if (!finite) atomicAdd(&S.counters[CNT_NONFINITE], 1);
 }
 
-// Adds the particles of one tile cell (list slots j0..j1) to this lane's
-// x-row (b, c) of the cell's 4x4x4 stencil: acc[a] holds node x = lx + a.
-// The semi-implicit solve's K u (float sums of A grad w).
-__device__ __forceinline__ void cell_sums_force(const ItemShared& sh, int j0, int j1, int b, int c,
-                                                float (&acc)[4][kAccFields]) {
-  for (int j = j0; j < j1; j++) {
-    const float4* d = sh.pd[j];
-    const float* df = reinterpret_cast<const float*>(d);
-    const float4 w4 = d[4], g4 = d[5];
-    const float wxa[4] = {w4.x, w4.y, w4.z, w4.w};
-    const float gxa[4] = {g4.x, g4.y, g4.z, g4.w};
-    const float wyb = df[6 * 4 + b], wzc = df[8 * 4 + c];
-    const float gyb = df[7 * 4 + b], gzc = df[9 * 4 + c];
-    const float t1 = wyb * wzc, t2 = gyb * wzc, t3 = wyb * gzc;
-    const float4 a1 = d[1], a2 = d[2];
-    const float a22 = df[3 * 4];
-    // A rows: r0 = (a1.x a1.y a1.z), r1 = (a1.w a2.x a2.y), r2 = (a2.z a2.w a22)
-    const float kk[3] = {a1.x * t1, a1.w * t1, a2.z * t1};
-    const float hh[3] = {a1.y * t2 + a1.z * t3, a2.x * t2 + a2.y * t3, a2.w * t2 + a22 * t3};
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int r = 0; r < 3; r++) acc[a][r] += gxa[a] * kk[r] + wxa[a] * hh[r];
-  }
+// Clears the halves of v outside the list slots [j0, j1) of the pair at slots (j, j + 1).
+__device__ __forceinline__ f32x2 mask2(f32x2 v, bool lo, bool hi) {
+  unsigned a, b;
+  unpack2(v, a, b);
+  return pack2(__uint_as_float(lo ? a : 0u), __uint_as_float(hi ? b : 0u));
 }
 
-// The same for the fixed-point sums (mass alone, or mass, momentum and force):
-// each contribution is rounded by the magic-offset FMA (fix_mass, fix_mom,
-// fix_force) and its bits are added to the unsigned accumulators, so every
-// accumulator gains kMagicBits per particle; np counts the particles summed.
+// Adds the particles of one tile cell (list slots j0..j1) to this lane's
+// x-row (b, c) of the cell's 4x4x4 stencil: acc[a] holds node x = lx + a. The
+// slots are taken two at a time (one record of sh.pd); a cell that starts or
+// ends inside a record clears the other cell's half by its y weights, on which
+// every term depends. Fixed point (mass alone, or mass, momentum and force):
+// each contribution is rounded by the magic-offset FMA with the operations of
+// row_factors, fix_mass, fix_mom and fix_force, and its bits are added to the
+// unsigned accumulators, so every accumulator gains kMagicBits per slot; np
+// counts the slots summed. K u (KIND kP2gForce): float sums of A grad w, the
+// two halves apart in facc.
+// Bound by the 128 bytes a cycle that shared memory returns to registers (the
+// 16 lanes of a cell each load the particle's values). Two particles per
+// packed instruction: 20 FMAs and 14 three-input adds per particle and lane
+// instead of 40 and 28; with the packed gather above it took 23% of the fused
+// kernel's instructions (162.6 to 125.3 million, 1M particles, 256^3).
 template <int KIND>
-__device__ __forceinline__ void cell_sums_fix(const ItemShared& sh, int j0, int j1, int b, int c,
-                                              unsigned (&acc)[4][kAccFields], int& np) {
-  constexpr bool mo = KIND == kP2gMass;
-  for (int j = j0; j < j1; j++, np++) {
-    const float4* d = sh.pd[j];
-    const float* df = reinterpret_cast<const float*>(d);
-    const float4 w4 = d[4];
-    const float wxa[4] = {w4.x, w4.y, w4.z, w4.w};
-    const float4 d0 = d[0];
-    const float mvs[3] = {d0.y, d0.z, d0.w};
-    float As[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
-    float gyb = 0.0f, gzc = 0.0f;
-    float gxa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (!mo) {
-      const float4 a1 = d[1], a2 = d[2], g4 = d[5];
-      As[0][0] = a1.x; As[0][1] = a1.y; As[0][2] = a1.z;
-      As[1][0] = a1.w; As[1][1] = a2.x; As[1][2] = a2.y;
-      As[2][0] = a2.z; As[2][1] = a2.w; As[2][2] = df[3 * 4];
-      gyb = df[7 * 4 + b];
-      gzc = df[9 * 4 + c];
-      gxa[0] = g4.x; gxa[1] = g4.y; gxa[2] = g4.z; gxa[3] = g4.w;
+__device__ __forceinline__ void cell_sums(const ItemShared& sh, int j0, int j1, int b, int c,
+                                          unsigned (&acc)[4][kAccFields], f32x2 (&facc)[4][3], unsigned& np) {
+  const f32x2 magic = pack2(kMagic, kMagic);
+  for (int j = j0 & ~1; j < j1; j += 2, np += 2) {
+    const float* rec = sh.pd + (j >> 1) * kPdStride;
+    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(rec);
+    const ulonglong2 yw = q[(kPdY >> 1) + b], zw = q[(kPdZ >> 1) + c];
+    f32x2 wy = yw.x, gy = yw.y;
+    const bool lo = j >= j0, hi = j + 1 < j1;
+    if (!(lo && hi)) {
+      wy = mask2(wy, lo, hi);
+      gy = mask2(gy, lo, hi);
     }
-    RowFactors f;
-    row_factors(d0.x, mvs, As, df[6 * 4 + b], gyb, df[8 * 4 + c], gzc, mo, f);
+    const f32x2 t1 = mul2(wy, zw.x);
+    const ulonglong2 q0 = q[0];  // A22, m
+    const ulonglong2 wx01 = q[kPdWx >> 1], wx23 = q[(kPdWx >> 1) + 1];
+    const f32x2 wx[4] = {wx01.x, wx01.y, wx23.x, wx23.y};
+    if (KIND != kP2gForce) {
+      const f32x2 mw = mul2(q0.y, t1);
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      acc[a][0] += (unsigned)fix_mass(wxa[a], f);
-      if (mo) continue;
+      for (int a = 0; a < 4; a++) {
+        unsigned u, v;
+        unpack2(fma2(wx[a], mw, magic), u, v);
+        acc[a][0] += u + v;
+      }
+    }
+    if (KIND == kP2gMass) continue;
+    const f32x2 t2 = mul2(gy, zw.x), t3 = mul2(wy, zw.y);
+    const ulonglong2 q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5], q6 = q[6];
+    if (KIND == kP2gFull) {
+      const f32x2 mv[3] = {q1.x, q1.y, q2.x};
 #pragma unroll
       for (int r = 0; r < 3; r++) {
-        acc[a][1 + r] += (unsigned)fix_mom(wxa[a], f, r);
-        acc[a][4 + r] += (unsigned)fix_force(wxa[a], gxa[a], f, r);
+        const f32x2 pv = mul2(mv[r], t1);
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          unsigned u, v;
+          unpack2(fma2(wx[a], pv, magic), u, v);
+          acc[a][1 + r] += u + v;
+        }
+      }
+    }
+    const ulonglong2 gx01 = q[kPdGx >> 1], gx23 = q[(kPdGx >> 1) + 1];
+    const f32x2 gx[4] = {gx01.x, gx01.y, gx23.x, gx23.y};
+    const f32x2 A[3][3] = {{q2.y, q3.x, q3.y}, {q4.x, q4.y, q5.x}, {q5.y, q6.x, q0.x}};
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const f32x2 kk = mul2(A[r][0], t1);
+      const f32x2 hh = fma2(A[r][1], t2, mul2(A[r][2], t3));
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        if (KIND == kP2gFull) {
+          unsigned u, v;
+          unpack2(fma2(gx[a], kk, fma2(wx[a], hh, magic)), u, v);
+          acc[a][4 + r] += u + v;
+        } else {
+          facc[a][r] = fma2(gx[a], kk, fma2(wx[a], hh, facc[a][r]));
+        }
       }
     }
   }
 }
 
+__device__ __forceinline__ float sum2(f32x2 v) { return lo2(v) + hi2(v); }
+
 // Adds the 4 nodes of this lane's row (tile nodes t0 .. t0 + 3) to the
 // shared tile and clears them (float sums).
-template <int NF>
-__device__ __forceinline__ void row_flush(ItemShared& sh, int t0, float (&acc)[4][kAccFields]) {
+__device__ __forceinline__ void row_flush(ItemShared& sh, int t0, f32x2 (&acc)[4][3]) {
 #pragma unroll
   for (int a = 0; a < 4; a++) {
 #pragma unroll
-    for (int f = 0; f < NF; f++) {
-      atomicAdd(&sh.tile[f * kTile3 + t0 + a], acc[a][f]);
-      acc[a][f] = 0.0f;
+    for (int f = 0; f < 3; f++) {
+      atomicAdd(&sh.tile[f * kTile3 + t0 + a], sum2(acc[a][f]));
+      acc[a][f] = 0ull;
     }
   }
 }
@@ -934,53 +1066,65 @@ __device__ __forceinline__ int cell_row_node(int ci, int b, int c) {
 
 // P2G of the item's particles into the shared tile (every thread of the CTA
 // calls it; thread i holds particle i of the item when `have`):
-//   1. each particle inside the tile whose contributions fit the fast
-//      path's range counts itself in its base cell; the others scatter
+//   1. each particle inside the tile whose contributions fit the fast path's
+//      range counts itself in its base cell (p2g_count); the others scatter
 //      straight to acc (scatter_fix; K u: scatter_force);
-//   2. a scan of the cell counts gives each cell its first slot and lists the
-//      occupied cells; each particle stores its (scaled) mass, momentum, A
-//      and axis weights at its slot, so the particles lie in tile-cell order;
+//   2. every warp scans the cell counts for itself: the first slot of each
+//      cell and the list of the occupied cells; each particle stores its
+//      (scaled) mass, momentum, A and axis weights at its slot, so the
+//      particles lie in tile-cell order;
 //   3. each half-warp owns one occupied cell at a time: lane l sums the
 //      x-row (b, c) = (l & 3, l >> 2) of the cell's stencil over the cell's
 //      particles in registers and adds the row to the shared tile.
 // The tile keeps accumulating until p2g_tile_flush adds it to acc, so the
-// items of one home block can share it. Returns false (at its first barrier,
-// before any write beyond the cell counts and the straight scatters) when a
-// copy wait of the CTA ran out (sh.abort): the caller then stops the CTA.
+// items of one home block can share it. A barrier separates p2g_count from
+// p2g_sum (2 and 3), at which the caller stops the CTA if a copy wait ran out
+// (sh.abort, sh.pabort; nothing but the cell counts and the straight scatters
+// has been written then).
 // RUN: the tile may already hold earlier items' sums (sh.run_bound bounds
 // them); when this item's particles could take a sum past kTileSumBound, the
-// tile is first added to acc and cleared. Ends with a barrier.
+// tile is first added to acc and cleared. p2g_sum ends with a barrier.
 template <int KIND>
 __device__ __forceinline__ void p2g_tile_flush(ItemShared& sh, const SceneDev& S, int bx, int by, int bz);
+
+// A particle's quantities as the tile stores them (fixed point: scaled).
+struct P2GStored {
+  float ms, mvs[3], As[3][3];
+  int cell, rank;  // its tile cell (-1: not in the tile) and its place among the cell's particles
+};
+
 template <int KIND, bool RUN = false>
-__device__ __forceinline__ bool p2g_tile_accumulate(ItemShared& sh, const SceneDev& S, int bx, int by, int bz,
-                                                    bool have, const P2GParticle& q, const AxisW& w,
-                                                    const int base[3], const FixScale& sc) {
-  constexpr int nf = P2gFields<KIND>::nf;
+__device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, bool have,
+                                          const P2GParticle& q, const AxisW& w, const int base[3], const FixScale& sc,
+                                          P2GStored& st) {
   constexpr bool fix = KIND != kP2gForce;
   const int ox = 4 * bx - 2, oy = 4 * by - 2, oz = 4 * bz - 2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int my_cell = -1, my_rank = 0;
+  st.cell = -1;
+  st.rank = 0;
+  st.ms = 0.0f;
   float tile_bound = 0.0f;  // the particle's contribution bound, if it goes to the tile
-  // the particle's quantities as the tile stores them (fixed point: scaled)
-  float ms = 0.0f, mvs[3] = {0.0f, 0.0f, 0.0f}, As[3][3];
 #pragma unroll
-  for (int r = 0; r < 3; r++)
+  for (int r = 0; r < 3; r++) {
+    st.mvs[r] = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 3; c++) As[r][c] = fix ? (q.force ? q.A[r][c] * sc.f : 0.0f) : q.A[r][c];
+    for (int c = 0; c < 3; c++) st.As[r][c] = q.force ? (fix ? q.A[r][c] * sc.f : q.A[r][c]) : 0.0f;
+  }
   if (fix) {
-    ms = q.m * sc.m;
+    st.ms = q.m * sc.m;
 #pragma unroll
-    for (int r = 0; r < 3; r++) mvs[r] = q.mv[r] * sc.p;
+    for (int r = 0; r < 3; r++) st.mvs[r] = q.mv[r] * sc.p;
   }
   if (have) {
     const float bound = fix ? fix_bound<KIND>(q, sc) : 0.0f;
     const bool fast = !fix || bound < kFastLimit;  // false for a non-finite particle as well
     const int lx = base[0] - 1 - ox, ly = base[1] - 1 - oy, lz = base[2] - 1 - oz;
     const bool inside = lx >= 0 && ly >= 0 && lz >= 0 && lx < kCellsPerAxis && ly < kCellsPerAxis && lz < kCellsPerAxis;
-    if (inside && fast) {
-      my_cell = lx + kCellsPerAxis * ly + kCellsPerAxis * kCellsPerAxis * lz;
-      my_rank = atomicAdd(&sh.ccount[my_cell], 1);
+    // a NaN position (cell 0 of the grid) stays out of the records, which pair
+    // particles of neighbouring cells
+    const bool finite_w = w.wx[1] + w.wy[1] + w.wz[1] < 4.0f;
+    if (inside && fast && finite_w) {
+      st.cell = lx + kCellsPerAxis * ly + kCellsPerAxis * kCellsPerAxis * lz;
+      st.rank = atomicAdd(&sh.ccount[st.cell], 1);
       tile_bound = bound;
     } else {
       // the particle drifted out of its home block's tile since the last
@@ -988,21 +1132,28 @@ __device__ __forceinline__ bool p2g_tile_accumulate(ItemShared& sh, const SceneD
       if (!inside) atomicAdd(&S.counters[CNT_FALLBACK], 1);
       if (!fix)
         scatter_force(S, q, w, base);
-      else if (fast)
-        scatter_fix<KIND, true>(S, ms, mvs, As, w, base);
+      else if (fast && finite_w)
+        scatter_fix<KIND, true>(S, st.ms, st.mvs, st.As, w, base);
       else {
         atomicAdd(&S.fix->wide, 1u);
-        scatter_fix<KIND, false>(S, ms, mvs, As, w, base);
+        scatter_fix<KIND, false>(S, st.ms, st.mvs, st.As, w, base);
       }
     }
   }
   if (RUN) {  // per warp: its tile particles times their largest bound (no lower than their sum)
-    const uint32_t in = __ballot_sync(0xffffffffu, my_cell >= 0);
+    const uint32_t in = __ballot_sync(0xffffffffu, st.cell >= 0);
     const float bmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(tile_bound)));
-    if (lane == 0 && in) atomicAdd(&sh.item_bound, (float)__popc(in) * bmax);
+    if ((threadIdx.x & 31) == 0 && in) atomicAdd(&sh.item_bound, (float)__popc(in) * bmax);
   }
-  __syncthreads();  // counts done
-  if (sh.abort) return false;  // a copy wait ran out
+}
+
+template <int KIND, bool RUN = false>
+__device__ __forceinline__ void p2g_sum(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, const P2GStored& st,
+                                        const AxisW& w) {
+  constexpr int nf = P2gFields<KIND>::nf;
+  constexpr bool fix = KIND != kP2gForce;
+  const int lane = threadIdx.x & 31;
+  const int my_cell = st.cell;
   if (RUN && sh.run_bound + sh.item_bound > kTileSumBound) {  // uniform across the CTA
     // this item's sums could wrap the tile's int32 sums: the earlier items'
     // go to acc first (integer sums: the split changes no bit of the result)
@@ -1011,58 +1162,67 @@ __device__ __forceinline__ bool p2g_tile_accumulate(ItemShared& sh, const SceneD
     if (threadIdx.x == 0) sh.run_bound = 0.0f;
     tile_zero(sh, nf);
   }
-  // exclusive scan of the cell counts and list of the occupied cells, one
-  // cell per thread
-  const int t = threadIdx.x;
-  const int cnt = t < kCells ? sh.ccount[t] : 0;
-  int incl = cnt;
+  // exclusive scan of the cell counts and list of the occupied cells, seven
+  // cells per lane. Every warp forms all of it and writes the same values, so
+  // that no barrier lies between the scan and the stores that use it.
+  constexpr int kPer = (kCells + 31) / 32;
+  int ncells;
+  {
+    int cnt[kPer], sum = 0, occ = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
+    for (int k = 0; k < kPer; k++) {
+      const int ci = lane * kPer + k;
+      cnt[k] = ci < kCells ? sh.ccount[ci] : 0;
+      sum += cnt[k] + (cnt[k] > 0 ? 1 << 16 : 0);  // particles below, occupied cells above
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    ncells = __shfl_sync(0xffffffffu, incl, 31) >> 16;
+    int at = (incl - sum) & 0xffff;
+    occ = (incl - sum) >> 16;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      const int ci = lane * kPer + k;
+      if (ci <= kCells) sh.cstart[ci] = at;  // cstart[kCells]: the count of all
+      if (cnt[k] > 0) sh.cells[occ++] = (short)ci;
+      at += cnt[k];
+    }
+    static_assert(32 * kPer > kCells, "the lane past the last cell writes the end");
+    __syncwarp();
   }
-  const uint32_t occ = __ballot_sync(0xffffffffu, cnt > 0);
-  if (lane == 31) {
-    sh.wsum[warp] = incl;
-    sh.wocc[warp] = __popc(occ);
+  if (my_cell >= 0) {
+    // the particle's P2G data, stored in tile-cell order
+    const int slot = sh.cstart[my_cell] + st.rank;
+    float* d = sh.pd + (slot >> 1) * kPdStride + (slot & 1);
+    d[2 * kPdM] = st.ms;
+    if (KIND != kP2gMass) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        d[2 * (kPdMv + r)] = st.mvs[r];
+#pragma unroll
+        for (int c = 0; c < 3; c++) d[2 * (r == 2 && c == 2 ? kPdA22 : kPdA + 3 * r + c)] = st.As[r][c];
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      d[2 * (kPdWx + a)] = w.wx[a];
+      d[2 * (kPdGx + a)] = w.gx[a];
+      d[2 * (kPdY + 2 * a)] = w.wy[a];
+      d[2 * (kPdY + 2 * a + 1)] = w.gy[a];
+      d[2 * (kPdZ + 2 * a)] = w.wz[a];
+      d[2 * (kPdZ + 2 * a + 1)] = w.gz[a];
+    }
   }
   __syncthreads();
-  int off = 0, ooff = 0;
-  for (int k = 0; k < warp; k++) {
-    off += sh.wsum[k];
-    ooff += sh.wocc[k];
-  }
-  if (t < kCells) {
-    sh.cstart[t] = off + incl - cnt;
-    sh.ccount[t] = 0;
-    if (cnt > 0) sh.cells[ooff + __popc(occ & ((1u << lane) - 1u))] = (short)t;
-  }
-  if (t == kCells - 1) sh.cstart[kCells] = off + incl;
-  if (t == blockDim.x - 1) sh.ncells = ooff + __popc(occ);
-  if (RUN && t == 0) {  // every thread has read both bounds (two barriers ago)
+  for (int i = threadIdx.x; i < kCells; i += blockDim.x) sh.ccount[i] = 0;  // every warp has scanned them
+  if (RUN && threadIdx.x == 0) {  // every thread has read both bounds
     sh.run_bound += sh.item_bound;
     sh.item_bound = 0.0f;
   }
-  __syncthreads();
-  if (my_cell >= 0) {
-    // the particle's P2G data, stored in tile-cell order
-    float4* d = sh.pd[sh.cstart[my_cell] + my_rank];
-    const bool f = KIND != kP2gMass && q.force;
-    if (KIND == kP2gMass)
-      d[0] = make_float4(ms, 0.0f, 0.0f, 0.0f);
-    else if (KIND == kP2gFull)
-      d[0] = make_float4(ms, mvs[0], mvs[1], mvs[2]);
-    d[1] = f ? make_float4(As[0][0], As[0][1], As[0][2], As[1][0]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    d[2] = f ? make_float4(As[1][1], As[1][2], As[2][0], As[2][1]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    d[3] = make_float4(f ? As[2][2] : 0.0f, __int_as_float(my_cell), 0.0f, 0.0f);
-    d[4] = make_float4(w.wx[0], w.wx[1], w.wx[2], w.wx[3]);
-    d[5] = make_float4(w.gx[0], w.gx[1], w.gx[2], w.gx[3]);
-    d[6] = make_float4(w.wy[0], w.wy[1], w.wy[2], w.wy[3]);
-    d[7] = make_float4(w.gy[0], w.gy[1], w.gy[2], w.gy[3]);
-    d[8] = make_float4(w.wz[0], w.wz[1], w.wz[2], w.wz[3]);
-    d[9] = make_float4(w.gz[0], w.gz[1], w.gz[2], w.gz[3]);
-  }
-  __syncthreads();
   {
     // half-warp h takes a contiguous slice of the occupied-cell list (the
     // two halves of a warp get neighbouring slices, whose particle counts
@@ -1073,68 +1233,58 @@ __device__ __forceinline__ bool p2g_tile_accumulate(ItemShared& sh, const SceneD
     const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
     const int b = l16 & 3, c = l16 >> 2;
     const int nhw = blockDim.x >> 4;
-    const int ncells = sh.ncells;
     const int k0 = (ncells * hw) / nhw, k1 = (ncells * (hw + 1)) / nhw;
     int cur = -1;
-    if (fix) {
-      unsigned acc[4][kAccFields];
+    unsigned acc[4][kAccFields];
+    f32x2 facc[4][3];
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+    for (int a = 0; a < 4; a++) {
 #pragma unroll
-        for (int f = 0; f < kAccFields; f++) acc[a][f] = 0u;
-      int np = 0;
-      for (int k = k0; k < k1; k++) {
-        const int ci = sh.cells[k];
-        if (cur >= 0) {
-          const unsigned base_bits = (unsigned)np * (unsigned)kMagicBits;
-          if (ci == cur + 1 && ci % kCellsPerAxis != 0) {
-            // only node 0 leaves the window: flush it, slide the rest
+      for (int f = 0; f < kAccFields; f++) acc[a][f] = 0u;
 #pragma unroll
-            for (int f = 0; f < NF; f++) {
-              atomicAdd(&sh.tilei[f * kTile3 + cell_row_node(cur, b, c)], (int)(acc[0][f] - base_bits));
+      for (int f = 0; f < 3; f++) facc[a][f] = 0ull;
+    }
+    unsigned np = 0;
+    for (int k = k0; k < k1; k++) {
+      const int ci = sh.cells[k];
+      if (cur >= 0) {
+        const int row = cell_row_node(cur, b, c);
+        const unsigned base_bits = np * (unsigned)kMagicBits;
+        if (ci == cur + 1 && ci % kCellsPerAxis != 0) {
+          // only node 0 leaves the window: flush it, slide the rest
+#pragma unroll
+          for (int f = 0; f < NF; f++) {
+            if (fix) {
+              atomicAdd(&sh.tilei[f * kTile3 + row], (int)(acc[0][f] - base_bits));
               acc[0][f] = acc[1][f];
               acc[1][f] = acc[2][f];
               acc[2][f] = acc[3][f];
               acc[3][f] = base_bits;
+            } else {
+              atomicAdd(&sh.tile[f * kTile3 + row], sum2(facc[0][f]));
+              facc[0][f] = facc[1][f];
+              facc[1][f] = facc[2][f];
+              facc[2][f] = facc[3][f];
+              facc[3][f] = 0ull;
             }
-          } else {
-            row_flush_fix<NF>(sh, cell_row_node(cur, b, c), acc, base_bits);
           }
+        } else if (fix) {
+          row_flush_fix<NF>(sh, row, acc, base_bits);
+        } else {
+          row_flush(sh, row, facc);
         }
-        cell_sums_fix<KIND>(sh, sh.cstart[ci], sh.cstart[ci + 1], b, c, acc, np);
-        cur = ci;
       }
-      if (cur >= 0) row_flush_fix<NF>(sh, cell_row_node(cur, b, c), acc, (unsigned)np * (unsigned)kMagicBits);
-    } else {
-      float acc[4][kAccFields];
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int f = 0; f < kAccFields; f++) acc[a][f] = 0.0f;
-      for (int k = k0; k < k1; k++) {
-        const int ci = sh.cells[k];
-        if (cur >= 0) {
-          if (ci == cur + 1 && ci % kCellsPerAxis != 0) {
-#pragma unroll
-            for (int f = 0; f < NF; f++) {
-              atomicAdd(&sh.tile[f * kTile3 + cell_row_node(cur, b, c)], acc[0][f]);
-              acc[0][f] = acc[1][f];
-              acc[1][f] = acc[2][f];
-              acc[2][f] = acc[3][f];
-              acc[3][f] = 0.0f;
-            }
-          } else {
-            row_flush<NF>(sh, cell_row_node(cur, b, c), acc);
-          }
-        }
-        cell_sums_force(sh, sh.cstart[ci], sh.cstart[ci + 1], b, c, acc);
-        cur = ci;
-      }
-      if (cur >= 0) row_flush<NF>(sh, cell_row_node(cur, b, c), acc);
+      cell_sums<KIND>(sh, sh.cstart[ci], sh.cstart[ci + 1], b, c, acc, facc, np);
+      cur = ci;
+    }
+    if (cur >= 0) {
+      if (fix)
+        row_flush_fix<NF>(sh, cell_row_node(cur, b, c), acc, np * (unsigned)kMagicBits);
+      else
+        row_flush(sh, cell_row_node(cur, b, c), facc);
     }
   }
   __syncthreads();
-  return true;
 }
 
 // Adds the tile's non-zero nodes that lie in the grid to acc and flags
@@ -1142,7 +1292,7 @@ __device__ __forceinline__ bool p2g_tile_accumulate(ItemShared& sh, const SceneD
 // words; K u: three float adds into the force words of blocks active in
 // this step). One tile node per thread, x fastest, so consecutive threads
 // add to consecutive words. Every thread of the CTA calls it after
-// p2g_tile_accumulate's closing barrier; the caller separates it from the
+// p2g_sum's closing barrier; the caller separates it from the
 // next use of the tile with a barrier.
 template <int KIND>
 __device__ __forceinline__ void p2g_tile_flush(ItemShared& sh, const SceneDev& S, int bx, int by, int bz) {
@@ -1162,7 +1312,7 @@ __device__ __forceinline__ void p2g_tile_flush(ItemShared& sh, const SceneDev& S
     if (!any) continue;
     const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
     unsigned long long* a = S.acc + (size_t)blk * kAccBlockWords + (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3);
-    if (KIND == kP2gForce) {
+    if constexpr (KIND == kP2gForce) {
       // K u goes only to blocks active in this step: the solve's node passes
       // read and clear the words of those alone (a block whose fixed-point
       // sums all rounded to zero is not active, although its K u may not be)
@@ -1170,12 +1320,12 @@ __device__ __forceinline__ void p2g_tile_flush(ItemShared& sh, const SceneDev& S
       float* fw = reinterpret_cast<float*>(a + 4 * kBlockNodes);
 #pragma unroll
       for (int f = 0; f < 3; f++) atomicAdd(fw + 2 * f * kBlockNodes, __int_as_float(v[f]));
-      continue;
-    }
+    } else {
 #pragma unroll
-    for (int f = 0; f < nf; f++)
-      if (v[f]) atomicAdd(a + f * kBlockNodes, (unsigned long long)(long long)v[f]);
-    S.blk_flag[blk] = 1;
+      for (int f = 0; f < nf; f++)
+        if (v[f]) atomicAdd(a + f * kBlockNodes, (unsigned long long)(long long)v[f]);
+      S.blk_flag[blk] = 1;
+    }
   }
 }
 }  // namespace

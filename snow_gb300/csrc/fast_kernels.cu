@@ -10,22 +10,23 @@
 //            it consumes.
 //   blk_flag blocks that received P2G sums (set by the P2G tile flush).
 //   compact  turns the flags into the active-block list and gives each
-//            active block a slot in the output pool.
-//   gout     the pool: per slot the grid update's output v* and
-//            d = v* - alpha p/m, one 6-float record per node (1536 bytes).
+//            active block a slot (its place in the list).
+//   gout     dense over the nodes, x fastest: the grid update's output v* and
+//            d = v* - alpha p/m, one 6-float record per node; zero in blocks
+//            that are not active.
 //
 // Kernels of one step (every scene of a batch in one launch each):
 //   compact      flags -> slots, active list             (thread per block)
 //   grid         per active block: v* = p/m + dt (f/m + g), colliders, d
 //   g2p2g        per work item (<= 256 particles binned to one home block):
-//                bulk-copy (TMA) the 27 pool blocks around the home block
+//                bulk-copy (TMA) the 81 rows of nodes around the home block
 //                into shared memory, gather v* and d (G2P), update F_E with
 //                the SVD clamp, J_p, velocity, colliders, position (particle
 //                advance), then scatter the updated particles (P2G of the
 //                next step) into a 9^3-node shared tile, cell by cell, and
 //                add the tile to acc. A CTA takes a contiguous range of
 //                items; consecutive items of one home block (a run) share
-//                the staged grid blocks and the tile, which is added to acc
+//                the staged grid rows and the tile, which is added to acc
 //                once per run.
 // Separate P2G and G2P kernels serve the first step after set-up and the
 // per-kernel dispatch entry point.
@@ -93,8 +94,23 @@ __global__ void k_gather_counters(const SceneDev* __restrict__ scenes, int nscen
   __threadfence_system();
 }
 
-// Flags -> active-block list and pool slots (one thread per block); the CTA
-// that finishes last forms the item and active-block prefixes.
+// The outputs of a block that is no longer active read as zero.
+__device__ __noinline__ void clear_block(const SceneDev& S, int b) {
+  int bx, by, bz;
+  home_coords(S, b, bx, by, bz);
+  for (int r = 0; r < 16; r++) {
+    const size_t row = node_index(S, 4 * bx, 4 * by + (r & 3), 4 * bz + (r >> 2));
+    float4* o = reinterpret_cast<float4*>(S.gout + row * kOutFields);
+    for (int k = 0; k < kOutFields; k++) o[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (!S.crs) continue;
+    float4* u = reinterpret_cast<float4*>(S.cru + row * kImpFields);
+    for (int k = 0; k < kImpFields; k++) u[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+}
+
+// Flags -> active-block list and slots (one thread per block); a block that
+// was active before and is not now has its outputs cleared (few blocks a
+// step). The CTA that finishes last forms the item and active-block prefixes.
 __global__ void k_compact(const SceneDev* __restrict__ scenes, const int* __restrict__ block_prefix, int nscenes,
                           long long total, int* items_prefix, int* active_prefix) {
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < total;
@@ -102,6 +118,7 @@ __global__ void k_compact(const SceneDev* __restrict__ scenes, const int* __rest
     const int s = find_scene(block_prefix, nscenes, u);
     const SceneDev& S = scenes[s];
     const int b = (int)(u - block_prefix[s]);
+    const int old = S.blk_slot[b];
     int slot = -1;
     if (S.blk_flag[b]) {
       S.blk_flag[b] = 0;
@@ -113,7 +130,8 @@ __global__ void k_compact(const SceneDev* __restrict__ scenes, const int* __rest
         S.active[slot] = b;
       }
     }
-    S.blk_slot[b] = slot;
+    if (slot != old) S.blk_slot[b] = slot;
+    if (slot < 0 && old >= 0) clear_block(S, b);
   }
   __shared__ bool last;
   __syncthreads();
@@ -165,7 +183,7 @@ __global__ void __launch_bounds__(256) k_fix_measure(const SceneDev* __restrict_
 // magnitudes give; the CTA that takes a scene's first item records them for
 // the grid update.
 template <bool MASS_ONLY>
-__global__ void __launch_bounds__(kItemMax, 2) k_p2g(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kItemMax, kItemCtas) k_p2g(const SceneDev* __restrict__ scenes,
                                                   const int* __restrict__ item_prefix, int nscenes) {
   extern __shared__ float4 smem_raw[];
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
@@ -203,7 +221,10 @@ __global__ void __launch_bounds__(kItemMax, 2) k_p2g(const SceneDev* __restrict_
         have = true;
       }
     }
-    p2g_tile_accumulate<KIND>(sh, S, bx, by, bz, have, q, w, base, sc);
+    P2GStored stored;
+    p2g_count<KIND>(sh, S, bx, by, bz, have, q, w, base, sc, stored);
+    __syncthreads();
+    p2g_sum<KIND>(sh, S, bx, by, bz, stored, w);
     p2g_tile_flush<KIND>(sh, S, bx, by, bz);
     __syncthreads();
   }
@@ -224,7 +245,11 @@ __device__ __forceinline__ void grid_node(const SceneDev& S, int slot, int b, in
                                (float)(long long)w[4] * isf,
                                (float)(long long)w[5] * isf,
                                (float)(long long)w[6] * isf};
-  float2* out = reinterpret_cast<float2*>(S.gout + (size_t)slot * kOutBlockFloats + kOutFields * node);
+  int bx, by, bz;
+  home_coords(S, b, bx, by, bz);
+  const int gi = 4 * bx + (node & 3), gj = 4 * by + ((node >> 2) & 3), gk = 4 * bz + (node >> 4);
+  const size_t ni = node_index(S, gi, gj, gk);
+  float2* out = reinterpret_cast<float2*>(S.gout + ni * kOutFields);
   const float mi = v[0];
   float vs[3] = {0.0f, 0.0f, 0.0f}, d[3] = {0.0f, 0.0f, 0.0f};
   if (mq > 0) {
@@ -232,8 +257,6 @@ __device__ __forceinline__ void grid_node(const SceneDev& S, int slot, int b, in
     const float vold[3] = {v[1] * inv, v[2] * inv, v[3] * inv};
 #pragma unroll
     for (int k = 0; k < 3; k++) vs[k] = vold[k] + S.dt * (v[4 + k] * inv + S.grav[k]);
-    const int bx = b % S.bdim[0], by = (b / S.bdim[0]) % S.bdim[1], bz = b / (S.bdim[0] * S.bdim[1]);
-    const int gi = 4 * bx + (node & 3), gj = 4 * by + ((node >> 2) & 3), gk = 4 * bz + (node >> 4);
     // node position as Grid::initSSBO forms it: x_off + h * (float)i
     const float xi[3] = {__fadd_rn(S.gpos[0], __fmul_rn(S.h, (float)gi)),
                          __fadd_rn(S.gpos[1], __fmul_rn(S.h, (float)gj)),
@@ -248,7 +271,7 @@ __device__ __forceinline__ void grid_node(const SceneDev& S, int slot, int b, in
   if (S.crs && !S.crs->skipping) {  // semi-implicit: the solve starts from x = v* and applies K to v* first
     const size_t i = (size_t)slot * kBlockNodes + node;
     S.crv[i] = make_float4(vs[0], vs[1], vs[2], mi > 0.0f ? mi : 0.0f);
-    float* u = S.cru + (size_t)slot * kImpBlockFloats + 3 * node;
+    float* u = S.cru + ni * kImpFields;
     u[0] = vs[0];
     u[1] = vs[1];
     u[2] = vs[2];
@@ -382,7 +405,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
     const int4 it = S.items[u - item_prefix[s]];
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);
-    if (threadIdx.x < 32) stage_issue(sh, S, tile_slot(S, it, threadIdx.x));
+    stage_issue<kOutFields>(sh, S, S.gout, it.x);
     load_colliders(sh, S);
     stage_wait(sh, S, phase);
     __syncthreads();
@@ -413,7 +436,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // diagonal up to the Jacobi residual, whose polar rotation is W V^T.
 // A CTA takes a contiguous range of work items. Consecutive items of one
 // home block form a run: they share
-// the staged pool blocks (copied once, by bulk copies issued while the
+// the staged grid rows (copied once, by bulk copies issued while the
 // previous run's last item sums its P2G) and the P2G tile (added to acc
 // once, at the run's end). The P2G sums are fixed
 // point at the scales step_scales gives; the CTA that takes a scene's first
@@ -422,7 +445,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // re-binned some scene; such a scene's particles are read from its binned
 // copies (CNT_BINNED) and, like every scene's, written to its streams.
 template <bool BINNED>
-__global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
                                                        const int* __restrict__ item_prefix, int nscenes) {
   extern __shared__ float4 smem_raw[];
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
@@ -432,21 +455,26 @@ __global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restric
   const int u0 = min(total, (int)blockIdx.x * chunk), u1 = min(total, u0 + chunk);
   if (u0 >= u1) return;
   // The last warp, which holds the fewest particles of an item (items are
-  // filled from thread 0), looks up the next item and its pool slots.
+  // filled from thread 0), looks up the next item and issues the copies of its
+  // particles.
   const int lane = threadIdx.x & 31;
   const bool lastw = (threadIdx.x >> 5) == (blockDim.x >> 5) - 1;
-  if (lastw) {
+  {
     const int s0 = find_scene(item_prefix, nscenes, u0);
-    const int4 it0 = scenes[s0].items[u0 - item_prefix[s0]];
-    stage_issue(sh, scenes[s0], tile_slot(scenes[s0], it0, lane));
-    if (lane == 0) {
-      sh.item_q[0] = it0;
-      sh.scene_q[0] = s0;
-      sh.coll_scene = -1;
-      sh.next_same = 0;
+    const SceneDev& S0 = scenes[s0];
+    const int4 it0 = S0.items[u0 - item_prefix[s0]];
+    stage_issue<kOutFields>(sh, S0, S0.gout, it0.x);
+    if (lastw) {
+      particles_issue(sh, S0, it0.y, min(it0.z, kItemMax), BINNED && particles_binned(S0));
+      if (lane == 0) {
+        sh.item_q[0] = it0;
+        sh.scene_q[0] = s0;
+        sh.coll_scene = -1;
+        sh.next_same = 0;
+      }
     }
   }
-  uint32_t phase = 0;
+  uint32_t phase = 0, pphase = 0;
   int par = 0;
   bool run_start = true;  // uniform across the CTA
   for (int u = u0; u < u1; u++, par ^= 1) {
@@ -475,27 +503,22 @@ __global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restric
     }
     const int4 it = sh.item_q[par];
     const int un = u + 1;
-    // the next item's descriptor and pool slots: loaded now, so that the
-    // loads' latency overlaps this item's G2P instead of delaying the last
-    // warp, and put in shared memory before this item's P2G
-    int sn = 0, slot = -1;
+    // the next item's descriptor: loaded now, so that the loads' latency
+    // overlaps this item's G2P instead of delaying the last warp, and put in
+    // shared memory before this item's P2G
+    int sn = 0;
     int4 itn = make_int4(0, 0, 0, 0);
-    bool same = false;
     if (lastw && un < u1) {
       sn = find_scene(item_prefix, nscenes, un);
       itn = scenes[sn].items[un - item_prefix[sn]];
-      same = sn == s && itn.x == it.x;
-      if (!same) slot = tile_slot(scenes[sn], itn, lane);
     }
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);
     const int i = threadIdx.x;
     const bool mine = i < min(it.z, kItemMax);
     const int p = it.y + i;
-    PState ps;
-    const bool binned = BINNED && particles_binned(S);
-    if (mine) ps = load_state(S, p, binned);
-    const bool landed = run_start ? stage_wait(sh, S, phase) : true;
+    bool landed = particles_wait(sh, S, pphase);
+    if (run_start) landed = stage_wait(sh, S, phase) && landed;
     bool have = false;
     P2GParticle q;
     q.force = false;
@@ -504,6 +527,8 @@ __global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restric
     int nbase[3] = {0, 0, 0};
     float rec_v = 0.0f;
     if (mine && landed) {
+      PState ps;
+      ps.xm = sh.pxm[i];
       float pg[3];
       int base[3];
       grid_coords(S, ps.xm, pg, base);
@@ -511,7 +536,8 @@ __global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restric
       all_weights(pg, base, w);
       float dv[3], L[3][3];
       g2p_gather(sh, S, bx, by, bz, base, w, dv, L);
-      const PDef def = load_def(S, p, binned);
+      ps.vv = sh.pvv[i];
+      const PDef def = {sh.pfa[i], sh.pfb[i], sh.pvq[i], sh.pfc[i + (it.y & 1)]};
       Advanced adv;
       advance_particle(S, p, ps, def, dv, L, sh, adv);
       // P2G quantities of the advanced particle
@@ -539,23 +565,31 @@ __global__ void __launch_bounds__(kItemMax, 2) k_g2p2g(const SceneDev* __restric
       }
     }
     // the next item's queue entry: every thread read this one's at the loop
-    // top, and the accumulation's barriers publish it before the flush
-    // decision below
-    if (lastw) {  // kept in shared memory, not registers, across the accumulation
-      sh.next_slot[lane] = slot;
-      if (lane == 0) {
-        sh.item_q[par ^ 1] = itn;
-        sh.scene_q[par ^ 1] = sn;
-        sh.next_same = same ? 1 : 0;
-        sh.next_issue = un < u1 && !same ? 1 : 0;
-      }
+    // top, and the barriers below publish it before the flush decision
+    if (lastw && lane == 0) {
+      const bool same = sn == s && itn.x == it.x;
+      sh.item_q[par ^ 1] = itn;
+      sh.scene_q[par ^ 1] = sn;
+      sh.next_same = un < u1 && same ? 1 : 0;
+      sh.next_issue = un < u1 && !same ? 1 : 0;
     }
-    if (!p2g_tile_accumulate<kP2gFull, true>(sh, S, bx, by, bz, have, q, wn, nbase, sh.fscale)) {
+    P2GStored stored;
+    p2g_count<kP2gFull, true>(sh, S, bx, by, bz, have, q, wn, nbase, sh.fscale, stored);
+    __syncthreads();  // counts done; the particle buffer is read
+    if (sh.abort | sh.pabort) {
       stage_abort(sh, S);  // a copy wait ran out: this item's particles keep their state, the CTA stops
       return;
     }
-    if (lastw && sh.next_issue)  // uniform in the warp
-      stage_issue(sh, scenes[sh.scene_q[par ^ 1]], lane < 27 ? sh.next_slot[lane] : -1);
+    if (lastw && un < u1) {
+      const int4 nx = sh.item_q[par ^ 1];
+      const SceneDev& N = scenes[sh.scene_q[par ^ 1]];
+      particles_issue(sh, N, nx.y, min(nx.z, kItemMax), BINNED && particles_binned(N));
+    }
+    p2g_sum<kP2gFull, true>(sh, S, bx, by, bz, stored, wn);
+    if (sh.next_issue) {  // uniform across the CTA
+      const SceneDev& N = scenes[sh.scene_q[par ^ 1]];
+      stage_issue<kOutFields>(sh, N, N.gout, sh.item_q[par ^ 1].x);
+    }
     if (threadIdx.x == 0) {  // only maxima above what this CTA already recorded go to HBM
       unsigned* cur[3] = {&S.fix->m_cur, &S.fix->v_cur, &S.fix->a_cur};
 #pragma unroll
@@ -689,7 +723,7 @@ __global__ void __launch_bounds__(256) k_unpack(const SceneDev* __restrict__ sd,
   }
 }
 
-// Dense copies of the P2G sums (acc) and of v* (pool) of the active blocks.
+// Dense copies of the P2G sums (acc) and of v* of the active blocks.
 __global__ void k_download_grid(const SceneDev* __restrict__ sd, float* mass, float* mom, float* force, float* vstar) {
   const SceneDev& S = *sd;
   const int count = min(S.counters[CNT_ACTIVE], S.pool_cap);
@@ -701,7 +735,7 @@ __global__ void k_download_grid(const SceneDev* __restrict__ sd, float* mass, fl
     const int gi = 4 * bx + (node & 3), gj = 4 * by + ((node >> 2) & 3), gk = 4 * bz + (node >> 4);
     if (gi >= S.dim[0] || gj >= S.dim[1] || gk >= S.dim[2]) continue;
     const long long g = gi + (long long)S.dim[0] * (gj + (long long)S.dim[1] * gk);
-    const float* out = S.gout + (size_t)slot * kOutBlockFloats + kOutFields * node;
+    const float* out = S.gout + node_index(S, gi, gj, gk) * kOutFields;
     if (vstar)
       for (int k = 0; k < 3; k++) vstar[3 * g + k] = out[k];
   }

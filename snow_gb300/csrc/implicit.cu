@@ -21,9 +21,9 @@
 // Layout in HBM, per active pool slot (the grid update's slots):
 //   crv  three float4 planes of pool_cap x 64 nodes: (v, m), (p, 0), (A p, 0)
 //        with p and A p in the scaled variables
-//   cru  pool_cap x 192 floats: u = M^-1/2 r, the vector K is applied to,
-//        3 floats per node, so that a work item bulk-copies (TMA) its 27
-//        blocks like the G2P gather does
+//   cru  dense over the nodes like gout: u = M^-1/2 r, the vector K is applied
+//        to, 3 floats per node, so that a work item bulk-copies (TMA) its rows
+//        like the G2P gather does
 //   acc  the dense P2G sums, zero between steps: K u accumulates in its
 //        force slots and is cleared by the pass that consumes it
 //   crs  per scene: |M^1/2 v*|^2 and per iteration (r, A r), |A p|^2, |r|^2 in FP64
@@ -97,21 +97,13 @@ __device__ __forceinline__ void hess_sums(const AxisW& w, Node node, float Gm[3]
 // lies in it (decided once per particle), else from cru.
 __device__ __forceinline__ void hess_gather(const ItemShared& sh, const SceneDev& S, int bx, int by, int bz,
                                             const int base[3], const AxisW& w, float Gm[3][3]) {
-  const int tx = base[0] - 1 - (4 * bx - 2), ty = base[1] - 1 - (4 * by - 2), tz = base[2] - 1 - (4 * bz - 2);
-  if (tx >= 0 && ty >= 0 && tz >= 0 && tx <= kTile - 4 && ty <= kTile - 4 && tz <= kTile - 4) {
-    // tile node t (0..8) lies in tile block floor((t + 2) / 4) at local (t + 2) & 3
-    int X[4], Y[4], Z[4];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int t = tx + a, q = ty + a, r = tz + a;
-      X[a] = ((t + 2) >> 2) * kOutBlockFloats + 3 * ((t + 2) & 3);
-      Y[a] = ((q + 2) >> 2) * 3 * kOutBlockFloats + 3 * 4 * ((q + 2) & 3);
-      Z[a] = ((r + 2) >> 2) * 9 * kOutBlockFloats + 3 * 16 * ((r + 2) & 3);
-    }
-    const float* st = &sh.stage[0][0];
+  using T = StageShape<kImpFields>;
+  int t[3];
+  if (stencil_in_tile(bx, by, bz, base, t)) {
+    const float* st = sh.stage + t[2] * T::plane + t[1] * T::row + (t[0] + T::x0 - 2) * kImpFields;
     hess_sums(w,
               [&](int a, int b, int c, float u[3]) {
-                const float* o = st + X[a] + Y[b] + Z[c];
+                const float* o = st + c * T::plane + b * T::row + a * kImpFields;
                 u[0] = o[0];
                 u[1] = o[1];
                 u[2] = o[2];
@@ -123,9 +115,7 @@ __device__ __forceinline__ void hess_gather(const ItemShared& sh, const SceneDev
                 const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
                 u[0] = u[1] = u[2] = 0.0f;
                 if (!node_in_grid(S, g0, g1, g2)) return;
-                const int sl = __ldg(&S.blk_slot[block_id(S, g0 >> 2, g1 >> 2, g2 >> 2)]);
-                if (sl < 0) return;
-                const float* o = S.cru + (size_t)sl * kImpBlockFloats + 3 * ((g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3));
+                const float* o = S.cru + node_index(S, g0, g1, g2) * kImpFields;
                 u[0] = __ldg(o);
                 u[1] = __ldg(o + 1);
                 u[2] = __ldg(o + 2);
@@ -239,9 +229,9 @@ __device__ __forceinline__ int next_running(const SceneDev* __restrict__ scenes,
 
 // K u for the items of every scene whose iteration k runs, into acc's force
 // slots (iteration 0: u = v*). Persistent over the items like the fused
-// explicit kernel: the bulk copies of the CTA's next item are issued by the
-// last warp while the current item's per-cell sums are flushed.
-__global__ void __launch_bounds__(kItemMax, 2) k_hess(const SceneDev* __restrict__ scenes,
+// explicit kernel: the bulk copies of the CTA's next item are under way while
+// the current item's per-cell sums are flushed.
+__global__ void __launch_bounds__(kItemMax, kItemCtas) k_hess(const SceneDev* __restrict__ scenes,
                                                       const int* __restrict__ item_prefix, int nscenes,
                                                       const int* __restrict__ iter) {
   const int k = iter ? *iter : 0;  // iteration 0: K v*
@@ -250,27 +240,21 @@ __global__ void __launch_bounds__(kItemMax, 2) k_hess(const SceneDev* __restrict
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
   tile_init(sh);
   const int total = item_prefix[nscenes];
-  const int lane = threadIdx.x & 31;
-  const bool lastw = (threadIdx.x >> 5) == (blockDim.x >> 5) - 1;
   int s = 0;
   int u = next_running(scenes, item_prefix, nscenes, k, blockIdx.x, total, s);
   if (u >= total) return;  // uniform across the CTA
   int4 it = scenes[s].items[u - item_prefix[s]];
-  if (lastw) stage_issue(sh, scenes[s].cru, kImpBlockFloats, tile_slot(scenes[s], it, lane), scenes[s].tx_unsent);
+  stage_issue<kImpFields>(sh, scenes[s], scenes[s].cru, it.x);
   uint32_t phase = 0;
   while (u < total) {
     __syncthreads();  // zero-filled stage blocks are visible; the last flush is done
     tile_zero(sh, 3);
     const SceneDev& S = scenes[s];
-    // the next item and (last warp) its pool slots, loaded ahead of use
+    // the next item, loaded ahead of use
     int sn = 0;
     const int un = next_running(scenes, item_prefix, nscenes, k, u + gridDim.x, total, sn);
     int4 itn = make_int4(0, 0, 0, 0);
-    int slot = -1;
-    if (un < total) {
-      itn = scenes[sn].items[un - item_prefix[sn]];
-      if (lastw) slot = tile_slot(scenes[sn], itn, lane);
-    }
+    if (un < total) itn = scenes[sn].items[un - item_prefix[sn]];
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);
     const int i = threadIdx.x;
@@ -293,12 +277,15 @@ __global__ void __launch_bounds__(kItemMax, 2) k_hess(const SceneDev* __restrict
       hess_gather(sh, S, bx, by, bz, base, w, Gm);
       have = hess_particle(S, it.y + i, binned, Gm, q);
     }
-    if (!p2g_tile_accumulate<kP2gForce>(sh, S, bx, by, bz, have, q, w, base, FixScale{1.0f, 1.0f, 1.0f})) {
+    P2GStored stored;
+    p2g_count<kP2gForce>(sh, S, bx, by, bz, have, q, w, base, FixScale{1.0f, 1.0f, 1.0f}, stored);
+    __syncthreads();
+    if (sh.abort) {
       stage_abort(sh, S);  // a copy wait ran out: the CTA stops
       return;
     }
-    if (lastw && un < total)
-      stage_issue(sh, scenes[sn].cru, kImpBlockFloats, lane < 27 ? slot : -1, scenes[sn].tx_unsent);
+    p2g_sum<kP2gForce>(sh, S, bx, by, bz, stored, w);
+    if (un < total) stage_issue<kImpFields>(sh, scenes[sn], scenes[sn].cru, itn.x);
     p2g_tile_flush<kP2gForce>(sh, S, bx, by, bz);
     u = un;
     s = sn;
@@ -369,6 +356,13 @@ __device__ __forceinline__ void take_ku(const SceneDev& S, int slot, int node, b
   }
 }
 
+// Index in gout and cru of node `node` of the active block at `slot`.
+__device__ __forceinline__ size_t slot_node(const SceneDev& S, int slot, int node) {
+  int bx, by, bz;
+  home_coords(S, S.active[slot], bx, by, bz);
+  return node_index(S, 4 * bx + (node & 3), 4 * by + ((node >> 2) & 3), 4 * bz + (node >> 4));
+}
+
 __device__ __forceinline__ float dot3f(const float a[3], const float b[3]) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
 // M^1/2 and M^-1/2 at a node (both 0 without mass).
@@ -392,7 +386,7 @@ __global__ void __launch_bounds__(256) k_cr_begin(const SceneDev* __restrict__ s
         mass_scales(vm.w, sq, isq);
         const float ci = -S.imp_beta * S.dt * S.dt * isq;
         const float r[3] = {ci * ku[0], ci * ku[1], ci * ku[2]};
-        float* u = S.cru + (size_t)slot * kImpBlockFloats + 3 * node;
+        float* u = S.cru + slot_node(S, slot, node) * kImpFields;
         u[0] = isq * r[0];
         u[1] = isq * r[1];
         u[2] = isq * r[2];
@@ -415,7 +409,7 @@ __device__ __forceinline__ void residual_and_ar(const SceneDev& S, int slot, int
   float sq, isq;
   mass_scales(S.crv[(size_t)slot * kBlockNodes + node].w, sq, isq);
   const float ci = S.imp_beta * S.dt * S.dt * isq;
-  const float* u = S.cru + (size_t)slot * kImpBlockFloats + 3 * node;
+  const float* u = S.cru + slot_node(S, slot, node) * kImpFields;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     r[k] = sq * u[k];
@@ -499,7 +493,7 @@ __global__ void __launch_bounds__(256) k_cr_update(const SceneDev* __restrict__ 
         vm.y += ai * p.y;
         vm.z += ai * p.z;
         S.crv[i] = vm;
-        float* u = S.cru + (size_t)slot * kImpBlockFloats + 3 * node;
+        float* u = S.cru + slot_node(S, slot, node) * kImpFields;
         const float r[3] = {sq * u[0] - alpha * ap.x, sq * u[1] - alpha * ap.y, sq * u[2] - alpha * ap.z};
         u[0] = isq * r[0];
         u[1] = isq * r[1];
@@ -531,7 +525,7 @@ __global__ void __launch_bounds__(256) k_cr_end(const SceneDev* __restrict__ sce
                                __fadd_rn(S.gpos[2], __fmul_rn(S.h, (float)gk))};
           float v[3] = {xm.x, xm.y, xm.z};
           collide(S.coll, S.ncoll, xi, v);
-          float* o = S.gout + (size_t)slot * kOutBlockFloats + kOutFields * node;
+          float* o = S.gout + node_index(S, gi, gj, gk) * kOutFields;
           const float vs[3] = {o[0], o[1], o[2]};
 #pragma unroll
           for (int k = 0; k < 3; k++) {

@@ -376,6 +376,10 @@ snow_status fast_alloc_pool(snow_scene* s, int cap_blocks) {
   if (d.crs && ((st = salloc(s, (size_t)cap_blocks * kBlockNodes * 3, &d.crv)) ||
                 (st = salloc(s, (size_t)cap_blocks * kImpBlockFloats, &d.cru))))
     return st;
+  // blocks that are not active read as zero
+  CK(cudaMemsetAsync(d.gout, 0, (size_t)cap_blocks * kOutBlockFloats * sizeof(float), ctx->stream));
+  if (d.cru) CK(cudaMemsetAsync(d.cru, 0, (size_t)cap_blocks * kImpBlockFloats * sizeof(float), ctx->stream));
+  CK(cudaMemsetAsync(d.blk_slot, 0xff, (size_t)d.nblocks * sizeof(int), ctx->stream));
   d.pool_cap = cap_blocks;
   return SNOW_OK;
 }

@@ -55,7 +55,7 @@ constexpr int kOutFields = 6;              // v* (3), d = v* - alpha p/m (3)
 // particles pile into a cell.
 constexpr int kAccWords = kAccFields;
 constexpr int kAccBlockWords = kAccWords * kBlockNodes;    // 448 (3584 bytes)
-constexpr int kOutBlockFloats = kOutFields * kBlockNodes;  // 384
+constexpr int kOutBlockFloats = kOutFields * kBlockNodes;  // 384: a block's share of gout
 
 // Fixed-point state of one scene's P2G sums. Magnitudes are the bits of
 // non-negative floats (they order like unsigned ints, so atomicMax records
@@ -110,7 +110,8 @@ struct CrScalars {
   int skip_left;               // steps still to skip (kept across steps)
   int pad;
 };
-constexpr int kImpBlockFloats = 3 * kBlockNodes;  // 192: one 3-vector per node
+constexpr int kImpFields = 3;                              // u of the solve: one 3-vector per node
+constexpr int kImpBlockFloats = kImpFields * kBlockNodes;  // 192: a block's share of cru
 constexpr uint32_t kDefaultWaitNs = 1000000000u;   // one second
 
 // Device-resident description of one FAST scene (read by every kernel).
@@ -154,7 +155,10 @@ struct SceneDev {
   unsigned long long* acc;  // nblocks x 320 words: the fixed-point P2G sums, word-major per block (dense)
   FixState* fix;            // their scales and the magnitudes the next scales are chosen from
   int* active;      // pool_cap: block id of each slot
-  float* gout;      // pool_cap x 384: grid-update output, per node (v*, d) as 6 floats
+  // grid-update output, dense over the nodes of the blocked grid (4 bdim per
+  // axis, x fastest), per node (v*, d) as 6 floats; zero in blocks that are
+  // not active, so that a node without mass reads as zero
+  float* gout;
   int pool_cap;
   // P2G work items: (home block, first particle, count, 0)
   int4* items;
@@ -170,16 +174,23 @@ struct SceneDev {
   float imp_tol;    // stop once |r| <= imp_tol |M^1/2 v*| (r of the mass-scaled system)
   int imp_maxit;    // at most this many iterations per step
   float4* crv;      // 3 planes of pool_cap x 64 float4 per node: (v, m), (p, 0), (A p, 0)
-  float* cru;       // pool_cap x 192: u = M^-1/2 r (the vector K is applied to), 3 floats per node
+  float* cru;       // u = M^-1/2 r (the vector K is applied to), 3 floats per node, dense as gout
   CrScalars* crs;
 };
 
 struct FastTuning {
   int sort_interval = 8;  // re-bin particles every k steps
-  int items_max = 256;    // most particles per work item (kMinItemMax .. 256)
-  int ctas_per_sm = 2;    // work-item CTAs launched per SM (1 or 2)
+  int items_max = 256;    // most particles per work item (kMinItemMax .. kItemMax)
+  int ctas_per_sm = 2;    // work-item CTAs launched per SM (1 .. kItemCtas)
 };
 constexpr int kMinItemMax = 64;
+// Threads of a work-item CTA (one particle each) and CTAs resident per SM:
+// registers (128 a thread) fit 16 warps an SM in any shape. 2 x 256 threads
+// against 3 x 160, 3 x 192 (96 registers, 0.4 KB of spills a thread) and
+// 2 x 320 (the same): 0.237 ms a step's fused kernel at 1M particles, 256^3,
+// against 0.26, 0.27 and 0.28.
+constexpr int kItemMax = 256;
+constexpr int kItemCtas = 2;
 
 // Work spaces over a batch: prefix[s] .. prefix[s+1] are scene s's units
 // (P2G work items, active blocks, grid blocks). Item and active-block counts

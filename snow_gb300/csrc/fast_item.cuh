@@ -563,6 +563,7 @@ struct ItemShared {
   short cells[kCells];               // occupied tile cells
   int4 item_q[2];                    // this and the next work item of the CTA
   int scene_q[2];                    // ... and their scenes
+  int index_q[2];                    // ... and their indices (total: no item)
   int coll_scene;                    // scene whose colliders sit in coll
   FixScale fscale;                   // fixed-point scales of coll_scene's P2G in this launch
   unsigned seen[3];                  // largest mass, |v|, force-term bound of coll_scene's particles (bits) ...

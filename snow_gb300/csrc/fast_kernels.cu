@@ -24,8 +24,8 @@
 //                the SVD clamp, J_p, velocity, colliders, position (particle
 //                advance), then scatter the updated particles (P2G of the
 //                next step) into a 9^3-node shared tile, cell by cell, and
-//                add the tile to acc. A CTA takes a contiguous range of
-//                items; consecutive items of one home block (a run) share
+//                add the tile to acc. The items of one home block (a run)
+//                share
 //                the staged grid rows and the tile, which is added to acc
 //                once per run.
 // Separate P2G and G2P kernels serve the first step after set-up and the
@@ -53,10 +53,6 @@ __device__ __forceinline__ void form_prefixes(const SceneDev* __restrict__ scene
   active[nscenes] = aa;
 }
 
-__global__ void k_prefix(const SceneDev* __restrict__ scenes, int nscenes, int* items, int* active) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) form_prefixes(scenes, nscenes, items, active);
-}
-
 // One CTA per scene: the step's counters reset, colliders advanced.
 __global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, int rigid) {
   const int s = blockIdx.x;
@@ -66,6 +62,7 @@ __global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, i
     S.counters[CNT_ACTIVE] = 0;
     S.counters[CNT_OVERFLOW] = 0;
     S.counters[CNT_BINNED] = 0;
+    S.counters[CNT_WORK] = 0;
     // the magnitudes of the particles the pending P2G scattered become the
     // ones this step's P2G chooses its fixed-point scales from
     FixState& f = *S.fix;
@@ -434,8 +431,8 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // P2G of the next, in one pass over the item's particles. The P2G stress uses
 // the rotation R = W V^T of the advance's SVD: F_E' = W S' V^T with S'
 // diagonal up to the Jacobi residual, whose polar rotation is W V^T.
-// A CTA takes a contiguous range of work items. Consecutive items of one
-// home block form a run: they share
+// The CTAs take units of work from a counter: all items of a home block (a run)
+// or, when the launch has few, single items. The items of a run share
 // the staged grid rows (copied once, by bulk copies issued while the
 // previous run's last item sums its P2G) and the P2G tile (added to acc
 // once, at the run's end). The P2G sums are fixed
@@ -444,6 +441,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // magnitudes of its particles for the next step's scales. BINNED: a step that
 // re-binned some scene; such a scene's particles are read from its binned
 // copies (CNT_BINNED) and, like every scene's, written to its streams.
+constexpr int kSingleItems = 5;
 template <bool BINNED>
 __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
                                                        const int* __restrict__ item_prefix, int nscenes) {
@@ -451,34 +449,56 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
   tile_init(sh);
   const int total = item_prefix[nscenes];
-  const int chunk = (total + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int u0 = min(total, (int)blockIdx.x * chunk), u1 = min(total, u0 + chunk);
-  if (u0 >= u1) return;
+  // Whole runs unless that leaves CTAs without work: a run of two or three
+  // items costs one copy of the grid rows and one flush, but the CTA that takes
+  // it last works alone: with at most 5 items a CTA single items are faster
+  // (262k particles, 4.6 items a CTA: 32 steps 4.36 against 4.54 ms; 32k: 4.60
+  // against 6.12), above that both take the same time. The counter instead of
+  // equal shares of consecutive items: the items differ (surface blocks hold
+  // few particles, compressed snow costs more), 24 steps of a 1.5M-particle
+  // block on a sphere 12.0 to 11.0 ms, 50 of 1M particles 17.2 to 16.3.
+  const bool single = total <= kSingleItems * (int)gridDim.x;
+  int* counter = &scenes[0].counters[CNT_WORK];
+  // the first item of the unit after the one that was handed out as u
+  auto next_unit = [&](int u, int& s, int4& it) {
+    for (;;) {
+      if (u >= total) return total;
+      s = find_scene(item_prefix, nscenes, u);
+      it = scenes[s].items[u - item_prefix[s]];
+      if (single || it.w > 0) return u;
+      u = (int)gridDim.x + atomicAdd(counter, 1);
+    }
+  };
   // The last warp, which holds the fewest particles of an item (items are
   // filled from thread 0), looks up the next item and issues the copies of its
   // particles.
   const int lane = threadIdx.x & 31;
   const bool lastw = (threadIdx.x >> 5) == (blockDim.x >> 5) - 1;
-  {
-    const int s0 = find_scene(item_prefix, nscenes, u0);
-    const SceneDev& S0 = scenes[s0];
-    const int4 it0 = S0.items[u0 - item_prefix[s0]];
-    stage_issue<kOutFields>(sh, S0, S0.gout, it0.x);
-    if (lastw) {
-      particles_issue(sh, S0, it0.y, min(it0.z, kItemMax), BINNED && particles_binned(S0));
-      if (lane == 0) {
-        sh.item_q[0] = it0;
-        sh.scene_q[0] = s0;
-        sh.coll_scene = -1;
-        sh.next_same = 0;
-      }
-    }
+  if (lastw && lane == 0) {
+    int s0 = 0;
+    int4 it0 = make_int4(0, 0, 0, 0);
+    sh.index_q[0] = next_unit((int)blockIdx.x, s0, it0);
+    sh.item_q[0] = it0;
+    sh.scene_q[0] = s0;
+    sh.coll_scene = -1;
+    sh.next_same = 0;
   }
+  __syncthreads();
+  if (sh.index_q[0] >= total) return;  // uniform across the CTA
+  {
+    const SceneDev& S0 = scenes[sh.scene_q[0]];
+    const int4 it0 = sh.item_q[0];
+    stage_issue<kOutFields>(sh, S0, S0.gout, it0.x);
+    if (lastw) particles_issue(sh, S0, it0.y, min(it0.z, kItemMax), BINNED && particles_binned(S0));
+  }
+  int left = 0;  // items of the unit after this one (the last warp's lane 0)
   uint32_t phase = 0, pphase = 0;
   int par = 0;
   bool run_start = true;  // uniform across the CTA
-  for (int u = u0; u < u1; u++, par ^= 1) {
+  for (;; par ^= 1) {
     __syncthreads();  // this item's queue entry is written; the last flush is done
+    const int u = sh.index_q[par];
+    if (u >= total) return;  // uniform across the CTA
     const int s = sh.scene_q[par];
     const SceneDev& S = scenes[s];
     if (s != sh.coll_scene) {  // uniform across the CTA
@@ -488,29 +508,30 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
         sh.pushed[0] = sh.pushed[1] = sh.pushed[2] = 0u;
       }
       load_colliders(sh, S);  // its closing barrier publishes fscale as well
-      if (threadIdx.x == 0) {
-        sh.coll_scene = s;
-        if (u == item_prefix[s]) {
-          S.fix->scale[0] = sh.fscale.m;
-          S.fix->scale[1] = sh.fscale.p;
-          S.fix->scale[2] = sh.fscale.f;
-        }
-      }
+      if (threadIdx.x == 0) sh.coll_scene = s;
+    }
+    if (threadIdx.x == 0 && u == item_prefix[s]) {
+      S.fix->scale[0] = sh.fscale.m;
+      S.fix->scale[1] = sh.fscale.p;
+      S.fix->scale[2] = sh.fscale.f;
     }
     if (run_start) {
       tile_zero(sh, kAccFields);
       if (threadIdx.x == 0) sh.run_bound = 0.0f;
     }
     const int4 it = sh.item_q[par];
-    const int un = u + 1;
-    // the next item's descriptor: loaded now, so that the loads' latency
-    // overlaps this item's G2P instead of delaying the last warp, and put in
-    // shared memory before this item's P2G
-    int sn = 0;
+    // the next item: looked up now, so that the latency overlaps this item's
+    // G2P, and put in shared memory before this item's P2G
+    int sn = s, un = u + 1;
     int4 itn = make_int4(0, 0, 0, 0);
-    if (lastw && un < u1) {
-      sn = find_scene(item_prefix, nscenes, un);
-      itn = scenes[sn].items[un - item_prefix[sn]];
+    if (lastw && lane == 0) {
+      if (run_start) left = single ? 0 : it.w - 1;
+      if (left > 0) {
+        left--;
+        itn = S.items[un - item_prefix[s]];
+      } else {
+        un = next_unit((int)gridDim.x + atomicAdd(counter, 1), sn, itn);
+      }
     }
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);
@@ -540,6 +561,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       const PDef def = {sh.pfa[i], sh.pfb[i], sh.pvq[i], sh.pfc[i + (it.y & 1)]};
       Advanced adv;
       advance_particle(S, p, ps, def, dv, L, sh, adv);
+      if (BINNED && particles_binned(S)) S.pid[p] = S.bpid[p];
       // P2G quantities of the advanced particle
       q.m = adv.xm.w;
       if (fabsf(q.m) <= 100.0f) {  // p2gTransfer.glsl:64-66
@@ -567,11 +589,12 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     // the next item's queue entry: every thread read this one's at the loop
     // top, and the barriers below publish it before the flush decision
     if (lastw && lane == 0) {
-      const bool same = sn == s && itn.x == it.x;
+      const bool same = un == u + 1 && sn == s && itn.x == it.x;  // (single items of a block may also come one after the other)
       sh.item_q[par ^ 1] = itn;
       sh.scene_q[par ^ 1] = sn;
-      sh.next_same = un < u1 && same ? 1 : 0;
-      sh.next_issue = un < u1 && !same ? 1 : 0;
+      sh.index_q[par ^ 1] = un;
+      sh.next_same = un < total && same ? 1 : 0;
+      sh.next_issue = un < total && !same ? 1 : 0;
     }
     P2GStored stored;
     p2g_count<kP2gFull, true>(sh, S, bx, by, bz, have, q, wn, nbase, sh.fscale, stored);
@@ -580,7 +603,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       stage_abort(sh, S);  // a copy wait ran out: this item's particles keep their state, the CTA stops
       return;
     }
-    if (lastw && un < u1) {
+    if (lastw && sh.index_q[par ^ 1] < total) {
       const int4 nx = sh.item_q[par ^ 1];
       const SceneDev& N = scenes[sh.scene_q[par ^ 1]];
       particles_issue(sh, N, nx.y, min(nx.z, kItemMax), BINNED && particles_binned(N));
@@ -798,10 +821,6 @@ int num_sms() {
   return n[dev];
 }
 
-
-void fast_prefix(const SceneDev* scenes, int nscenes, int* items_prefix, int* active_prefix, cudaStream_t st) {
-  k_prefix<<<1, 32, 0, st>>>(scenes, nscenes, items_prefix, active_prefix);
-}
 
 void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st) {
   if (nscenes > 0) k_begin_step<<<nscenes, 32, 0, st>>>(scenes, nscenes, rigid ? 1 : 0);

@@ -43,12 +43,6 @@ struct snow_ctx {
   bool stat_pending[SNOW_STATS_SLOTS] = {};
   int* h_counters = nullptr;      // pinned, kCounterStride ints
   cudaEvent_t ev[8] = {};
-  // side streams for independent per-scene work inside a batch step (the
-  // re-binning of several scenes runs as parallel graph branches)
-  static constexpr int kAux = 8;
-  cudaStream_t aux[kAux] = {};
-  cudaEvent_t fork_ev = nullptr;
-  cudaEvent_t join_ev[kAux] = {};
   // the semi-implicit solve: its iteration counter and the stream its loop
   // body is captured from (all solves of a context run on `stream`, in order)
   int* d_iter = nullptr;
@@ -81,7 +75,8 @@ struct snow_scene {
   BinScratch bin{};
   FastTuning tune{};
   int key_bits = 0;
-  int* d_prefix = nullptr;  // [0,2) items, [2,4) active, [6,8) blocks
+  int* d_prefix = nullptr;  // the prefixes of `work`, two entries each
+  WorkSpace work{};
   int steps_since_sort = 1 << 30;
   // re-binning interval in use (1 .. tune.sort_interval): dropped to 1 when
   // particles leave their work items' tiles between binnings, doubled back
@@ -115,9 +110,9 @@ struct snow_batch {
   snow_ctx* ctx = nullptr;
   std::vector<snow_scene*> scenes;
   SceneDev* d_scenes = nullptr;
-  int* d_prefix = nullptr;  // items (n+1), active (n+1), unused (n+1), blocks (n+1)
+  int* d_prefix = nullptr;  // the prefixes of `work`, n + 1 entries each
+  WorkSpace work{};
   std::vector<int> versions;
-  long long total_blocks = 0;
   int step_count = 0;
   std::map<int, cudaGraphExec_t> graphs;  // 0: the step that re-bins every scene, 1: the others
   std::vector<float> g_dt;
@@ -267,6 +262,8 @@ void fill_sd_params(snow_scene* s) {
   d.h = s->p.grid_spacing;
   d.inv_h = 1.0f / s->p.grid_spacing;
   d.nblocks = d.bdim[0] * d.bdim[1] * d.bdim[2];
+  d.nchunks = (d.nblocks + kBinChunk - 1) / kBinChunk;
+  d.items_max = s->tune.items_max;
   d.young = s->p.young;
   // mu0 = E / (2 (1 + nu)), lambda0 = E nu / ((1 + nu)(1 - 2 nu)), in the
   // order and precision lame.include.glsl evaluates them per particle
@@ -324,6 +321,11 @@ snow_status fast_alloc_particles(snow_scene* s, size_t cap) {
   d.bfb = b.tmp4[3];
   d.bvq = b.tmp4[4];
   d.bfc = b.tmp2;
+  d.bpid = b.tmp_pid;
+  d.bkey = b.keys[0];
+  d.brank = b.vals[0];
+  d.bidx = b.vals[1];
+  d.bskey = b.keys[1];
   d.item_cap = (int)(cap / kMinItemMax + std::min<size_t>(cap, (size_t)d.nblocks) + 1);
   if ((st = salloc(s, (size_t)d.item_cap, &d.items))) return st;
   return SNOW_OK;
@@ -336,9 +338,10 @@ snow_status fast_alloc_grid(snow_scene* s) {
   const size_t nb = (size_t)d.nblocks;
   if ((st = salloc(s, nb, &d.blk_slot)) || (st = salloc(s, nb, &d.blk_flag)) ||
       (st = salloc(s, nb * kAccBlockWords, &d.acc)) || (st = salloc(s, (size_t)1, &d.fix)) ||
-      (st = salloc(s, nb, &s->bin.bstart)) ||
-      (st = salloc(s, nb, &s->bin.bend)) || (st = salloc(s, nb, &s->bin.home)) ||
-      (st = salloc(s, (size_t)kCounterStride, &d.counters)) || (st = salloc(s, (size_t)8, &s->d_prefix)) ||
+      (st = salloc(s, nb, &d.bstart)) || (st = salloc(s, nb, &d.bend)) || (st = salloc(s, nb, &d.bcount)) ||
+      (st = salloc(s, (size_t)d.nchunks, &d.bchunk)) ||
+      (st = salloc(s, (size_t)kCounterStride, &d.counters)) ||
+      (st = salloc(s, (size_t)kWorkPrefixes * 2, &s->d_prefix)) ||
       (st = salloc(s, (size_t)1, &s->sd_dev)))
     return st;
   if (is_implicit(s->p) && (st = salloc(s, (size_t)1, &d.crs))) return st;
@@ -346,6 +349,7 @@ snow_status fast_alloc_grid(snow_scene* s) {
   if (d.crs) CK(cudaMemsetAsync(d.crs, 0, sizeof(CrScalars), ctx->stream));
   CK(cudaMemsetAsync(d.blk_flag, 0, nb * sizeof(int), ctx->stream));
   CK(cudaMemsetAsync(d.blk_slot, 0xff, nb * sizeof(int), ctx->stream));
+  CK(cudaMemsetAsync(d.bcount, 0, nb * sizeof(int), ctx->stream));
   CK(cudaMemsetAsync(d.acc, 0, nb * kAccBlockWords * sizeof(unsigned long long), ctx->stream));
   {
     FixState f{};
@@ -384,12 +388,37 @@ snow_status fast_alloc_pool(snow_scene* s, int cap_blocks) {
   return SNOW_OK;
 }
 
-// Prefix arrays of a one-scene work space: [items 0,1][active 2,3][blocks 6,7];
-// items and active are written on the device.
+// The work space of n scenes whose prefixes lie in d_prefix (items and active
+// are written on the device).
+WorkSpace make_work(const SceneDev* scenes, int n, int* d_prefix) {
+  WorkSpace w{};
+  w.scenes = scenes;
+  w.nscenes = n;
+  w.items = d_prefix;
+  w.active = d_prefix + (n + 1);
+  w.particles = d_prefix + 2 * (n + 1);
+  w.blocks = d_prefix + 3 * (n + 1);
+  w.chunks = d_prefix + 4 * (n + 1);
+  return w;
+}
+// Appends scene `sd` as the i-th of n to the host copy of the prefixes.
+void add_work(WorkSpace& w, std::vector<int>& pre, int i, const SceneDev& sd) {
+  const int n = w.nscenes;
+  pre.resize((size_t)kWorkPrefixes * (n + 1), 0);
+  w.total_particles += sd.n;
+  w.total_blocks += sd.nblocks;
+  w.total_chunks += sd.nchunks;
+  pre[2 * (n + 1) + i + 1] = (int)w.total_particles;
+  pre[3 * (n + 1) + i + 1] = (int)w.total_blocks;
+  pre[4 * (n + 1) + i + 1] = (int)w.total_chunks;
+}
+
 snow_status fast_single_prefix(snow_scene* s) {
   snow_ctx* ctx = s->ctx;
-  int h[2] = {0, s->sd.nblocks};
-  CK(cudaMemcpyAsync(s->d_prefix + 6, h, 2 * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+  s->work = make_work(s->sd_dev, 1, s->d_prefix);
+  std::vector<int> pre;
+  add_work(s->work, pre, 0, s->sd);
+  CK(cudaMemcpyAsync(s->d_prefix, pre.data(), pre.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return SNOW_OK;
 }
@@ -397,20 +426,15 @@ snow_status fast_single_prefix(snow_scene* s) {
 int item_ctas(const FastTuning& t) { return num_sms() * t.ctas_per_sm; }
 int grid_ctas() { return num_sms() * 8; }
 
-// Binning: keys, radix sort, permutation, work items, item prefix.
-// in_step: the step's fused kernel follows in the same stream and reads the
-// particles from the binned copies (no copy back); else they are copied back
-// for the per-kernel P2G that follows.
-void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) {
-  fast_sort_keys(s->sd, s->sd_dev, s->bin, s->key_bits, st);
-  fast_apply_bins(s->sd, s->sd_dev, s->bin, s->tune.items_max, !in_step, st);
-  fast_prefix(s->sd_dev, 1, s->d_prefix + 0, s->d_prefix + 2, st);
-}
+// Binning of one scene. in_step: the step's fused kernel follows in the same
+// stream and reads the particles from the binned copies (no copy back); else
+// they are copied back for the per-kernel P2G that follows.
+void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) { fast_bin_scenes(s->work, !in_step, st); }
 
 // Active blocks of the pending P2G sums -> pool slots (and prefixes).
 void fast_enqueue_compact(snow_scene* s, cudaStream_t st, bool counters_reset = false) {
   if (!counters_reset) fast_begin_step(s->sd_dev, 1, false, st);
-  fast_compact(s->sd_dev, s->d_prefix + 6, 1, s->sd.nblocks, s->d_prefix + 0, s->d_prefix + 2, st);
+  fast_compact(s->sd_dev, s->work.blocks, 1, s->work.total_blocks, s->work.items, s->work.active, st);
 }
 void fast_enqueue_p2g(snow_scene* s, bool mass_only, cudaStream_t st) {
   fast_p2g(s->sd_dev, s->sd, s->d_prefix + 0, 1, item_ctas(s->tune), mass_only, st);
@@ -676,11 +700,6 @@ snow_status snow_ctx_create(int device, size_t hbm_budget_bytes, snow_ctx** out)
     e = cudaEventCreateWithFlags(&ctx->stat_ev[i], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_counters, kCounterStride * sizeof(int));
   for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&ctx->ev[i]);
-  for (int i = 0; i < snow_ctx::kAux && e == cudaSuccess; i++) {
-    e = cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_ev[i], cudaEventDisableTiming);
-  }
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_iter, sizeof(int));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->body_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->gate_stream, cudaStreamNonBlocking);
@@ -700,14 +719,6 @@ void snow_ctx_destroy(snow_ctx* ctx) {
   while (!ctx->scenes.empty()) snow_scene_destroy(*ctx->scenes.begin());
   for (int i = 0; i < 8; i++)
     if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
-  for (int i = 0; i < snow_ctx::kAux; i++) {
-    if (ctx->aux[i]) {
-      cudaStreamSynchronize(ctx->aux[i]);
-      cudaStreamDestroy(ctx->aux[i]);
-    }
-    if (ctx->join_ev[i]) cudaEventDestroy(ctx->join_ev[i]);
-  }
-  if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   if (ctx->body_stream) cudaStreamDestroy(ctx->body_stream);
   if (ctx->gate_stream) cudaStreamDestroy(ctx->gate_stream);
   if (ctx->d_iter) cudaFree(ctx->d_iter);
@@ -760,7 +771,7 @@ size_t snow_scene_footprint(const snow_params* p, size_t n) {
   // A semi-implicit scene adds per pool block its solver planes (64 nodes x
   // (3 float4 + 3 floats)) and one scalar record.
   const double solver = is_implicit(*p) ? nb * (64 * (48.0 + 12.0)) + sizeof(CrScalars) : 0.0;
-  return (size_t)(n * (92.0 + 108.0 + 100.0) + tiles * 256 * 4.0 + 4096.0 + items * 16.0 + nb * (kAccBlockWords * 8.0 + 5 * 4.0) +
+  return (size_t)(n * (92.0 + 108.0 + 100.0) + tiles * 256 * 4.0 + 4096.0 + items * 16.0 + nb * (kAccBlockWords * 8.0 + 5 * 4.0 + 4.0 / kBinChunk) +
                   nb * (384 * 4.0 + 4.0) + solver + 1024.0);
 }
 
@@ -1441,7 +1452,7 @@ snow_status snow_batch_create(snow_ctx* ctx, snow_scene* const* scenes, int n, s
   b->scenes.assign(scenes, scenes + n);
   snow_status st;
   if ((st = dalloc(ctx, b->allocs, b->bytes, sizeof(SceneDev) * n, (void**)&b->d_scenes)) ||
-      (st = dalloc(ctx, b->allocs, b->bytes, sizeof(int) * 4 * (n + 1), (void**)&b->d_prefix))) {
+      (st = dalloc(ctx, b->allocs, b->bytes, sizeof(int) * kWorkPrefixes * (n + 1), (void**)&b->d_prefix))) {
     snow_batch_destroy(b);
     return st;
   }
@@ -1483,18 +1494,15 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
   if (want != b->g_dt) changed = true;
   if (!changed) return SNOW_OK;
   std::vector<SceneDev> sds(n);
-  std::vector<int> pre(4 * (n + 1), 0);
-  long long blocks = 0;
+  b->work = make_work(b->d_scenes, n, b->d_prefix);
+  std::vector<int> pre;
   for (int i = 0; i < n; i++) {
     snow_scene* s = b->scenes[i];
     s->sd.dt = want[i];
     s->last_dt = want[i];
     sds[i] = s->sd;
-    pre[3 * (n + 1) + i] = (int)blocks;
-    blocks += s->sd.nblocks;
+    add_work(b->work, pre, i, s->sd);
   }
-  pre[3 * (n + 1) + n] = (int)blocks;
-  b->total_blocks = blocks;
   CK(cudaMemcpyAsync(b->d_scenes, sds.data(), sizeof(SceneDev) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(b->d_prefix, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, ctx->stream));
   for (int i = 0; i < n; i++) {
@@ -1514,35 +1522,16 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
 
 void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   const int n = (int)b->scenes.size();
-  int* pre = b->d_prefix;
-  int* items = pre;
-  int* active = pre + (n + 1);
-  int* blocks = pre + 3 * (n + 1);
+  int* items = b->work.items;
+  int* active = b->work.active;
   fast_begin_step(b->d_scenes, n, true, st);
   // every scene re-binned in the same step, every sort_interval steps, so
   // the other steps run the fused kernel's plain instantiation (re-binning a
   // staggered subset of the scenes each step made every step take the
   // binned one: 3% slower on 16 scenes of 2M-8M particles and on 64 of
-  // 10k-500k, A/B on one GPU); the scenes' binnings are independent, so they
-  // run on side streams (parallel branches of the step's graph) and join
-  // before the compaction
-  std::vector<int> bins;
-  if (bin_all)
-    for (int i = 0; i < n; i++) bins.push_back(i);
-  snow_ctx* ctx = b->ctx;
-  if (bins.size() < 2) {
-    for (int i : bins) fast_bin(b->scenes[i], st, true);
-  } else {
-    const int lanes = std::min((int)bins.size(), (int)snow_ctx::kAux);
-    cudaEventRecord(ctx->fork_ev, st);
-    for (int k = 0; k < lanes; k++) cudaStreamWaitEvent(ctx->aux[k], ctx->fork_ev, 0);
-    for (size_t k = 0; k < bins.size(); k++) fast_bin(b->scenes[bins[k]], ctx->aux[k % lanes], true);
-    for (int k = 0; k < lanes; k++) {
-      cudaEventRecord(ctx->join_ev[k], ctx->aux[k]);
-      cudaStreamWaitEvent(st, ctx->join_ev[k], 0);
-    }
-  }
-  fast_compact(b->d_scenes, blocks, n, b->total_blocks, items, active, st);
+  // 10k-500k, A/B on one GPU)
+  if (bin_all) fast_bin_scenes(b->work, false, st);
+  fast_compact(b->d_scenes, b->work.blocks, n, b->work.total_blocks, items, active, st);
   fast_grid(b->d_scenes, active, n, grid_ctas(), false, st);
   int iters = 0;  // the solve runs while any semi-implicit scene still iterates
   for (snow_scene* s : b->scenes)
@@ -1550,7 +1539,7 @@ void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   if (iters > 0)
     fast_implicit_solve(b->d_scenes, items, active, n, iters, item_ctas(b->scenes[0]->tune), grid_ctas(),
                         b->ctx->d_iter, b->ctx->body_stream, b->ctx->gate_stream, st);
-  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), !bins.empty(), st);
+  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), bin_all, st);
 }
 
 }  // namespace
@@ -1632,6 +1621,11 @@ snow_status snow_scene_set_tuning(snow_scene* s, const snow_tuning* t) {
   s->tune.ctas_per_sm = t->ctas_per_sm;
   s->bin_interval = t->sort_interval;
   s->clean_checks = 0;
+  if (s->sd.items_max != t->items_max) {
+    s->sd.items_max = t->items_max;
+    snow_status r = push_sd(s);
+    if (r) return r;
+  }
   // the next step re-bins with the new work split
   if (s->p2g_ready) s->steps_since_sort = s->bin_interval;
   if (split_changed) drop_graphs(s);
@@ -1647,6 +1641,8 @@ snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t) {
     s->tune.items_max = t->items_max;
     s->tune.ctas_per_sm = t->ctas_per_sm;
     s->bin_interval = t->sort_interval;
+    s->sd.items_max = t->items_max;
+    s->version++;  // the batch's next step copies the descriptors
     drop_graphs(s);
   }
   for (auto& g : b->graphs) cudaGraphExecDestroy(g.second);

@@ -78,12 +78,13 @@ enum {
   CNT_OVERFLOW = 1,   // blocks that found no slot in the pool
   CNT_ITEMS = 2,      // P2G work items since the last binning
   CNT_NONFINITE = 3,  // particles with a non-finite field (cumulative)
-  CNT_HOME = 4,       // occupied home blocks at the last binning
+  CNT_HOME = 4,       // unused
   CNT_FALLBACK = 5,   // particles that left their P2G tile (diagnostic, cumulative)
   CNT_TIMEOUT = 6,    // bounded waits that ran out (cumulative)
   CNT_DONE = 7,       // CTAs of the compaction finished (the last forms the prefixes)
   CNT_BINNED = 8,     // 1: this step's binning left the particles in the binned copies
-  kCounterStride = 9
+  CNT_WORK = 9,       // hands out the fused kernel's work to its CTAs (scene 0's)
+  kCounterStride = 10
 };
 
 // Semi-implicit velocity solve: conjugate residuals on the mass-scaled form
@@ -143,12 +144,27 @@ struct SceneDev {
   // a step leaves the particles there (counters[CNT_BINNED] = 1), and the
   // kernels of that step read them from there until the fused kernel, which
   // writes every particle, has put them back into the streams above
-  const float4* bxm;
-  const float4* bvv;
-  const float4* bfa;
-  const float4* bfb;
-  const float2* bfc;
-  const float4* bvq;
+  float4* bxm;
+  float4* bvv;
+  float4* bfa;
+  float4* bfb;
+  float2* bfc;
+  float4* bvq;
+  uint32_t* bpid;
+  // binning (k_bin_*): per particle its key and its place among its block's,
+  // and the block-ordered particle indices and keys; per block its count (zero
+  // between binnings) and range; per kBinChunk blocks their count; most
+  // particles per work item
+  uint32_t* bkey;
+  uint32_t* brank;
+  uint32_t* bidx;
+  uint32_t* bskey;
+  int* bcount;
+  int* bstart;
+  int* bend;
+  int* bchunk;
+  int nchunks;
+  int items_max;
   // blocked grid
   int* blk_slot;    // nblocks: pool slot of the block this step, -1 if inactive
   int* blk_flag;    // nblocks: block received P2G sums since the last compaction
@@ -160,7 +176,8 @@ struct SceneDev {
   // not active, so that a node without mass reads as zero
   float* gout;
   int pool_cap;
-  // P2G work items: (home block, first particle, count, 0)
+  // P2G work items: (home block, first particle, count, and in a block's first
+  // item the number of its items, else 0)
   int4* items;
   int item_cap;
   int* counters;    // kCounterStride ints
@@ -192,10 +209,23 @@ constexpr int kMinItemMax = 64;
 constexpr int kItemMax = 256;
 constexpr int kItemCtas = 2;
 
-// Work spaces over a batch: prefix[s] .. prefix[s+1] are scene s's units
-// (P2G work items, active blocks, grid blocks). Item and active-block counts
-// are only known on the device; fast_prefix() forms both prefixes there.
-void fast_prefix(const SceneDev* scenes, int nscenes, int* items_prefix, int* active_prefix, cudaStream_t st);
+// Work spaces over nscenes scenes: prefix[s] .. prefix[s+1] are scene s's units
+// (P2G work items, active blocks, particles, grid blocks, chunks of grid
+// blocks), in one device array of five prefixes of nscenes + 1 entries. Item
+// and active-block counts are only known on the device; the binning and the
+// compaction form those two prefixes there.
+struct WorkSpace {
+  const SceneDev* scenes;
+  int nscenes;
+  int* items;
+  int* active;
+  const int* particles;
+  const int* blocks;
+  const int* chunks;
+  long long total_particles, total_blocks, total_chunks;
+};
+constexpr int kWorkPrefixes = 5;
+constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
 // Start of a step: resets the per-step counters and, with `rigid`, moves the
 // colliders by dt * velocity (rigidAdvance.glsl:14-18).
 void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st);
@@ -278,16 +308,12 @@ inline bool capture_handle(cudaStream_t st, cudaGraphConditionalHandle* cond) {
   return cudaGraphConditionalHandleCreate(cond, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
 }
 
-// Binning of one scene (host-side sizes known): keys -> radix sort ->
-// permutation of the particle streams -> P2G work items.
+// Scratch of a scene's binning and of the radix sort of its cell keys.
 struct BinScratch {
   uint32_t* keys[2];
   uint32_t* vals[2];
   uint32_t* hist;      // 256 x tiles
   uint32_t* scan_tmp;  // partial sums of the scan
-  int* bstart;         // nblocks
-  int* bend;           // nblocks
-  int* home;           // nblocks
   float4* tmp4[5];     // permutation targets for xm, vv, fa, fb, vq
   float2* tmp2;        // ... and fc
   uint32_t* tmp_pid;   // ... and pid
@@ -298,10 +324,11 @@ size_t radix_tiles(size_t n);
 // copy of the device descriptor) and leaves the sorted keys in keys[0] and
 // the permutation in vals[0].
 void fast_sort_keys(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, int key_bits, cudaStream_t st);
-// copy_back false: the particles stay in the binned copies (CNT_BINNED) for the
-// step's fused kernel; only valid when that kernel follows in the same step.
-void fast_apply_bins(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, int items_max, bool copy_back,
-                     cudaStream_t st);
+// Binning of every scene of the work space: particles into the order of the
+// stable sort by cell key, work items, the item prefix. copy_back false: the
+// particles stay in the binned copies (CNT_BINNED) for the step's fused kernel,
+// which must follow in the same step.
+void fast_bin_scenes(const WorkSpace& w, bool copy_back, cudaStream_t st);
 
 // Radix sort of arbitrary (key, value) pairs; the result lands in k[0]/v[0].
 void radix_sort_pairs(uint32_t* k[2], uint32_t* v[2], size_t n, int key_bits, uint32_t* hist, uint32_t* scan_tmp,

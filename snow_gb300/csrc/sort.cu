@@ -1,6 +1,7 @@
-// Particle binning for SNOW_MODE_FAST on sm_103a: cell keys, a stable LSD
-// radix sort of (key, particle index) pairs, the permutation of the particle
-// streams into key order and the P2G work items (home block, particle range).
+// Particle binning for SNOW_MODE_FAST on sm_103a: the particle streams in the
+// order of their cell keys and the P2G work items (home block, particle range);
+// and a stable LSD radix sort of (key, particle index) pairs for the callers
+// who ask for the sorted keys themselves.
 //
 // The reference has no sort (it scatters every (particle, neighbour) pair with
 // global int atomics, p2gTransfer.cpp:22-23); binning is what makes the
@@ -183,97 +184,291 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __res
   }
 }
 
-// ---- keys, permutation, work items -----------------------------------------
+// ---- cell keys ---------------------------------------------------------------
+__device__ __forceinline__ uint32_t cell_key(const SceneDev& S, float4 xm) {
+  const float x[3] = {xm.x, xm.y, xm.z};
+  int c[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    int v = (int)((x[k] - S.gpos[k]) / S.h);
+    v = v < 0 ? 0 : (v > S.dim[k] - 1 ? S.dim[k] - 1 : v);
+    c[k] = v;
+  }
+  const uint32_t b =
+      ((uint32_t)(c[2] >> 2) * (uint32_t)S.bdim[1] + (uint32_t)(c[1] >> 2)) * (uint32_t)S.bdim[0] + (uint32_t)(c[0] >> 2);
+  return b * 64u + (uint32_t)(c[0] & 3) + 4u * (uint32_t)(c[1] & 3) + 16u * (uint32_t)(c[2] & 3);
+}
+
 __global__ void k_keys(const SceneDev* __restrict__ sd, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   const SceneDev& S = *sd;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < S.n; p += gridDim.x * blockDim.x) {
-    const float4 xm = S.xm[p];
-    const float x[3] = {xm.x, xm.y, xm.z};
-    int c[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      int v = (int)((x[k] - S.gpos[k]) / S.h);
-      v = v < 0 ? 0 : (v > S.dim[k] - 1 ? S.dim[k] - 1 : v);
-      c[k] = v;
-    }
-    const uint32_t b = ((uint32_t)(c[2] >> 2) * (uint32_t)S.bdim[1] + (uint32_t)(c[1] >> 2)) * (uint32_t)S.bdim[0] +
-                       (uint32_t)(c[0] >> 2);
-    keys[p] = b * 64u + (uint32_t)(c[0] & 3) + 4u * (uint32_t)(c[1] & 3) + 16u * (uint32_t)(c[2] & 3);
+    keys[p] = cell_key(S, S.xm[p]);
     vals[p] = (uint32_t)p;
   }
 }
 
-// Gathers the particle streams into key order (into the scratch copies;
-// k_heads copies them back, or the step's fused kernel reads them there)
-// and zeroes the item and home counters.
-__global__ void k_permute(const SceneDev* __restrict__ sd, const uint32_t* __restrict__ perm, float4* __restrict__ xm,
-                          float4* __restrict__ vv, float4* __restrict__ fa, float4* __restrict__ fb,
-                          float2* __restrict__ fc, uint32_t* __restrict__ pid, float4* __restrict__ vq) {
-  const SceneDev& S = *sd;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    S.counters[CNT_ITEMS] = 0;
-    S.counters[CNT_HOME] = 0;
+// ---- binning -----------------------------------------------------------------
+// The order of the stable sort by cell key, in six kernels over all scenes of
+// a step instead of the radix sort's passes (five launches each, three or four
+// passes a scene): the particles are counted per grid block, the blocks' starts
+// are scanned, the particle indices are put into their blocks, one CTA per block
+// orders its few hundred by (cell, index), and the streams are moved. Bound by
+// launches in small scenes and by the 184 bytes a particle that the streams'
+// move reads and writes in large ones. A binning of 32k / 262k / 1M particles
+// took 67 / 81 / 126 us in 20 launches, now 20 / 28 / 69 in 6.
+__device__ __forceinline__ int scene_of(const int* __restrict__ prefix, int nscenes, long long u) {
+  int lo = 0, hi = nscenes;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if ((long long)prefix[mid] <= u)
+      lo = mid;
+    else
+      hi = mid;
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.n; i += gridDim.x * blockDim.x) {
-    const uint32_t src = perm[i];
-    xm[i] = S.xm[src];
-    vv[i] = S.vv[src];
-    fa[i] = S.fa[src];
-    fb[i] = S.fb[src];
-    fc[i] = S.fc[src];
-    pid[i] = S.pid[src];
-    vq[i] = S.vq[src];
+  return lo;
+}
+
+// Keys, and each particle's place among those of its block (in no particular
+// order): the lanes of a warp that share a block take their places with one
+// atomic.
+__global__ void __launch_bounds__(256) k_bin_count(const WorkSpace w) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long u0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; u0 < w.total_particles;
+       u0 += warps * 32) {
+    const bool valid = u0 + lane < w.total_particles;
+    const long long u = valid ? u0 + lane : w.total_particles - 1;
+    const int s = scene_of(w.particles, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int p = (int)(u - w.particles[s]);
+    const uint32_t key = cell_key(S, S.xm[p]);
+    const int b = (int)(key >> 6);
+    const unsigned long long id = valid ? (unsigned long long)s << 32 | (unsigned)b : ~0ull;
+    const uint32_t peers = __match_any_sync(0xffffffffu, id);
+    const int leader = __ffs(peers) - 1;
+    int base = 0;
+    if (valid && lane == leader) base = atomicAdd(&S.bcount[b], __popc(peers));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!valid) continue;
+    S.bkey[p] = key;
+    S.brank[p] = (uint32_t)(base + __popc(peers & ((1u << lane) - 1u)));
+    if (p == 0) S.counters[CNT_ITEMS] = 0;
   }
 }
 
-// Block ranges of the sorted keys and the list of home blocks; also copies
-// the permuted particle ids back, and with copy_back the permuted streams
-// (else the particles stay in the binned copies, flagged by CNT_BINNED, for
-// the step's fused kernel to read and write back).
-__global__ void k_heads(const SceneDev* __restrict__ sd, const uint32_t* __restrict__ keys, int* __restrict__ bstart,
-                        int* __restrict__ bend, int* __restrict__ home, const float4* __restrict__ xm,
-                        const float4* __restrict__ vv, const float4* __restrict__ fa, const float4* __restrict__ fb,
-                        const float2* __restrict__ fc, const uint32_t* __restrict__ pid,
-                        const float4* __restrict__ vq, int copy_back) {
-  const SceneDev& S = *sd;
-  const int n = S.n;
-  if (!copy_back && blockIdx.x == 0 && threadIdx.x == 0) S.counters[CNT_BINNED] = 1;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    S.pid[i] = pid[i];
-    if (copy_back) {
-      S.xm[i] = xm[i];
-      S.vv[i] = vv[i];
-      S.fa[i] = fa[i];
-      S.fb[i] = fb[i];
-      S.fc[i] = fc[i];
-      S.vq[i] = vq[i];
-    }
-    const uint32_t b = keys[i] >> 6;
-    if (i == 0 || (keys[i - 1] >> 6) != b) {
-      bstart[b] = i;
-      home[atomicAdd(&S.counters[CNT_HOME], 1)] = (int)b;
-    }
-    if (i == n - 1 || (keys[i + 1] >> 6) != b) bend[b] = i + 1;
+// Particles per chunk of blocks.
+__global__ void __launch_bounds__(kBinChunk / 2) k_bin_reduce(const WorkSpace w) {
+  for (long long u = blockIdx.x; u < w.total_chunks; u += gridDim.x) {
+    const int s = scene_of(w.chunks, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int c = (int)(u - w.chunks[s]), b0 = c * kBinChunk + 2 * (int)threadIdx.x;
+    int2 n = make_int2(0, 0);
+    if (b0 + 1 < S.nblocks)
+      n = *reinterpret_cast<const int2*>(S.bcount + b0);
+    else if (b0 < S.nblocks)
+      n.x = S.bcount[b0];
+    const int any = __syncthreads_or(n.x | n.y);
+    uint32_t sum = 0;
+    if (any) block_exclusive_scan((uint32_t)(n.x + n.y), &sum);
+    if (threadIdx.x == 0) S.bchunk[c] = (int)sum;
   }
 }
 
-__global__ void k_items(const SceneDev* __restrict__ sd, const int* __restrict__ bstart, const int* __restrict__ bend,
-                        const int* __restrict__ home, int items_max) {
-  const SceneDev& S = *sd;
-  const int nh = S.counters[CNT_HOME];
-  for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += gridDim.x * blockDim.x) {
-    const int b = home[h];
-    const int s = bstart[b], e = bend[b];
-    // split the block's particles into nit near-equal items of <= items_max
-    const int cnt = e - s;
-    const int nit = (cnt + items_max - 1) / items_max;
-    const int at = atomicAdd(&S.counters[CNT_ITEMS], nit);
-    for (int j = 0; j < nit; j++) {
-      if (at + j >= S.item_cap) break;  // cannot happen: item_cap covers the bound
-      const int first = s + (int)(((long long)j * cnt) / nit);
-      const int last = s + (int)(((long long)(j + 1) * cnt) / nit);
-      S.items[at + j] = make_int4(b, first, last - first, 0);
+// Block ranges and work items, a CTA per chunk of blocks: the chunk starts
+// after the particles of the chunks before it. Each block's particles are split
+// into near-equal items of at most S.items_max.
+__global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
+  __shared__ int first_item;
+  for (long long u = blockIdx.x; u < w.total_chunks; u += gridDim.x) {
+    const int s = scene_of(w.chunks, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int c = (int)(u - w.chunks[s]);
+    if (S.bchunk[c] == 0) continue;  // uniform across the CTA
+    uint32_t sum = 0, before;
+    for (int k = threadIdx.x; k < c; k += blockDim.x) sum += (uint32_t)S.bchunk[k];
+    block_exclusive_scan(sum, &before);
+    const int b0 = c * kBinChunk + 2 * (int)threadIdx.x;
+    int cnt[2], nit[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      cnt[k] = b0 + k < S.nblocks ? S.bcount[b0 + k] : 0;
+      nit[k] = (cnt[k] + S.items_max - 1) / S.items_max;
     }
+    uint32_t items;
+    uint32_t at = before + block_exclusive_scan((uint32_t)(cnt[0] + cnt[1]), nullptr);
+    const uint32_t ahead = block_exclusive_scan((uint32_t)(nit[0] + nit[1]), &items);
+    if (threadIdx.x == 0) first_item = atomicAdd(&S.counters[CNT_ITEMS], (int)items);
+    __syncthreads();
+    int it = first_item + (int)ahead;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      if (cnt[k] == 0) continue;
+      const int b = b0 + k;
+      S.bcount[b] = 0;
+      S.bstart[b] = (int)at;
+      S.bend[b] = (int)at + cnt[k];
+      for (int j = 0; j < nit[k]; j++, it++) {
+        if (it >= S.item_cap) break;  // cannot happen: item_cap covers the bound
+        const int first = (int)(((long long)j * cnt[k]) / nit[k]), last = (int)(((long long)(j + 1) * cnt[k]) / nit[k]);
+        S.items[it] = make_int4(b, (int)at + first, last - first, j == 0 ? nit[k] : 0);
+      }
+      at += (uint32_t)cnt[k];
+    }
+    __syncthreads();
+  }
+}
+
+// Particle indices and keys into block order. The CTA that finishes last forms
+// the item prefix.
+__global__ void __launch_bounds__(256) k_bin_place(const WorkSpace w) {
+  const long long stride = (long long)gridDim.x * blockDim.x, u0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (long long u = u0; u < w.total_particles; u += stride) {
+    const int s = scene_of(w.particles, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int p = (int)(u - w.particles[s]);
+    const uint32_t key = S.bkey[p];
+    const int d = S.bstart[key >> 6] + (int)S.brank[p];
+    S.bidx[d] = (uint32_t)p;
+    S.bskey[d] = key;
+  }
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&w.scenes[0].counters[CNT_DONE], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (last && threadIdx.x == 0) {
+    __threadfence();
+    int a = 0;
+    for (int s = 0; s < w.nscenes; s++) {
+      w.items[s] = a;
+      a += *(volatile int*)&w.scenes[s].counters[CNT_ITEMS];
+    }
+    w.items[w.nscenes] = a;
+    w.scenes[0].counters[CNT_DONE] = 0;
+  }
+}
+
+// One CTA per occupied block (by its first work item): its particle indices in
+// the order of their cells, and of the indices within a cell (a cell of more
+// than kMaxRanked keeps the order it came in). The moves that follow have a
+// thread per particle: done here, by the few hundred threads of a block's CTA,
+// they took 69 us at 1M particles against 35.
+constexpr int kCellThreads = 128;
+constexpr int kCellHeld = 6;  // particles a thread holds in registers: blocks up to 768 are read once
+constexpr int kMaxRanked = 128;
+__global__ void __launch_bounds__(kCellThreads) k_bin_cells(const WorkSpace w, int in_step) {
+  __shared__ int count[64], start[64], cursor[64];
+  __shared__ uint32_t sidx[kCellThreads * kCellHeld];
+  const int total = w.items[w.nscenes];
+  for (int u = blockIdx.x; u < total; u += gridDim.x) {
+    const int s = scene_of(w.items, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    if (in_step && u == w.items[s] && threadIdx.x == 0) S.counters[CNT_BINNED] = 1;
+    const int4 it = S.items[u - w.items[s]];
+    const int n0 = S.bstart[it.x], n = S.bend[it.x] - n0;
+    if (it.y != n0) continue;  // uniform across the CTA
+    const bool small = n <= kCellThreads * kCellHeld;
+    uint32_t p[kCellHeld];
+    int c[kCellHeld];
+    if (threadIdx.x < 64) count[threadIdx.x] = 0;
+    __syncthreads();
+    if (small) {
+#pragma unroll
+      for (int k = 0; k < kCellHeld; k++) {
+        const int i = k * kCellThreads + (int)threadIdx.x;
+        if (i < n) {
+          p[k] = S.bidx[n0 + i];
+          c[k] = (int)(S.bskey[n0 + i] & 63u);
+          atomicAdd(&count[c[k]], 1);
+        }
+      }
+    } else {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&count[S.bskey[n0 + i] & 63u], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int c0 = count[2 * threadIdx.x], c1 = count[2 * threadIdx.x + 1];
+      int incl = c0 + c1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)threadIdx.x >= o) incl += v;
+      }
+      const int at = incl - c0 - c1;
+      start[2 * threadIdx.x] = cursor[2 * threadIdx.x] = at;
+      start[2 * threadIdx.x + 1] = cursor[2 * threadIdx.x + 1] = at + c0;
+    }
+    __syncthreads();
+    if (small) {
+#pragma unroll
+      for (int k = 0; k < kCellHeld; k++)
+        if (k * kCellThreads + (int)threadIdx.x < n) sidx[atomicAdd(&cursor[c[k]], 1)] = p[k];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kCellHeld; k++) {
+        if (k * kCellThreads + (int)threadIdx.x >= n) break;
+        const int a = start[c[k]], m = count[c[k]];
+        int r = 0;
+        for (int j = a; j < a + m; j++) r += sidx[j] < p[k];
+        S.bidx[n0 + a + r] = p[k];
+      }
+    } else {
+      uint32_t* far = S.brank + n0;  // the places are no longer needed
+      for (int i = threadIdx.x; i < n; i += blockDim.x)
+        far[atomicAdd(&cursor[S.bskey[n0 + i] & 63u], 1)] = S.bidx[n0 + i];
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t q = far[i];
+        const int cell = (int)(S.bkey[q] & 63u), a = start[cell], m = count[cell];
+        int r = i - a;
+        if (m <= kMaxRanked) {
+          r = 0;
+          for (int j = a; j < a + m; j++) r += far[j] < q;
+        }
+        S.bidx[n0 + a + r] = q;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The particle streams into the binned copies, in the order bidx.
+__global__ void __launch_bounds__(256) k_bin_move(const WorkSpace w) {
+  for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < w.total_particles;
+       u += (long long)gridDim.x * blockDim.x) {
+    const int s = scene_of(w.particles, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int i = (int)(u - w.particles[s]);
+    const uint32_t p = S.bidx[i];
+    const float4 xm = S.xm[p], vv = S.vv[p], fa = S.fa[p], fb = S.fb[p], vq = S.vq[p];
+    const float2 fc = S.fc[p];
+    const uint32_t pid = S.pid[p];
+    S.bxm[i] = xm;
+    S.bvv[i] = vv;
+    S.bfa[i] = fa;
+    S.bfb[i] = fb;
+    S.bfc[i] = fc;
+    S.bvq[i] = vq;
+    S.bpid[i] = pid;
+  }
+}
+
+// The binned copies back into the streams.
+__global__ void __launch_bounds__(256) k_bin_back(const WorkSpace w) {
+  for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < w.total_particles;
+       u += (long long)gridDim.x * blockDim.x) {
+    const int s = scene_of(w.particles, w.nscenes, u);
+    const SceneDev& S = w.scenes[s];
+    const int i = (int)(u - w.particles[s]);
+    S.xm[i] = S.bxm[i];
+    S.vv[i] = S.bvv[i];
+    S.fa[i] = S.bfa[i];
+    S.fb[i] = S.bfb[i];
+    S.fc[i] = S.bfc[i];
+    S.vq[i] = S.bvq[i];
+    S.pid[i] = S.bpid[i];
   }
 }
 
@@ -317,16 +512,17 @@ void fast_sort_keys(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, i
   radix_sort_pairs(b.keys, b.vals, (size_t)sd.n, key_bits, b.hist, b.scan_tmp, st, start);
 }
 
-void fast_apply_bins(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, int items_max, bool copy_back,
-                     cudaStream_t st) {
-  if (sd.n <= 0) return;
-  const size_t n = (size_t)sd.n;
-  k_permute<<<grid_for(n, 256, 8), 256, 0, st>>>(sd_dev, b.vals[0], b.tmp4[0], b.tmp4[1], b.tmp4[2], b.tmp4[3],
-                                                  b.tmp2, b.tmp_pid, b.tmp4[4]);
-  k_heads<<<grid_for(n, 256, 8), 256, 0, st>>>(sd_dev, b.keys[0], b.bstart, b.bend, b.home, b.tmp4[0], b.tmp4[1],
-                                                b.tmp4[2], b.tmp4[3], b.tmp2, b.tmp_pid, b.tmp4[4], copy_back ? 1 : 0);
-  const size_t maxhome = n < (size_t)sd.nblocks ? n : (size_t)sd.nblocks;
-  k_items<<<grid_for(maxhome, 256, 4), 256, 0, st>>>(sd_dev, b.bstart, b.bend, b.home, items_max);
+void fast_bin_scenes(const WorkSpace& w, bool copy_back, cudaStream_t st) {
+  if (w.total_particles <= 0) return;
+  const size_t n = (size_t)w.total_particles;
+  k_bin_count<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
+  k_bin_reduce<<<grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st>>>(w);
+  k_bin_scan<<<grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st>>>(w);
+  k_bin_place<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
+  // an occupied block holds some hundred particles; at most one CTA for each 64
+  k_bin_cells<<<grid_for(n, 64, 16), kCellThreads, 0, st>>>(w, copy_back ? 0 : 1);
+  k_bin_move<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
+  if (copy_back) k_bin_back<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
 }
 
 }  // namespace snow

@@ -88,10 +88,11 @@ typedef struct snow_params {
   float alpha;            /* PIC/FLIP blend, 0.95 in the shaders  */
   float gravity[3];       /* (0, -9.81, 0) in gForceCompute.glsl  */
   int mode;               /* snow_mode                            */
-  int sort_interval;      /* FAST: re-bin particles at least every k steps (0 = library
-                           * default). snow_scene_step re-bins every step while particles
-                           * leave their work items' tiles between binnings (fast particles,
-                           * long steps) and returns to k once they stay put */
+  int sort_interval;      /* FAST: re-bin particles at least every k steps (0 = chosen from
+                           * the particles' speeds, at most 32). snow_scene_step re-bins more
+                           * often while particles leave their work items' tiles between
+                           * binnings (fast particles, long steps) and returns to k once they
+                           * stay put */
   /* Semi-implicit velocity update (the reference's SemiImplicitTimeUpdate,
    * an empty stub in semiimplicittimeupdate.cpp:3-5; Stomakhin et al. 2013,
    * eq. 9): with implicit_beta > 0 each step solves
@@ -195,15 +196,14 @@ snow_status snow_scene_init(snow_scene* s);
  * work is queued. Conditions counted on the device (non-finite particles:
  * SNOW_ENUMERIC, grid block pool overflow: SNOW_ECAPACITY, an expired
  * bounded wait: SNOW_ETIMEDOUT) are returned by a later step call, at the
- * second re-binning point after they occurred (the counters are read there
+ * second look after they occurred (every eight steps the counters are read
  * without waiting for the queued steps); snow_scene_stats counts non-finite
  * particles at once. CUDA errors surface at the next call that synchronises
  * (download, stats, snow_ctx_synchronize). */
 snow_status snow_scene_step(snow_scene* s, double dt, int n_steps);
 /* Waits for the scene's queued work and returns the first condition its
  * device counters hold (SNOW_ETIMEDOUT, SNOW_ECAPACITY, SNOW_ENUMERIC) or
- * SNOW_OK: the same checks snow_scene_step makes at its re-binning points,
- * at once. (No counterpart in the reference, which reports no errors.) */
+ * SNOW_OK: the same checks snow_scene_step makes every eight steps, at once. (No counterpart in the reference, which reports no errors.) */
 snow_status snow_scene_check(snow_scene* s);
 /* Bounded waits of the FAST kernels. A work item's wait for the bulk copies
  * of its grid tile into shared memory gives up after `wait_ns` nanoseconds
@@ -394,7 +394,7 @@ typedef struct snow_tuning {
 snow_status snow_scene_set_tuning(snow_scene* s, const snow_tuning* t);
 /* Applies a tuning to every scene of the batch (e.g. one kept from an
  * earlier autotune); the batch's next step starts the re-binning cycle
- * again (scene i re-bins at cycle step i mod sort_interval). */
+ * again. */
 snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t);
 /* Times candidate tunings (sort interval 1/2/4/8/12/16/24/32 x 128/256 particles per work
  * item x 1/2 CTAs per SM) on real steps of the batch and keeps the fastest;

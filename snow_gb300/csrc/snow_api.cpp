@@ -78,11 +78,16 @@ struct snow_scene {
   int* d_prefix = nullptr;  // the prefixes of `work`, two entries each
   WorkSpace work{};
   int steps_since_sort = 1 << 30;
-  // re-binning interval in use (1 .. tune.sort_interval): dropped to 1 when
+  // re-binning interval in use (1 .. tune.sort_interval): lowered when
   // particles leave their work items' tiles between binnings, doubled back
-  // after a run of clean checks
+  // after a run of clean checks (clean_needed, longer after each time that
+  // failed)
   int bin_interval = 8;
   int clean_checks = 0;
+  int clean_needed = 8;
+  int steps_since_check = 0;
+  float vmax = 0.0f;         // largest particle speed at the last look (init, checks)
+  float interval_dt = -1.0f;  // time step bin_interval was chosen for
   // the device counters as copied (without a wait) at the last binning point
   // and read at the next one
   int* h_cnt = nullptr;
@@ -113,7 +118,11 @@ struct snow_batch {
   int* d_prefix = nullptr;  // the prefixes of `work`, n + 1 entries each
   WorkSpace work{};
   std::vector<int> versions;
-  int step_count = 0;
+  int steps_since_check = 0;
+  int interval = 8;  // re-binning interval in use
+  bool interval_set = false;
+  long long fallbacks_seen = 0;
+  int steps_at_snapshot = 0;
   std::map<int, cudaGraphExec_t> graphs;  // 0: the step that re-bins every scene, 1: the others
   std::vector<float> g_dt;
   int g_threads = 0;
@@ -337,13 +346,16 @@ snow_status fast_alloc_grid(snow_scene* s) {
   snow_status st;
   const size_t nb = (size_t)d.nblocks;
   if ((st = salloc(s, nb, &d.blk_slot)) || (st = salloc(s, nb, &d.blk_flag)) ||
-      (st = salloc(s, nb * kAccBlockWords, &d.acc)) || (st = salloc(s, (size_t)1, &d.fix)) ||
+      (st = salloc(s, nb * kAccBlockWords, &d.acc)) ||
       (st = salloc(s, nb, &d.bstart)) || (st = salloc(s, nb, &d.bend)) || (st = salloc(s, nb, &d.bcount)) ||
       (st = salloc(s, (size_t)d.nchunks, &d.bchunk)) ||
       (st = salloc(s, (size_t)kCounterStride, &d.counters)) ||
       (st = salloc(s, (size_t)kWorkPrefixes * 2, &s->d_prefix)) ||
       (st = salloc(s, (size_t)1, &s->sd_dev)))
     return st;
+  static_assert(kCounters <= kFixOffset && kFixOffset * sizeof(int) + sizeof(FixState) <= kCounterStride * sizeof(int),
+                "the fixed-point state fits behind the counters");
+  d.fix = reinterpret_cast<FixState*>(d.counters + kFixOffset);
   if (is_implicit(s->p) && (st = salloc(s, (size_t)1, &d.crs))) return st;
   snow_ctx* ctx = s->ctx;
   if (d.crs) CK(cudaMemsetAsync(d.crs, 0, sizeof(CrScalars), ctx->stream));
@@ -351,13 +363,13 @@ snow_status fast_alloc_grid(snow_scene* s) {
   CK(cudaMemsetAsync(d.blk_slot, 0xff, nb * sizeof(int), ctx->stream));
   CK(cudaMemsetAsync(d.bcount, 0, nb * sizeof(int), ctx->stream));
   CK(cudaMemsetAsync(d.acc, 0, nb * kAccBlockWords * sizeof(unsigned long long), ctx->stream));
+  CK(cudaMemsetAsync(d.counters, 0, kCounterStride * sizeof(int), ctx->stream));
   {
     FixState f{};
     f.scale[0] = f.scale[1] = f.scale[2] = 1.0f;
     CK(cudaMemcpyAsync(d.fix, &f, sizeof f, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
-  CK(cudaMemsetAsync(d.counters, 0, kCounterStride * sizeof(int), ctx->stream));
   return SNOW_OK;
 }
 
@@ -478,26 +490,56 @@ snow_status check_counters(snow_scene* s, const int* h) {
   return SNOW_OK;
 }
 
-// At a binning point of snow_scene_step: checks the counters copied at the
-// previous binning point (that copy has long landed, so there is no wait for
-// the queued steps), adapts the re-binning interval to the share of
-// particle-steps that left their work item's tile since then (above 1/256:
-// re-bin every step; below 1/4096 eight times in a row: double the interval,
-// up to the tuned one), and copies the counters again for the next point.
-snow_status fast_check_async(snow_scene* s, int steps_since_last) {
+float fix_vmax(const int* counters) {
+  FixState f;
+  std::memcpy(&f, counters + kFixOffset, sizeof f);
+  const uint32_t bits = std::max(f.v_cur, f.v_prev);
+  float v;
+  std::memcpy(&v, &bits, sizeof v);
+  return v;
+}
+
+// Steps a scene can take between binnings before its fastest particles can
+// leave their work items' tiles, which reach one cell beyond the home block:
+// 1 / (vmax dt / h), and four fifths of that where it is more than the checks'
+// distance (the order of the particles within the block ages). A binning costs
+// a fifth (1M particles) to a half (32k) of a step: 100 steps of 32k particles
+// take 4.39 ms at the chosen interval, 4.60 at the fixed 8 it replaces, 50 of
+// 1M 16.20 against 16.35. Past the limit each particle outside its tile is
+// scattered with 448 global atomics: 20 steps of half a cell and 300k particles
+// took 4.34 ms until the counters showed it, 3.41 now; 8 semi-implicit steps
+// of a third of a cell and 131k particles 6.52, now 3.66.
+int safe_interval(const snow_scene* s, float dt) {
+  const double d = (double)s->vmax * dt / s->p.grid_spacing;
+  if (!(d > 1.0 / 128.0)) return kAutoInterval;  // (also for a scene that is not finite)
+  int n = (int)(1.0 / d);
+  if (n > kCheckSteps) n = std::max(kCheckSteps, (int)(0.8 / d));
+  return std::max(1, std::min(n, kAutoInterval));
+}
+
+// Every kCheckSteps steps and at each binning point of snow_scene_step: checks
+// the counters copied at the previous such point (that copy has long landed, so
+// there is no wait for the queued steps), adapts the re-binning interval to
+// the share of particle-steps that left their work item's tile since then (above
+// 1/256: as short as the speeds ask; below 1/4096 clean_needed times in a row:
+// doubled, up to the tuned one), and copies the counters again for the next one.
+snow_status fast_check_async(snow_scene* s) {
   snow_ctx* ctx = s->ctx;
   if (s->cnt_pending) {
     CK(cudaEventSynchronize(s->cnt_ev));
     s->cnt_pending = false;
     const int* h = s->h_cnt;
+    s->vmax = fix_vmax(h);
     const long long fb = (long long)(unsigned)h[CNT_FALLBACK];
     const long long delta = fb - s->fallbacks_seen;
     s->fallbacks_seen = fb;
     const double work = (double)s->steps_at_snapshot * (double)std::max<size_t>(s->n, 1);
     if (s->steps_at_snapshot > 0 && delta > work / 256.0) {
-      s->bin_interval = 1;
+      const int safe = safe_interval(s, s->last_dt);
+      s->clean_needed = std::min(1024, 4 * s->clean_needed);
+      s->bin_interval = s->tune.chosen || safe >= s->bin_interval ? 1 : safe;
       s->clean_checks = 0;
-    } else if (delta <= work / 4096.0 && ++s->clean_checks >= 8) {
+    } else if (delta <= work / 4096.0 && ++s->clean_checks >= s->clean_needed) {
       s->bin_interval = std::min(s->tune.sort_interval, 2 * s->bin_interval);
       s->clean_checks = 0;
     }
@@ -507,7 +549,8 @@ snow_status fast_check_async(snow_scene* s, int steps_since_last) {
   CK(cudaMemcpyAsync(s->h_cnt, s->sd.counters, kCounterStride * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaEventRecord(s->cnt_ev, ctx->stream));
   s->cnt_pending = true;
-  s->steps_at_snapshot = steps_since_last;
+  s->steps_at_snapshot = s->steps_since_check;
+  s->steps_since_check = 0;
   return SNOW_OK;
 }
 
@@ -547,7 +590,14 @@ snow_status fast_init(snow_scene* s) {
   fast_enqueue_grid(s, true, st);                                // clear acc
   fast_enqueue_p2g(s, false, st);                                // P2G of step 1
   CK(cudaGetLastError());
+  // the particles' largest speed, which the re-binning interval is chosen from
+  CK(cudaMemcpyAsync(s->h_cnt, s->sd.counters, kCounterStride * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  s->cnt_pending = false;
+  s->fallbacks_seen = (long long)(unsigned)s->h_cnt[CNT_FALLBACK];
+  s->vmax = fix_vmax(s->h_cnt);
+  s->interval_dt = -1.0f;
+  s->steps_since_check = 0;
   s->steps_since_sort = 0;
   s->p2g_ready = true;
   return SNOW_OK;
@@ -790,7 +840,10 @@ snow_status snow_scene_create(snow_ctx* ctx, const snow_params* p, const snow_co
   s->G = (long long)p->grid_dim[0] * p->grid_dim[1] * p->grid_dim[2];
   s->coll_h.assign(colliders, colliders + n_colliders);
   s->ncoll = n_colliders;
-  if (p->sort_interval > 0) s->tune.sort_interval = p->sort_interval;
+  if (p->sort_interval > 0) {
+    s->tune.sort_interval = p->sort_interval;
+    s->tune.chosen = true;
+  }
   s->bin_interval = s->tune.sort_interval;
   snow_status st = SNOW_OK;
   if (n_colliders > 0) st = salloc(s, (size_t)n_colliders, &s->coll_d);
@@ -1038,7 +1091,8 @@ snow_status snow_dispatch(snow_scene* s, int kernel, double dt) {
         fast_enqueue_compact(s, st);
         fast_enqueue_grid(s, true, st);
       }
-      if (s->steps_since_sort >= s->bin_interval) {
+      // (single kernels: the speeds are not looked at between the calls)
+      if (s->steps_since_sort >= (s->tune.chosen ? s->bin_interval : std::min(s->bin_interval, kCheckSteps))) {
         fast_bin(s, st, false);
         s->steps_since_sort = 0;
       }
@@ -1095,13 +1149,18 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
     fast_enqueue_p2g(s, false, st);
     s->p2g_ready = true;
   }
+  if (!s->tune.chosen && s->interval_dt != fdt) {
+    s->bin_interval = safe_interval(s, fdt);
+    s->clean_checks = 0;
+    s->clean_needed = 8;
+    s->interval_dt = fdt;
+  }
   for (int i = 0; i < n_steps; i++) {
-    const bool bin = s->steps_since_sort >= s->bin_interval;
-    if (bin) {
-      // binning points are where the host looks at the device counters
-      r = fast_check_async(s, std::min(s->steps_since_sort, 1 << 20));
+    if (s->steps_since_check >= kCheckSteps || s->steps_since_sort >= s->bin_interval) {
+      r = fast_check_async(s);
       if (r) return r;
     }
+    const bool bin = s->steps_since_sort >= s->bin_interval;
     if (ctx->profiling) {
       cudaEvent_t* ev = ctx->ev;
       CK(cudaEventRecord(ev[0], st));
@@ -1145,6 +1204,7 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       s->times.binnings++;
     }
     s->steps_since_sort++;
+    s->steps_since_check++;
   }
   CK(cudaGetLastError());
   return SNOW_OK;
@@ -1493,6 +1553,7 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
   }
   if (want != b->g_dt) changed = true;
   if (!changed) return SNOW_OK;
+  if (want != b->g_dt) b->interval_set = false;
   std::vector<SceneDev> sds(n);
   b->work = make_work(b->d_scenes, n, b->d_prefix);
   std::vector<int> pre;
@@ -1518,6 +1579,18 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
   for (auto& g : b->graphs) cudaGraphExecDestroy(g.second);
   b->graphs.clear();
   return SNOW_OK;
+}
+
+// The interval at which a batch re-bins all its scenes: the tuned one, or what
+// the fastest of its scenes allows, but no less than 8 while the particles stay
+// in their tiles (`leaving`: more than 1/256 of them do not).
+void batch_interval(snow_batch* b, bool leaving) {
+  int n = kAutoInterval;
+  for (size_t i = 0; i < b->scenes.size(); i++) n = std::min(n, safe_interval(b->scenes[i], b->scenes[i]->last_dt));
+  if (n < 8 && !leaving) n = std::max(n, b->interval_set ? std::min(b->interval, 8) : 8);
+  if (b->scenes[0]->tune.chosen) n = std::max(1, b->scenes[0]->tune.sort_interval);
+  b->interval = n;
+  b->interval_set = true;
 }
 
 void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
@@ -1563,42 +1636,58 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
   }
   snow_status r = batch_refresh(b, dt);
   if (r) return r;
-  const int interval = std::max(1, b->scenes[0]->tune.sort_interval);
+  if (!b->interval_set) batch_interval(b, false);
   for (int i = 0; i < n_steps; i++) {
-    const int phase = b->step_count % interval;
-    if (phase == 0 && b->step_count > 0) {
+    int since = 0;
+    for (snow_scene* s : b->scenes) since = std::max(since, s->steps_since_sort);
+    if (b->steps_since_check >= kCheckSteps || (since >= b->interval && b->steps_since_check > 0)) {
       // the counters gathered at the previous checking point (long landed:
       // no wait for the queued steps), then a new gather for the next one
       if (b->cnt_pending) {
         CK(cudaEventSynchronize(b->cnt_ev));
         b->cnt_pending = false;
+        long long fb = 0;
+        double parts = 0.0;
         for (size_t k = 0; k < b->scenes.size(); k++) {
-          r = check_counters(b->scenes[k], b->h_cnt + k * kCounterStride);
+          const int* h = b->h_cnt + k * kCounterStride;
+          r = check_counters(b->scenes[k], h);
           if (r) return r;
+          b->scenes[k]->vmax = fix_vmax(h);
+          fb += (unsigned)h[CNT_FALLBACK];
+          parts += (double)b->scenes[k]->n;
         }
+        const bool leaving = b->steps_at_snapshot > 0 && (double)(fb - b->fallbacks_seen) > parts * b->steps_at_snapshot / 256.0;
+        b->fallbacks_seen = fb;
+        batch_interval(b, leaving);
       }
       fast_gather_counters(b->d_scenes, (int)b->scenes.size(), b->d_hcnt, st);
       CK(cudaEventRecord(b->cnt_ev, st));
       b->cnt_pending = true;
+      b->steps_at_snapshot = b->steps_since_check;
+      b->steps_since_check = 0;
       r = batch_refresh(b, dt);
       if (r) return r;
     }
-    const int key = phase == 0 ? 0 : 1;  // a step that re-bins every scene, or none
+    const bool bin = since >= b->interval;
+    const int key = bin ? 0 : 1;  // a step that re-bins every scene, or none
     auto it = b->graphs.find(key);
     if (it == b->graphs.end()) {
       cudaGraph_t graph;
       cudaGraphExec_t exec;
       CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      batch_enqueue_step(b, phase == 0, st);
+      batch_enqueue_step(b, bin, st);
       CK(cudaStreamEndCapture(st, &graph));
       CK(cudaGraphInstantiate(&exec, graph, 0));
       cudaGraphDestroy(graph);
       it = b->graphs.emplace(key, exec).first;
     }
     CK(cudaGraphLaunch(it->second, st));
-    b->step_count++;
+    b->steps_since_check++;
+    for (snow_scene* s : b->scenes) {
+      s->steps_since_sort = bin ? 1 : s->steps_since_sort + 1;
+      s->steps_since_check++;
+    }
   }
-  for (snow_scene* s : b->scenes) s->steps_since_sort = 1;  // single-scene stepping re-bins on its own schedule
   CK(cudaGetLastError());
   return SNOW_OK;
 }
@@ -1617,6 +1706,7 @@ snow_status snow_scene_set_tuning(snow_scene* s, const snow_tuning* t) {
   // needs new ones
   const bool split_changed = s->tune.items_max != t->items_max || s->tune.ctas_per_sm != t->ctas_per_sm;
   s->tune.sort_interval = t->sort_interval;
+  s->tune.chosen = true;
   s->tune.items_max = t->items_max;
   s->tune.ctas_per_sm = t->ctas_per_sm;
   s->bin_interval = t->sort_interval;
@@ -1638,6 +1728,8 @@ snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t) {
   CK(cudaStreamSynchronize(ctx->stream));
   for (snow_scene* s : b->scenes) {
     s->tune.sort_interval = t->sort_interval;
+    s->tune.chosen = true;
+    s->steps_since_sort = 1 << 30;  // the next step re-bins with the new work split
     s->tune.items_max = t->items_max;
     s->tune.ctas_per_sm = t->ctas_per_sm;
     s->bin_interval = t->sort_interval;
@@ -1647,7 +1739,7 @@ snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t) {
   }
   for (auto& g : b->graphs) cudaGraphExecDestroy(g.second);
   b->graphs.clear();
-  b->step_count = 0;
+  b->interval_set = false;
   return SNOW_OK;
 }
 

@@ -84,7 +84,9 @@ enum {
   CNT_DONE = 7,       // CTAs of the compaction finished (the last forms the prefixes)
   CNT_BINNED = 8,     // 1: this step's binning left the particles in the binned copies
   CNT_WORK = 9,       // hands out the fused kernel's work to its CTAs (scene 0's)
-  kCounterStride = 10
+  kCounters = 10,
+  kFixOffset = 16,    // a scene's FixState follows its counters (one copy reads both)
+  kCounterStride = 32
 };
 
 // Semi-implicit velocity solve: conjugate residuals on the mass-scaled form
@@ -195,8 +197,13 @@ struct SceneDev {
   CrScalars* crs;
 };
 
+// Re-binning intervals when the caller names none, and the steps between the
+// host's looks at the device counters.
+constexpr int kAutoInterval = 32;
+constexpr int kCheckSteps = 8;
 struct FastTuning {
-  int sort_interval = 8;  // re-bin particles every k steps
+  int sort_interval = kAutoInterval;  // re-bin particles at least every k steps ...
+  bool chosen = false;                // ... asked for by the caller (else chosen from the speeds, up to kAutoInterval)
   int items_max = 256;    // most particles per work item (kMinItemMax .. kItemMax)
   int ctas_per_sm = 2;    // work-item CTAs launched per SM (1 .. kItemCtas)
 };
@@ -229,7 +236,7 @@ constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
 // Start of a step: resets the per-step counters and, with `rigid`, moves the
 // colliders by dt * velocity (rigidAdvance.glsl:14-18).
 void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st);
-// Copies every scene's counters into out[s * kCounterStride ...] (mapped
+// Copies every scene's counters and FixState into out[s * kCounterStride ...] (mapped
 // pinned memory: a batch reads them one re-binning interval later, without
 // draining the stream).
 void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStream_t st);

@@ -363,12 +363,13 @@ snow_status snow_server_drain(snow_server* srv, double timeout_s);
  * default stream) and the call returns without waiting.
  *
  * Scratch lives in one fixed device array inside the library, sized for
- * SNOW_SORT_STATIC_MAX_KEYS keys (about 2.1 MB, held by every GPU that loads
+ * SNOW_SORT_STATIC_MAX_KEYS keys (about 130 KB, held by every GPU that loads
  * the library until the process exits). n above that limit returns
  * SNOW_EINVAL and queues nothing. All calls share the array, so calls whose
  * work overlaps on the GPU (other streams, other host threads) race and must
- * be ordered by the caller; every pass overwrites the scratch it reads, so
- * nothing carried over from an earlier call needs clearing. The first call in
+ * be ordered by the caller; every call clears the scratch it relies on, so
+ * nothing carried over from an earlier call matters. The sort is one
+ * cooperative launch (at most 128 blocks). The first call in
  * a device context (and the first after that device's context was reset)
  * looks up the array's device address; make that first call before any
  * stream capture. Returns SNOW_ECUDA if a CUDA call fails. */

@@ -30,6 +30,8 @@
 //                once per run.
 // Separate P2G and G2P kernels serve the first step after set-up and the
 // per-kernel dispatch entry point.
+#include <algorithm>
+
 #include "snow_internal.h"
 #include "snow_math.cuh"
 #include "snow_stats.cuh"
@@ -159,19 +161,24 @@ __global__ void __launch_bounds__(256) k_fix_measure(const SceneDev* __restrict_
     v0 = fmaxf(v0, vv.w);
     if (with_stress) am = fmaxf(am, p2g_particle(S, p, xm, false).a);
   }
-  const unsigned bm = __reduce_max_sync(0xffffffffu, __float_as_uint(mm));
-  const unsigned bv = __reduce_max_sync(0xffffffffu, __float_as_uint(vm));
-  const unsigned ba = __reduce_max_sync(0xffffffffu, __float_as_uint(am));
-  const unsigned b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(v0));
-  if ((threadIdx.x & 31) == 0) {
+  // one warp's maxima per block, and only those above what is recorded: the
+  // same seven words for every warp of the GPU (39 us at 262k particles,
+  // now 12)
+  __shared__ unsigned best[4];
+  if (threadIdx.x < 4) best[threadIdx.x] = 0u;
+  __syncthreads();
+  const unsigned b[4] = {__reduce_max_sync(0xffffffffu, __float_as_uint(mm)), __reduce_max_sync(0xffffffffu, __float_as_uint(vm)),
+                         __reduce_max_sync(0xffffffffu, __float_as_uint(am)), __reduce_max_sync(0xffffffffu, __float_as_uint(v0))};
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < 4; k++) atomicMax(&best[k], b[k]);
+  __syncthreads();
+  if (threadIdx.x < 7) {
     FixState& f = *S.fix;
-    atomicMax(&f.m_prev, bm);
-    atomicMax(&f.m_cur, bm);
-    atomicMax(&f.v_prev, bv);
-    atomicMax(&f.v_cur, bv);
-    atomicMax(&f.a_prev, ba);
-    atomicMax(&f.a_cur, ba);
-    atomicMax(&f.v0max, b0);
+    uint32_t* to[7] = {&f.m_prev, &f.m_cur, &f.v_prev, &f.v_cur, &f.a_prev, &f.a_cur, &f.v0max};
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+      if ((int)threadIdx.x == k && best[k / 2] > *(volatile uint32_t*)to[k]) atomicMax(to[k], best[k / 2]);
   }
 }
 
@@ -359,32 +366,54 @@ __global__ void __launch_bounds__(kGridGroups * kBlockNodes) k_grid(const SceneD
 
 // pVolumeCompute.glsl:32-83: rho0 = sum_i m_i w_ip / h^3 from the grid mass,
 // stored as V0 = m / rho0 (0 when rho0 <= 0, which disables the force as
-// p2gTransfer.glsl:126 does).
-__global__ void __launch_bounds__(256) k_volume(const SceneDev* __restrict__ sd) {
+// p2gTransfer.glsl:126 does). Per work item: the masses of its tile's nodes go to
+// shared memory once instead of being read (as int64 words) 64 times a particle:
+// 167 us at 1M particles, now 51. A particle whose stencil leaves the
+// tile (outside the grid, binned to its border) reads them from the grid.
+__device__ __forceinline__ float node_mass(const SceneDev& S, int g0, int g1, int g2, float scale_inv) {
+  if (!node_in_grid(S, g0, g1, g2)) return 0.0f;
+  const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
+  const long long mq = (long long)S.acc[(size_t)blk * kAccBlockWords + (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3)];
+  return (float)mq * scale_inv;  // the scale is a power of two
+}
+__global__ void __launch_bounds__(256) k_volume(const SceneDev* __restrict__ sd, const int* __restrict__ item_prefix) {
+  __shared__ float mass[kTile3];
   const SceneDev& S = *sd;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < S.n; p += gridDim.x * blockDim.x) {
-    const float4 xm = S.xm[p];
-    float pg[3];
-    int base[3];
-    grid_coords(S, xm, pg, base);
-    AxisW w;
-    all_weights(pg, base, w);
-    float rho = 0.0f;
-    for (int c = 0; c < 4; c++)
-      for (int b = 0; b < 4; b++)
-        for (int a = 0; a < 4; a++) {
-          const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
-          if (!node_in_grid(S, g0, g1, g2)) continue;
-          const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
-          const long long mq = (long long)S.acc[(size_t)blk * kAccBlockWords + (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3)];
-          const float mi = (float)mq / S.fix->scale[0];
-          rho += mi * (sel4(a, w.wx[0], w.wx[1], w.wx[2], w.wx[3]) * sel4(b, w.wy[0], w.wy[1], w.wy[2], w.wy[3]) *
-                       sel4(c, w.wz[0], w.wz[1], w.wz[2], w.wz[3]));
-        }
-    rho = rho / (S.h * S.h * S.h);
-    float4 vv = S.vv[p];
-    vv.w = rho > 0.0f ? xm.w / rho : 0.0f;
-    S.vv[p] = vv;
+  const float si = 1.0f / S.fix->scale[0];
+  const int total = item_prefix[1];
+  for (int u = blockIdx.x; u < total; u += gridDim.x) {
+    const int4 it = S.items[u];
+    int bx, by, bz;
+    home_coords(S, it.x, bx, by, bz);
+    for (int t = threadIdx.x; t < kTile3; t += blockDim.x)
+      mass[t] = node_mass(S, 4 * bx - 2 + t % kTile, 4 * by - 2 + (t / kTile) % kTile, 4 * bz - 2 + t / (kTile * kTile), si);
+    __syncthreads();
+    for (int i = threadIdx.x; i < it.z; i += blockDim.x) {
+      const int p = it.y + i;
+      const float4 xm = S.xm[p];
+      float pg[3];
+      int base[3], t[3];
+      grid_coords(S, xm, pg, base);
+      AxisW w;
+      all_weights(pg, base, w);
+      const bool inside = stencil_in_tile(bx, by, bz, base, t);
+      float rho = 0.0f;
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+#pragma unroll
+          for (int a = 0; a < 4; a++) {
+            const float mi = inside ? mass[t[0] + a + kTile * (t[1] + b) + kTile * kTile * (t[2] + c)]
+                                    : node_mass(S, base[0] - 1 + a, base[1] - 1 + b, base[2] - 1 + c, si);
+            rho += mi * (w.wx[a] * w.wy[b] * w.wz[c]);
+          }
+      rho = rho / (S.h * S.h * S.h);
+      float4 vv = S.vv[p];
+      vv.w = rho > 0.0f ? xm.w / rho : 0.0f;
+      S.vv[p] = vv;
+    }
+    __syncthreads();
   }
 }
 
@@ -681,68 +710,122 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const SceneDev* __restr
 }
 
 // Upload: the caller's arrays (x, v: N x 3; m: N; FE, FP: N x 9 row-major or
-// null for identity), copied to the device as they are, packed into the
+// null for identity), in device or page-locked host memory, packed into the
 // particle streams. J_p = det F_P in double without contraction, as the
-// host formerly computed it.
-__global__ void __launch_bounds__(256) k_pack(const float* __restrict__ x, const float* __restrict__ v,
-                                              const float* __restrict__ m, const float* __restrict__ FE,
-                                              const float* __restrict__ FP, size_t n, float4* xm, float4* vv,
-                                              float4* fa, float4* fb, float2* fc, uint32_t* pid, float4* vq) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    xm[i] = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], m[i]);
-    vv[i] = make_float4(v[3 * i], v[3 * i + 1], v[3 * i + 2], 0.0f);
-    float F[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-    if (FE)
+// host formerly computed it. Bound by the CPU-GPU link (210 GB/s for reads in
+// whole lines): a block's stretch of every array is read by consecutive threads
+// into shared memory and picked up there per particle; each thread reading its
+// own particle's 12 and 36 bytes reached 168 GB/s (624 us for 1M particles with
+// F_E and F_P, now 505).
+constexpr int kIoTile = 256;  // particles per block and turn
+// Words [0, n) of src, which starts at any 4-byte boundary, by all threads.
+__device__ __forceinline__ void io_read(float* dst, const float* __restrict__ src, int n) {
+  for (int k = threadIdx.x; k < n; k += kIoTile) dst[k] = __ldcs(src + k);
+}
+__global__ void __launch_bounds__(kIoTile) k_pack(const float* __restrict__ x, const float* __restrict__ v,
+                                                  const float* __restrict__ m, const float* __restrict__ FE,
+                                                  const float* __restrict__ FP, size_t n, float4* xm, float4* vv,
+                                                  float4* fa, float4* fb, float2* fc, uint32_t* pid, float4* vq) {
+  __shared__ float sx[3 * kIoTile], sv[3 * kIoTile], sm[kIoTile], se[9 * kIoTile], sp[9 * kIoTile];
+  for (size_t i0 = blockIdx.x * (size_t)kIoTile; i0 < n; i0 += (size_t)gridDim.x * kIoTile) {
+    const int cnt = (int)min((size_t)kIoTile, n - i0);
+    io_read(sx, x + 3 * i0, 3 * cnt);
+    io_read(sv, v + 3 * i0, 3 * cnt);
+    io_read(sm, m + i0, cnt);
+    if (FE) io_read(se, FE + 9 * i0, 9 * cnt);
+    if (FP) io_read(sp, FP + 9 * i0, 9 * cnt);
+    __syncthreads();
+    const int k = threadIdx.x;
+    if (k < cnt) {
+      const size_t i = i0 + k;
+      xm[i] = make_float4(sx[3 * k], sx[3 * k + 1], sx[3 * k + 2], sm[k]);
+      vv[i] = make_float4(sv[3 * k], sv[3 * k + 1], sv[3 * k + 2], 0.0f);
+      float F[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
+      if (FE)
 #pragma unroll
-      for (int k = 0; k < 9; k++) F[k] = FE[9 * i + k];
-    fa[i] = make_float4(F[0], F[3], F[6], F[1]);
-    fb[i] = make_float4(F[4], F[7], F[2], F[5]);
-    float jp = 1.0f;
-    if (FP) {
-      const float* f = FP + 9 * i;
-      const double a = f[0], b = f[1], c = f[2], d = f[3], e = f[4], g = f[5], h = f[6], ii = f[7], j = f[8];
-      const double t0 = __dsub_rn(__dmul_rn(e, j), __dmul_rn(g, ii));
-      const double t1 = __dsub_rn(__dmul_rn(d, j), __dmul_rn(g, h));
-      const double t2 = __dsub_rn(__dmul_rn(d, ii), __dmul_rn(e, h));
-      jp = (float)__dadd_rn(__dsub_rn(__dmul_rn(a, t0), __dmul_rn(b, t1)), __dmul_rn(c, t2));
+        for (int c = 0; c < 9; c++) F[c] = se[9 * k + c];
+      fa[i] = make_float4(F[0], F[3], F[6], F[1]);
+      fb[i] = make_float4(F[4], F[7], F[2], F[5]);
+      float jp = 1.0f;
+      if (FP) {
+        const float* f = sp + 9 * k;
+        const double a = f[0], b = f[1], c = f[2], d = f[3], e = f[4], g = f[5], h = f[6], ii = f[7], j = f[8];
+        const double t0 = __dsub_rn(__dmul_rn(e, j), __dmul_rn(g, ii));
+        const double t1 = __dsub_rn(__dmul_rn(d, j), __dmul_rn(g, h));
+        const double t2 = __dsub_rn(__dmul_rn(d, ii), __dmul_rn(e, h));
+        jp = (float)__dadd_rn(__dsub_rn(__dmul_rn(a, t0), __dmul_rn(b, t1)), __dmul_rn(c, t2));
+      }
+      fc[i] = make_float2(F[8], jp);
+      pid[i] = (uint32_t)i;
+      vq[i] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);  // no previous SVD: identity frame
     }
-    fc[i] = make_float2(F[8], jp);
-    pid[i] = (uint32_t)i;
-    vq[i] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);  // no previous SVD: identity frame
+    __syncthreads();
   }
 }
 
-// Download: the particle streams back to the caller's layout and order
-// (slot i holds upload index pid[i]); any output may be null.
-__global__ void __launch_bounds__(256) k_unpack(const SceneDev* __restrict__ sd, size_t n, float* x, float* v,
-                                                float* FE, float* Jp, float* volume) {
+// Download: the particle streams back to the caller's layout and order (slot i
+// holds upload index pid[i]); any output may be null, and each lies in device or
+// page-locked host memory. k_invert finds the slot of every upload index; a
+// block then gathers its stretch of upload indices into shared memory and
+// writes it out by consecutive threads, which fills whole lines of the CPU-GPU
+// link (190 GB/s, what a DMA reaches), so that pinned arrays are written in
+// place: 374 us for 1M particles instead of 107 for unpacking to a staging
+// buffer and 386 for five copies; a viewer's frame of 4k particles 79 to 60 us.
+__global__ void __launch_bounds__(256) k_invert(const SceneDev* __restrict__ sd, size_t n, uint32_t* __restrict__ slot) {
   const SceneDev& S = *sd;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const size_t j = S.pid[i];
-    if (j >= n) continue;  // cannot happen: pid is a permutation
-    const float4 xm = S.xm[i], vv = S.vv[i];
-    if (x) {
-      x[3 * j] = xm.x;
-      x[3 * j + 1] = xm.y;
-      x[3 * j + 2] = xm.z;
-    }
-    if (v) {
-      v[3 * j] = vv.x;
-      v[3 * j + 1] = vv.y;
-      v[3 * j + 2] = vv.z;
-    }
-    const float2 c = S.fc[i];
-    if (FE) {
-      // fa = (m00, m01, m02, m10), fb = (m11, m12, m20, m21), fc = (m22, Jp); m[c][r]
-      const float4 a = S.fa[i], b = S.fb[i];
-      const float mcr[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x};
+    if (j < n) slot[j] = (uint32_t)i;  // (always: pid is a permutation)
+  }
+}
+__device__ __forceinline__ void io_write(float* dst, const float* src, int n) {
+  if (!dst) return;
+  for (int k = threadIdx.x; k < n; k += kIoTile) __stcs(dst + k, src[k]);
+}
+__global__ void __launch_bounds__(kIoTile) k_unpack(const SceneDev* __restrict__ sd, size_t n,
+                                                    const uint32_t* __restrict__ slot, float* x, float* v, float* FE,
+                                                    float* Jp, float* volume) {
+  const SceneDev& S = *sd;
+  __shared__ float sx[3 * kIoTile], sv[3 * kIoTile], se[9 * kIoTile], sj[kIoTile], so[kIoTile];
+  for (size_t j0 = blockIdx.x * (size_t)kIoTile; j0 < n; j0 += (size_t)gridDim.x * kIoTile) {
+    const int cnt = (int)min((size_t)kIoTile, n - j0);
+    const int k = threadIdx.x;
+    if (k < cnt) {
+      const uint32_t i = slot[j0 + k];
+      if (x) {
+        const float4 xm = S.xm[i];
+        sx[3 * k] = xm.x;
+        sx[3 * k + 1] = xm.y;
+        sx[3 * k + 2] = xm.z;
+      }
+      if (v || volume) {
+        const float4 vv = S.vv[i];
+        sv[3 * k] = vv.x;
+        sv[3 * k + 1] = vv.y;
+        sv[3 * k + 2] = vv.z;
+        so[k] = vv.w;
+      }
+      if (FE || Jp) {
+        const float2 c = S.fc[i];
+        sj[k] = c.y;
+        if (FE) {
+          // fa = (m00, m01, m02, m10), fb = (m11, m12, m20, m21), fc = (m22, Jp); m[c][r]
+          const float4 a = S.fa[i], b = S.fb[i];
+          const float mcr[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x};
 #pragma unroll
-      for (int r = 0; r < 3; r++)
+          for (int r = 0; r < 3; r++)
 #pragma unroll
-        for (int q = 0; q < 3; q++) FE[9 * j + 3 * r + q] = mcr[3 * q + r];
+            for (int q = 0; q < 3; q++) se[9 * k + 3 * r + q] = mcr[3 * q + r];
+        }
+      }
     }
-    if (Jp) Jp[j] = c.y;
-    if (volume) volume[j] = vv.w;
+    __syncthreads();
+    io_write(x ? x + 3 * j0 : nullptr, sx, 3 * cnt);
+    io_write(v ? v + 3 * j0 : nullptr, sv, 3 * cnt);
+    io_write(FE ? FE + 9 * j0 : nullptr, se, 9 * cnt);
+    io_write(Jp ? Jp + j0 : nullptr, sj, cnt);
+    io_write(volume ? volume + j0 : nullptr, so, cnt);
+    __syncthreads();
   }
 }
 
@@ -859,11 +942,10 @@ void fast_grid(const SceneDev* scenes, const int* active_prefix, int nscenes, in
   k_grid<<<grid_ctas, kGridGroups * kBlockNodes, 0, st>>>(scenes, active_prefix, nscenes, clear_only ? 1 : 0);
 }
 
-void fast_volume(const SceneDev* sd_dev, int n, cudaStream_t st) {
+void fast_volume(const SceneDev* sd_dev, const int* item_prefix, int n, cudaStream_t st) {
   if (n <= 0) return;
-  int g = (n + 255) / 256;
-  if (g > num_sms() * 8) g = num_sms() * 8;
-  k_volume<<<g, 256, 0, st>>>(sd_dev);
+  const int g = std::min(n / 32 + 1, num_sms() * 8);
+  k_volume<<<g, 256, 0, st>>>(sd_dev, item_prefix);
 }
 
 void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, cudaStream_t st) {
@@ -890,17 +972,16 @@ void fast_stats(const SceneDev* sd_dev, int n, StatsSlot* slot, StatsAccum* host
 void fast_pack(const float* x, const float* v, const float* m, const float* FE, const float* FP, size_t n,
                const SceneDev& sd, cudaStream_t st) {
   if (n == 0) return;
-  size_t g = (n + 255) / 256;
-  if (g > (size_t)num_sms() * 8) g = (size_t)num_sms() * 8;
-  k_pack<<<(int)g, 256, 0, st>>>(x, v, m, FE, FP, n, sd.xm, sd.vv, sd.fa, sd.fb, sd.fc, sd.pid, sd.vq);
+  const size_t g = std::min((n + kIoTile - 1) / kIoTile, (size_t)num_sms() * 8);
+  k_pack<<<(int)g, kIoTile, 0, st>>>(x, v, m, FE, FP, n, sd.xm, sd.vv, sd.fa, sd.fb, sd.fc, sd.pid, sd.vq);
 }
 
-void fast_unpack(const SceneDev* sd_dev, size_t n, float* x, float* v, float* FE, float* Jp, float* volume,
-                 cudaStream_t st) {
+void fast_unpack(const SceneDev* sd_dev, size_t n, uint32_t* slot, float* x, float* v, float* FE, float* Jp,
+                 float* volume, cudaStream_t st) {
   if (n == 0) return;
-  size_t g = (n + 255) / 256;
-  if (g > (size_t)num_sms() * 8) g = (size_t)num_sms() * 8;
-  k_unpack<<<(int)g, 256, 0, st>>>(sd_dev, n, x, v, FE, Jp, volume);
+  const size_t g = std::min((n + kIoTile - 1) / kIoTile, (size_t)num_sms() * 8);
+  k_invert<<<(int)g, 256, 0, st>>>(sd_dev, n, slot);
+  k_unpack<<<(int)g, kIoTile, 0, st>>>(sd_dev, n, slot, x, v, FE, Jp, volume);
 }
 
 void fast_download_grid(const SceneDev* sd_dev, float* mass, float* mom, float* force, float* vstar,

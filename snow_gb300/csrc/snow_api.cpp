@@ -586,7 +586,7 @@ snow_status fast_init(snow_scene* s) {
     if ((r = push_sd(s))) return r;
   }
   fast_enqueue_compact(s, st);
-  if (!s->volume_given) fast_volume(s->sd_dev, (int)s->n, st);  // pVolumeCompute
+  if (!s->volume_given) fast_volume(s->sd_dev, s->work.items, (int)s->n, st);  // pVolumeCompute
   fast_enqueue_grid(s, true, st);                                // clear acc
   fast_enqueue_p2g(s, false, st);                                // P2G of step 1
   CK(cudaGetLastError());
@@ -1214,8 +1214,8 @@ snow_status snow_scene_download(snow_scene* s, float* x, float* v, float* FE, fl
   if (!s) return SNOW_EINVAL;
   snow_ctx* ctx = s->ctx;
   const size_t n = s->n;
-  CK(cudaStreamSynchronize(ctx->stream));
   if (s->mode == SNOW_MODE_REFERENCE) {
+    CK(cudaStreamSynchronize(ctx->stream));
     std::vector<float4> pxm(n), pfe(4 * n), pfp(4 * n);
     std::vector<int4> pv(n);
     RefArgs& a = ref_args(s);
@@ -1253,32 +1253,35 @@ snow_status snow_scene_download(snow_scene* s, float* x, float* v, float* FE, fl
   }
   if (FP) return fail(ctx, SNOW_EUNSUPPORTED, "F_P is not kept in SNOW_MODE_FAST (J_p is)");
   if (n == 0) return SNOW_OK;
-  // unpacked on the device into upload order in a staging buffer, then one
-  // copy per requested array into the caller's memory (a DMA when it is
-  // pinned; the unpack kernel writing pinned memory directly was 6x slower:
-  // its per-particle stores cross the CPU-GPU link in small pieces; the
-  // copies spread over several streams were no faster than in one)
+  // written in upload order by the unpack kernel: arrays in page-locked memory
+  // in place, the others to a staging buffer and from there by one copy each
   if (!x && !v && !FE && !Jp && !volume) return SNOW_OK;
   float* out[5] = {x, v, FE, Jp, volume};
   const size_t width[5] = {3, 3, 9, 1, 1};
   float* dev[5] = {};
   size_t words = 0;
-  for (int k = 0; k < 5; k++)
-    if (out[k]) words += width[k] * n;
+  for (int k = 0; k < 5; k++) {
+    if (!out[k]) continue;
+    dev[k] = static_cast<float*>(pinned_device_ptr(out[k]));
+    if (!dev[k]) words += width[k] * n;
+  }
   std::vector<std::pair<void*, size_t>> tmp;
   size_t tmp_bytes = 0;
   float* stage = nullptr;
   snow_status st = dalloc(ctx, tmp, tmp_bytes, words * sizeof(float), (void**)&stage);
   if (st) return st;
+  bool staged[5] = {};
   for (int k = 0; k < 5; k++) {
-    if (!out[k]) continue;
+    if (!out[k] || dev[k]) continue;
     dev[k] = stage;
+    staged[k] = true;
     stage += width[k] * n;
   }
-  fast_unpack(s->sd_dev, n, dev[0], dev[1], dev[2], dev[3], dev[4], ctx->stream);
+  // (the sort's second value buffer is free between binnings)
+  fast_unpack(s->sd_dev, n, s->bin.vals[1], dev[0], dev[1], dev[2], dev[3], dev[4], ctx->stream);
   cudaError_t e = cudaGetLastError();
   for (int k = 0; k < 5 && e == cudaSuccess; k++)
-    if (out[k])
+    if (staged[k])
       e = cudaMemcpyAsync(out[k], dev[k], width[k] * n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   dfree_all(ctx, tmp, tmp_bytes);

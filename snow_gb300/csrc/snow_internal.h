@@ -252,7 +252,7 @@ void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_p
               bool mass_only, cudaStream_t st);
 void fast_grid(const SceneDev* scenes, const int* active_prefix, int nscenes, int grid_ctas, bool clear_only,
                cudaStream_t st);
-void fast_volume(const SceneDev* sd_dev, int n, cudaStream_t st);
+void fast_volume(const SceneDev* sd_dev, const int* item_prefix, int n, cudaStream_t st);
 void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, cudaStream_t st);
 // binned: some scene of the launch was re-binned in this step (its particles
 // are in its binned copies)
@@ -368,8 +368,9 @@ void ref_stats(const RefArgs& a, StatsSlot* slot, StatsAccum* host, cudaStream_t
 void fast_download_grid(const SceneDev* sd_dev, float* mass, float* mom, float* force, float* vstar, cudaStream_t st);
 void fast_pack(const float* x, const float* v, const float* m, const float* FE, const float* FP, size_t n,
                const SceneDev& sd, cudaStream_t st);
-void fast_unpack(const SceneDev* sd_dev, size_t n, float* x, float* v, float* FE, float* Jp, float* volume,
-                 cudaStream_t st);
+// slot: n words of scratch
+void fast_unpack(const SceneDev* sd_dev, size_t n, uint32_t* slot, float* x, float* v, float* FE, float* Jp,
+                 float* volume, cudaStream_t st);
 
 constexpr int kMaxDevices = 64;
 // The calling thread's current device (0 .. kMaxDevices - 1).

@@ -6,8 +6,9 @@
 // and from atomics being integer (order-independent).
 //
 // Differences in structure, not in results:
-//   * one thread per particle walks the 64 neighbours (the reference launches
-//     one invocation per particle x neighbour, (N/1024+1, 64, 1));
+//   * a block of particles is scattered by one thread per particle x neighbour
+//     pair at a time, and gathered by eight lanes per particle (the reference
+//     launches one invocation per pair, (N/1024+1, 64, 1));
 //   * the polar decomposition of F_E is computed once per particle instead
 //     of once per neighbour (p2gTransfer.glsl:109-110 recomputes it 64x);
 //   * every grid kernel is bounds-checked (gReset.glsl and gForceCompute.glsl
@@ -91,74 +92,121 @@ __global__ void k_rigid(snow_collider* coll, int ncoll, float dt) {  // rigidAdv
 }
 
 // p2gTransfer.glsl:44-151; with MASS_ONLY, gMassCompute.glsl:33-84.
+// A block takes kPairs particles: their stresses by one thread each, then their
+// 64 x kPairs pairs by all threads, the 32 lanes of a warp on 32 neighbours of
+// one particle. The lanes then trade their seven values each through shared
+// memory, so that one atomic instruction adds all words of four neighbouring
+// nodes (two whole sectors of each array). A thread walking its particle's
+// neighbours alone made the lanes of a cell's particles add to the same words,
+// and left a scene of 32k particles one warp per scheduler: 129 us a call, 73
+// with a word of 32 nodes per instruction, 51 now.
+constexpr int kPairs = 64;
+struct PairParticle {
+  float pg[3], mp, vp[3], vol_scale;
+  float stress[9];
+  int base[3];
+  int kind;  // 0: not scattered, 1: mass and momentum, 2: and force
+};
 template <bool MASS_ONLY>
 __global__ void __launch_bounds__(kThreads) k_p2g(RefArgs a) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-    const float4 xm = a.pxm[p];
-    const float mp = xm.w;
-    if (!MASS_ONLY && fabsf(mp) > 100.0f) continue;
-    const int4 pvi = a.pv[p];
-    const float vp[3] = {(float)pvi.x * 1e-8f, (float)pvi.y * 1e-8f, (float)pvi.z * 1e-8f};
-    const float pp0 = (float)pvi.w * 1e-6f;
-    const float pg[3] = {(xm.x - a.gpos[0]) / a.h, (xm.y - a.gpos[1]) / a.h, (xm.z - a.gpos[2]) / a.h};
-    const int base[3] = {(int)pg[0], (int)pg[1], (int)pg[2]};
-    M3 stress;
-    float vol_scale = 0.0f;
-    if (!MASS_ONLY) {
-      const M3 FE = load_mat4(a.pfe + 4 * (size_t)p);
-      const M3 FP = load_mat4(a.pfp + 4 * (size_t)p);
-      M3 W, S, V;
-      svd3<true>(FE, W, S, V);
-      M3 R = m3_mul(W, m3_transpose(V));
+  __shared__ PairParticle part[kPairs];
+  __shared__ int add[MASS_ONLY ? 1 : kThreads / 32][32][9];  // per warp: a node's values (m at 3), padded
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long p0 = blockIdx.x * (long long)kPairs; p0 < a.n; p0 += (long long)gridDim.x * kPairs) {
+    const int cnt = (int)min((long long)kPairs, a.n - p0);
+    if ((int)threadIdx.x < cnt) {
+      const size_t p = (size_t)p0 + threadIdx.x;
+      PairParticle& q = part[threadIdx.x];
+      const float4 xm = a.pxm[p];
+      const float mp = xm.w;
+      q.mp = mp;
+      q.kind = MASS_ONLY || !(fabsf(mp) > 100.0f) ? 1 : 0;
+      const int4 pvi = a.pv[p];
+      q.vp[0] = (float)pvi.x * 1e-8f;
+      q.vp[1] = (float)pvi.y * 1e-8f;
+      q.vp[2] = (float)pvi.z * 1e-8f;
+      const float pp0 = (float)pvi.w * 1e-6f;
+      q.pg[0] = (xm.x - a.gpos[0]) / a.h;
+      q.pg[1] = (xm.y - a.gpos[1]) / a.h;
+      q.pg[2] = (xm.z - a.gpos[2]) / a.h;
 #pragma unroll
-      for (int c = 0; c < 3; c++)
+      for (int k = 0; k < 3; k++) q.base[k] = (int)q.pg[k];
+      if (!MASS_ONLY && q.kind && pp0 > 0.0f) {
+        q.kind = 2;
+        const M3 FE = load_mat4(a.pfe + 4 * p);
+        const M3 FP = load_mat4(a.pfp + 4 * p);
+        M3 W, S, V;
+        svd3<true>(FE, W, S, V);
+        M3 R = m3_mul(W, m3_transpose(V));
 #pragma unroll
-        for (int r = 0; r < 3; r++) R.m[c][r] = quantize(R.m[c][r], 1e9f);
-      const float jpp = m3_det(FP);
-      const float jep = m3_det(FE);
-      const float s1 = 2.0f * lame_mu(a.young, a.poisson, a.hardening, jpp);
-      M3 t;
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-      for (int c = 0; c < 3; c++)
+          for (int r = 0; r < 3; r++) R.m[c][r] = quantize(R.m[c][r], 1e9f);
+        const float jpp = m3_det(FP);
+        const float jep = m3_det(FE);
+        const float s1 = 2.0f * lame_mu(a.young, a.poisson, a.hardening, jpp);
+        M3 t;
 #pragma unroll
-        for (int r = 0; r < 3; r++) t.m[c][r] = s1 * (FE.m[c][r] - R.m[c][r]);
-      const M3 A = m3_mul(t, m3_transpose(FE));
-      const float s2 = lame_lambda(a.young, a.poisson, a.hardening, jpp) * (jep - 1.0f) * jep;
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-      for (int c = 0; c < 3; c++)
+          for (int r = 0; r < 3; r++) t.m[c][r] = s1 * (FE.m[c][r] - R.m[c][r]);
+        const M3 A = m3_mul(t, m3_transpose(FE));
+        const float s2 = lame_lambda(a.young, a.poisson, a.hardening, jpp) * (jep - 1.0f) * jep;
 #pragma unroll
-        for (int r = 0; r < 3; r++) stress.m[c][r] = A.m[c][r] + s2 * (c == r ? 1.0f : 0.0f);
-      vol_scale = -(mp / pp0);
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+          for (int r = 0; r < 3; r++) q.stress[3 * c + r] = A.m[c][r] + s2 * (c == r ? 1.0f : 0.0f);
+        q.vol_scale = -(mp / pp0);
+      }
     }
-    for (int y = 0; y < 64; y++) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < 64 * cnt; i += kThreads) {
+      const PairParticle& q = part[i >> 6];  // the same for the lanes of a warp
+      if (!q.kind) continue;
       int o[3];
-      neighbour(y, o);
-      const int g[3] = {base[0] + o[0], base[1] + o[1], base[2] + o[2]};
-      if (!(g[0] >= 0 && g[1] >= 0 && g[2] >= 0 && g[0] < a.dim[0] && g[1] < a.dim[1] && g[2] < a.dim[2]))
-        continue;
-      const float d[3] = {(float)g[0] - pg[0], (float)g[1] - pg[1], (float)g[2] - pg[2]};
+      neighbour(i & 63, o);
+      const int g[3] = {q.base[0] + o[0], q.base[1] + o[1], q.base[2] + o[2]};
+      const bool in = g[0] >= 0 && g[1] >= 0 && g[2] >= 0 && g[0] < a.dim[0] && g[1] < a.dim[1] && g[2] < a.dim[2];
+      const float d[3] = {(float)g[0] - q.pg[0], (float)g[1] - q.pg[1], (float)g[2] - q.pg[2]};
       const float w = bspline(d[0]) * bspline(d[1]) * bspline(d[2]);
-      const long long gI = (long long)g[0] + (long long)g[1] * a.dim[0] + (long long)g[2] * a.dim[1] * a.dim[0];
-      atomicAdd(&a.gv[gI].w, (int)(mp * w * 1e8f));
-      if (MASS_ONLY) continue;
-      atomicAdd(&a.gv[gI].x, (int)(vp[0] * mp * w * 1e8f));
-      atomicAdd(&a.gv[gI].y, (int)(vp[1] * mp * w * 1e8f));
-      atomicAdd(&a.gv[gI].z, (int)(vp[2] * mp * w * 1e8f));
-      if (pp0 > 0.0f) {
+      const int gI = in ? g[0] + (g[1] + g[2] * a.dim[1]) * a.dim[0] : -1;  // (a grid holds fewer than 2^31 nodes)
+      if (MASS_ONLY) {
+        if (in) atomicAdd(&a.gv[gI].w, (int)(q.mp * w * 1e8f));
+        continue;
+      }
+      int v[7];
+      v[3] = (int)(q.mp * w * 1e8f);
+#pragma unroll
+      for (int k = 0; k < 3; k++) v[k] = (int)(q.vp[k] * q.mp * w * 1e8f);
+      v[4] = v[5] = v[6] = 0;
+      if (q.kind == 2) {
         const float nd[3] = {-d[0], -d[1], -d[2]};
         const float wg[3] = {bspline_d(nd[0]) * bspline(nd[1]) * bspline(nd[2]),
                              bspline(nd[0]) * bspline_d(nd[1]) * bspline(nd[2]),
                              bspline(nd[0]) * bspline(nd[1]) * bspline_d(nd[2])};
         float f[3];
 #pragma unroll
-        for (int r = 0; r < 3; r++)
-          f[r] = vol_scale *
-                 (stress.m[0][r] * wg[0] + stress.m[1][r] * wg[1] + stress.m[2][r] * wg[2]);
-        atomicAdd(&a.gf[gI].x, (int)(f[0] * 1e6f));
-        atomicAdd(&a.gf[gI].y, (int)(f[1] * 1e6f));
-        atomicAdd(&a.gf[gI].z, (int)(f[2] * 1e6f));
+        for (int r = 0; r < 3; r++) {
+          f[r] = q.vol_scale *
+                 (q.stress[r] * wg[0] + q.stress[3 + r] * wg[1] + q.stress[6 + r] * wg[2]);
+          v[4 + r] = (int)(f[r] * 1e6f);
+        }
       }
+#pragma unroll
+      for (int k = 0; k < 7; k++) add[warp][lane][k] = v[k];
+      add[warp][lane][7] = gI;
+      __syncwarp();
+      const int word = lane & 7;
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int node = 4 * k + (lane >> 3), at = add[warp][node][7];
+        if (word == 7 || at < 0) continue;
+        const int x = add[warp][node][word];
+        if (x != 0) atomicAdd((word < 4 ? &a.gv[at].x : &a.gf[at].x) + (word & 3), x);
+      }
+      __syncwarp();
     }
+    __syncthreads();
   }
 }
 
@@ -213,16 +261,25 @@ __global__ void __launch_bounds__(kThreads) k_grid(RefArgs a, float dt) {
   }
 }
 
-// g2pTransfer.glsl:53-143: per-particle sums of truncated contributions.
+// g2pTransfer.glsl:53-143: per-particle sums of truncated contributions, eight
+// of the 64 neighbours per lane (integer sums: the split changes no bit). One
+// thread a particle waited for 64 loads in turn: 75 us for 32k particles,
+// now 31.
+constexpr int kGatherLanes = 8;
 __global__ void __launch_bounds__(kThreads) k_g2p(RefArgs a) {
   const float alpha = a.alpha;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
+  const int part = threadIdx.x % kGatherLanes;
+  const long long stride = (long long)gridDim.x * (kThreads / kGatherLanes);
+  for (long long p0 = blockIdx.x * (long long)(kThreads / kGatherLanes); p0 < a.n; p0 += stride) {
+    const long long mine = p0 + threadIdx.x / kGatherLanes;
+    const size_t p = (size_t)min(mine, (long long)a.n - 1);  // (all lanes of a warp take part in the sums)
     const float4 xm = a.pxm[p];
     const float pg[3] = {(xm.x - a.gpos[0]) / a.h, (xm.y - a.gpos[1]) / a.h, (xm.z - a.gpos[2]) / a.h};
     const int base[3] = {(int)pg[0], (int)pg[1], (int)pg[2]};
     unsigned av[3] = {0u, 0u, 0u};
     unsigned ad[3][3] = {{0u, 0u, 0u}, {0u, 0u, 0u}, {0u, 0u, 0u}};
-    for (int y = 0; y < 64; y++) {
+#pragma unroll 2
+    for (int y = part; y < 64; y += kGatherLanes) {
       int o[3];
       neighbour(y, o);
       const int g[3] = {base[0] + o[0], base[1] + o[1], base[2] + o[2]};
@@ -252,6 +309,16 @@ __global__ void __launch_bounds__(kThreads) k_g2p(RefArgs a) {
           for (int r = 0; r < 3; r++) ad[c][r] += (unsigned)(int)(vin[r] * gw[c] * 1e8f);
       }
     }
+#pragma unroll
+    for (int o = 1; o < kGatherLanes; o <<= 1) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) av[k] += __shfl_xor_sync(0xffffffffu, av[k], o);
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) ad[c][r] += __shfl_xor_sync(0xffffffffu, ad[c][r], o);
+    }
+    if (part != 0 || mine >= a.n) continue;
     a.pvn[p] = make_int4((int)av[0], (int)av[1], (int)av[2], a.pvn[p].w);
     a.pd0[p] = make_int4((int)ad[0][0], (int)ad[0][1], (int)ad[0][2], a.pd0[p].w);
     a.pd1[p] = make_int4((int)ad[1][0], (int)ad[1][1], (int)ad[1][2], a.pd1[p].w);
@@ -362,16 +429,16 @@ void ref_reset(const RefArgs& a, cudaStream_t st) {  // gReset.glsl:11-16
 void ref_p2g(const RefArgs& a, bool mass_only, cudaStream_t st) {
   if (a.n <= 0) return;
   if (mass_only)
-    k_p2g<true><<<grid_for(a.n), kThreads, 0, st>>>(a);
+    k_p2g<true><<<grid_for((long long)a.n * (kThreads / kPairs)), kThreads, 0, st>>>(a);
   else
-    k_p2g<false><<<grid_for(a.n), kThreads, 0, st>>>(a);
+    k_p2g<false><<<grid_for((long long)a.n * (kThreads / kPairs)), kThreads, 0, st>>>(a);
 }
 void ref_volume(const RefArgs& a, cudaStream_t st) {
   if (a.n > 0) k_volume<<<grid_for(a.n), kThreads, 0, st>>>(a);
 }
 void ref_grid(const RefArgs& a, float dt, cudaStream_t st) { k_grid<<<grid_for(a.G), kThreads, 0, st>>>(a, dt); }
 void ref_g2p(const RefArgs& a, cudaStream_t st) {
-  if (a.n > 0) k_g2p<<<grid_for(a.n), kThreads, 0, st>>>(a);
+  if (a.n > 0) k_g2p<<<grid_for((long long)a.n * kGatherLanes), kThreads, 0, st>>>(a);
 }
 void ref_stats(const RefArgs& a, StatsSlot* slot, StatsAccum* host, cudaStream_t st) {
   // at least one block (it publishes empty sums), at most one partial per slot entry

@@ -16,7 +16,8 @@
 //            that are not active.
 //
 // Kernels of one step (every scene of a batch in one launch each):
-//   compact      flags -> slots, active list             (thread per block)
+//   compact      flags -> slots, active list; the step's start (counters,
+//                scales, colliders)                (thread per four blocks)
 //   grid         per active block: v* = p/m + dt (f/m + g), colliders, d
 //   g2p2g        per work item (<= 256 particles binned to one home block):
 //                bulk-copy (TMA) the 81 rows of nodes around the home block
@@ -55,16 +56,18 @@ __device__ __forceinline__ void form_prefixes(const SceneDev* __restrict__ scene
   active[nscenes] = aa;
 }
 
-// One CTA per scene: the step's counters reset, colliders advanced.
-__global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, int rigid) {
-  const int s = blockIdx.x;
-  if (s >= nscenes) return;
-  const SceneDev& S = scenes[s];
-  if (threadIdx.x == 0) {
-    S.counters[CNT_ACTIVE] = 0;
+// The start of a step for scene S, by one warp: counters reset, the magnitudes
+// moved on and the scales of this step's P2G formed from them, colliders
+// advanced, the solve's scalars cleared.
+__device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool binned) {
+  const int lane = threadIdx.x & 31;
+  if (rigid)  // rigidAdvance.glsl:14-18
+    for (int i = lane; i < S.ncoll; i += 32)
+      for (int k = 0; k < 3; k++) S.coll[i].pos[k] = S.coll[i].pos[k] + S.dt * S.coll[i].vel[k];
+  if (lane == 0) {
     S.counters[CNT_OVERFLOW] = 0;
-    S.counters[CNT_BINNED] = 0;
     S.counters[CNT_WORK] = 0;
+    if (!binned) S.counters[CNT_BINNED] = 0;
     // the magnitudes of the particles the pending P2G scattered become the
     // ones this step's P2G chooses its fixed-point scales from
     FixState& f = *S.fix;
@@ -72,19 +75,28 @@ __global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, i
     f.v_prev = f.v_cur;
     f.a_prev = f.a_cur;
     f.m_cur = f.v_cur = f.a_cur = 0u;
+    const FixScale sc = step_scales(S);
+    f.next[0] = sc.m;
+    f.next[1] = sc.p;
+    f.next[2] = sc.f;
   }
-  if (rigid)  // rigidAdvance.glsl:14-18
-    for (int i = threadIdx.x; i < S.ncoll; i += blockDim.x)
-      for (int k = 0; k < 3; k++) S.coll[i].pos[k] = S.coll[i].pos[k] + S.dt * S.coll[i].vel[k];
   if (S.crs) {  // the semi-implicit solve's scalars start from zero each step
     int* c = reinterpret_cast<int*>(S.crs);
-    for (int i = threadIdx.x; i < (int)(offsetof(CrScalars, skipping) / sizeof(int)); i += blockDim.x) c[i] = 0;
-    if (threadIdx.x == 0) {  // a step within kCrSkipSteps of a start below kCrSkipFactor * tol skips the solve
+    for (int i = lane; i < (int)(offsetof(CrScalars, skipping) / sizeof(int)); i += 32) c[i] = 0;
+    if (lane == 0) {  // a step within kCrSkipSteps of a start below kCrSkipFactor * tol skips the solve
       CrScalars& cs = *S.crs;
       cs.skipping = cs.skip_left > 0 ? 1 : 0;
       if (cs.skip_left > 0) cs.skip_left--;
     }
   }
+}
+
+// The same alone (per-kernel dispatches of the rigid advance).
+__global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, int rigid) {
+  const int s = blockIdx.x;
+  if (s >= nscenes) return;
+  begin_scene(scenes[s], rigid != 0, false);
+  if (threadIdx.x == 0) scenes[s].counters[CNT_ACTIVE] = 0;
 }
 
 __global__ void k_gather_counters(const SceneDev* __restrict__ scenes, int nscenes, int* out) {
@@ -107,30 +119,52 @@ __device__ __noinline__ void clear_block(const SceneDev& S, int b) {
   }
 }
 
-// Flags -> active-block list and slots (one thread per block); a block that
+// Flags -> active-block list and slots, four blocks per thread; a block that
 // was active before and is not now has its outputs cleared (few blocks a
-// step). The CTA that finishes last forms the item and active-block prefixes.
-__global__ void k_compact(const SceneDev* __restrict__ scenes, const int* __restrict__ block_prefix, int nscenes,
-                          long long total, int* items_prefix, int* active_prefix) {
+// step). The first warps also start the step of the scenes (a launch of its own
+// for that took 3 us of a step; at this kernel's end it took as long), and the
+// CTA that finishes last forms the item and active-block prefixes. Bound by
+// launch latency in small grids and by the 8 bytes a block it reads in large
+// ones: 5.1 us on 64^3 nodes and 7.6 on 256^3, against 4.4 + 2.1 and 6.7 + 2.2
+// (and a launch's gap) for the two kernels.
+// BINNED: the step's binning has left the particles in the binned copies.
+__global__ void __launch_bounds__(256) k_compact(const SceneDev* __restrict__ scenes, const int* __restrict__ quad_prefix,
+                                                 int nscenes, long long total, int* items_prefix, int* active_prefix,
+                                                 int rigid, int binned) {
+  const int warps = blockDim.x >> 5;
+  for (int s = blockIdx.x * warps + (threadIdx.x >> 5); s < nscenes; s += gridDim.x * warps)
+    begin_scene(scenes[s], rigid != 0, binned != 0);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < total;
        u += (long long)gridDim.x * blockDim.x) {
-    const int s = find_scene(block_prefix, nscenes, u);
+    const int s = find_scene(quad_prefix, nscenes, u);
     const SceneDev& S = scenes[s];
-    const int b = (int)(u - block_prefix[s]);
-    const int old = S.blk_slot[b];
-    int slot = -1;
-    if (S.blk_flag[b]) {
-      S.blk_flag[b] = 0;
-      slot = atomicAdd(&S.counters[CNT_ACTIVE], 1);
-      if (slot >= S.pool_cap) {
-        atomicAdd(&S.counters[CNT_OVERFLOW], 1);
-        slot = -1;
-      } else {
-        S.active[slot] = b;
+    const int q = (int)(u - quad_prefix[s]);
+    // (the arrays are whole 256-byte units long)
+    const int4 f4 = reinterpret_cast<const int4*>(S.blk_flag)[q], o4 = reinterpret_cast<const int4*>(S.blk_slot)[q];
+    const int flag[4] = {f4.x, f4.y, f4.z, f4.w}, old[4] = {o4.x, o4.y, o4.z, o4.w};
+    int want = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) want += 4 * q + k < S.nblocks && flag[k] != 0;
+    if (want == 0 && (old[0] & old[1] & old[2] & old[3]) == -1) continue;  // nothing active before or now
+    int slot = want ? atomicAdd(&S.counters[CNT_SLOTS], want) : 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int b = 4 * q + k;
+      if (b >= S.nblocks) break;
+      int now = -1;
+      if (flag[k]) {
+        S.blk_flag[b] = 0;
+        now = slot++;
+        if (now >= S.pool_cap) {
+          atomicAdd(&S.counters[CNT_OVERFLOW], 1);
+          now = -1;
+        } else {
+          S.active[now] = b;
+        }
       }
+      if (now != old[k]) S.blk_slot[b] = now;
+      if (now < 0 && old[k] >= 0) clear_block(S, b);
     }
-    if (slot != old) S.blk_slot[b] = slot;
-    if (slot < 0 && old >= 0) clear_block(S, b);
   }
   __shared__ bool last;
   __syncthreads();
@@ -139,8 +173,15 @@ __global__ void k_compact(const SceneDev* __restrict__ scenes, const int* __rest
     last = atomicAdd(&scenes[0].counters[CNT_DONE], 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
+  if (!last) return;
+  __threadfence();
+  for (int s = threadIdx.x; s < nscenes; s += blockDim.x) {
+    int* c = scenes[s].counters;
+    c[CNT_ACTIVE] = *(volatile int*)&c[CNT_SLOTS];
+    c[CNT_SLOTS] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     form_prefixes(scenes, nscenes, items_prefix, active_prefix);
     scenes[0].counters[CNT_DONE] = 0;
   }
@@ -532,7 +573,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     const SceneDev& S = scenes[s];
     if (s != sh.coll_scene) {  // uniform across the CTA
       if (threadIdx.x == 0) {
-        sh.fscale = step_scales(S);
+        sh.fscale = FixScale{S.fix->next[0], S.fix->next[1], S.fix->next[2]};
         sh.seen[0] = sh.seen[1] = sh.seen[2] = 0u;
         sh.pushed[0] = sh.pushed[1] = sh.pushed[2] = 0u;
       }
@@ -914,11 +955,10 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
   k_gather_counters<<<(n + 255) / 256, 256, 0, st>>>(scenes, nscenes, out);
 }
 
-void fast_compact(const SceneDev* scenes, const int* block_prefix, int nscenes, long long total_blocks,
-                  int* items_prefix, int* active_prefix, cudaStream_t st) {
-  long long g = (total_blocks + 255) / 256;
-  g = g > (long long)num_sms() * 16 ? (long long)num_sms() * 16 : (g < 1 ? 1 : g);
-  k_compact<<<(int)g, 256, 0, st>>>(scenes, block_prefix, nscenes, total_blocks, items_prefix, active_prefix);
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, cudaStream_t st) {
+  const long long g = std::max(1ll, std::min((w.total_quads + 255) / 256, (long long)num_sms() * 8));
+  k_compact<<<(int)g, 256, 0, st>>>(w.scenes, w.quads, w.nscenes, w.total_quads, w.items, w.active, rigid ? 1 : 0,
+                                    binned ? 1 : 0);
 }
 
 void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_prefix, int nscenes, int grid_ctas,

@@ -409,7 +409,7 @@ WorkSpace make_work(const SceneDev* scenes, int n, int* d_prefix) {
   w.items = d_prefix;
   w.active = d_prefix + (n + 1);
   w.particles = d_prefix + 2 * (n + 1);
-  w.blocks = d_prefix + 3 * (n + 1);
+  w.quads = d_prefix + 3 * (n + 1);
   w.chunks = d_prefix + 4 * (n + 1);
   return w;
 }
@@ -418,10 +418,10 @@ void add_work(WorkSpace& w, std::vector<int>& pre, int i, const SceneDev& sd) {
   const int n = w.nscenes;
   pre.resize((size_t)kWorkPrefixes * (n + 1), 0);
   w.total_particles += sd.n;
-  w.total_blocks += sd.nblocks;
+  w.total_quads += (sd.nblocks + 3) / 4;
   w.total_chunks += sd.nchunks;
   pre[2 * (n + 1) + i + 1] = (int)w.total_particles;
-  pre[3 * (n + 1) + i + 1] = (int)w.total_blocks;
+  pre[3 * (n + 1) + i + 1] = (int)w.total_quads;
   pre[4 * (n + 1) + i + 1] = (int)w.total_chunks;
 }
 
@@ -443,11 +443,8 @@ int grid_ctas() { return num_sms() * 8; }
 // they are copied back for the per-kernel P2G that follows.
 void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) { fast_bin_scenes(s->work, !in_step, st); }
 
-// Active blocks of the pending P2G sums -> pool slots (and prefixes).
-void fast_enqueue_compact(snow_scene* s, cudaStream_t st, bool counters_reset = false) {
-  if (!counters_reset) fast_begin_step(s->sd_dev, 1, false, st);
-  fast_compact(s->sd_dev, s->work.blocks, 1, s->work.total_blocks, s->work.items, s->work.active, st);
-}
+// Active blocks of the pending P2G sums -> slots (and prefixes); the step's start.
+void fast_enqueue_compact(snow_scene* s, cudaStream_t st) { fast_compact(s->work, false, false, st); }
 void fast_enqueue_p2g(snow_scene* s, bool mass_only, cudaStream_t st) {
   fast_p2g(s->sd_dev, s->sd, s->d_prefix + 0, 1, item_ctas(s->tune), mass_only, st);
 }
@@ -463,9 +460,8 @@ void fast_enqueue_solve(snow_scene* s, cudaStream_t st) {
 // One step of a scene whose P2G sums of the current state are pending in
 // acc: rigid advance, [binning], grid update, G2P + advance + next P2G.
 void fast_enqueue_step(snow_scene* s, bool bin, cudaStream_t st) {
-  fast_begin_step(s->sd_dev, 1, s->ncoll > 0, st);
   if (bin) fast_bin(s, st, true);
-  fast_enqueue_compact(s, st, true);
+  fast_compact(s->work, s->ncoll > 0, bin, st);
   fast_enqueue_grid(s, false, st);
   fast_enqueue_solve(s, st);
   fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, st);
@@ -1164,10 +1160,9 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
     if (ctx->profiling) {
       cudaEvent_t* ev = ctx->ev;
       CK(cudaEventRecord(ev[0], st));
-      fast_begin_step(s->sd_dev, 1, s->ncoll > 0, st);
       if (bin) fast_bin(s, st, true);
       CK(cudaEventRecord(ev[1], st));
-      fast_enqueue_compact(s, st, true);
+      fast_compact(s->work, s->ncoll > 0, bin, st);
       fast_enqueue_grid(s, false, st);
       CK(cudaEventRecord(ev[2], st));
       fast_enqueue_solve(s, st);
@@ -1600,14 +1595,13 @@ void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   const int n = (int)b->scenes.size();
   int* items = b->work.items;
   int* active = b->work.active;
-  fast_begin_step(b->d_scenes, n, true, st);
   // every scene re-binned in the same step, every sort_interval steps, so
   // the other steps run the fused kernel's plain instantiation (re-binning a
   // staggered subset of the scenes each step made every step take the
   // binned one: 3% slower on 16 scenes of 2M-8M particles and on 64 of
   // 10k-500k, A/B on one GPU)
   if (bin_all) fast_bin_scenes(b->work, false, st);
-  fast_compact(b->d_scenes, b->work.blocks, n, b->work.total_blocks, items, active, st);
+  fast_compact(b->work, true, bin_all, st);
   fast_grid(b->d_scenes, active, n, grid_ctas(), false, st);
   int iters = 0;  // the solve runs while any semi-implicit scene still iterates
   for (snow_scene* s : b->scenes)

@@ -70,6 +70,7 @@ struct FixState {
   uint32_t a_cur;
   uint32_t v0max;     // largest initial particle volume
   uint32_t wide;      // particles scattered with int64 contributions (outgrew the fast range), cumulative
+  float next[3];      // s_m, s_p, s_f of the step's P2G, formed at the step's start
 };
 
 // Per-scene counters (int32), one row of kCounterStride per scene.
@@ -84,7 +85,8 @@ enum {
   CNT_DONE = 7,       // CTAs of the compaction finished (the last forms the prefixes)
   CNT_BINNED = 8,     // 1: this step's binning left the particles in the binned copies
   CNT_WORK = 9,       // hands out the fused kernel's work to its CTAs (scene 0's)
-  kCounters = 10,
+  CNT_SLOTS = 10,     // slots the compaction has given out (zero between compactions)
+  kCounters = 11,
   kFixOffset = 16,    // a scene's FixState follows its counters (one copy reads both)
   kCounterStride = 32
 };
@@ -217,7 +219,7 @@ constexpr int kItemMax = 256;
 constexpr int kItemCtas = 2;
 
 // Work spaces over nscenes scenes: prefix[s] .. prefix[s+1] are scene s's units
-// (P2G work items, active blocks, particles, grid blocks, chunks of grid
+// (P2G work items, active blocks, particles, quads and chunks of grid
 // blocks), in one device array of five prefixes of nscenes + 1 entries. Item
 // and active-block counts are only known on the device; the binning and the
 // compaction form those two prefixes there.
@@ -227,24 +229,24 @@ struct WorkSpace {
   int* items;
   int* active;
   const int* particles;
-  const int* blocks;
+  const int* quads;
   const int* chunks;
-  long long total_particles, total_blocks, total_chunks;
+  long long total_particles, total_quads, total_chunks;
 };
 constexpr int kWorkPrefixes = 5;
 constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
-// Start of a step: resets the per-step counters and, with `rigid`, moves the
-// colliders by dt * velocity (rigidAdvance.glsl:14-18).
+// Start of a step alone: resets the per-step counters and, with `rigid`, moves
+// the colliders by dt * velocity (rigidAdvance.glsl:14-18). A step's compaction
+// does the same at its end.
 void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st);
 // Copies every scene's counters and FixState into out[s * kCounterStride ...] (mapped
 // pinned memory: a batch reads them one re-binning interval later, without
 // draining the stream).
 void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStream_t st);
-// Flags -> active list and pool slots; its last CTA then forms the item and
-// active-block prefixes (as fast_prefix does).
-void fast_compact(const SceneDev* scenes, const int* block_prefix, int nscenes, long long total_blocks,
-                  int* items_prefix, int* active_prefix,
-                  cudaStream_t st);
+// Flags -> active list and slots; its last CTA then starts the step of every
+// scene (fast_begin_step) and forms the item and active-block prefixes. binned:
+// the step's binning ran before and left the particles in the binned copies.
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, cudaStream_t st);
 // P2G of the stored particle state (set-up, per-kernel dispatches), after a
 // pass over the particles that measures the magnitudes its fixed-point
 // scales are chosen from.

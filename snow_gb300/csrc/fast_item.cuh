@@ -270,8 +270,8 @@ __device__ __forceinline__ void collide_packed(const snow_collider* coll, const 
 // already carry a growth margin (1.25 max|v| + margins, twice the largest
 // stress term) into [2^21, 2^22), the fast range's limit. A particle whose
 // contributions reach the limit (it outgrew the magnitudes the scales were
-// chosen from) is scattered with int64 contributions rounded in double
-// precision ("wide"), which depends only on the particle itself, so it is
+// chosen from) is scattered with exactly rounded int64 contributions ("wide"),
+// which depends only on the particle itself, so it is
 // as deterministic.
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
@@ -450,86 +450,102 @@ __device__ __forceinline__ int fix_force(float wxa, float gxa, const RowFactors&
   return __float_as_int(__fmaf_rn(gxa, f.kk[r], __fmaf_rn(wxa, f.hh[r], kMagic)));
 }
 
-// Scatter of one particle's 64 stencil nodes straight into acc (global
-// atomics; loops not unrolled, the code's size counts), for a particle outside its work item's tile. FAST: the particle
-// fits the fast path's range and its contributions are rounded exactly as
-// the tile path rounds them; otherwise (wide) each contribution is rounded in
-// double precision to int64. ms, mvs, As: the scaled quantities.
-template <int KIND, bool FAST>
-__device__ __forceinline__ void scatter_fix(const SceneDev& S, float ms, const float mvs[3], const float As[3][3],
-                                            const AxisW& w, const int base[3]) {
-  constexpr bool mo = KIND == kP2gMass;
-#pragma unroll 1
-  for (int c = 0; c < 4; c++)
-#pragma unroll 1
-    for (int b = 0; b < 4; b++) {
-      const int g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
-      if (g1 < 0 || g2 < 0 || g1 >= S.dim[1] || g2 >= S.dim[2]) continue;
-      RowFactors f;
-      row_factors(ms, mvs, As, sel4(b, w.wy[0], w.wy[1], w.wy[2], w.wy[3]), sel4(b, w.gy[0], w.gy[1], w.gy[2], w.gy[3]),
-                  sel4(c, w.wz[0], w.wz[1], w.wz[2], w.wz[3]), sel4(c, w.gz[0], w.gz[1], w.gz[2], w.gz[3]), mo, f);
-#pragma unroll 1
-      for (int a = 0; a < 4; a++) {
-        const int g0 = base[0] - 1 + a;
-        if (g0 < 0 || g0 >= S.dim[0]) continue;
-        const float wxa = sel4(a, w.wx[0], w.wx[1], w.wx[2], w.wx[3]);
-        const float gxa = sel4(a, w.gx[0], w.gx[1], w.gx[2], w.gx[3]);
-        long long v[7] = {0, 0, 0, 0, 0, 0, 0};
-        if (FAST) {
-          v[0] = fix_mass(wxa, f) - kMagicBits;
-          if (!mo)
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-              v[1 + r] = fix_mom(wxa, f, r) - kMagicBits;
-              v[4 + r] = fix_force(wxa, gxa, f, r) - kMagicBits;
-            }
-        } else {
-          auto wide = [](double x) { return isfinite(x) && fabs(x) < 4.0e18 ? __double2ll_rn(x) : 0ll; };
-          v[0] = wide((double)wxa * (double)f.mw);
-          if (!mo)
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-              v[1 + r] = wide((double)wxa * (double)f.pv[r]);
-              const double h = (double)wide((double)wxa * (double)f.hh[r]);
-              v[4 + r] = wide(fma((double)gxa, (double)f.kk[r], h));
-            }
-        }
-        if (!(v[0] | v[1] | v[2] | v[3] | v[4] | v[5] | v[6])) continue;
-        const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
-        acc_add(S, blk, (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3), v, mo);
-        S.blk_flag[blk] = 1;
-      }
-    }
+// Scatter of the 64 stencil nodes of a warp's particles that do not go to the
+// tile straight into acc (global atomics), one particle at a time with two nodes
+// per lane, whose words lie in whole sectors. FAR_FAST: the particle lies outside
+// its work item's tile; its contributions are rounded exactly as the tile path
+// rounds them. FAR_WIDE: it outgrew the fast path's range; each contribution is
+// rounded exactly to int64. K u (kP2gForce): float sums into the
+// low 4 bytes of acc's force words (free between the grid update and the next
+// P2G; the solve's node passes read and clear them), in active blocks alone.
+// A thread per particle took the 448 atomics of each in turn, those of a cell's
+// particles to the same words, and rounded the wide ones in double precision: 8
+// steps of half a cell without a binning (300k particles) took 0.69 ms each, now
+// 0.36; a step whose 131k particles are all wide 1.44, now 0.85.
+//
+// round(a b + h) to an integer, ties to even, with one rounding, in integer
+// arithmetic (a 24 x 24 bit product and a shift): this GPU's double precision is
+// 64 times slower than its single. 0 for what is not finite or reaches 4e18.
+__device__ __forceinline__ long long round_product(float a, float b, long long h) {
+  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+  const int xa = (int)(ua >> 23 & 255u), xb = (int)(ub >> 23 & 255u);
+  if (xa == 255 || xb == 255) return 0;
+  const uint32_t ma = (ua & 0x7fffffu) | (xa ? 0x800000u : 0u), mb = (ub & 0x7fffffu) | (xb ? 0x800000u : 0u);
+  const unsigned long long p = (unsigned long long)ma * mb;
+  const int e = max(xa, 1) + max(xb, 1) - 300;  // |a b| = p 2^e
+  const bool neg = ((ua ^ ub) >> 31) != 0u;
+  constexpr long long kLimit = 4000000000000000000ll;
+  long long q;
+  if (e >= 0) {
+    if (p != 0 && (e > 62 || (p >> (62 - e)) != 0)) return 0;
+    const long long v = e > 62 ? 0ll : (long long)(p << e);
+    q = h + (neg ? -v : v);
+  } else if (e <= -50) {
+    q = h;  // below a quarter
+  } else {
+    const int s = -e;
+    const long long t = neg ? -(long long)p : (long long)p;
+    const long long fl = t >> s, rem = t - (fl << s), half = 1ll << (s - 1);
+    q = h + fl;
+    if (rem > half || (rem == half && (q & 1))) q++;
+  }
+  return q < kLimit && q > -kLimit ? q : 0;
 }
 
-// The semi-implicit solve's K u scatter for a particle outside its tile:
-// float sums into the low 4 bytes of acc's force words (free between the
-// grid update and the next P2G; the solve's node passes read and clear them).
-__device__ __forceinline__ void scatter_force(const SceneDev& S, const P2GParticle& q, const AxisW& w, const int base[3]) {
-  if (!q.force) return;
-#pragma unroll 1
-  for (int c = 0; c < 4; c++)
-#pragma unroll 1
-    for (int b = 0; b < 4; b++)
-#pragma unroll 1
-      for (int a = 0; a < 4; a++) {
-        const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
-        if (!node_in_grid(S, g0, g1, g2)) continue;
-        const float wxa = sel4(a, w.wx[0], w.wx[1], w.wx[2], w.wx[3]);
-        const float gxa = sel4(a, w.gx[0], w.gx[1], w.gx[2], w.gx[3]);
-        const float wyb = sel4(b, w.wy[0], w.wy[1], w.wy[2], w.wy[3]);
-        const float gyb = sel4(b, w.gy[0], w.gy[1], w.gy[2], w.gy[3]);
-        const float wzc = sel4(c, w.wz[0], w.wz[1], w.wz[2], w.wz[3]);
-        const float gzc = sel4(c, w.gz[0], w.gz[1], w.gz[2], w.gz[3]);
-        const float gw[3] = {gxa * wyb * wzc, wxa * gyb * wzc, wxa * wyb * gzc};
-        const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
-        if (__ldg(&S.blk_slot[blk]) < 0) continue;  // only active blocks' words are read and cleared by the solve
-        float* dst = reinterpret_cast<float*>(S.acc + (size_t)blk * kAccBlockWords + 4 * kBlockNodes +
-                                              (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3));
+enum { kFarNone = 0, kFarFast = 1, kFarWide = 2 };
+struct FarParticle {
+  float wx[4], gx[4], wy[4], gy[4], wz[4], gz[4];
+  float ms, mvs[3], As[9];
+  int base[3];
+};
+template <int KIND>
+__device__ __noinline__ void scatter_far(const SceneDev& S, const FarParticle& f, int kind) {
+  constexpr bool mo = KIND == kP2gMass;
+  const int lane = threadIdx.x & 31;
+  float As[3][3];
 #pragma unroll
-        for (int r = 0; r < 3; r++)
-          atomicAdd(dst + 2 * r * kBlockNodes, q.A[r][0] * gw[0] + q.A[r][1] * gw[1] + q.A[r][2] * gw[2]);
+  for (int k = 0; k < 9; k++) As[k / 3][k % 3] = f.As[k];
+  const int a = lane & 3, b = (lane >> 2) & 3;
+  const float wxa = f.wx[a], gxa = f.gx[a], wyb = f.wy[b], gyb = f.gy[b];
+  const int g0 = f.base[0] - 1 + a, g1 = f.base[1] - 1 + b;
+#pragma unroll 1
+  for (int c = lane >> 4; c < 4; c += 2) {
+    const int g2 = f.base[2] - 1 + c;
+    if (!node_in_grid(S, g0, g1, g2)) continue;
+    const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2), node = (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3);
+    const float wzc = f.wz[c], gzc = f.gz[c];
+    if constexpr (KIND == kP2gForce) {
+      if (__ldg(&S.blk_slot[blk]) < 0) continue;  // only active blocks' words are read and cleared by the solve
+      const float gw[3] = {gxa * wyb * wzc, wxa * gyb * wzc, wxa * wyb * gzc};
+      float* dst = reinterpret_cast<float*>(S.acc + (size_t)blk * kAccBlockWords + 4 * kBlockNodes + node);
+#pragma unroll
+      for (int r = 0; r < 3; r++) atomicAdd(dst + 2 * r * kBlockNodes, As[r][0] * gw[0] + As[r][1] * gw[1] + As[r][2] * gw[2]);
+    } else {
+      RowFactors rf;
+      row_factors(f.ms, f.mvs, As, wyb, gyb, wzc, gzc, mo, rf);
+      long long v[7] = {0, 0, 0, 0, 0, 0, 0};
+      if (kind == kFarFast) {
+        v[0] = fix_mass(wxa, rf) - kMagicBits;
+        if (!mo)
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            v[1 + r] = fix_mom(wxa, rf, r) - kMagicBits;
+            v[4 + r] = fix_force(wxa, gxa, rf, r) - kMagicBits;
+          }
+      } else {
+        v[0] = round_product(wxa, rf.mw, 0);
+        if (!mo)
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            v[1 + r] = round_product(wxa, rf.pv[r], 0);
+            v[4 + r] = round_product(gxa, rf.kk[r], round_product(wxa, rf.hh[r], 0));
+          }
       }
+      if (!(v[0] | v[1] | v[2] | v[3] | v[4] | v[5] | v[6])) continue;
+      acc_add(S, blk, node, v, mo);
+      S.blk_flag[blk] = 1;
+    }
+  }
 }
 
 // ---- shared memory of one work item --------------------------------------
@@ -1068,8 +1084,8 @@ __device__ __forceinline__ int cell_row_node(int ci, int b, int c) {
 // P2G of the item's particles into the shared tile (every thread of the CTA
 // calls it; thread i holds particle i of the item when `have`):
 //   1. each particle inside the tile whose contributions fit the fast path's
-//      range counts itself in its base cell (p2g_count); the others scatter
-//      straight to acc (scatter_fix; K u: scatter_force);
+//      range counts itself in its base cell (p2g_count); the others are
+//      scattered straight to acc (scatter_far);
 //   2. every warp scans the cell counts for itself: the first slot of each
 //      cell and the list of the occupied cells; each particle stores its
 //      (scaled) mass, momentum, A and axis weights at its slot, so the
@@ -1104,6 +1120,7 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
   st.rank = 0;
   st.ms = 0.0f;
   float tile_bound = 0.0f;  // the particle's contribution bound, if it goes to the tile
+  int far = kFarNone;       // ... or how it is scattered
 #pragma unroll
   for (int r = 0; r < 3; r++) {
     st.mvs[r] = 0.0f;
@@ -1131,14 +1148,41 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
       // the particle drifted out of its home block's tile since the last
       // binning, or outgrew the fast path's range
       if (!inside) atomicAdd(&S.counters[CNT_FALLBACK], 1);
-      if (!fix)
-        scatter_force(S, q, w, base);
-      else if (fast && finite_w)
-        scatter_fix<KIND, true>(S, st.ms, st.mvs, st.As, w, base);
-      else {
-        atomicAdd(&S.fix->wide, 1u);
-        scatter_fix<KIND, false>(S, st.ms, st.mvs, st.As, w, base);
+      far = fast && finite_w ? kFarFast : kFarWide;
+      if (KIND != kP2gForce && far == kFarWide) atomicAdd(&S.fix->wide, 1u);
+      if (KIND == kP2gForce && !q.force) far = kFarNone;
+    }
+  }
+  uint32_t todo = __ballot_sync(0xffffffffu, far != kFarNone);
+  if (todo) {
+    // through the warp's part of the particle buffer, which its lanes have read
+    static_assert(sizeof(FarParticle) <= 32 * sizeof(float4), "one particle in the warp's part of a stream");
+    FarParticle* f = reinterpret_cast<FarParticle*>(sh.pfa + (threadIdx.x & ~31u));
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      __syncwarp();
+      if ((int)(threadIdx.x & 31) == src) {
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          f->wx[a] = w.wx[a];
+          f->gx[a] = w.gx[a];
+          f->wy[a] = w.wy[a];
+          f->gy[a] = w.gy[a];
+          f->wz[a] = w.wz[a];
+          f->gz[a] = w.gz[a];
+        }
+        f->ms = st.ms;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          f->mvs[r] = st.mvs[r];
+          f->base[r] = base[r];
+#pragma unroll
+          for (int c = 0; c < 3; c++) f->As[3 * r + c] = st.As[r][c];
+        }
       }
+      __syncwarp();
+      scatter_far<KIND>(S, *f, __shfl_sync(0xffffffffu, far, src));
     }
   }
   if (RUN) {  // per warp: its tile particles times their largest bound (no lower than their sum)

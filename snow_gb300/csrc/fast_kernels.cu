@@ -43,17 +43,42 @@ namespace snow {
 namespace {
 
 // ===========================================================================
+// Item and active-block prefixes of the scenes, by one full warp; the slots
+// handed out become the scenes' active blocks.
 __device__ __forceinline__ void form_prefixes(const SceneDev* __restrict__ scenes, int nscenes, int* items,
                                               int* active) {
-  int ai = 0, aa = 0;
-  for (int s = 0; s < nscenes; s++) {
-    items[s] = ai;
-    active[s] = aa;
-    ai += *(volatile int*)&scenes[s].counters[CNT_ITEMS];
-    aa += min(*(volatile int*)&scenes[s].counters[CNT_ACTIVE], scenes[s].pool_cap);
+  const int lane = threadIdx.x & 31;
+  int items0 = 0, active0 = 0;
+  for (int s0 = 0; s0 < nscenes; s0 += 32) {
+    int ni = 0, na = 0;
+    if (s0 + lane < nscenes) {
+      const SceneDev& S = scenes[s0 + lane];
+      ni = *(volatile int*)&S.counters[CNT_ITEMS];
+      na = *(volatile int*)&S.counters[CNT_SLOTS];
+      S.counters[CNT_ACTIVE] = na;
+      S.counters[CNT_SLOTS] = 0;
+      na = min(na, S.pool_cap);
+    }
+    int ei = ni, ea = na;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int vi = __shfl_up_sync(0xffffffffu, ei, o), va = __shfl_up_sync(0xffffffffu, ea, o);
+      if (lane >= o) {
+        ei += vi;
+        ea += va;
+      }
+    }
+    if (s0 + lane < nscenes) {
+      items[s0 + lane] = items0 + ei - ni;
+      active[s0 + lane] = active0 + ea - na;
+    }
+    items0 += __shfl_sync(0xffffffffu, ei, 31);
+    active0 += __shfl_sync(0xffffffffu, ea, 31);
   }
-  items[nscenes] = ai;
-  active[nscenes] = aa;
+  if (lane == 0) {
+    items[nscenes] = items0;
+    active[nscenes] = active0;
+  }
 }
 
 // The start of a step for scene S, by one warp: counters reset, the magnitudes
@@ -121,32 +146,44 @@ __device__ __noinline__ void clear_block(const SceneDev& S, int b) {
 
 // Flags -> active-block list and slots, four blocks per thread; a block that
 // was active before and is not now has its outputs cleared (few blocks a
-// step). The first warps also start the step of the scenes (a launch of its own
-// for that took 3 us of a step; at this kernel's end it took as long), and the
-// CTA that finishes last forms the item and active-block prefixes. Bound by
-// launch latency in small grids and by the 8 bytes a block it reads in large
-// ones: 5.1 us on 64^3 nodes and 7.6 on 256^3, against 4.4 + 2.1 and 6.7 + 2.2
-// (and a launch's gap) for the two kernels.
+// step). The first CTAs start the step of the scenes instead (a launch of its own
+// for that took 3 us of a step), and the CTA that takes its slots last forms
+// the item and active-block prefixes. Bound by a chain of round trips to L2
+// (flags, slots, count of the CTAs, prefixes) in small grids and by the 8 bytes a
+// block it reads in large ones. The scenes' start in CTAs of its own, the CTAs
+// counted before they write their lists and the prefixes formed by a warp:
+// 5.1 to 3.9 us on 64^3 nodes, 7.5 to 5.7 on 256^3, 17.0 to 15.6 on 512^3.
 // BINNED: the step's binning has left the particles in the binned copies.
-__global__ void __launch_bounds__(256) k_compact(const SceneDev* __restrict__ scenes, const int* __restrict__ quad_prefix,
-                                                 int nscenes, long long total, int* items_prefix, int* active_prefix,
-                                                 int rigid, int binned) {
-  const int warps = blockDim.x >> 5;
-  for (int s = blockIdx.x * warps + (threadIdx.x >> 5); s < nscenes; s += gridDim.x * warps)
-    begin_scene(scenes[s], rigid != 0, binned != 0);
-  for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < total;
-       u += (long long)gridDim.x * blockDim.x) {
-    const int s = find_scene(quad_prefix, nscenes, u);
-    const SceneDev& S = scenes[s];
-    const int q = (int)(u - quad_prefix[s]);
-    // (the arrays are whole 256-byte units long)
-    const int4 f4 = reinterpret_cast<const int4*>(S.blk_flag)[q], o4 = reinterpret_cast<const int4*>(S.blk_slot)[q];
-    const int flag[4] = {f4.x, f4.y, f4.z, f4.w}, old[4] = {o4.x, o4.y, o4.z, o4.w};
-    int want = 0;
+constexpr int kCompactThreads = 256;
+__global__ void __launch_bounds__(kCompactThreads) k_compact(const SceneDev* __restrict__ scenes, const int* quad_prefix,
+                                                             int nscenes, long long total, int* items_prefix,
+                                                             int* active_prefix, int rigid, int binned) {
+  constexpr int kWarps = kCompactThreads / 32;
+  const int begin_ctas = (nscenes + kWarps - 1) / kWarps;
+  if ((int)blockIdx.x < begin_ctas) {
+    const int s = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
+    if (s < nscenes) begin_scene(scenes[s], rigid != 0, binned != 0);
+    return;
+  }
+  const long long u = ((long long)blockIdx.x - begin_ctas) * kCompactThreads + threadIdx.x;
+  const int s = find_scene(quad_prefix, nscenes, min(u, total - 1));
+  const SceneDev& S = scenes[s];
+  const int q = (int)(min(u, total - 1) - (nscenes == 1 ? 0 : quad_prefix[s]));
+  // (the arrays are whole 256-byte units long)
+  const int4 f4 = reinterpret_cast<const int4*>(S.blk_flag)[q], o4 = reinterpret_cast<const int4*>(S.blk_slot)[q];
+  const int flag[4] = {f4.x, f4.y, f4.z, f4.w}, old[4] = {o4.x, o4.y, o4.z, o4.w};
+  int want = 0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) want += 4 * q + k < S.nblocks && flag[k] != 0;
-    if (want == 0 && (old[0] & old[1] & old[2] & old[3]) == -1) continue;  // nothing active before or now
-    int slot = want ? atomicAdd(&S.counters[CNT_SLOTS], want) : 0;
+  for (int k = 0; k < 4; k++) want += u < total && 4 * q + k < S.nblocks && flag[k] != 0;
+  int slot = want ? atomicAdd(&S.counters[CNT_SLOTS], want) : 0;
+  // the CTA's slots are taken: counted before the lists are written
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&scenes[0].counters[CNT_DONE], 1) == (int)gridDim.x - begin_ctas - 1;
+  }
+  if (u < total && (want || (old[0] & old[1] & old[2] & old[3]) != -1)) {  // active now or before
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const int b = 4 * q + k;
@@ -166,25 +203,11 @@ __global__ void __launch_bounds__(256) k_compact(const SceneDev* __restrict__ sc
       if (now < 0 && old[k] >= 0) clear_block(S, b);
     }
   }
-  __shared__ bool last;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&scenes[0].counters[CNT_DONE], 1) == (int)gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
+  if (!last || threadIdx.x >= 32) return;
   __threadfence();
-  for (int s = threadIdx.x; s < nscenes; s += blockDim.x) {
-    int* c = scenes[s].counters;
-    c[CNT_ACTIVE] = *(volatile int*)&c[CNT_SLOTS];
-    c[CNT_SLOTS] = 0;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    form_prefixes(scenes, nscenes, items_prefix, active_prefix);
-    scenes[0].counters[CNT_DONE] = 0;
-  }
+  form_prefixes(scenes, nscenes, items_prefix, active_prefix);
+  if (threadIdx.x == 0) scenes[0].counters[CNT_DONE] = 0;
 }
 
 // Largest mass, |v|, force-term bound and initial volume of the particles a
@@ -956,9 +979,10 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
 }
 
 void fast_compact(const WorkSpace& w, bool rigid, bool binned, cudaStream_t st) {
-  const long long g = std::max(1ll, std::min((w.total_quads + 255) / 256, (long long)num_sms() * 8));
-  k_compact<<<(int)g, 256, 0, st>>>(w.scenes, w.quads, w.nscenes, w.total_quads, w.items, w.active, rigid ? 1 : 0,
-                                    binned ? 1 : 0);
+  const long long g = std::max(1ll, (w.total_quads + kCompactThreads - 1) / kCompactThreads);
+  const int begin_ctas = (w.nscenes + kCompactThreads / 32 - 1) / (kCompactThreads / 32);
+  k_compact<<<(int)g + begin_ctas, kCompactThreads, 0, st>>>(w.scenes, w.quads, w.nscenes, w.total_quads, w.items,
+                                                             w.active, rigid ? 1 : 0, binned ? 1 : 0);
 }
 
 void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_prefix, int nscenes, int grid_ctas,

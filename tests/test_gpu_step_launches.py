@@ -1,0 +1,30 @@
+"""How the FAST step is launched does not show in its results: scenes are the
+same bit for bit alone and in a batch of any size (the step's start and its
+prefixes are formed by warps over 8 and 32 scenes)."""
+import numpy as np
+import pytest
+
+from snow_gb300 import scenes
+
+gpu = pytest.mark.gpu
+KEYS = ("x", "v", "FE", "Jp")
+
+
+def _same(a, b):
+    return all(np.array_equal(a[k], b[k]) for k in KEYS)
+
+
+@gpu
+@pytest.mark.parametrize("count", [1, 8, 9, 32, 33, 70])
+def test_batches_of_any_number_of_scenes_match_each_alone(count):
+    from snow_gb300 import api
+    kinds = [scenes.small_scene(n=200 + 37 * i, grid_edge=(17, 24, 9)[i % 3], seed=300 + i, v0=(0.5, -1.0 - i, 0.0))
+             for i in range(5)]
+    ctx = api.Context(0)
+    alone = [api.SimScene(ctx, s).upload().init().step(s.dt, 11).download() for s in kinds]
+    scs = [kinds[i % 5] for i in range(count)]
+    sims = [api.SimScene(ctx, s).upload().init() for s in scs]
+    api.Batch(ctx, sims).step(11, dt=[s.dt for s in scs])
+    for i, g in enumerate(sims):
+        assert _same(g.check().download(), alone[i % 5]), i
+    ctx.close()

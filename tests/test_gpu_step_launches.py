@@ -28,3 +28,30 @@ def test_batches_of_any_number_of_scenes_match_each_alone(count):
     for i, g in enumerate(sims):
         assert _same(g.check().download(), alone[i % 5]), i
     ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("interval", [0, 1, 3, 6, 32])
+def test_steps_in_one_call_or_in_many_are_the_same(interval):
+    """One call of 75 steps (graphs of several steps from its first on), calls of
+    one step, mixed calls (a graph of several steps from some point on), and
+    plain launches."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=2500, grid_edge=32, seed=41, v0=(1.0, -3.0, 0.5))
+    ctx = api.Context(0)
+    runs = []
+    for calls, graphs in (([75], True), ([1] * 75, True), ([5, 7, 4, 4, 4, 4, 4, 4, 4, 20, 15], True), ([75], False),
+                          ([40, 35], False)):
+        assert sum(calls) == 75
+        ctx.set_graphs(graphs)
+        g = api.SimScene(ctx, s, sort_interval=interval).upload().init()
+        for n in calls:
+            g.step(s.dt, n)
+        runs.append(g.check().download())
+        g.step(0.5 * s.dt, 40)  # another time step: other graphs
+        runs[-1]["then"] = g.check().download()
+        g.close()
+    ctx.set_graphs(True)
+    for r in runs[1:]:
+        assert _same(r, runs[0]) and _same(r["then"], runs[0]["then"])
+    ctx.close()

@@ -38,7 +38,7 @@ constexpr int kPdStride = 2 * kPdPairs;  // words per record (304 bytes: 16-byte
 enum { kPdA22 = 0, kPdM = 1, kPdMv = 2, kPdA = 5, kPdWx = 14, kPdGx = 18, kPdY = 22, kPdZ = 30 };
 constexpr int kShColliders = 16;  // colliders cached in shared memory
 
-__device__ __forceinline__ int find_scene(const int* __restrict__ prefix, int nscenes, long long u) {
+__device__ __forceinline__ int find_scene(const int* prefix, int nscenes, long long u) {
   int lo = 0, hi = nscenes;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -843,9 +843,9 @@ __device__ __forceinline__ void g2p_gather(const ItemShared& sh, const SceneDev&
                const int g0 = base[0] - 1 + a, g1 = base[1] - 1 + b, g2 = base[2] - 1 + c;
                if (!node_in_grid(S, g0, g1, g2)) return false;
                const f32x2* o = reinterpret_cast<const f32x2*>(S.gout + node_index(S, g0, g1, g2) * kOutFields);
-               p[0] = __ldg(o);
-               p[1] = __ldg(o + 1);
-               p[2] = __ldg(o + 2);
+               p[0] = o[0];
+               p[1] = o[1];
+               p[2] = o[2];
                return true;
              },
              dv, L);

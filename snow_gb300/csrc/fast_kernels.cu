@@ -160,6 +160,8 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(const SceneDev* __r
                                                              int* active_prefix, int rigid, int binned) {
   constexpr int kWarps = kCompactThreads / 32;
   const int begin_ctas = (nscenes + kWarps - 1) / kWarps;
+  chain_next();
+  chain_wait();
   if ((int)blockIdx.x < begin_ctas) {
     const int s = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
     if (s < nscenes) begin_scene(scenes[s], rigid != 0, binned != 0);
@@ -355,12 +357,19 @@ __device__ __forceinline__ void grid_node(const SceneDev& S, int slot, int b, in
 // nothing is staged or written (scene set-up).
 constexpr int kGridGroups = 4;  // 64-thread groups per CTA
 __global__ void __launch_bounds__(kGridGroups * kBlockNodes) k_grid(const SceneDev* __restrict__ scenes,
-                                                                    const int* __restrict__ active_prefix,
-                                                                    int nscenes, int clear_only) {
+                                                                    const int* active_prefix, int nscenes,
+                                                                    int clear_only) {
   __shared__ __align__(128) unsigned long long buf[kGridGroups][kAccBlockWords];
   __shared__ uint64_t bar[kGridGroups];
   __shared__ int gabort[kGridGroups];
   const int g = threadIdx.x / kBlockNodes, node = threadIdx.x % kBlockNodes;
+  chain_next();
+  if (node == 0) {
+    mbar_init(&bar[g], 1);
+    gabort[g] = 0;
+  }
+  __syncthreads();
+  chain_wait();
   const long long total = active_prefix[nscenes];
   const long long stride = (long long)gridDim.x * kGridGroups;
   long long u = (long long)blockIdx.x * kGridGroups + g;
@@ -376,11 +385,6 @@ __global__ void __launch_bounds__(kGridGroups * kBlockNodes) k_grid(const SceneD
   }
   constexpr uint32_t kBytes = kAccBlockWords * sizeof(unsigned long long);
   static_assert(kBytes % 16 == 0, "bulk copies move multiples of 16 bytes");
-  if (node == 0) {
-    mbar_init(&bar[g], 1);
-    gabort[g] = 0;
-  }
-  __syncthreads();
   // the block of work unit uu: its scene, pool slot and block id
   auto locate = [&](long long uu, int& s, int& slot, int& b) {
     s = find_scene(active_prefix, nscenes, uu);
@@ -537,10 +541,12 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 constexpr int kSingleItems = 5;
 template <bool BINNED>
 __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
-                                                       const int* __restrict__ item_prefix, int nscenes) {
+                                                       const int* item_prefix, int nscenes) {
   extern __shared__ float4 smem_raw[];
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
+  chain_next();
   tile_init(sh);
+  chain_wait();
   const int total = item_prefix[nscenes];
   // Whole runs unless that leaves CTAs without work: a run of two or three
   // items costs one copy of the grid rows and one flush, but the CTA that takes
@@ -978,11 +984,11 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
   k_gather_counters<<<(n + 255) / 256, 256, 0, st>>>(scenes, nscenes, out);
 }
 
-void fast_compact(const WorkSpace& w, bool rigid, bool binned, cudaStream_t st) {
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st) {
   const long long g = std::max(1ll, (w.total_quads + kCompactThreads - 1) / kCompactThreads);
   const int begin_ctas = (w.nscenes + kCompactThreads / 32 - 1) / (kCompactThreads / 32);
-  k_compact<<<(int)g + begin_ctas, kCompactThreads, 0, st>>>(w.scenes, w.quads, w.nscenes, w.total_quads, w.items,
-                                                             w.active, rigid ? 1 : 0, binned ? 1 : 0);
+  launch_after(chained, k_compact, (int)g + begin_ctas, kCompactThreads, 0, st, w.scenes, w.quads, w.nscenes,
+               w.total_quads, w.items, w.active, rigid ? 1 : 0, binned ? 1 : 0);
 }
 
 void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_prefix, int nscenes, int grid_ctas,
@@ -1002,8 +1008,9 @@ void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_p
 }
 
 void fast_grid(const SceneDev* scenes, const int* active_prefix, int nscenes, int grid_ctas, bool clear_only,
-               cudaStream_t st) {
-  k_grid<<<grid_ctas, kGridGroups * kBlockNodes, 0, st>>>(scenes, active_prefix, nscenes, clear_only ? 1 : 0);
+               bool chained, cudaStream_t st) {
+  launch_after(chained, k_grid, grid_ctas, kGridGroups * kBlockNodes, 0, st, scenes, active_prefix, nscenes,
+               clear_only ? 1 : 0);
 }
 
 void fast_volume(const SceneDev* sd_dev, const int* item_prefix, int n, cudaStream_t st) {
@@ -1017,11 +1024,9 @@ void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscene
 }
 
 void fast_g2p2g(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, bool binned,
-                cudaStream_t st) {
-  if (binned)
-    k_g2p2g<true><<<grid_ctas, kItemMax, item_smem(), st>>>(scenes, item_prefix, nscenes);
-  else
-    k_g2p2g<false><<<grid_ctas, kItemMax, item_smem(), st>>>(scenes, item_prefix, nscenes);
+                bool chained, cudaStream_t st) {
+  launch_after(chained, binned ? k_g2p2g<true> : k_g2p2g<false>, grid_ctas, kItemMax, item_smem(), st, scenes,
+               item_prefix, nscenes);
 }
 
 void fast_stats(const SceneDev* sd_dev, int n, StatsSlot* slot, StatsAccum* host, cudaStream_t st) {

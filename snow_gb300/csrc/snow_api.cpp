@@ -444,15 +444,15 @@ int grid_ctas() { return num_sms() * 8; }
 // Binning of one scene. in_step: the step's fused kernel follows in the same
 // stream and reads the particles from the binned copies (no copy back); else
 // they are copied back for the per-kernel P2G that follows.
-void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) { fast_bin_scenes(s->work, !in_step, st); }
+void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) { fast_bin_scenes(s->work, !in_step, false, st); }
 
 // Active blocks of the pending P2G sums -> slots (and prefixes); the step's start.
-void fast_enqueue_compact(snow_scene* s, cudaStream_t st) { fast_compact(s->work, false, false, st); }
+void fast_enqueue_compact(snow_scene* s, cudaStream_t st) { fast_compact(s->work, false, false, false, st); }
 void fast_enqueue_p2g(snow_scene* s, bool mass_only, cudaStream_t st) {
   fast_p2g(s->sd_dev, s->sd, s->d_prefix + 0, 1, item_ctas(s->tune), mass_only, st);
 }
-void fast_enqueue_grid(snow_scene* s, bool clear_only, cudaStream_t st) {
-  fast_grid(s->sd_dev, s->d_prefix + 2, 1, grid_ctas(), clear_only, st);
+void fast_enqueue_grid(snow_scene* s, bool clear_only, bool chained, cudaStream_t st) {
+  fast_grid(s->sd_dev, s->d_prefix + 2, 1, grid_ctas(), clear_only, chained, st);
 }
 // The semi-implicit solve after the grid update (explicit scenes: nothing).
 void fast_enqueue_solve(snow_scene* s, cudaStream_t st) {
@@ -462,12 +462,15 @@ void fast_enqueue_solve(snow_scene* s, cudaStream_t st) {
 }
 // One step of a scene whose P2G sums of the current state are pending in
 // acc: rigid advance, [binning], grid update, G2P + advance + next P2G.
-void fast_enqueue_step(snow_scene* s, bool bin, cudaStream_t st) {
-  if (bin) fast_bin(s, st, true);
-  fast_compact(s->work, s->ncoll > 0, bin, st);
-  fast_enqueue_grid(s, false, st);
+// follows: st's last kernel is that of the step before.
+void fast_enqueue_step(snow_scene* s, bool bin, bool follows, cudaStream_t st) {
+  bin = bin && s->n > 0;
+  const bool chain = s->n <= kChainParticles;
+  if (bin) fast_bin_scenes(s->work, false, follows, st);
+  fast_compact(s->work, s->ncoll > 0, bin, chain && (bin || follows), st);
+  fast_enqueue_grid(s, false, chain, st);
   fast_enqueue_solve(s, st);
-  fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, st);
+  fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, chain && !s->sd.crs, st);
 }
 
 snow_status set_dt(snow_scene* s, float dt) {
@@ -586,7 +589,7 @@ snow_status fast_init(snow_scene* s) {
   }
   fast_enqueue_compact(s, st);
   if (!s->volume_given) fast_volume(s->sd_dev, s->work.items, (int)s->n, st);  // pVolumeCompute
-  fast_enqueue_grid(s, true, st);                                // clear acc
+  fast_enqueue_grid(s, true, false, st);                         // clear acc
   fast_enqueue_p2g(s, false, st);                                // P2G of step 1
   CK(cudaGetLastError());
   // the particles' largest speed, which the re-binning interval is chosen from
@@ -1081,14 +1084,14 @@ snow_status snow_dispatch(snow_scene* s, int kernel, double dt) {
     case SNOW_K_G_RESET:  // discard pending P2G sums
       if (s->p2g_ready) {
         fast_enqueue_compact(s, st);
-        fast_enqueue_grid(s, true, st);
+        fast_enqueue_grid(s, true, false, st);
         s->p2g_ready = false;
       }
       break;
     case SNOW_K_P2G:
       if (s->p2g_ready) {
         fast_enqueue_compact(s, st);
-        fast_enqueue_grid(s, true, st);
+        fast_enqueue_grid(s, true, false, st);
       }
       // (single kernels: the speeds are not looked at between the calls)
       if (s->steps_since_sort >= (s->tune.chosen ? s->bin_interval : std::min(s->bin_interval, kCheckSteps))) {
@@ -1100,7 +1103,7 @@ snow_status snow_dispatch(snow_scene* s, int kernel, double dt) {
       break;
     case SNOW_K_G_FORCE:
       fast_enqueue_compact(s, st);
-      fast_enqueue_grid(s, false, st);
+      fast_enqueue_grid(s, false, false, st);
       fast_enqueue_solve(s, st);
       s->p2g_ready = false;
       break;
@@ -1167,9 +1170,11 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
     s->clean_needed = 8;
     s->interval_dt = fdt;
   }
+  bool follows = false;  // the kernel launched last is that of the step before
   for (int i = 0; i < n_steps;) {
     int k = 1;  // steps this pass takes
     if (s->steps_since_check >= kCheckSteps || s->steps_since_sort >= s->bin_interval) {
+      follows = false;
       r = fast_check_async(s);
       if (r) return r;
     }
@@ -1179,12 +1184,12 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       CK(cudaEventRecord(ev[0], st));
       if (bin) fast_bin(s, st, true);
       CK(cudaEventRecord(ev[1], st));
-      fast_compact(s->work, s->ncoll > 0, bin, st);
-      fast_enqueue_grid(s, false, st);
+      fast_compact(s->work, s->ncoll > 0, bin, false, st);
+      fast_enqueue_grid(s, false, false, st);
       CK(cudaEventRecord(ev[2], st));
       fast_enqueue_solve(s, st);
       CK(cudaEventRecord(ev[3], st));
-      fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, st);
+      fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, false, st);
       CK(cudaEventRecord(ev[4], st));
       CK(cudaEventSynchronize(ev[4]));
       float t[4];
@@ -1196,7 +1201,8 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       s->times.total_ms += t[0] + t[1] + t[2] + t[3];
       s->times.steps++;
     } else if (!ctx->graphs) {
-      fast_enqueue_step(s, bin, st);
+      fast_enqueue_step(s, bin, follows, st);
+      follows = true;
     } else {
       if (s->g_dt != fdt) drop_graphs(s);
       if (!bin && !s->sd.crs && n_steps - i >= kGraphSteps && kCheckSteps - s->steps_since_check >= kGraphSteps &&
@@ -1207,7 +1213,7 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       if (!g) {
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < k; j++) fast_enqueue_step(s, bin, st);
+        for (int j = 0; j < k; j++) fast_enqueue_step(s, bin, j > 0, st);
         CK(cudaStreamEndCapture(st, &graph));
         CK(cudaGraphInstantiate(&g, graph, 0));
         cudaGraphDestroy(graph);
@@ -1622,16 +1628,18 @@ void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   // staggered subset of the scenes each step made every step take the
   // binned one: 3% slower on 16 scenes of 2M-8M particles and on 64 of
   // 10k-500k, A/B on one GPU)
-  if (bin_all) fast_bin_scenes(b->work, false, st);
-  fast_compact(b->work, true, bin_all, st);
-  fast_grid(b->d_scenes, active, n, grid_ctas(), false, st);
+  bin_all = bin_all && b->work.total_particles > 0;
+  if (bin_all) fast_bin_scenes(b->work, false, false, st);
+  const bool chain = b->work.total_particles <= kChainParticles;
+  fast_compact(b->work, true, bin_all, chain && bin_all, st);
+  fast_grid(b->d_scenes, active, n, grid_ctas(), false, chain, st);
   int iters = 0;  // the solve runs while any semi-implicit scene still iterates
   for (snow_scene* s : b->scenes)
     if (s->sd.crs) iters = std::max(iters, s->sd.imp_maxit);
   if (iters > 0)
     fast_implicit_solve(b->d_scenes, items, active, n, iters, item_ctas(b->scenes[0]->tune), grid_ctas(),
                         b->ctx->d_iter, b->ctx->body_stream, b->ctx->gate_stream, st);
-  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), bin_all, st);
+  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), bin_all, chain && iters == 0, st);
 }
 
 }  // namespace

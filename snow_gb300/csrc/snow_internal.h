@@ -246,20 +246,20 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
 // Flags -> active list and slots; its last CTA then starts the step of every
 // scene (fast_begin_step) and forms the item and active-block prefixes. binned:
 // the step's binning ran before and left the particles in the binned copies.
-void fast_compact(const WorkSpace& w, bool rigid, bool binned, cudaStream_t st);
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st);
 // P2G of the stored particle state (set-up, per-kernel dispatches), after a
 // pass over the particles that measures the magnitudes its fixed-point
 // scales are chosen from.
 void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_prefix, int nscenes, int grid_ctas,
               bool mass_only, cudaStream_t st);
 void fast_grid(const SceneDev* scenes, const int* active_prefix, int nscenes, int grid_ctas, bool clear_only,
-               cudaStream_t st);
+               bool chained, cudaStream_t st);
 void fast_volume(const SceneDev* sd_dev, const int* item_prefix, int n, cudaStream_t st);
 void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, cudaStream_t st);
 // binned: some scene of the launch was re-binned in this step (its particles
 // are in its binned copies)
 void fast_g2p2g(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, bool binned,
-                cudaStream_t st);
+                bool chained, cudaStream_t st);
 // The semi-implicit velocity solve between the grid update (which leaves
 // v*, m and u = v* in the solver planes) and G2P: iterations of conjugate
 // residuals (each a K u pass over the items and three passes over the active
@@ -276,6 +276,39 @@ void fast_implicit_solve(const SceneDev* scenes, const int* item_prefix, const i
                          cudaStream_t gate, cudaStream_t st);
 // Kernel attributes of the solve (outside any stream capture).
 void fast_implicit_setup();
+
+// Launches k after the kernel launched before it in st. chained: that kernel is
+// one that calls chain_next and chain_wait, and nothing lies between the two; k's
+// CTAs then start once all of that kernel's have started (as far as there is
+// room) and set themselves up while it runs. Every thread of such a kernel calls
+// chain_wait before it reads or writes global memory: it returns when the kernel
+// before has finished, which by then has waited for the one before it. What these
+// kernels read and another of them wrote is read by plain loads, through pointers
+// that are not __restrict__ (a load of read-only memory could move above the
+// wait); the scenes' descriptors are written by copies, which nothing is chained to.
+// It takes launches and the kernels' set-up out of a short step: one step of 4k
+// particles with its download 56 to 54 us, 100 steps of 32k 3.70 to 3.64 ms, 20
+// steps of 300k with a binning in most 3.20 to 3.16, 50 of 1M 15.58 to 15.46. A
+// long one loses (12 steps of 16M particles 63.1 to 63.4 ms): hence the limit.
+constexpr long long kChainParticles = 1 << 20;
+template <typename... P, typename... A>
+inline void launch_after(bool chained, void (*k)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = (size_t)smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
 
 // While `st` captures a graph: appends a conditional node (IF or WHILE) on
 // `cond` after the work captured so far, and captures `fill`'s launches on
@@ -337,7 +370,7 @@ void fast_sort_keys(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, i
 // stable sort by cell key, work items, the item prefix. copy_back false: the
 // particles stay in the binned copies (CNT_BINNED) for the step's fused kernel,
 // which must follow in the same step.
-void fast_bin_scenes(const WorkSpace& w, bool copy_back, cudaStream_t st);
+void fast_bin_scenes(const WorkSpace& w, bool copy_back, bool chained, cudaStream_t st);
 
 // Radix sort of arbitrary (key, value) pairs; the result lands in k[0]/v[0].
 void radix_sort_pairs(uint32_t* k[2], uint32_t* v[2], size_t n, int key_bits, uint32_t* hist, uint32_t* scan_tmp,

@@ -217,7 +217,7 @@ __global__ void k_keys(const SceneDev* __restrict__ sd, uint32_t* __restrict__ k
 // launches in small scenes and by the 184 bytes a particle that the streams'
 // move reads and writes in large ones. A binning of 32k / 262k / 1M particles
 // took 67 / 81 / 126 us in 20 launches, now 20 / 28 / 69 in 6.
-__device__ __forceinline__ int scene_of(const int* __restrict__ prefix, int nscenes, long long u) {
+__device__ __forceinline__ int scene_of(const int* prefix, int nscenes, long long u) {
   int lo = 0, hi = nscenes;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -233,6 +233,8 @@ __device__ __forceinline__ int scene_of(const int* __restrict__ prefix, int nsce
 // order): the lanes of a warp that share a block take their places with one
 // atomic.
 __global__ void __launch_bounds__(256) k_bin_count(const WorkSpace w) {
+  chain_next();
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long u0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; u0 < w.total_particles;
@@ -259,6 +261,8 @@ __global__ void __launch_bounds__(256) k_bin_count(const WorkSpace w) {
 
 // Particles per chunk of blocks.
 __global__ void __launch_bounds__(kBinChunk / 2) k_bin_reduce(const WorkSpace w) {
+  chain_next();
+  chain_wait();
   for (long long u = blockIdx.x; u < w.total_chunks; u += gridDim.x) {
     const int s = scene_of(w.chunks, w.nscenes, u);
     const SceneDev& S = w.scenes[s];
@@ -280,6 +284,8 @@ __global__ void __launch_bounds__(kBinChunk / 2) k_bin_reduce(const WorkSpace w)
 // into near-equal items of at most S.items_max.
 __global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
   __shared__ int first_item;
+  chain_next();
+  chain_wait();
   for (long long u = blockIdx.x; u < w.total_chunks; u += gridDim.x) {
     const int s = scene_of(w.chunks, w.nscenes, u);
     const SceneDev& S = w.scenes[s];
@@ -322,6 +328,8 @@ __global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
 // Particle indices and keys into block order. The CTA that finishes last forms
 // the item prefix.
 __global__ void __launch_bounds__(256) k_bin_place(const WorkSpace w) {
+  chain_next();
+  chain_wait();
   const long long stride = (long long)gridDim.x * blockDim.x, u0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (long long u = u0; u < w.total_particles; u += stride) {
     const int s = scene_of(w.particles, w.nscenes, u);
@@ -360,6 +368,8 @@ constexpr int kCellThreads = 128;
 constexpr int kCellHeld = 6;  // particles a thread holds in registers: blocks up to 768 are read once
 constexpr int kMaxRanked = 128;
 __global__ void __launch_bounds__(kCellThreads) k_bin_cells(const WorkSpace w, int in_step) {
+  chain_next();
+  chain_wait();
   __shared__ int count[64], start[64], cursor[64];
   __shared__ uint32_t sidx[kCellThreads * kCellHeld];
   const int total = w.items[w.nscenes];
@@ -437,6 +447,8 @@ __global__ void __launch_bounds__(kCellThreads) k_bin_cells(const WorkSpace w, i
 
 // The particle streams into the binned copies, in the order bidx.
 __global__ void __launch_bounds__(256) k_bin_move(const WorkSpace w) {
+  chain_next();
+  chain_wait();
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < w.total_particles;
        u += (long long)gridDim.x * blockDim.x) {
     const int s = scene_of(w.particles, w.nscenes, u);
@@ -458,6 +470,8 @@ __global__ void __launch_bounds__(256) k_bin_move(const WorkSpace w) {
 
 // The binned copies back into the streams.
 __global__ void __launch_bounds__(256) k_bin_back(const WorkSpace w) {
+  chain_next();
+  chain_wait();
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < w.total_particles;
        u += (long long)gridDim.x * blockDim.x) {
     const int s = scene_of(w.particles, w.nscenes, u);
@@ -513,17 +527,18 @@ void fast_sort_keys(const SceneDev& sd, const SceneDev* sd_dev, BinScratch& b, i
   radix_sort_pairs(b.keys, b.vals, (size_t)sd.n, key_bits, b.hist, b.scan_tmp, st, start);
 }
 
-void fast_bin_scenes(const WorkSpace& w, bool copy_back, cudaStream_t st) {
+void fast_bin_scenes(const WorkSpace& w, bool copy_back, bool chained, cudaStream_t st) {
   if (w.total_particles <= 0) return;
   const size_t n = (size_t)w.total_particles;
-  k_bin_count<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
-  k_bin_reduce<<<grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st>>>(w);
-  k_bin_scan<<<grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st>>>(w);
-  k_bin_place<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
+  const bool chain = w.total_particles <= kChainParticles;
+  launch_after(chain && chained, k_bin_count, grid_for(n, 256, 8), 256, 0, st, w);
+  launch_after(chain, k_bin_reduce, grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st, w);
+  launch_after(chain, k_bin_scan, grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st, w);
+  launch_after(chain, k_bin_place, grid_for(n, 256, 8), 256, 0, st, w);
   // an occupied block holds some hundred particles; at most one CTA for each 64
-  k_bin_cells<<<grid_for(n, 64, 16), kCellThreads, 0, st>>>(w, copy_back ? 0 : 1);
-  k_bin_move<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
-  if (copy_back) k_bin_back<<<grid_for(n, 256, 8), 256, 0, st>>>(w);
+  launch_after(chain, k_bin_cells, grid_for(n, 64, 16), kCellThreads, 0, st, w, copy_back ? 0 : 1);
+  launch_after(chain, k_bin_move, grid_for(n, 256, 8), 256, 0, st, w);
+  if (copy_back) launch_after(chain, k_bin_back, grid_for(n, 256, 8), 256, 0, st, w);
 }
 
 }  // namespace snow

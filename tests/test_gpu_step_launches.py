@@ -55,3 +55,24 @@ def test_steps_in_one_call_or_in_many_are_the_same(interval):
     for r in runs[1:]:
         assert _same(r, runs[0]) and _same(r["then"], runs[0]["then"])
     ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("interval", [0, 1])
+@pytest.mark.parametrize("n", [1, 2500, (1 << 20) - 1, 1 << 20, (1 << 20) + 1])
+def test_chained_launches_match_separate_ones(n, interval):
+    """A profiled step waits for each of its kernels' groups; the others' kernels
+    are chained up to 2^20 particles."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=n, grid_edge=128 if n > 10000 else 32, seed=43, v0=(1.0, -3.0, 0.5))
+    ctx = api.Context(0)
+    runs = []
+    for profiled, graphs in ((True, True), (False, True), (False, False)):
+        ctx.set_profiling(profiled)
+        ctx.set_graphs(graphs)
+        g = api.SimScene(ctx, s, sort_interval=interval).upload().init().step(s.dt, 41)
+        runs.append(g.check().download())
+        g.close()
+    for r in runs[1:]:
+        assert _same(r, runs[0])
+    ctx.close()

@@ -28,6 +28,8 @@
 
 #include "../../include/snow_mpm.h"
 
+void scene_will_batch(snow_scene* s);  // snow_api.cpp
+
 namespace {
 
 double now_s() {
@@ -143,6 +145,7 @@ void run(snow_server* srv) {
     for (Job* j : admit) {
       j->t_admit = now_s();
       snow_status s = snow_scene_create(ctx, &j->p, j->coll.data(), (int)j->coll.size(), j->n, &j->scene);
+      if (s == SNOW_OK) scene_will_batch(j->scene);
       if (s == SNOW_OK) s = snow_scene_upload(j->scene, j->x.data(), j->v.data(), j->m.data(), nullptr, nullptr, j->n);
       if (s == SNOW_OK) s = snow_scene_init(j->scene);
       if (s != SNOW_OK) {

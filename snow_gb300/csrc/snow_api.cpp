@@ -95,6 +95,8 @@ struct snow_scene {
   bool cnt_pending = false;
   long long fallbacks_seen = 0;
   int steps_at_snapshot = 0;  // steps between the last two snapshots
+  int batches = 0;      // batches it is in (counted by their creation)
+  bool fitted = false;  // its items were sized for a launch of its own
   int version = 0;
   bool volume_given = false;
   // FAST: acc holds the P2G sums of the current particle state (the next
@@ -127,6 +129,7 @@ struct snow_batch {
   std::map<int, cudaGraphExec_t> graphs;  // 0: the step that re-bins every scene, 1: the others
   std::vector<float> g_dt;
   int g_threads = 0;
+  bool counted = false;  // in its scenes' `batches`
   size_t bytes = 0;
   std::vector<std::pair<void*, size_t>> allocs;
   // every scene's counters, written by a kernel into mapped pinned memory at
@@ -353,7 +356,7 @@ snow_status fast_alloc_grid(snow_scene* s) {
       (st = salloc(s, nb, &d.bstart)) || (st = salloc(s, nb, &d.bend)) || (st = salloc(s, nb, &d.bcount)) ||
       (st = salloc(s, (size_t)d.nchunks, &d.bchunk)) ||
       (st = salloc(s, (size_t)kCounterStride, &d.counters)) ||
-      (st = salloc(s, (size_t)kWorkPrefixes * 2, &s->d_prefix)) ||
+      (st = salloc(s, (size_t)kWorkPrefixes * 2 + kSizeChoices, &s->d_prefix)) ||
       (st = salloc(s, (size_t)1, &s->sd_dev)))
     return st;
   static_assert(kCounters <= kFixOffset && kFixOffset * sizeof(int) + sizeof(FixState) <= kCounterStride * sizeof(int),
@@ -414,12 +417,13 @@ WorkSpace make_work(const SceneDev* scenes, int n, int* d_prefix) {
   w.particles = d_prefix + 2 * (n + 1);
   w.quads = d_prefix + 3 * (n + 1);
   w.chunks = d_prefix + 4 * (n + 1);
+  w.sizes = d_prefix + kWorkPrefixes * (n + 1);
   return w;
 }
 // Appends scene `sd` as the i-th of n to the host copy of the prefixes.
 void add_work(WorkSpace& w, std::vector<int>& pre, int i, const SceneDev& sd) {
   const int n = w.nscenes;
-  pre.resize((size_t)kWorkPrefixes * (n + 1), 0);
+  pre.resize((size_t)kWorkPrefixes * (n + 1) + kSizeChoices, 0);
   w.total_particles += sd.n;
   w.total_quads += (sd.nblocks + 3) / 4;
   w.total_chunks += sd.nchunks;
@@ -444,7 +448,12 @@ int grid_ctas() { return num_sms() * 8; }
 // Binning of one scene. in_step: the step's fused kernel follows in the same
 // stream and reads the particles from the binned copies (no copy back); else
 // they are copied back for the per-kernel P2G that follows.
-void fast_bin(snow_scene* s, cudaStream_t st, bool in_step) { fast_bin_scenes(s->work, !in_step, false, st); }
+void fast_bin(snow_scene* s, cudaStream_t st, bool in_step, bool follows = false) {
+  const int ctas = item_ctas(s->tune);
+  s->work.fit = !s->tune.items_chosen && s->batches == 0 && fits_items((long long)s->n, ctas) ? ctas : 0;
+  s->fitted = s->work.fit > 0;
+  fast_bin_scenes(s->work, !in_step, follows, st);
+}
 
 // Active blocks of the pending P2G sums -> slots (and prefixes); the step's start.
 void fast_enqueue_compact(snow_scene* s, cudaStream_t st) { fast_compact(s->work, false, false, false, st); }
@@ -466,7 +475,7 @@ void fast_enqueue_solve(snow_scene* s, cudaStream_t st) {
 void fast_enqueue_step(snow_scene* s, bool bin, bool follows, cudaStream_t st) {
   bin = bin && s->n > 0;
   const bool chain = s->n <= kChainParticles;
-  if (bin) fast_bin_scenes(s->work, false, follows, st);
+  if (bin) fast_bin(s, st, true, follows);
   fast_compact(s->work, s->ncoll > 0, bin, chain && (bin || follows), st);
   fast_enqueue_grid(s, false, chain, st);
   fast_enqueue_solve(s, st);
@@ -678,6 +687,12 @@ snow_status fast_upload_soa(snow_scene* s, const std::vector<float4>& xm, const 
 }
 
 }  // namespace
+
+// The scene is, or (told before its set-up) will be, stepped in batches: its
+// binnings do not fit its items to launches of its own.
+void scene_will_batch(snow_scene* s) {
+  if (s->batches++ == 0) drop_graphs(s);
+}
 
 // ===========================================================================
 extern "C" {
@@ -1538,7 +1553,7 @@ snow_status snow_batch_create(snow_ctx* ctx, snow_scene* const* scenes, int n, s
   b->scenes.assign(scenes, scenes + n);
   snow_status st;
   if ((st = dalloc(ctx, b->allocs, b->bytes, sizeof(SceneDev) * n, (void**)&b->d_scenes)) ||
-      (st = dalloc(ctx, b->allocs, b->bytes, sizeof(int) * kWorkPrefixes * (n + 1), (void**)&b->d_prefix))) {
+      (st = dalloc(ctx, b->allocs, b->bytes, sizeof(int) * (kWorkPrefixes * (n + 1) + kSizeChoices), (void**)&b->d_prefix))) {
     snow_batch_destroy(b);
     return st;
   }
@@ -1549,7 +1564,9 @@ snow_status snow_batch_create(snow_ctx* ctx, snow_scene* const* scenes, int n, s
     snow_batch_destroy(b);
     return st;
   }
+  for (snow_scene* s : b->scenes) scene_will_batch(s);
   ctx->batches.insert(b);
+  b->counted = true;
   *out = b;
   return SNOW_OK;
 }
@@ -1558,6 +1575,9 @@ void snow_batch_destroy(snow_batch* b) {
   if (!b) return;
   cudaStreamSynchronize(b->ctx->stream);
   for (auto& g : b->graphs) cudaGraphExecDestroy(g.second);
+  if (b->counted)
+    for (snow_scene* s : b->scenes)
+      if (--s->batches == 0) drop_graphs(s);  // its binnings fit the items to its own launches again
   dfree_all(b->ctx, b->allocs, b->bytes);
   if (b->h_cnt) cudaFreeHost(b->h_cnt);
   if (b->cnt_ev) cudaEventDestroy(b->cnt_ev);
@@ -1583,13 +1603,17 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
   std::vector<SceneDev> sds(n);
   b->work = make_work(b->d_scenes, n, b->d_prefix);
   std::vector<int> pre;
+  bool chosen = false;
   for (int i = 0; i < n; i++) {
     snow_scene* s = b->scenes[i];
+    chosen = chosen || s->tune.items_chosen;
     s->sd.dt = want[i];
     s->last_dt = want[i];
     sds[i] = s->sd;
     add_work(b->work, pre, i, s->sd);
   }
+  const int ctas = item_ctas(b->scenes[0]->tune);
+  b->work.fit = !chosen && fits_items(b->work.total_particles, ctas) ? ctas : 0;
   CK(cudaMemcpyAsync(b->d_scenes, sds.data(), sizeof(SceneDev) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(b->d_prefix, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, ctx->stream));
   for (int i = 0; i < n; i++) {
@@ -1653,6 +1677,10 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
   cudaStream_t st = ctx->stream;
   for (size_t i = 0; i < b->scenes.size(); i++) {
     snow_scene* s = b->scenes[i];
+    if (s->fitted) {  // binned before it was in a batch: the next step re-bins
+      s->fitted = false;
+      s->steps_since_sort = 1 << 30;
+    }
     if (s->p2g_ready) continue;  // left behind by per-kernel dispatches: scatter its state first
     snow_status r0 = set_dt(s, dt ? (float)dt[i] : s->last_dt);
     if (r0) return r0;
@@ -1731,10 +1759,12 @@ snow_status snow_scene_set_tuning(snow_scene* s, const snow_tuning* t) {
   CK(cudaStreamSynchronize(ctx->stream));
   // the captured step graphs bake in the launch shapes: a changed work split
   // needs new ones
-  const bool split_changed = s->tune.items_max != t->items_max || s->tune.ctas_per_sm != t->ctas_per_sm;
+  const bool split_changed =
+      !s->tune.items_chosen || s->tune.items_max != t->items_max || s->tune.ctas_per_sm != t->ctas_per_sm;
   s->tune.sort_interval = t->sort_interval;
   s->tune.chosen = true;
   s->tune.items_max = t->items_max;
+  s->tune.items_chosen = true;
   s->tune.ctas_per_sm = t->ctas_per_sm;
   s->bin_interval = t->sort_interval;
   s->clean_checks = 0;
@@ -1758,6 +1788,7 @@ snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t) {
     s->tune.chosen = true;
     s->steps_since_sort = 1 << 30;  // the next step re-bins with the new work split
     s->tune.items_max = t->items_max;
+    s->tune.items_chosen = true;
     s->tune.ctas_per_sm = t->ctas_per_sm;
     s->bin_interval = t->sort_interval;
     s->sd.items_max = t->items_max;

@@ -206,7 +206,8 @@ constexpr int kCheckSteps = 8;
 struct FastTuning {
   int sort_interval = kAutoInterval;  // re-bin particles at least every k steps ...
   bool chosen = false;                // ... asked for by the caller (else chosen from the speeds, up to kAutoInterval)
-  int items_max = 256;    // most particles per work item (kMinItemMax .. kItemMax)
+  int items_max = 256;    // most particles per work item (kMinItemMax .. kItemMax) ...
+  bool items_chosen = false;  // ... asked for by the caller (else fewer where all items then run at once, size_choice)
   int ctas_per_sm = 2;    // work-item CTAs launched per SM (1 .. kItemCtas)
 };
 constexpr int kMinItemMax = 64;
@@ -232,8 +233,25 @@ struct WorkSpace {
   const int* quads;
   const int* chunks;
   long long total_particles, total_quads, total_chunks;
+  int fit;     // CTAs that the items are fitted to (0: the scenes' items_max as it is)
+  int* sizes;  // items there would be at each size_choice (zero between binnings)
 };
 constexpr int kWorkPrefixes = 5;
+// Item sizes that a binning of few particles chooses from: the smallest at which
+// the items take no more rounds of the fused kernel's CTAs than at the largest, if
+// those are at most kFitRounds. A round lasts as long as its largest items, whose
+// time falls with their size down to about 96 (below, their fixed part outweighs
+// it), and a size that needs a round more loses 5 to 25%. A step with items of up
+// to 256 and as chosen: 4k particles 26.8 to 23.3 us, 32k 33.2 to 29.9, 65k 49.9
+// to 42.3, 80k 50.7 to 46.5, 131k 63.7 to 60.4, the same from 160k on.
+constexpr int kSizeChoices = 8;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int size_choice(int k) { return k <= 4 ? 96 + 16 * k : 160 + 32 * (k - 4); }
+constexpr int kFitRounds = 3;
+// Whether a binning of n particles over `ctas` CTAs looks for one.
+inline bool fits_items(long long n, int ctas) { return n <= (long long)kFitRounds * ctas * size_choice(kSizeChoices - 1); }
 constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
 // Start of a step alone: resets the per-step counters and, with `rigid`, moves
 // the colliders by dt * velocity (rigidAdvance.glsl:14-18). A step's compaction

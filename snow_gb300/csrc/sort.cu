@@ -276,12 +276,31 @@ __global__ void __launch_bounds__(kBinChunk / 2) k_bin_reduce(const WorkSpace w)
     uint32_t sum = 0;
     if (any) block_exclusive_scan((uint32_t)(n.x + n.y), &sum);
     if (threadIdx.x == 0) S.bchunk[c] = (int)sum;
+    if (w.fit && any)
+#pragma unroll
+      for (int k = 0; k < kSizeChoices; k++) {
+        const int z = size_choice(k);
+        const int items = __reduce_add_sync(0xffffffffu, (n.x + z - 1) / z + (n.y + z - 1) / z);
+        if ((threadIdx.x & 31) == 0 && items) atomicAdd(&w.sizes[k], items);
+      }
   }
+}
+
+// The most particles of a work item (size_choice).
+__device__ __forceinline__ int item_size(const WorkSpace& w, int items_max) {
+  if (!w.fit) return items_max;
+  const int rounds = (w.sizes[kSizeChoices - 1] + w.fit - 1) / w.fit;
+  if (rounds > kFitRounds) return items_max;
+  int size = items_max;
+#pragma unroll
+  for (int k = kSizeChoices - 1; k >= 0; k--)
+    if (w.sizes[k] <= rounds * w.fit) size = size_choice(k);
+  return size;
 }
 
 // Block ranges and work items, a CTA per chunk of blocks: the chunk starts
 // after the particles of the chunks before it. Each block's particles are split
-// into near-equal items of at most S.items_max.
+// into near-equal items of at most item_size.
 __global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
   __shared__ int first_item;
   chain_next();
@@ -295,11 +314,12 @@ __global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
     for (int k = threadIdx.x; k < c; k += blockDim.x) sum += (uint32_t)S.bchunk[k];
     block_exclusive_scan(sum, &before);
     const int b0 = c * kBinChunk + 2 * (int)threadIdx.x;
+    const int most = item_size(w, S.items_max);
     int cnt[2], nit[2];
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       cnt[k] = b0 + k < S.nblocks ? S.bcount[b0 + k] : 0;
-      nit[k] = (cnt[k] + S.items_max - 1) / S.items_max;
+      nit[k] = (cnt[k] + most - 1) / most;
     }
     uint32_t items;
     uint32_t at = before + block_exclusive_scan((uint32_t)(cnt[0] + cnt[1]), nullptr);
@@ -355,6 +375,7 @@ __global__ void __launch_bounds__(256) k_bin_place(const WorkSpace w) {
       a += *(volatile int*)&w.scenes[s].counters[CNT_ITEMS];
     }
     w.items[w.nscenes] = a;
+    for (int k = 0; k < kSizeChoices; k++) w.sizes[k] = 0;
     w.scenes[0].counters[CNT_DONE] = 0;
   }
 }

@@ -76,3 +76,34 @@ def test_chained_launches_match_separate_ones(n, interval):
     for r in runs[1:]:
         assert _same(r, runs[0])
     ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("n", [40, 4096, 33000, 70000, 3 * 304 * 256, 3 * 304 * 256 + 1])
+def test_fitted_items_give_the_results_of_full_ones(n):
+    """Items sized by the binning (up to three rounds of the GPU's CTAs) against
+    items of up to 256: alone, in a batch that the scenes enter after their set-up,
+    and alone again."""
+    from snow_gb300 import api
+    edge = 32 if n < 10000 else 64 if n < 100000 else 96
+    s = scenes.small_scene(n=n, grid_edge=edge, seed=47, v0=(1.0, -3.0, 0.5))
+    t = scenes.small_scene(n=900, grid_edge=24, seed=48)
+    ctx = api.Context(0)
+    out = []
+    for full in (True, False):
+        sims = [api.SimScene(ctx, c) for c in (s, t)]
+        if full:
+            for g in sims:
+                g.set_tuning(8, 256, 2)
+        for g in sims:
+            g.upload().init().step(s.dt, 10)
+        got = [g.check().download() for g in sims]
+        b = api.Batch(ctx, sims)
+        b.step(13, dt=[s.dt, t.dt])
+        got += [g.check().download() for g in sims]
+        b.close()
+        got += [g.step(s.dt, 20).check().download() for g in sims]
+        out.append(got)
+    for a, b in zip(*out):
+        assert _same(a, b)
+    ctx.close()

@@ -586,6 +586,9 @@ struct ItemShared {
   unsigned pushed[3];                // ... and the part of them already recorded in FixState
   int next_same;                     // the CTA's next work item continues this item's home-block run
   int next_issue;                    // ... or starts a run whose grid rows the last warp copies
+  int unit_left;                     // items of the unit in hand after the one looked up last
+  int unit_tail;                     // runs from this item on are handed out item by item
+  int unit_pairs;                    // 1: the others two items at a time
   float run_bound;                   // sum of the contribution bounds of the particles in the tile's sums
   float item_bound;                  // ... and of this item's particles headed for the tile
   int abort;                         // 1 + parity of a wait for grid rows that ran out, else 0

@@ -528,8 +528,8 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // P2G of the next, in one pass over the item's particles. The P2G stress uses
 // the rotation R = W V^T of the advance's SVD: F_E' = W S' V^T with S'
 // diagonal up to the Jacobi residual, whose polar rotation is W V^T.
-// The CTAs take units of work from a counter: all items of a home block (a run)
-// or, when the launch has few, single items. The items of a run share
+// The CTAs take units of work from a counter: the items of a home block (a run)
+// or some of them. The items of a unit share
 // the staged grid rows (copied once, by bulk copies issued while the
 // previous run's last item sums its P2G) and the P2G tile (added to acc
 // once, at the run's end). The P2G sums are fixed
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // magnitudes of its particles for the next step's scales. BINNED: a step that
 // re-binned some scene; such a scene's particles are read from its binned
 // copies (CNT_BINNED) and, like every scene's, written to its streams.
-constexpr int kSingleItems = 5;
+constexpr int kSingleRounds = 3, kPairRounds = 5;
 template <bool BINNED>
 __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
                                                        const int* item_prefix, int nscenes) {
@@ -548,23 +548,34 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   tile_init(sh);
   chain_wait();
   const int total = item_prefix[nscenes];
-  // Whole runs unless that leaves CTAs without work: a run of two or three
-  // items costs one copy of the grid rows and one flush, but the CTA that takes
-  // it last works alone: with at most 5 items a CTA single items are faster
-  // (262k particles, 4.6 items a CTA: 32 steps 4.36 against 4.54 ms; 32k: 4.60
-  // against 6.12), above that both take the same time. The counter instead of
-  // equal shares of consecutive items: the items differ (surface blocks hold
-  // few particles, compressed snow costs more), 24 steps of a 1.5M-particle
-  // block on a sphere 12.0 to 11.0 ms, 50 of 1M particles 17.2 to 16.3.
-  const bool single = total <= kSingleItems * (int)gridDim.x;
+  // A unit is a run; in the last round of the CTAs (runs that start in the
+  // last gridDim.x items), and in launches of up to three rounds, a single item; and in
+  // launches of up to five rounds, before the last, two of a run's items. A run
+  // costs one copy of the grid rows and one flush, but the CTA that takes it last
+  // works on alone: with whole runs to the end 50 steps of 1M particles took 15.46
+  // ms, with single items in the last round 15.08, in the last two or four 15.13
+  // and 15.21; 16M the same. 32 steps of 262k particles (4.6 rounds): 3.97 ms
+  // all single, 3.85 now; 20 steps of 300k (4.8): 3.16, now 3.12, with whole runs 3.41.
+  // The counter instead of equal shares of consecutive items: the items differ
+  // (surface blocks hold few particles, compressed snow costs more), 24 steps of a
+  // 1.5M-particle block on a sphere 12.0 to 11.0 ms, 50 of 1M particles 17.2 to 16.3.
   int* counter = &scenes[0].counters[CNT_WORK];
-  // the first item of the unit after the one that was handed out as u
-  auto next_unit = [&](int u, int& s, int4& it) {
+  // the first item of the unit that starts at item u or at one handed out after
+  // it, and the unit's length
+  auto next_unit = [&](int u, int& s, int4& it, int& len) {
     for (;;) {
       if (u >= total) return total;
       s = find_scene(item_prefix, nscenes, u);
       it = scenes[s].items[u - item_prefix[s]];
-      if (single || it.w > 0) return u;
+      const int at = it.w > 0 ? 0 : -it.w;  // its place in its run
+      len = 1;
+      if (u - at >= sh.unit_tail) return u;
+      len = sh.unit_pairs ? min(2, it.w) : it.w;
+      if (at == 0) return u;
+      if (sh.unit_pairs && (at & 1) == 0) {
+        len = min(2, scenes[s].items[u - at - item_prefix[s]].w - at);
+        return u;
+      }
       u = (int)gridDim.x + atomicAdd(counter, 1);
     }
   };
@@ -574,9 +585,13 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   const int lane = threadIdx.x & 31;
   const bool lastw = (threadIdx.x >> 5) == (blockDim.x >> 5) - 1;
   if (lastw && lane == 0) {
-    int s0 = 0;
+    const int round = (int)gridDim.x;
+    sh.unit_tail = total <= kSingleRounds * round ? 0 : total - round;
+    sh.unit_pairs = total <= kPairRounds * round ? 1 : 0;
+    int s0 = 0, len = 1;
     int4 it0 = make_int4(0, 0, 0, 0);
-    sh.index_q[0] = next_unit((int)blockIdx.x, s0, it0);
+    sh.index_q[0] = next_unit((int)blockIdx.x, s0, it0, len);
+    sh.unit_left = len - 1;
     sh.item_q[0] = it0;
     sh.scene_q[0] = s0;
     sh.coll_scene = -1;
@@ -590,7 +605,6 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     stage_issue<kOutFields>(sh, S0, S0.gout, it0.x);
     if (lastw) particles_issue(sh, S0, it0.y, min(it0.z, kItemMax), BINNED && particles_binned(S0));
   }
-  int left = 0;  // items of the unit after this one (the last warp's lane 0)
   uint32_t phase = 0, pphase = 0;
   int par = 0;
   bool run_start = true;  // uniform across the CTA
@@ -624,13 +638,12 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     int sn = s, un = u + 1;
     int4 itn = make_int4(0, 0, 0, 0);
     if (lastw && lane == 0) {
-      if (run_start) left = single ? 0 : it.w - 1;
-      if (left > 0) {
-        left--;
+      int left = sh.unit_left;
+      if (left > 0)
         itn = S.items[un - item_prefix[s]];
-      } else {
-        un = next_unit((int)gridDim.x + atomicAdd(counter, 1), sn, itn);
-      }
+      else
+        un = next_unit((int)gridDim.x + atomicAdd(counter, 1), sn, itn, left);
+      sh.unit_left = left - 1;
     }
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);

@@ -182,7 +182,7 @@ struct SceneDev {
   int pool_cap;
   // P2G work items: (home block, first particle, count, and in a block's first
   // item the number of its items, else 0)
-  int4* items;
+  int4* items;  // home block, first particle, particles; its block's items (the first of them) or minus its place among them
   int item_cap;
   int* counters;    // kCounterStride ints
   // bounded waits for bulk copies into shared memory: give up after wait_ns

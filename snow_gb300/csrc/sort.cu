@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kBinChunk / 2) k_bin_scan(const WorkSpace w) {
       for (int j = 0; j < nit[k]; j++, it++) {
         if (it >= S.item_cap) break;  // cannot happen: item_cap covers the bound
         const int first = (int)(((long long)j * cnt[k]) / nit[k]), last = (int)(((long long)(j + 1) * cnt[k]) / nit[k]);
-        S.items[it] = make_int4(b, (int)at + first, last - first, j == 0 ? nit[k] : 0);
+        S.items[it] = make_int4(b, (int)at + first, last - first, j == 0 ? nit[k] : -j);
       }
       at += (uint32_t)cnt[k];
     }

@@ -107,3 +107,29 @@ def test_fitted_items_give_the_results_of_full_ones(n):
     for a, b in zip(*out):
         assert _same(a, b)
     ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("kind,n", [("dense", 200_003), ("dense", 70_001), ("sphere", 300_000), ("sphere", 9000)])
+def test_the_work_split_does_not_show_in_the_results(kind, n):
+    """Units of whole runs, of two items and of single ones: item sizes and CTAs
+    that take the items through three, five and more rounds of the CTAs; dense
+    snow has runs of hundreds of items, an odd number among them."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=n, grid_edge=32 if kind == "dense" else 96, seed=51, v0=(0.5, -2.0, 0.0))
+    if kind == "dense":  # five blocks, 16,000 to 64,000 particles each (at 200k), masses to match
+        rng = np.random.default_rng(52)
+        cells = np.array([[8, 8, 8], [12, 8, 8], [16, 8, 8], [8, 16, 12], [20, 20, 20]])[rng.choice(
+            5, n, p=[0.1, 0.1, 0.2, 0.28, 0.32])]
+        s.x = ((cells + rng.uniform(0.6, 3.4, (n, 3))) * s.grid_spacing).astype(np.float32) + np.float32(s.grid_pos[0])
+        s.m = (s.m / 100).astype(np.float32)
+    ctx = api.Context(0)
+    first = None
+    for items, ctas in ((256, 2), (256, 1), (128, 2), (64, 2), (64, 1)):
+        g = api.SimScene(ctx, s)
+        g.set_tuning(4, items, ctas)
+        out = g.upload().init().step(s.dt, 9).check().download()
+        g.close()
+        first = first or out
+        assert _same(out, first), (items, ctas)
+    ctx.close()

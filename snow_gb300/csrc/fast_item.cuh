@@ -492,7 +492,19 @@ __device__ __forceinline__ long long round_product(float a, float b, long long h
   return q < kLimit && q > -kLimit ? q : 0;
 }
 
-enum { kFarNone = 0, kFarFast = 1, kFarWide = 2 };
+// The same for finite a and b with |a b| < 2^46, without branches.
+__device__ __forceinline__ long long round_bounded(float a, float b, long long h) {
+  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+  const int xa = (int)(ua >> 23 & 255u), xb = (int)(ub >> 23 & 255u);
+  const uint32_t ma = (ua & 0x7fffffu) | (xa ? 0x800000u : 0u), mb = (ub & 0x7fffffu) | (xb ? 0x800000u : 0u);
+  const long long p = (long long)((unsigned long long)ma * mb);
+  const int s = min(300 - max(xa, 1) - max(xb, 1), 50);  // |a b| = p 2^-s, s > 0; rounds to 0 from 50 on
+  const long long t = ((ua ^ ub) >> 31) != 0u ? -p : p;
+  const long long odd = (h + (t >> s)) & 1;
+  return h + ((t + (1ll << (s - 1)) - 1 + odd) >> s);
+}
+
+enum { kFarNone = 0, kFarFast = 1, kFarWide = 2, kFarTile = 3 };
 struct FarParticle {
   float wx[4], gx[4], wy[4], gy[4], wz[4], gz[4];
   float ms, mvs[3], As[9];
@@ -591,6 +603,7 @@ struct ItemShared {
   int unit_pairs;                    // 1: the others two items at a time
   float run_bound;                   // sum of the contribution bounds of the particles in the tile's sums
   float item_bound;                  // ... and of this item's particles headed for the tile
+  int wide;                          // some of the item's particles go through wide_scatter
   int abort;                         // 1 + parity of a wait for grid rows that ran out, else 0
   int pabort;                        // ... for particles
   uint64_t bar, pbar;                // completion of the grid rows' copies, of the particles'
@@ -748,6 +761,7 @@ __device__ __forceinline__ void tile_init(ItemShared& sh) {
     mbar_init(&sh.pbar, 1);
     sh.abort = sh.pabort = 0;
     sh.run_bound = sh.item_bound = 0.0f;
+    sh.wide = 0;
   }
   __syncthreads();
 }
@@ -1110,10 +1124,118 @@ __device__ __forceinline__ void p2g_tile_flush(ItemShared& sh, const SceneDev& S
 // A particle's quantities as the tile stores them (fixed point: scaled).
 struct P2GStored {
   float ms, mvs[3], As[3][3];
-  int cell, rank;  // its tile cell (-1: not in the tile) and its place among the cell's particles
+  int cell, rank;  // its tile cell (-1: not in the tile) and its place among the cell's particles;
+                   // kCellWide: its contributions outgrew 32 bits, and its stencil's first tile node
 };
+constexpr int kCellWide = -2;
 
-template <int KIND, bool RUN = false>
+__device__ __forceinline__ void far_put(FarParticle* f, const P2GStored& st, const AxisW& w) {
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    f->wx[a] = w.wx[a];
+    f->gx[a] = w.gx[a];
+    f->wy[a] = w.wy[a];
+    f->gy[a] = w.gy[a];
+    f->wz[a] = w.wz[a];
+    f->gz[a] = w.gz[a];
+  }
+  f->ms = st.ms;
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    f->mvs[r] = st.mvs[r];
+#pragma unroll
+    for (int c = 0; c < 3; c++) f->As[3 * r + c] = st.As[r][c];
+  }
+}
+
+// Particles in the tile whose force outgrew the scale (the first steps from
+// rest: the scale follows the largest force of the step before): summed in shared
+// memory, each force contribution as its low 20 bits and the rest, in two words of
+// a tile of their own in pd, which is not in use yet. Not the mass and momentum,
+// which stay in the fast range for these (wide_force) and round there to the
+// same integers. 256 contributions below 2^42 fit both words. At kWideWarp such
+// particles in a warp the zeroing and the flush cost less than their 448
+// atomics each on 64-bit words in HBM: a step whose 131k particles are all wide
+// took 544 us, now 220; the first of 32k particles from rest 115, now 53. WIDE: in an
+// instantiation of its own, which a single scene's first step after its set-up takes:
+// in every step's it cost 1% (registers).
+constexpr int kWideWarp = 8;
+constexpr int kWideShift = 20;
+constexpr int kWideWords = 10 * kTile3;  // mass, momentum, force (low), force (rest)
+static_assert(kWideWords + (int)(kItemMax / 32 * sizeof(FarParticle) / sizeof(float)) <= kItemMax / 2 * kPdStride,
+              "the wide tile and a particle per warp fit pd");
+__device__ __forceinline__ bool wide_force(const P2GParticle& q, const FixScale& sc, float bound) {
+  const float mv = fmaxf(fabsf(q.mv[0]), fmaxf(fabsf(q.mv[1]), fabsf(q.mv[2])));
+  return fmaxf(fabsf(q.m) * sc.m, mv * sc.p) * kWmax < kFastLimit && bound < 4.0e12f;  // 2^42 = 4.4e12
+}
+__device__ __noinline__ void wide_scatter(ItemShared& sh, const FarParticle& f, int origin) {
+  int* const sum = reinterpret_cast<int*>(sh.pd);
+  const int lane = threadIdx.x & 31;
+  float As[3][3];
+#pragma unroll
+  for (int k = 0; k < 9; k++) As[k / 3][k % 3] = f.As[k];
+  const int a = lane & 3, b = (lane >> 2) & 3;
+  const float wxa = f.wx[a], gxa = f.gx[a], wyb = f.wy[b], gyb = f.gy[b];
+#pragma unroll 1
+  for (int c = lane >> 4; c < 4; c += 2) {
+    RowFactors rf;
+    row_factors(f.ms, f.mvs, As, wyb, gyb, f.wz[c], f.gz[c], false, rf);
+    int* const at = sum + origin + a + kTile * b + kTile * kTile * c;
+    atomicAdd(at, fix_mass(wxa, rf) - kMagicBits);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      atomicAdd(at + (1 + r) * kTile3, fix_mom(wxa, rf, r) - kMagicBits);
+      const long long v = round_bounded(gxa, rf.kk[r], round_bounded(wxa, rf.hh[r], 0));
+      atomicAdd(at + (4 + r) * kTile3, (int)(v & ((1 << kWideShift) - 1)));
+      atomicAdd(at + (7 + r) * kTile3, (int)(v >> kWideShift));
+    }
+  }
+}
+// The wide tile into acc; pd is left zero (finite) for the records.
+__device__ __noinline__ void wide_flush(ItemShared& sh, const SceneDev& S, int bx, int by, int bz) {
+  int* const sum = reinterpret_cast<int*>(sh.pd);
+  for (int t = threadIdx.x; t < kTile3; t += blockDim.x) {
+    long long v[7];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+      v[k] = sum[k * kTile3 + t];
+      sum[k * kTile3 + t] = 0;
+      if (k >= 4) {
+        v[k] += (long long)sum[(k + 3) * kTile3 + t] * (1 << kWideShift);
+        sum[(k + 3) * kTile3 + t] = 0;
+      }
+      any = any || v[k] != 0;
+    }
+    const int g0 = 4 * bx - 2 + t % kTile, g1 = 4 * by - 2 + t / kTile % kTile, g2 = 4 * bz - 2 + t / (kTile * kTile);
+    if (!any || !node_in_grid(S, g0, g1, g2)) continue;
+    const int blk = block_id(S, g0 >> 2, g1 >> 2, g2 >> 2);
+    acc_add(S, blk, (g0 & 3) + 4 * (g1 & 3) + 16 * (g2 & 3), v, false);
+    S.blk_flag[blk] = 1;
+  }
+}
+// By the whole CTA after the counts' barrier, when the item has such particles.
+__device__ __forceinline__ void wide_sums(ItemShared& sh, const SceneDev& S, int bx, int by, int bz,
+                                          const P2GStored& st, const AxisW& w) {
+  for (int k = threadIdx.x; k < kWideWords; k += blockDim.x) sh.pd[k] = 0.0f;
+  __syncthreads();
+  if (threadIdx.x == 0) sh.wide = 0;  // every thread has read it
+  FarParticle* f = reinterpret_cast<FarParticle*>(sh.pd + kWideWords) + (threadIdx.x >> 5);
+  uint32_t todo = __ballot_sync(0xffffffffu, st.cell == kCellWide);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    __syncwarp();
+    if ((int)(threadIdx.x & 31) == src) far_put(f, st, w);
+    __syncwarp();
+    wide_scatter(sh, *f, __shfl_sync(0xffffffffu, st.rank, src));
+  }
+  __syncthreads();
+  wide_flush(sh, S, bx, by, bz);
+  __syncthreads();
+}
+
+template <int KIND, bool RUN = false, bool WIDE = false>
 __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, bool have,
                                           const P2GParticle& q, const AxisW& w, const int base[3], const FixScale& sc,
                                           P2GStored& st) {
@@ -1154,6 +1276,20 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
       far = fast && finite_w ? kFarFast : kFarWide;
       if (KIND != kP2gForce && far == kFarWide) atomicAdd(&S.fix->wide, 1u);
       if (KIND == kP2gForce && !q.force) far = kFarNone;
+      if (WIDE && inside && finite_w && wide_force(q, sc, bound)) {
+        far = kFarTile;
+        st.rank = lx + kTile * ly + kTile * kTile * lz;
+      }
+    }
+  }
+  if (WIDE) {
+    const int n = __popc(__ballot_sync(0xffffffffu, far == kFarTile));
+    if (far == kFarTile) {
+      far = n >= kWideWarp ? kFarNone : kFarWide;
+      if (n >= kWideWarp) {
+        st.cell = kCellWide;
+        sh.wide = 1;
+      }
     }
   }
   uint32_t todo = __ballot_sync(0xffffffffu, far != kFarNone);
@@ -1166,23 +1302,9 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
       todo &= todo - 1;
       __syncwarp();
       if ((int)(threadIdx.x & 31) == src) {
+        far_put(f, st, w);
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-          f->wx[a] = w.wx[a];
-          f->gx[a] = w.gx[a];
-          f->wy[a] = w.wy[a];
-          f->gy[a] = w.gy[a];
-          f->wz[a] = w.wz[a];
-          f->gz[a] = w.gz[a];
-        }
-        f->ms = st.ms;
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-          f->mvs[r] = st.mvs[r];
-          f->base[r] = base[r];
-#pragma unroll
-          for (int c = 0; c < 3; c++) f->As[3 * r + c] = st.As[r][c];
-        }
+        for (int r = 0; r < 3; r++) f->base[r] = base[r];
       }
       __syncwarp();
       scatter_far<KIND>(S, *f, __shfl_sync(0xffffffffu, far, src));
@@ -1195,13 +1317,14 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
   }
 }
 
-template <int KIND, bool RUN = false>
+template <int KIND, bool RUN = false, bool WIDE = false>
 __device__ __forceinline__ void p2g_sum(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, const P2GStored& st,
                                         const AxisW& w) {
   constexpr int nf = P2gFields<KIND>::nf;
   constexpr bool fix = KIND != kP2gForce;
   const int lane = threadIdx.x & 31;
   const int my_cell = st.cell;
+  if (WIDE && sh.wide) wide_sums(sh, S, bx, by, bz, st, w);  // uniform across the CTA
   if (RUN && sh.run_bound + sh.item_bound > kTileSumBound) {  // uniform across the CTA
     // this item's sums could wrap the tile's int32 sums: the earlier items'
     // go to acc first (integer sums: the split changes no bit of the result)

@@ -537,9 +537,10 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // item records them for the next grid update, and every CTA records the
 // magnitudes of its particles for the next step's scales. BINNED: a step that
 // re-binned some scene; such a scene's particles are read from its binned
-// copies (CNT_BINNED) and, like every scene's, written to its streams.
+// copies (CNT_BINNED) and, like every scene's, written to its streams. WIDE: with
+// the sums of kCellWide particles (in shared memory; else by atomics on acc).
 constexpr int kSingleRounds = 3, kPairRounds = 5;
-template <bool BINNED>
+template <bool BINNED, bool WIDE>
 __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
                                                        const int* item_prefix, int nscenes) {
   extern __shared__ float4 smem_raw[];
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       sh.next_issue = un < total && !same ? 1 : 0;
     }
     P2GStored stored;
-    p2g_count<kP2gFull, true>(sh, S, bx, by, bz, have, q, wn, nbase, sh.fscale, stored);
+    p2g_count<kP2gFull, true, WIDE>(sh, S, bx, by, bz, have, q, wn, nbase, sh.fscale, stored);
     __syncthreads();  // counts done; the particle buffer is read
     if (sh.abort | sh.pabort) {
       stage_abort(sh, S);  // a copy wait ran out: this item's particles keep their state, the CTA stops
@@ -720,7 +721,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       const SceneDev& N = scenes[sh.scene_q[par ^ 1]];
       particles_issue(sh, N, nx.y, min(nx.z, kItemMax), BINNED && particles_binned(N));
     }
-    p2g_sum<kP2gFull, true>(sh, S, bx, by, bz, stored, wn);
+    p2g_sum<kP2gFull, true, WIDE>(sh, S, bx, by, bz, stored, wn);
     if (sh.next_issue) {  // uniform across the CTA
       const SceneDev& N = scenes[sh.scene_q[par ^ 1]];
       stage_issue<kOutFields>(sh, N, N.gout, sh.item_q[par ^ 1].x);
@@ -959,8 +960,9 @@ int item_smem() {
     smem_opt_in(k_p2g<true>, bytes);
     smem_opt_in(k_p2g<false>, bytes);
     smem_opt_in(k_g2p_advance, bytes);
-    smem_opt_in(k_g2p2g<false>, bytes);
-    smem_opt_in(k_g2p2g<true>, bytes);
+    smem_opt_in(k_g2p2g<false, false>, bytes);
+    smem_opt_in(k_g2p2g<true, false>, bytes);
+    smem_opt_in(k_g2p2g<true, true>, bytes);
     configured[dev] = true;
   }
   return bytes;
@@ -1037,9 +1039,9 @@ void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscene
 }
 
 void fast_g2p2g(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, bool binned,
-                bool chained, cudaStream_t st) {
-  launch_after(chained, binned ? k_g2p2g<true> : k_g2p2g<false>, grid_ctas, kItemMax, item_smem(), st, scenes,
-               item_prefix, nscenes);
+                bool wide, bool chained, cudaStream_t st) {
+  launch_after(chained, wide ? k_g2p2g<true, true> : binned ? k_g2p2g<true, false> : k_g2p2g<false, false>, grid_ctas,
+               kItemMax, item_smem(), st, scenes, item_prefix, nscenes);
 }
 
 void fast_stats(const SceneDev* sd_dev, int n, StatsSlot* slot, StatsAccum* host, cudaStream_t st) {

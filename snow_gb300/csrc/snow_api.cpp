@@ -105,6 +105,8 @@ struct snow_scene {
   // graphs of one step, keyed by (dt, with binning), and of kGraphSteps plain ones
   cudaGraphExec_t g_plain = nullptr, g_sort = nullptr, g_many = nullptr;
   float g_dt = NAN;
+  cudaGraphExec_t g_first = nullptr;  // of a semi-implicit scene's first step
+  bool first_step = false;            // the next step is the first since the set-up
   int g_steps = 0;  // steps launched one by one that g_many could have taken
   snow_phase_times times{};
   uint32_t wide_base = 0;  // FixState::wide at the last phase-times reset
@@ -243,7 +245,8 @@ void drop_graphs(snow_scene* s) {
   if (s->g_plain) cudaGraphExecDestroy(s->g_plain);
   if (s->g_sort) cudaGraphExecDestroy(s->g_sort);
   if (s->g_many) cudaGraphExecDestroy(s->g_many);
-  s->g_plain = s->g_sort = s->g_many = nullptr;
+  if (s->g_first) cudaGraphExecDestroy(s->g_first);
+  s->g_plain = s->g_sort = s->g_many = s->g_first = nullptr;
   s->g_steps = 0;
   s->g_dt = NAN;
 }
@@ -472,14 +475,14 @@ void fast_enqueue_solve(snow_scene* s, cudaStream_t st) {
 // One step of a scene whose P2G sums of the current state are pending in
 // acc: rigid advance, [binning], grid update, G2P + advance + next P2G.
 // follows: st's last kernel is that of the step before.
-void fast_enqueue_step(snow_scene* s, bool bin, bool follows, cudaStream_t st) {
+void fast_enqueue_step(snow_scene* s, bool bin, bool follows, cudaStream_t st, bool wide = false) {
   bin = bin && s->n > 0;
   const bool chain = s->n <= kChainParticles;
   if (bin) fast_bin(s, st, true, follows);
   fast_compact(s->work, s->ncoll > 0, bin, chain && (bin || follows), st);
   fast_enqueue_grid(s, false, chain, st);
   fast_enqueue_solve(s, st);
-  fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, chain && !s->sd.crs, st);
+  fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, wide, chain && !s->sd.crs, st);
 }
 
 snow_status set_dt(snow_scene* s, float dt) {
@@ -601,6 +604,7 @@ snow_status fast_init(snow_scene* s) {
   fast_enqueue_grid(s, true, false, st);                         // clear acc
   fast_enqueue_p2g(s, false, st);                                // P2G of step 1
   CK(cudaGetLastError());
+  s->first_step = true;
   // the particles' largest speed, which the re-binning interval is chosen from
   CK(cudaMemcpyAsync(s->h_cnt, s->sd.counters, kCounterStride * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1194,6 +1198,8 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       if (r) return r;
     }
     const bool bin = s->steps_since_sort >= s->bin_interval;
+    const bool first = s->first_step;
+    s->first_step = false;
     if (ctx->profiling) {
       cudaEvent_t* ev = ctx->ev;
       CK(cudaEventRecord(ev[0], st));
@@ -1204,7 +1210,7 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       CK(cudaEventRecord(ev[2], st));
       fast_enqueue_solve(s, st);
       CK(cudaEventRecord(ev[3], st));
-      fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, false, st);
+      fast_g2p2g(s->sd_dev, s->d_prefix + 0, 1, item_ctas(s->tune), bin, first, false, st);
       CK(cudaEventRecord(ev[4], st));
       CK(cudaEventSynchronize(ev[4]));
       float t[4];
@@ -1215,20 +1221,21 @@ snow_status snow_scene_step(snow_scene* s, double dt, int n_steps) {
       s->times.g2p_ms += t[3];
       s->times.total_ms += t[0] + t[1] + t[2] + t[3];
       s->times.steps++;
-    } else if (!ctx->graphs) {
-      fast_enqueue_step(s, bin, follows, st);
+    } else if (!ctx->graphs || (first && !s->sd.crs)) {  // (the first step runs while the others' graphs are made)
+      fast_enqueue_step(s, bin, follows, st, first);
       follows = true;
     } else {
       if (s->g_dt != fdt) drop_graphs(s);
+      follows = false;
       if (!bin && !s->sd.crs && n_steps - i >= kGraphSteps && kCheckSteps - s->steps_since_check >= kGraphSteps &&
           s->bin_interval - s->steps_since_sort >= kGraphSteps &&
           (s->g_many || n_steps - i >= kManyFrom || s->g_steps++ >= kManyFrom))
         k = kGraphSteps;
-      cudaGraphExec_t& g = k > 1 ? s->g_many : bin ? s->g_sort : s->g_plain;
+      cudaGraphExec_t& g = first && !bin ? s->g_first : k > 1 ? s->g_many : bin ? s->g_sort : s->g_plain;
       if (!g) {
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < k; j++) fast_enqueue_step(s, bin, j > 0, st);
+        for (int j = 0; j < k; j++) fast_enqueue_step(s, bin, j > 0, st, first && !bin);
         CK(cudaStreamEndCapture(st, &graph));
         CK(cudaGraphInstantiate(&g, graph, 0));
         cudaGraphDestroy(graph);
@@ -1663,7 +1670,7 @@ void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   if (iters > 0)
     fast_implicit_solve(b->d_scenes, items, active, n, iters, item_ctas(b->scenes[0]->tune), grid_ctas(),
                         b->ctx->d_iter, b->ctx->body_stream, b->ctx->gate_stream, st);
-  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), bin_all, chain && iters == 0, st);
+  fast_g2p2g(b->d_scenes, items, n, item_ctas(b->scenes[0]->tune), bin_all, false, chain && iters == 0, st);
 }
 
 }  // namespace
@@ -1677,6 +1684,7 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
   cudaStream_t st = ctx->stream;
   for (size_t i = 0; i < b->scenes.size(); i++) {
     snow_scene* s = b->scenes[i];
+    s->first_step = false;
     if (s->fitted) {  // binned before it was in a batch: the next step re-bins
       s->fitted = false;
       s->steps_since_sort = 1 << 30;

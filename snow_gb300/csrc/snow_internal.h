@@ -181,8 +181,8 @@ struct SceneDev {
   float* gout;
   int pool_cap;
   // P2G work items: (home block, first particle, count, and in a block's first
-  // item the number of its items, else 0)
-  int4* items;  // home block, first particle, particles; its block's items (the first of them) or minus its place among them
+  // item the number of its items, else minus its place among them)
+  int4* items;
   int item_cap;
   int* counters;    // kCounterStride ints
   // bounded waits for bulk copies into shared memory: give up after wait_ns
@@ -277,7 +277,7 @@ void fast_g2p_advance(const SceneDev* scenes, const int* item_prefix, int nscene
 // binned: some scene of the launch was re-binned in this step (its particles
 // are in its binned copies)
 void fast_g2p2g(const SceneDev* scenes, const int* item_prefix, int nscenes, int grid_ctas, bool binned,
-                bool chained, cudaStream_t st);
+                bool wide, bool chained, cudaStream_t st);
 // The semi-implicit velocity solve between the grid update (which leaves
 // v*, m and u = v* in the solver planes) and G2P: iterations of conjugate
 // residuals (each a K u pass over the items and three passes over the active

@@ -133,3 +133,32 @@ def test_the_work_split_does_not_show_in_the_results(kind, n):
         first = first or out
         assert _same(out, first), (items, ctas)
     ctx.close()
+
+
+@gpu
+@pytest.mark.parametrize("graphs", [True, False])
+@pytest.mark.parametrize("n,speed,young", [(3000, 0.01, 1.4e5), (3000, 2.0, 1.4e5), (20_001, 5.0, 1.4e5),
+                                           (20_001, 20.0, 1.4e7), (60_000, 3.0, 1e3)])
+def test_first_steps_with_forces_that_outgrow_the_scale(n, speed, young, graphs):
+    """Snow at rest in itself that is given random velocities: its first step's
+    forces are orders of magnitude above the scale chosen from a state without
+    any. A scene's own first step sums such particles in shared memory, a batch's by
+    atomics on the grid: the same integers."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=n, grid_edge=32 if n < 10000 else 64, seed=61, young=young, dt=2e-5)
+    s.v = np.random.default_rng(62).uniform(-speed, speed, (n, 3)).astype(np.float32)
+    s.v[: n // 3] *= 1e-3  # and some that stay in range, in the same warps' neighbourhoods
+    ctx = api.Context(0)
+    ctx.set_graphs(graphs)
+    alone = api.SimScene(ctx, s).upload().init()
+    other = api.SimScene(ctx, s).upload().init()
+    batch = api.Batch(ctx, [other])
+    wide = []
+    for steps in (1, 1, 6):
+        alone.step(s.dt, steps)
+        batch.step(steps, dt=[s.dt])
+        assert _same(alone.check().download(), other.check().download())
+        wide.append((alone.phase_times()["wide"], other.phase_times()["wide"]))
+    assert all(a == b for a, b in wide)
+    assert wide[0][0] > n // 2 or speed < 1
+    ctx.close()

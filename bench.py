@@ -18,7 +18,6 @@ from __future__ import annotations
 
 import argparse
 import json
-import math
 import os
 import statistics
 import subprocess
@@ -47,10 +46,10 @@ BYTES_GRID = (0, 40)
 # work split named in TRAFFIC_SOURCE, keyed by (particles, grid edge); other
 # workloads report null: DRAM bytes (read + write) per launch, and warp
 # instructions per launch for the issue roofline.
-TRAFFIC_MEASURED = {(1 << 20, 256): 144.3e6}
-INSTRUCTIONS_MEASURED = {(1 << 20, 256): 173.2e6}
+TRAFFIC_MEASURED = {(1 << 20, 256): 142.7e6}
+INSTRUCTIONS_MEASURED = {(1 << 20, 256): 143.4e6}
 TRAFFIC_SOURCE = ("not counted in this run: separate ncu --set full captures of one k_g2p2g launch of this "
-                  "workload (256 particles per item, 2 CTAs per SM; sort interval 8 and 32 alike)")
+                  "workload (256 particles per item, 2 CTAs per SM, sort interval 8)")
 # warp-instruction issue peak: 152 SMs x 4 schedulers x 2.07 GHz
 ISSUE_PEAK = 152 * 4 * 2.07e9
 # FP32 peak: 152 SMs x 128 lanes x 2 flops per FMA x 2.07 GHz; the algorithmic
@@ -131,13 +130,10 @@ def measured_peak_hbm():
         return 6800.0, "fallback"
 
 
-def kernels_per_step(n_colliders, sort_step, key_bits):
-    plain = 4  # begin (counters, colliders), compact (+ prefixes), grid, g2p2g
-    if not sort_step:
-        return plain
-    passes = (key_bits + 7) // 8
-    # keys, (hist + 3 scan + scatter) per pass, permute, heads, items, prefix
-    return plain + 1 + passes * 5 + 4
+def kernels_per_step(sort_step):
+    plain = 3  # compact (step start, active blocks, prefixes), grid, g2p2g
+    # re-binning: count, reduce, scan, place, cells, move
+    return plain + 6 if sort_step else plain
 
 
 def reduce_max_ms(total_ms, dist_mod, device):
@@ -296,9 +292,8 @@ def bench_ours(args, local_rank, barrier=lambda: None):
     sim2.close()
     del out
 
-    key_bits = math.ceil(math.log2(((args.grid + 3) // 4) ** 3 * 64))
-    plain_k = kernels_per_step(len(s.colliders), False, key_bits)
-    bin_k = kernels_per_step(len(s.colliders), True, key_bits)
+    plain_k = kernels_per_step(False)
+    bin_k = kernels_per_step(True)
     launches = args.steps * plain_k + binnings * (bin_k - plain_k)
     res = dict(total_ms=total_ms, step_ms=step_ms, n=n, A=A, per=per, dominant=dominant, alg_bytes=alg_bytes,
                achieved=achieved, peak=peak, peak_kind=peak_kind, clocks=clocks.summary(), e2e_s=e2e_s,

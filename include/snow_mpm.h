@@ -157,7 +157,8 @@ const char* snow_last_error(const snow_ctx* ctx);
 size_t snow_ctx_bytes_in_use(const snow_ctx* ctx);
 snow_status snow_ctx_set_profiling(snow_ctx* ctx, int on);
 /* on = 0: snow_scene_step launches each step's kernels one by one instead of
- * replaying the step's captured CUDA graph (default on). Batches always
+ * replaying captured CUDA graphs of one or more steps (default on; the first
+ * step after a set-up is launched directly either way). Batches always
  * replay graphs. */
 snow_status snow_ctx_set_graphs(snow_ctx* ctx, int on);
 /* The cudaStream_t every call of this context launches on, for callers that
@@ -385,7 +386,8 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps);
 /* Work decomposition of the FAST step (no counterpart in the reference). */
 typedef struct snow_tuning {
   int sort_interval;   /* steps between re-binnings of each scene's particles (1..64) */
-  int items_max;       /* most particles per work item (64..256) */
+  int items_max;       /* most particles per work item (64..256; without a tuning: 256,
+                        * and fewer where all items then run at once) */
   int ctas_per_sm;     /* work-item CTAs per SM (1 or 2) */
   int steps_taken;     /* autotune: steps the batch advanced while timing */
   double ms_per_step;  /* autotune: measured time per step of the choice */

@@ -223,7 +223,8 @@ constexpr int kItemCtas = 2;
 // (P2G work items, active blocks, particles, quads and chunks of grid
 // blocks), in one device array of five prefixes of nscenes + 1 entries. Item
 // and active-block counts are only known on the device; the binning and the
-// compaction form those two prefixes there.
+// compaction form those two prefixes there. The binning's item counts at each
+// size follow them.
 struct WorkSpace {
   const SceneDev* scenes;
   int nscenes;
@@ -255,7 +256,7 @@ inline bool fits_items(long long n, int ctas) { return n <= (long long)kFitRound
 constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
 // Start of a step alone: resets the per-step counters and, with `rigid`, moves
 // the colliders by dt * velocity (rigidAdvance.glsl:14-18). A step's compaction
-// does the same at its end.
+// does the same in its first CTAs.
 void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st);
 // Copies every scene's counters and FixState into out[s * kCounterStride ...] (mapped
 // pinned memory: a batch reads them one re-binning interval later, without

@@ -561,6 +561,14 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   // (surface blocks hold few particles, compressed snow costs more), 24 steps of a
   // 1.5M-particle block on a sphere 12.0 to 11.0 ms, 50 of 1M particles 17.2 to 16.3.
   int* counter = &scenes[0].counters[CNT_WORK];
+  // the length of the unit that starts at item u (`it`, of scene s); 0: none does
+  auto unit_at = [&](int u, int s, const int4& it) {
+    const int at = it.w > 0 ? 0 : -it.w;  // its place in its run
+    if (u - at >= sh.unit_tail) return 1;
+    if (at == 0) return sh.unit_pairs ? min(2, it.w) : it.w;
+    if (sh.unit_pairs && (at & 1) == 0) return min(2, scenes[s].items[u - at - item_prefix[s]].w - at);
+    return 0;
+  };
   // the first item of the unit that starts at item u or at one handed out after
   // it, and the unit's length
   auto next_unit = [&](int u, int& s, int4& it, int& len) {
@@ -568,15 +576,8 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       if (u >= total) return total;
       s = find_scene(item_prefix, nscenes, u);
       it = scenes[s].items[u - item_prefix[s]];
-      const int at = it.w > 0 ? 0 : -it.w;  // its place in its run
-      len = 1;
-      if (u - at >= sh.unit_tail) return u;
-      len = sh.unit_pairs ? min(2, it.w) : it.w;
-      if (at == 0) return u;
-      if (sh.unit_pairs && (at & 1) == 0) {
-        len = min(2, scenes[s].items[u - at - item_prefix[s]].w - at);
-        return u;
-      }
+      len = unit_at(u, s, it);
+      if (len > 0) return u;
       u = (int)gridDim.x + atomicAdd(counter, 1);
     }
   };
@@ -634,18 +635,13 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       if (threadIdx.x == 0) sh.run_bound = 0.0f;
     }
     const int4 it = sh.item_q[par];
-    // the next item: looked up now, so that the latency overlaps this item's
-    // G2P, and put in shared memory before this item's P2G
-    int sn = s, un = u + 1;
-    int4 itn = make_int4(0, 0, 0, 0);
-    if (lastw && lane == 0) {
-      int left = sh.unit_left;
-      if (left > 0)
-        itn = S.items[un - item_prefix[s]];
-      else
-        un = next_unit((int)gridDim.x + atomicAdd(counter, 1), sn, itn, left);
-      sh.unit_left = left - 1;
-    }
+    // the next item: handed out (at the end of a unit) while this one's particles
+    // and grid values are waited for, copied to its queue entry during the gather and
+    // looked at after it. Looked up at the item's start, the last warp waited for the
+    // atomic and the load in turn and the others for it: 12 steps of 16M particles
+    // 63.0 to 62.3 ms, 24 of a 1.5M block 9.70 to 9.60, 50 of 1M 15.06 to 14.94.
+    int un = u + 1;
+    if (lastw && lane == 0 && sh.unit_left <= 0) un = (int)gridDim.x + atomicAdd(counter, 1);
     int bx, by, bz;
     home_coords(S, it.x, bx, by, bz);
     const int i = threadIdx.x;
@@ -653,6 +649,11 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     const int p = it.y + i;
     bool landed = particles_wait(sh, S, pphase);
     if (run_start) landed = stage_wait(sh, S, phase) && landed;
+    if (lastw && lane == 0 && un < total) {
+      const int sn = find_scene(item_prefix, nscenes, un);
+      copy_async16(&sh.item_q[par ^ 1], &scenes[sn].items[un - item_prefix[sn]]);
+      sh.scene_q[par ^ 1] = sn;
+    }
     bool have = false;
     P2GParticle q;
     q.force = false;
@@ -699,9 +700,17 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
         atomicMax(&sh.seen[2], ba);
       }
     }
-    // the next item's queue entry: every thread read this one's at the loop
+    // the rest of the queue entry: every thread read this one's at the loop
     // top, and the barriers below publish it before the flush decision
     if (lastw && lane == 0) {
+      copy_async_wait();
+      int sn = sh.scene_q[par ^ 1], left = sh.unit_left;
+      int4 itn = sh.item_q[par ^ 1];
+      if (left <= 0 && un < total) {
+        left = unit_at(un, sn, itn);
+        if (left == 0) un = next_unit((int)gridDim.x + atomicAdd(counter, 1), sn, itn, left);
+      }
+      sh.unit_left = left - 1;
       const bool same = un == u + 1 && sn == s && itn.x == it.x;  // (single items of a block may also come one after the other)
       sh.item_q[par ^ 1] = itn;
       sh.scene_q[par ^ 1] = sn;

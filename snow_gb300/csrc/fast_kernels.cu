@@ -546,6 +546,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   extern __shared__ float4 smem_raw[];
   ItemShared& sh = *reinterpret_cast<ItemShared*>(smem_raw);
   chain_next();
+  tile_zero(sh, kAccFields);
   tile_init(sh);
   chain_wait();
   const int total = item_prefix[nscenes];
@@ -630,10 +631,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
       S.fix->scale[1] = sh.fscale.p;
       S.fix->scale[2] = sh.fscale.f;
     }
-    if (run_start) {
-      tile_zero(sh, kAccFields);
-      if (threadIdx.x == 0) sh.run_bound = 0.0f;
-    }
+    if (run_start && threadIdx.x == 0) sh.run_bound = 0.0f;
     const int4 it = sh.item_q[par];
     // the next item: handed out (at the end of a unit) while this one's particles
     // and grid values are waited for, copied to its queue entry during the gather and
@@ -745,7 +743,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
         }
     }
     const bool cont = sh.next_same != 0;  // uniform across the CTA
-    if (!cont) p2g_tile_flush<kP2gFull>(sh, S, bx, by, bz);
+    if (!cont) p2g_tile_flush<kP2gFull, true>(sh, S, bx, by, bz);
     run_start = !cont;
   }
 }

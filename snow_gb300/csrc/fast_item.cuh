@@ -346,11 +346,16 @@ __device__ __forceinline__ void acc_add(const SceneDev& S, int blk, int node, co
 }
 
 // ---- P2G quantities of one particle -----------------------------------------
+__device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf drops NaN)
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // mass, momentum and A = -V0 * stress, stress = 2 mu(Jp) (FE - R) FE^T +
 // lambda(Jp) (JE - 1) JE I with R the polar rotation of FE
 // (p2gTransfer.glsl:109-141); V0 = m / rho0. `a` = max over rows r of
 // |A_r0| + |A_r1| + |A_r2| bounds a force contribution and both its terms
-// (in units of the weight products' bound (2/3)^3).
+// (in units of the weight products' bound (2/3)^3); NaN if any term is.
 struct P2GParticle {
   float m, mv[3];
   float A[3][3];  // A[r][c]
@@ -376,7 +381,7 @@ __device__ __forceinline__ void p2g_stress(const SceneDev& S, const M3& F, const
   for (int r = 0; r < 3; r++) {
 #pragma unroll
     for (int c = 0; c < 3; c++) q.A[r][c] = -vol * (2.0f * mu * P.m[c][r] + (r == c ? s2 : 0.0f));
-    a = fmaxf(a, fabsf(q.A[r][0]) + fabsf(q.A[r][1]) + fabsf(q.A[r][2]));
+    a = max_nan(a, fabsf(q.A[r][0]) + fabsf(q.A[r][1]) + fabsf(q.A[r][2]));
   }
   q.a = a;
   q.force = true;
@@ -412,11 +417,18 @@ template <int KIND>
 __device__ __forceinline__ float fix_bound(const P2GParticle& q, const FixScale& sc) {
   float b = fabsf(q.m) * sc.m;
   if (KIND == kP2gFull) {
-    const float mv = fmaxf(fabsf(q.mv[0]), fmaxf(fabsf(q.mv[1]), fabsf(q.mv[2])));
-    b = fmaxf(b, mv * sc.p);
-    if (q.force) b = fmaxf(b, q.a * sc.f);
+    const float mv = max_nan(fabsf(q.mv[0]), max_nan(fabsf(q.mv[1]), fabsf(q.mv[2])));
+    b = max_nan(b, mv * sc.p);
+    if (q.force) b = max_nan(b, q.a * sc.f);
   }
   return b * kWmax;
+}
+// The size of a force-like particle's A (K u): not finite if any term is not.
+__device__ __forceinline__ float force_size(const P2GParticle& q) {
+  float sum = 0.0f;
+#pragma unroll
+  for (int r = 0; r < 3; r++) sum += fabsf(q.A[r][0]) + fabsf(q.A[r][1]) + fabsf(q.A[r][2]);
+  return q.force ? sum : 0.0f;
 }
 
 // The per-lane factors of one particle's contributions in stencil row
@@ -1258,12 +1270,15 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
     for (int r = 0; r < 3; r++) st.mvs[r] = q.mv[r] * sc.p;
   }
   if (have) {
-    const float bound = fix ? fix_bound<KIND>(q, sc) : 0.0f;
-    const bool fast = !fix || bound < kFastLimit;  // false for a non-finite particle as well
+    // what is not finite stays out of the records: cell_sums multiplies the
+    // particle that shares a record by zero weights, be it of the cell beside, of an
+    // item before or of another scene. It is scattered straight to its own nodes,
+    // where what is not finite counts as nothing (K u: stays what it is). A NaN position
+    // lies in cell 0 of the grid
+    const float bound = fix ? fix_bound<KIND>(q, sc) : force_size(q);
+    const bool fast = bound < (fix ? kFastLimit : INFINITY);  // false for NaN and infinite values as well
     const int lx = base[0] - 1 - ox, ly = base[1] - 1 - oy, lz = base[2] - 1 - oz;
     const bool inside = lx >= 0 && ly >= 0 && lz >= 0 && lx < kCellsPerAxis && ly < kCellsPerAxis && lz < kCellsPerAxis;
-    // a NaN position (cell 0 of the grid) stays out of the records, which pair
-    // particles of neighbouring cells
     const bool finite_w = w.wx[1] + w.wy[1] + w.wz[1] < 4.0f;
     if (inside && fast && finite_w) {
       st.cell = lx + kCellsPerAxis * ly + kCellsPerAxis * kCellsPerAxis * lz;
@@ -1271,7 +1286,7 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
       tile_bound = bound;
     } else {
       // the particle drifted out of its home block's tile since the last
-      // binning, or outgrew the fast path's range
+      // binning, outgrew the fast path's range or is not finite
       if (!inside) atomicAdd(&S.counters[CNT_FALLBACK], 1);
       far = fast && finite_w ? kFarFast : kFarWide;
       if (KIND != kP2gForce && far == kFarWide) atomicAdd(&S.fix->wide, 1u);

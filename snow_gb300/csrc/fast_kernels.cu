@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
     {  // the magnitudes the next step's scales are chosen from (per warp, then per CTA)
       const unsigned bm = __reduce_max_sync(0xffffffffu, have ? __float_as_uint(fabsf(q.m)) : 0u);
       const unsigned bv = __reduce_max_sync(0xffffffffu, __float_as_uint(rec_v));
-      const unsigned ba = __reduce_max_sync(0xffffffffu, __float_as_uint(q.a));
+      const unsigned ba = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(q.a, 0.0f)));  // (0 for NaN)
       if (lane == 0) {
         atomicMax(&sh.seen[0], bm);
         atomicMax(&sh.seen[1], bv);

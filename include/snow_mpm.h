@@ -370,12 +370,24 @@ snow_status snow_server_drain(snow_server* srv, double timeout_s);
  * work overlaps on the GPU (other streams, other host threads) race and must
  * be ordered by the caller; every call clears the scratch it relies on, so
  * nothing carried over from an earlier call matters. The sort is one
- * cooperative launch (at most 128 blocks). The first call in
+ * cooperative launch (at most 128 blocks), whose blocks wait for one another
+ * for at most one second at a time: if the GPU is taken away for longer, the sort
+ * stops, its outputs (and keys sorted in place) hold nothing to be relied on, and
+ * snow_sort_static_check says so. The first call in
  * a device context (and the first after that device's context was reset)
  * looks up the array's device address; make that first call before any
  * stream capture. Returns SNOW_ECUDA if a CUDA call fails. */
 snow_status snow_sort_keys_static(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm, size_t n,
                                   int key_bits, void* stream);
+/* Waits for `stream` and returns SNOW_ETIMEDOUT if a sort queued on the current
+ * device since the last check gave up a wait (SNOW_OK otherwise; SNOW_ECUDA if a
+ * CUDA call fails, and while the stream is capturing). */
+snow_status snow_sort_static_check(void* stream);
+/* snow_sort_keys_static with the waits' limit in nanoseconds (0: one second);
+ * `absent` (0 in normal use) makes every wait expect as many more arrivals than
+ * there are blocks, so that it runs out (a test of the timeout path). */
+snow_status snow_sort_keys_static_limited(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm, size_t n,
+                                          int key_bits, void* stream, uint32_t wait_ns, uint32_t absent);
 
 /* Batched stepping of many independent scenes (all SNOW_MODE_FAST): one
  * launch per phase covers every scene, the whole step is a CUDA graph. */

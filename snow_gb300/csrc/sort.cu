@@ -588,15 +588,23 @@ constexpr int kOneSplit = kOneThreads / 256;          // threads per digit where
 constexpr int kOneCtas = (int)(kStaticKeys / kOneTile);  // 128: all resident at once
 static_assert(kStaticKeys % kOneTile == 0, "whole tiles");
 constexpr int kOneBarriers = 8;                       // two per pass, four passes
-// layout: [digit counts kOneCtas x 256][barrier counters]
-constexpr size_t kStaticWords = (size_t)kOneCtas * 256 + kOneBarriers;
+// layout: [digit counts kOneCtas x 256][barrier counters][CTAs whose wait ran out, until it is read]
+constexpr size_t kStaticWords = (size_t)kOneCtas * 256 + kOneBarriers + 1;
 
 __device__ __align__(256) uint32_t g_sort_scratch[kStaticWords];
 
 // All CTAs of the (cooperative) launch meet at counter `bar`, zero before it.
-// The wait is bounded like the copy waits; a CTA that runs out of it returns
-// false and does no more work.
-__device__ __forceinline__ bool grid_meet(uint32_t* bar) {
+// The wait is bounded like the copy waits; a CTA that runs out of it is counted,
+// returns false and does no more work. LIMITED: with the limit and the arrivals of
+// `wait`, in an instantiation of its own: as parameters of the one in use they
+// took 262,144 keys from 47 to 54 us (its loads are scheduled otherwise).
+constexpr int kSortExpired = kOneCtas * 256 + kOneBarriers;
+struct SortWait {
+  uint32_t limit_ns;
+  uint32_t absent;  // arrivals waited for beyond those of the CTAs (a test of the timeout path)
+};
+template <bool LIMITED>
+__device__ __forceinline__ bool grid_meet(uint32_t* bar, const SortWait& wait) {
   __shared__ bool met;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -604,9 +612,10 @@ __device__ __forceinline__ bool grid_meet(uint32_t* bar) {
     atomicAdd(bar, 1u);
     const uint64_t t0 = global_ns();
     met = true;
-    for (uint32_t round = 0; *(volatile uint32_t*)bar < gridDim.x; round++)
-      if ((round & 63u) == 63u && (round > (1u << 26) || global_ns() - t0 > (uint64_t)kDefaultWaitNs)) {
+    for (uint32_t round = 0; *(volatile uint32_t*)bar < gridDim.x + (LIMITED ? wait.absent : 0u); round++)
+      if ((round & 63u) == 63u && (round > (1u << 26) || global_ns() - t0 > (uint64_t)(LIMITED ? wait.limit_ns : kDefaultWaitNs))) {
         met = false;
+        atomicAdd(&g_sort_scratch[kSortExpired], 1u);
         break;
       }
     __threadfence();
@@ -615,8 +624,10 @@ __device__ __forceinline__ bool grid_meet(uint32_t* bar) {
   return met;
 }
 
+template <bool LIMITED>
 __global__ void __launch_bounds__(kOneThreads) k_sort_one(const uint32_t* keys, uint32_t* sorted, uint32_t* perm,
-                                                          uint32_t n, int passes, uint32_t* hist, uint32_t* bars) {
+                                                          uint32_t n, int passes, uint32_t* hist, uint32_t* bars,
+                                                          const SortWait wait) {
   __shared__ uint32_t wcount[kOneWarps][256];
   __shared__ uint32_t part[kOneSplit][256], ahead[kOneSplit][256], wsum[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -665,7 +676,7 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(const uint32_t* keys, 
       tile += part[k][digit];
     }
     if (split == 0) __stcg(hist + blockIdx.x * 256 + digit, tile);
-    if (!grid_meet(bars + 2 * pass)) return;
+    if (!grid_meet<LIMITED>(bars + 2 * pass, wait)) return;
     uint32_t total = 0, before = 0;
 #pragma unroll 8
     for (int c = split; c < (int)gridDim.x; c += kOneSplit) {
@@ -714,7 +725,7 @@ __global__ void __launch_bounds__(kOneThreads) k_sort_one(const uint32_t* keys, 
       __stcg(sorted + pos, key[j]);
       __stcg(perm + pos, val[j]);
     }
-    if (pass + 1 < passes && !grid_meet(bars + 2 * pass + 1)) return;
+    if (pass + 1 < passes && !grid_meet<LIMITED>(bars + 2 * pass + 1, wait)) return;
   }
 }
 
@@ -778,12 +789,8 @@ bool ranges_overlap(const void* a, const void* b, size_t n) {
   return x < y + bytes && y < x + bytes;
 }
 
-}  // namespace
-}  // namespace snow
-
-extern "C" snow_status snow_sort_keys_static(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm, size_t n,
-                                             int key_bits, void* stream) {
-  using namespace snow;
+snow_status sort_static(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm, size_t n, int key_bits, void* stream,
+                        const SortWait* limited) {
   if (!keys || !sorted_keys || !perm || key_bits < 1 || key_bits > 32) return SNOW_EINVAL;
   if (n > kStaticKeys) return SNOW_EINVAL;
   if (n == 0) return SNOW_OK;
@@ -801,14 +808,48 @@ extern "C" snow_status snow_sort_keys_static(const uint32_t* keys, uint32_t* sor
   uint32_t* bars = scratch + (size_t)kOneCtas * 256;
   uint32_t count = (uint32_t)n;
   int passes = (key_bits + 7) / 8;
-  void* args[] = {&keys, &sorted_keys, &perm, &count, &passes, &scratch, &bars};
+  SortWait wait = limited ? *limited : SortWait{};
+  const void* kernel = limited ? reinterpret_cast<const void*>(&k_sort_one<true>) : reinterpret_cast<const void*>(&k_sort_one<false>);
+  void* args[] = {&keys, &sorted_keys, &perm, &count, &passes, &scratch, &bars, &wait};
   const unsigned ctas = (unsigned)((n + kOneTile - 1) / kOneTile);
   if (cudaMemsetAsync(bars, 0, kOneBarriers * sizeof(uint32_t), st) != cudaSuccess ||
-      cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_sort_one), dim3(ctas), dim3(kOneThreads), args, 0, st) !=
-          cudaSuccess) {
+      cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kOneThreads), args, 0, st) != cudaSuccess) {
     cudaGetLastError();
     return SNOW_ECUDA;
   }
   if (cudaGetLastError() != cudaSuccess) return SNOW_ECUDA;
   return SNOW_OK;
+}
+
+}  // namespace
+}  // namespace snow
+
+extern "C" snow_status snow_sort_keys_static(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm, size_t n,
+                                             int key_bits, void* stream) {
+  return snow::sort_static(keys, sorted_keys, perm, n, key_bits, stream, nullptr);
+}
+
+extern "C" snow_status snow_sort_keys_static_limited(const uint32_t* keys, uint32_t* sorted_keys, uint32_t* perm,
+                                                     size_t n, int key_bits, void* stream, uint32_t wait_ns,
+                                                     uint32_t absent) {
+  const snow::SortWait wait = {wait_ns ? wait_ns : snow::kDefaultWaitNs, absent};
+  return snow::sort_static(keys, sorted_keys, perm, n, key_bits, stream, &wait);
+}
+
+extern "C" snow_status snow_sort_static_check(void* stream) {
+  using namespace snow;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  uint32_t* scratch = nullptr;
+  uint32_t expired = 0;
+  cudaError_t e = static_scratch(&scratch);
+  uint32_t* word = scratch + kSortExpired;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&expired, word, sizeof expired, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && expired) e = cudaMemsetAsync(word, 0, sizeof expired, st);
+  if (e == cudaSuccess && expired) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return SNOW_ECUDA;
+  }
+  return expired ? SNOW_ETIMEDOUT : SNOW_OK;
 }

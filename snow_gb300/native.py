@@ -32,6 +32,7 @@ EXPORTS = [
     "snow_server_submit", "snow_server_poll", "snow_server_fetch", "snow_server_stats", "snow_server_drain",
     "snow_scene_set_tuning", "snow_batch_set_tuning", "snow_ctx_set_graphs", "snow_scene_stats_enqueue",
     "snow_ctx_stats_read", "snow_scene_solver_report", "snow_scene_check", "snow_scene_set_wait_limit",
+    "snow_sort_keys_static_limited", "snow_sort_static_check",
 ]
 SORT_STATIC_MAX_KEYS = 262144  # SNOW_SORT_STATIC_MAX_KEYS
 
@@ -163,6 +164,8 @@ def load(path: str = LIB_PATH):
     L.snow_batch_set_tuning.argtypes = [vp, C.POINTER(SnowTuning)]
     L.snow_scene_set_tuning.argtypes = [vp, C.POINTER(SnowTuning)]
     L.snow_sort_keys_static.argtypes = [vp, vp, vp, sz, C.c_int, vp]
+    L.snow_sort_keys_static_limited.argtypes = [vp, vp, vp, sz, C.c_int, vp, C.c_uint32, C.c_uint32]
+    L.snow_sort_static_check.argtypes = [vp]
     L.snow_scene_check.argtypes = [vp]
     L.snow_scene_set_wait_limit.argtypes = [vp, C.c_uint32, C.c_uint32]
     L.snow_server_create.argtypes = [C.POINTER(SnowServerConfig), C.POINTER(vp)]

@@ -244,12 +244,18 @@ snow_status snow_scene_stats_enqueue(snow_scene* s, int slot);
 snow_status snow_ctx_stats_read(snow_ctx* ctx, int slot, snow_stats* out);
 size_t snow_scene_size(const snow_scene* s);
 
-/* Particle -> cell binning as used by the FAST path: per-particle block-major
+/* Particle -> cell binning of the FAST path: per-particle block-major
  * cell key (block (i>>2, j>>2, k>>2) numbered x fastest, times 64, plus
  * (i&3) + 4(j&3) + 16(k&3), cell = trunc((x - grid_pos)/h) clamped to the
  * grid) and the stable sort permutation (perm[k] = particle at rank k).
  * Computed on the device from the current positions. */
 snow_status snow_scene_cell_keys(snow_scene* s, uint32_t* keys, uint32_t* perm);
+
+/* The order in which a FAST scene's particles lie on the device: order[k] = upload
+ * index of the particle stored at place k. An upload stores them as they come; every
+ * binning (at init and every few steps) reorders them as the stable sort of the
+ * stored particles by cell key does. Waits for the stream. */
+snow_status snow_scene_storage_order(snow_scene* s, uint32_t* order);
 
 snow_status snow_scene_phase_times(snow_scene* s, snow_phase_times* out, int reset);
 

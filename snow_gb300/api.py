@@ -238,6 +238,12 @@ class SimScene:
         self.ctx.check(self.L.snow_scene_cell_keys(self.h, N.ptr(keys, C.c_uint32), N.ptr(perm, C.c_uint32)))
         return keys, perm
 
+    def storage_order(self) -> np.ndarray:
+        """Upload index of the particle stored at each place."""
+        order = np.zeros(self.n, np.uint32)
+        self.ctx.check(self.L.snow_scene_storage_order(self.h, N.ptr(order, C.c_uint32)))
+        return order
+
     def phase_times(self, reset: bool = False) -> dict:
         t = N.SnowPhaseTimes()
         self.ctx.check(self.L.snow_scene_phase_times(self.h, C.byref(t), int(bool(reset))))

@@ -1496,6 +1496,16 @@ snow_status snow_scene_cell_keys(snow_scene* s, uint32_t* keys, uint32_t* perm) 
   return SNOW_OK;
 }
 
+snow_status snow_scene_storage_order(snow_scene* s, uint32_t* order) {
+  if (!s || !order) return SNOW_EINVAL;
+  snow_ctx* ctx = s->ctx;
+  if (s->mode != SNOW_MODE_FAST) return fail(ctx, SNOW_EUNSUPPORTED, "binning runs in SNOW_MODE_FAST");
+  if (!s->uploaded) return fail(ctx, SNOW_ESTATE, "snow_scene_storage_order before upload");
+  CK(cudaMemcpyAsync(order, s->sd.pid, s->n * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return SNOW_OK;
+}
+
 snow_status snow_scene_phase_times(snow_scene* s, snow_phase_times* out, int reset) {
   if (!s || !out) return SNOW_EINVAL;
   *out = s->times;

@@ -212,8 +212,9 @@ __global__ void k_keys(const SceneDev* __restrict__ sd, uint32_t* __restrict__ k
 // The order of the stable sort by cell key, in six kernels over all scenes of
 // a step instead of the radix sort's passes (five launches each, three or four
 // passes a scene): the particles are counted per grid block, the blocks' starts
-// are scanned, the particle indices are put into their blocks, one CTA per block
-// orders its few hundred by (cell, index), and the streams are moved. Bound by
+// are scanned, the particle indices are put into their blocks, a group of threads
+// per block orders its few hundred by (cell, index) (a CTA's groups together those
+// of a crowded block), and the streams are moved. Bound by
 // launches in small scenes and by the 184 bytes a particle that the streams'
 // move reads and writes in large ones. A binning of 32k / 262k / 1M particles
 // took 67 / 81 / 126 us in 20 launches, now 20 / 28 / 69 in 6.
@@ -380,90 +381,239 @@ __global__ void __launch_bounds__(256) k_bin_place(const WorkSpace w) {
   }
 }
 
-// One CTA per occupied block (by its first work item): its particle indices in
-// the order of their cells, and of the indices within a cell (a cell of more
-// than kMaxRanked keeps the order it came in). The moves that follow have a
-// thread per particle: done here, by the few hundred threads of a block's CTA,
-// they took 69 us at 1M particles against 35.
+// A group of 128 threads per occupied block (by its first work item): its particle
+// indices in the order of their cells, and of the indices within a cell. The moves
+// that follow have a thread per particle: done here, by the few hundred threads of a
+// block's CTA, they took 69 us at 1M particles against 35. A particle's place in its
+// cell is counted against all the cell's others; where a block of more than
+// kCellThreads * kCellHeld particles has a cell of more than kMaxRanked, whose square
+// that would cost, and where it has more than kMaxBlock, the CTA's groups together
+// sort the whole block afterwards (order_crowded).
 constexpr int kCellThreads = 128;
+constexpr int kCellGroups = 4;
+constexpr int kCellCta = kCellThreads * kCellGroups;
+constexpr int kCellCtas = 3;  // per SM (40 registers)
 constexpr int kCellHeld = 6;  // particles a thread holds in registers: blocks up to 768 are read once
 constexpr int kMaxRanked = 128;
-__global__ void __launch_bounds__(kCellThreads) k_bin_cells(const WorkSpace w, int in_step) {
+constexpr int kMaxBlock = 4096;
+struct CellGroup {
+  int count[64], start[64], cursor[64];
+  uint32_t idx[kCellThreads * kCellHeld];
+};
+struct CrowdCounts {
+  uint32_t next[4 * 256];                   // [digits + 1][values]: where the next index of each value goes
+  uint32_t warps[kCellCta / 32 * 256];      // [warps][values]: the warps' counts in a tile, then their starts
+};
+
+// The n particle indices at S.bidx[n0 ..] into the order of their cells, and of the
+// indices within a cell: a stable radix sort by the CTA, three digits of the index
+// (five, beyond 2^24 particles) and then the cell, between bidx and brank (whose
+// places are no longer needed). Bound by the latency of its reads and of the counts,
+// and by one SM's scattered writes. A binning of 3.2M particles in 1,000 blocks with
+// 200 to a cell takes 365 us, of 1M in 16 blocks 734, in one 9,230 (without any order
+// in such cells 263, 688 and 7,980; by one group of 128 threads 465, 1,760 and 27,000;
+// in a kernel of its own with 1,024 threads 351, 505 and 7,190, but then all binnings
+// take a launch more: 20 steps of 300k with a binning in most 3.08 ms, 3.095).
+constexpr int kCrowdedHeld = 8;  // indices of a thread under way
+__device__ __noinline__ void order_crowded(CrowdCounts& sh, const SceneDev& S, int n0, int n) {
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int bits = 32 - __clz(S.n - 1), digits = bits <= 24 ? 3 : 5, width = max(6, (bits + digits - 1) / digits);
+  const int values = 1 << width;  // of a digit: at most 256, and 128 where there are five
+  auto digit = [&](uint32_t p, int k) { return k == digits ? S.bkey[p] & 63u : p >> (k * width) & (uint32_t)(values - 1); };
+  for (int k = threadIdx.x; k < (digits + 1) * values; k += kCellCta) sh.next[k] = 0u;
+  __syncthreads();
+  for (int t = 0; t < n; t += kCellCta * kCrowdedHeld) {  // all digits are counted in one read
+    uint32_t p[kCrowdedHeld];
+#pragma unroll
+    for (int j = 0; j < kCrowdedHeld; j++) {
+      const int i = t + j * kCellCta + (int)threadIdx.x;
+      p[j] = i < n ? S.bidx[n0 + i] : ~0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kCrowdedHeld; j++) {
+      const uint32_t in = __ballot_sync(0xffffffffu, p[j] != ~0u);
+      if (p[j] == ~0u) continue;
+      for (int k = 0; k <= digits; k++) {  // often one value for the whole warp
+        const uint32_t d = digit(p[j], k);
+        int same;
+        __match_all_sync(in, d, &same);
+        if (!same)
+          atomicAdd(&sh.next[k * values + d], 1u);
+        else if (lane == 0)
+          atomicAdd(&sh.next[k * values + d], (uint32_t)__popc(in));
+      }
+    }
+  }
+  __syncthreads();
+  for (int k = wi; k <= digits; k += (kCellCta / 32)) {  // a warp scans a digit's counts: where its values start
+    uint32_t run = 0u;
+    for (int v = k * values + lane; v < (k + 1) * values; v += 32) {
+      const uint32_t c = sh.next[v];
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+      }
+      sh.next[v] = run + incl - c;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  }
+  __syncthreads();
+  uint32_t* const mine = sh.warps + wi * values;
+#pragma unroll 1
+  for (int pass = 0; pass <= digits; pass++) {  // an even number of passes: the last ends in bidx
+    const uint32_t* const from = (pass & 1 ? S.brank : S.bidx) + n0;
+    uint32_t* const to = (pass & 1 ? S.bidx : S.brank) + n0;
+    uint32_t* const base = sh.next + pass * values;
+    const int mine0 = wi * 32 * kCrowdedHeld + lane;  // the warp's stretch of a tile
+    for (int t = 0; t < n; t += kCellCta * kCrowdedHeld) {
+      uint32_t p[kCrowdedHeld], d[kCrowdedHeld], rank[kCrowdedHeld];
+#pragma unroll
+      for (int j = 0; j < kCrowdedHeld; j++) {
+        const int i = t + mine0 + 32 * j;
+        p[j] = i < n ? from[i] : ~0u;
+      }
+#pragma unroll
+      for (int j = 0; j < kCrowdedHeld; j++) d[j] = p[j] != ~0u ? digit(p[j], pass) : ~0u;
+      for (int v = lane; v < values; v += 32) mine[v] = 0u;
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kCrowdedHeld; j++) {  // stable within the stretch
+        const uint32_t peers = __match_any_sync(0xffffffffu, d[j]), below = peers & ((1u << lane) - 1u);
+        const uint32_t before = d[j] != ~0u ? mine[d[j]] : 0u;
+        __syncwarp();
+        if (d[j] != ~0u && below == 0u) mine[d[j]] = before + __popc(peers);
+        __syncwarp();
+        rank[j] = before + __popc(below);
+      }
+      __syncthreads();
+      for (int v = threadIdx.x; v < values; v += kCellCta) {  // the warps' counts become their starts
+        uint32_t at = base[v];
+#pragma unroll
+        for (int k = 0; k < (kCellCta / 32); k++) {
+          const uint32_t c = sh.warps[k * values + v];
+          sh.warps[k * values + v] = at;
+          at += c;
+        }
+        base[v] = at;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kCrowdedHeld; j++)
+        if (d[j] != ~0u) to[mine[d[j]] + rank[j]] = p[j];
+      __syncthreads();
+    }
+  }
+}
+
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kCellThreads) : "memory");
+}
+__global__ void __launch_bounds__(kCellCta, kCellCtas) k_bin_cells(const WorkSpace w, int in_step) {
   chain_next();
   chain_wait();
-  __shared__ int count[64], start[64], cursor[64];
-  __shared__ uint32_t sidx[kCellThreads * kCellHeld];
+  __shared__ union {
+    CellGroup group[kCellGroups];
+    CrowdCounts crowd;
+  } sh;
+  __shared__ int crowded;
+  if (threadIdx.x == 0) crowded = 0;
+  __syncthreads();
+  const int g = threadIdx.x / kCellThreads, tid = threadIdx.x % kCellThreads;
+  CellGroup& cg = sh.group[g];
+  auto leave = [&](const SceneDev& S, int n0) {  // a block to order_crowded
+    S.bskey[n0] |= 0x80000000u;
+    crowded = 1;
+  };
   const int total = w.items[w.nscenes];
-  for (int u = blockIdx.x; u < total; u += gridDim.x) {
+  for (int u = blockIdx.x * kCellGroups + g; u < total; u += gridDim.x * kCellGroups) {
     const int s = scene_of(w.items, w.nscenes, u);
     const SceneDev& S = w.scenes[s];
-    if (in_step && u == w.items[s] && threadIdx.x == 0) S.counters[CNT_BINNED] = 1;
+    if (in_step && u == w.items[s] && tid == 0) S.counters[CNT_BINNED] = 1;
     const int4 it = S.items[u - w.items[s]];
     const int n0 = S.bstart[it.x], n = S.bend[it.x] - n0;
-    if (it.y != n0) continue;  // uniform across the CTA
+    if (it.y != n0) continue;  // uniform across the group
+    if (n > kMaxBlock) {
+      if (tid == 0) leave(S, n0);
+      continue;
+    }
     const bool small = n <= kCellThreads * kCellHeld;
     uint32_t p[kCellHeld];
     int c[kCellHeld];
-    if (threadIdx.x < 64) count[threadIdx.x] = 0;
-    __syncthreads();
+    if (tid < 64) cg.count[tid] = 0;
+    group_sync(g);
     if (small) {
 #pragma unroll
       for (int k = 0; k < kCellHeld; k++) {
-        const int i = k * kCellThreads + (int)threadIdx.x;
+        const int i = k * kCellThreads + tid;
         if (i < n) {
           p[k] = S.bidx[n0 + i];
           c[k] = (int)(S.bskey[n0 + i] & 63u);
-          atomicAdd(&count[c[k]], 1);
+          atomicAdd(&cg.count[c[k]], 1);
         }
       }
     } else {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&count[S.bskey[n0 + i] & 63u], 1);
+      for (int i = tid; i < n; i += kCellThreads) atomicAdd(&cg.count[S.bskey[n0 + i] & 63u], 1);
     }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      const int c0 = count[2 * threadIdx.x], c1 = count[2 * threadIdx.x + 1];
+    group_sync(g);
+    bool crowd = false;
+    if (tid < 32) {
+      const int c0 = cg.count[2 * tid], c1 = cg.count[2 * tid + 1];
       int incl = c0 + c1;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)threadIdx.x >= o) incl += v;
+        if (tid >= o) incl += v;
       }
       const int at = incl - c0 - c1;
-      start[2 * threadIdx.x] = cursor[2 * threadIdx.x] = at;
-      start[2 * threadIdx.x + 1] = cursor[2 * threadIdx.x + 1] = at + c0;
+      cg.start[2 * tid] = cg.cursor[2 * tid] = at;
+      cg.start[2 * tid + 1] = cg.cursor[2 * tid + 1] = at + c0;
     }
-    __syncthreads();
-    if (small) {
+    if (!small) {
+      const int most = __reduce_max_sync(0xffffffffu, max(cg.count[2 * (tid & 31)], cg.count[2 * (tid & 31) + 1]));
+      crowd = most > kMaxRanked;  // uniform across the group
+    }
+    group_sync(g);
+    if (crowd) {
+      if (tid == 0) leave(S, n0);
+    } else if (small) {
 #pragma unroll
       for (int k = 0; k < kCellHeld; k++)
-        if (k * kCellThreads + (int)threadIdx.x < n) sidx[atomicAdd(&cursor[c[k]], 1)] = p[k];
-      __syncthreads();
+        if (k * kCellThreads + tid < n) cg.idx[atomicAdd(&cg.cursor[c[k]], 1)] = p[k];
+      group_sync(g);
 #pragma unroll
       for (int k = 0; k < kCellHeld; k++) {
-        if (k * kCellThreads + (int)threadIdx.x >= n) break;
-        const int a = start[c[k]], m = count[c[k]];
+        if (k * kCellThreads + tid >= n) break;
+        const int a = cg.start[c[k]], m = cg.count[c[k]];
         int r = 0;
-        for (int j = a; j < a + m; j++) r += sidx[j] < p[k];
+        for (int j = a; j < a + m; j++) r += cg.idx[j] < p[k];
         S.bidx[n0 + a + r] = p[k];
       }
     } else {
       uint32_t* far = S.brank + n0;  // the places are no longer needed
-      for (int i = threadIdx.x; i < n; i += blockDim.x)
-        far[atomicAdd(&cursor[S.bskey[n0 + i] & 63u], 1)] = S.bidx[n0 + i];
-      __syncthreads();
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      for (int i = tid; i < n; i += kCellThreads) far[atomicAdd(&cg.cursor[S.bskey[n0 + i] & 63u], 1)] = S.bidx[n0 + i];
+      group_sync(g);
+      for (int i = tid; i < n; i += kCellThreads) {
         const uint32_t q = far[i];
-        const int cell = (int)(S.bkey[q] & 63u), a = start[cell], m = count[cell];
-        int r = i - a;
-        if (m <= kMaxRanked) {
-          r = 0;
-          for (int j = a; j < a + m; j++) r += far[j] < q;
-        }
+        const int cell = (int)(S.bkey[q] & 63u), a = cg.start[cell], m = cg.count[cell];
+        int r = 0;
+        for (int j = a; j < a + m; j++) r += far[j] < q;
         S.bidx[n0 + a + r] = q;
       }
     }
-    __syncthreads();
+    group_sync(g);
   }
+  __syncthreads();
+  if (!crowded) return;
+  for (int k = 0; k < kCellGroups; k++)  // the groups' blocks again, those that were left
+    for (int u = blockIdx.x * kCellGroups + k; u < total; u += gridDim.x * kCellGroups) {
+      const int s = scene_of(w.items, w.nscenes, u);
+      const SceneDev& S = w.scenes[s];
+      const int4 it = S.items[u - w.items[s]];
+      const int n0 = S.bstart[it.x], n = S.bend[it.x] - n0;
+      if (it.y == n0 && S.bskey[n0] >> 31 != 0u) order_crowded(sh.crowd, S, n0, n);
+    }
 }
 
 // The particle streams into the binned copies, in the order bidx.
@@ -556,8 +706,8 @@ void fast_bin_scenes(const WorkSpace& w, bool copy_back, bool chained, cudaStrea
   launch_after(chain, k_bin_reduce, grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st, w);
   launch_after(chain, k_bin_scan, grid_for((size_t)w.total_chunks, 1, 8), kBinChunk / 2, 0, st, w);
   launch_after(chain, k_bin_place, grid_for(n, 256, 8), 256, 0, st, w);
-  // an occupied block holds some hundred particles; at most one CTA for each 64
-  launch_after(chain, k_bin_cells, grid_for(n, 64, 16), kCellThreads, 0, st, w, copy_back ? 0 : 1);
+  // an occupied block holds some hundred particles; at most a group for each 64
+  launch_after(chain, k_bin_cells, grid_for(n, 64 * kCellGroups, kCellCtas), kCellCta, 0, st, w, copy_back ? 0 : 1);
   launch_after(chain, k_bin_move, grid_for(n, 256, 8), 256, 0, st, w);
   if (copy_back) launch_after(chain, k_bin_back, grid_for(n, 256, 8), 256, 0, st, w);
 }

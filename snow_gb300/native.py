@@ -32,7 +32,7 @@ EXPORTS = [
     "snow_server_submit", "snow_server_poll", "snow_server_fetch", "snow_server_stats", "snow_server_drain",
     "snow_scene_set_tuning", "snow_batch_set_tuning", "snow_ctx_set_graphs", "snow_scene_stats_enqueue",
     "snow_ctx_stats_read", "snow_scene_solver_report", "snow_scene_check", "snow_scene_set_wait_limit",
-    "snow_sort_keys_static_limited", "snow_sort_static_check",
+    "snow_sort_keys_static_limited", "snow_sort_static_check", "snow_scene_storage_order",
 ]
 SORT_STATIC_MAX_KEYS = 262144  # SNOW_SORT_STATIC_MAX_KEYS
 
@@ -154,6 +154,7 @@ def load(path: str = LIB_PATH):
     L.snow_scene_size.argtypes = [vp]
     L.snow_scene_size.restype = sz
     L.snow_scene_cell_keys.argtypes = [vp, up, up]
+    L.snow_scene_storage_order.argtypes = [vp, up]
     L.snow_scene_phase_times.argtypes = [vp, C.POINTER(SnowPhaseTimes), C.c_int]
     L.snow_scene_solver_report.argtypes = [vp, C.POINTER(SnowSolverReport)]
     L.snow_batch_create.argtypes = [vp, C.POINTER(vp), C.c_int, C.POINTER(vp)]

@@ -81,14 +81,18 @@ __device__ __forceinline__ void form_prefixes(const SceneDev* __restrict__ scene
   }
 }
 
+// rigidAdvance.glsl:14-18, by one warp.
+__device__ __forceinline__ void advance_colliders(const SceneDev& S, int lane) {
+  for (int i = lane; i < S.ncoll; i += 32)
+    for (int k = 0; k < 3; k++) S.coll[i].pos[k] = S.coll[i].pos[k] + S.dt * S.coll[i].vel[k];
+}
+
 // The start of a step for scene S, by one warp: counters reset, the magnitudes
 // moved on and the scales of this step's P2G formed from them, colliders
 // advanced, the solve's scalars cleared.
 __device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool binned) {
   const int lane = threadIdx.x & 31;
-  if (rigid)  // rigidAdvance.glsl:14-18
-    for (int i = lane; i < S.ncoll; i += 32)
-      for (int k = 0; k < 3; k++) S.coll[i].pos[k] = S.coll[i].pos[k] + S.dt * S.coll[i].vel[k];
+  if (rigid) advance_colliders(S, lane);
   if (lane == 0) {
     S.counters[CNT_OVERFLOW] = 0;
     S.counters[CNT_WORK] = 0;
@@ -116,13 +120,9 @@ __device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool 
   }
 }
 
-// The same alone (per-kernel dispatches of the rigid advance).
-__global__ void k_begin_step(const SceneDev* __restrict__ scenes, int nscenes, int rigid) {
-  const int s = blockIdx.x;
-  if (s >= nscenes) return;
-  begin_scene(scenes[s], rigid != 0, false);
-  if (threadIdx.x == 0) scenes[s].counters[CNT_ACTIVE] = 0;
-}
+// The rigid advance alone (per-kernel dispatches): it starts no step, so what the
+// start of one moves on (the magnitudes, the solve's count of steps to skip) stays.
+__global__ void k_rigid(const SceneDev* __restrict__ sd) { advance_colliders(*sd, threadIdx.x); }
 
 __global__ void k_gather_counters(const SceneDev* __restrict__ scenes, int nscenes, int* out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nscenes * kCounterStride; i += gridDim.x * blockDim.x)
@@ -997,9 +997,7 @@ int num_sms() {
 }
 
 
-void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st) {
-  if (nscenes > 0) k_begin_step<<<nscenes, 32, 0, st>>>(scenes, nscenes, rigid ? 1 : 0);
-}
+void fast_rigid(const SceneDev* sd_dev, cudaStream_t st) { k_rigid<<<1, 32, 0, st>>>(sd_dev); }
 
 void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStream_t st) {
   const int n = nscenes * kCounterStride;

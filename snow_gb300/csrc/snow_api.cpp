@@ -1098,7 +1098,7 @@ snow_status snow_dispatch(snow_scene* s, int kernel, double dt) {
   if (r) return r;
   switch (kernel) {
     case SNOW_K_RIGID_ADVANCE:
-      if (s->ncoll > 0) fast_begin_step(s->sd_dev, 1, true, st);
+      if (s->ncoll > 0) fast_rigid(s->sd_dev, st);
       break;
     case SNOW_K_G_RESET:  // discard pending P2G sums
       if (s->p2g_ready) {

@@ -254,17 +254,17 @@ constexpr int kFitRounds = 3;
 // Whether a binning of n particles over `ctas` CTAs looks for one.
 inline bool fits_items(long long n, int ctas) { return n <= (long long)kFitRounds * ctas * size_choice(kSizeChoices - 1); }
 constexpr int kBinChunk = 512;  // grid blocks per chunk of the binning's scan
-// Start of a step alone: resets the per-step counters and, with `rigid`, moves
-// the colliders by dt * velocity (rigidAdvance.glsl:14-18). A step's compaction
-// does the same in its first CTAs.
-void fast_begin_step(const SceneDev* scenes, int nscenes, bool rigid, cudaStream_t st);
+// Moves a scene's colliders by dt * velocity (rigidAdvance.glsl:14-18). A step's
+// compaction does the same in its first CTAs.
+void fast_rigid(const SceneDev* sd_dev, cudaStream_t st);
 // Copies every scene's counters and FixState into out[s * kCounterStride ...] (mapped
 // pinned memory: a batch reads them one re-binning interval later, without
 // draining the stream).
 void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStream_t st);
-// Flags -> active list and slots; its last CTA then starts the step of every
-// scene (fast_begin_step) and forms the item and active-block prefixes. binned:
-// the step's binning ran before and left the particles in the binned copies.
+// Flags -> active list and slots; its first CTAs start the step of every scene
+// (counters, scales of the step's P2G; rigid: the colliders), and the CTA that takes
+// its slots last forms the item and active-block prefixes. binned: the step's binning
+// ran before and left the particles in the binned copies.
 void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st);
 // P2G of the stored particle state (set-up, per-kernel dispatches), after a
 // pass over the particles that measures the magnitudes its fixed-point

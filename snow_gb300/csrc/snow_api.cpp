@@ -587,6 +587,12 @@ snow_status fast_init(snow_scene* s) {
   snow_status r;
   s->sd.n = (int)s->n;
   if (s->sd.crs) fast_implicit_setup();
+  if (s->p2g_ready) {
+    // the sums of the state before lie in acc, to which the masses would be added
+    fast_enqueue_compact(s, st);
+    fast_enqueue_grid(s, true, false, st);
+    s->p2g_ready = false;
+  }
   if ((r = fast_single_prefix(s))) return r;
   if ((r = push_sd(s))) return r;
   fast_bin(s, st, false);

@@ -1,0 +1,46 @@
+"""A scene that is set up again starts as a new one does: nothing of the state
+before shows."""
+import numpy as np
+import pytest
+
+from snow_gb300 import scenes
+
+gpu = pytest.mark.gpu
+KEYS = ("x", "v", "FE", "Jp", "volume")
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from snow_gb300 import api
+    return api.Context(0)
+
+
+def _scene(seed, n=3000):
+    s = scenes.small_scene(n=n, grid_edge=32, seed=seed, v0=(0.5, -2.0, 0.0))
+    s.v += np.random.default_rng(seed).uniform(-0.5, 0.5, s.v.shape).astype(np.float32)
+    return s
+
+
+def _same(a, b):
+    return all(np.array_equal(a[k], b[k]) for k in KEYS)
+
+
+@gpu
+@pytest.mark.parametrize("how", ["init twice", "mass and volume kernels", "other state", "fewer particles", "after a grid reset"])
+@pytest.mark.parametrize("steps", [0, 5])
+def test_set_up_again_is_a_new_scene(ctx, how, steps):
+    from snow_gb300 import api, native as N
+    s = _scene(621)
+    want = api.SimScene(ctx, s).upload().init().step(s.dt, 7).check().download()
+    first = _scene(622, 4000 if how == "fewer particles" else s.n)
+    g = api.SimScene(ctx, s).upload(first.x, first.v, first.m).init().step(s.dt, steps)
+    if how == "after a grid reset":
+        g.dispatch(N.K_G_RESET, s.dt)
+    g.upload()
+    if how == "mass and volume kernels":
+        g.dispatch(N.K_G_MASS, s.dt).dispatch(N.K_P_VOLUME, s.dt)
+    else:
+        g.init()
+        if how == "init twice":
+            g.init()
+    assert _same(g.step(s.dt, 7).check().download(), want)

@@ -586,7 +586,11 @@ snow_status fast_init(snow_scene* s) {
   cudaStream_t st = ctx->stream;
   snow_status r;
   s->sd.n = (int)s->n;
-  if (s->sd.crs) fast_implicit_setup();
+  if (s->sd.crs) {
+    fast_implicit_setup();
+    // the state before may have left steps to skip
+    CK(cudaMemsetAsync(s->sd.crs, 0, sizeof(CrScalars), st));
+  }
   if (s->p2g_ready) {
     // the sums of the state before lie in acc, to which the masses would be added
     fast_enqueue_compact(s, st);

@@ -1,5 +1,5 @@
 """A scene that is set up again starts as a new one does: nothing of the state
-before shows."""
+before shows (sums not yet consumed, steps the solve may skip)."""
 import numpy as np
 import pytest
 
@@ -44,3 +44,19 @@ def test_set_up_again_is_a_new_scene(ctx, how, steps):
         if how == "init twice":
             g.init()
     assert _same(g.step(s.dt, 7).check().download(), want)
+
+
+@gpu
+def test_a_solve_after_steps_that_skipped_it(ctx):
+    """Snow in free flight skips its solve for up to 240 steps; the state uploaded
+    then does not."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=3000, grid_edge=32, seed=623, young=1.4e7, v0=(0.0, -1.0, 0.0))
+    s.implicit_beta, s.implicit_tolerance, s.implicit_max_iters = 1.0, 1e-5, 30
+    v = np.random.default_rng(624).uniform(-2.0, 2.0, s.v.shape).astype(np.float32)
+    new = api.SimScene(ctx, s).upload(v=v).init().step(s.dt, 1).solver_report()
+    assert new["iterations"] > 0
+    g = api.SimScene(ctx, s).upload().init().step(s.dt, 3)
+    assert g.solver_report()["iterations"] == 0
+    again = g.upload(v=v).init().step(s.dt, 1).solver_report()
+    assert again["iterations"] == new["iterations"]

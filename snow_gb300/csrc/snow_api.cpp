@@ -95,6 +95,7 @@ struct snow_scene {
   bool cnt_pending = false;
   long long fallbacks_seen = 0;
   int steps_at_snapshot = 0;  // steps between the last two snapshots
+  int set_ups = 0;      // of this scene (fast_init)
   int batches = 0;      // batches it is in (counted by their creation)
   bool fitted = false;  // its items were sized for a launch of its own
   int version = 0;
@@ -123,6 +124,7 @@ struct snow_batch {
   int* d_prefix = nullptr;  // the prefixes of `work`, n + 1 entries each
   WorkSpace work{};
   std::vector<int> versions;
+  std::vector<int> set_ups;  // the scenes' when the re-binning state below began
   int steps_since_check = 0;
   int interval = 8;  // re-binning interval in use
   bool interval_set = false;
@@ -622,8 +624,12 @@ snow_status fast_init(snow_scene* s) {
   s->fallbacks_seen = (long long)(unsigned)s->h_cnt[CNT_FALLBACK];
   s->vmax = fix_vmax(s->h_cnt);
   s->interval_dt = -1.0f;
+  s->bin_interval = s->tune.sort_interval;
+  s->clean_checks = 0;
+  s->clean_needed = 8;
   s->steps_since_check = 0;
   s->steps_since_sort = 0;
+  s->set_ups++;
   s->p2g_ready = true;
   return SNOW_OK;
 }
@@ -1670,6 +1676,24 @@ void batch_interval(snow_batch* b, bool leaving) {
   b->interval_set = true;
 }
 
+// At the start of a batch's steps: where scenes have been set up (again) since the
+// last, what the batch knows of their speeds and counters is of the states before.
+// The interval is chosen anew, from the speeds that the set-up measured, and the
+// counters as they are now become what the next look compares with.
+snow_status batch_follow_set_ups(snow_batch* b) {
+  std::vector<int> now;
+  for (snow_scene* s : b->scenes) now.push_back(s->set_ups);
+  if (now == b->set_ups) return SNOW_OK;
+  snow_ctx* ctx = b->ctx;
+  b->set_ups = now;
+  b->interval_set = false;
+  b->steps_since_check = b->steps_at_snapshot = 0;
+  fast_gather_counters(b->d_scenes, (int)b->scenes.size(), b->d_hcnt, ctx->stream);
+  CK(cudaEventRecord(b->cnt_ev, ctx->stream));
+  b->cnt_pending = true;
+  return SNOW_OK;
+}
+
 void batch_enqueue_step(snow_batch* b, bool bin_all, cudaStream_t st) {
   const int n = (int)b->scenes.size();
   int* items = b->work.items;
@@ -1718,6 +1742,7 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
     s->p2g_ready = true;
   }
   snow_status r = batch_refresh(b, dt);
+  if (!r) r = batch_follow_set_ups(b);
   if (r) return r;
   if (!b->interval_set) batch_interval(b, false);
   for (int i = 0; i < n_steps; i++) {

@@ -1,0 +1,64 @@
+"""A set-up starts the re-binning schedule anew: what was learned of the state before
+(speeds, particles outside their tiles) is not that of the new one. Read from the
+order in which the particles lie, which a binning changes once they have moved."""
+import numpy as np
+import pytest
+
+from snow_gb300 import scenes
+
+gpu = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from snow_gb300 import api
+    return api.Context(0)
+
+
+def _scene(seed, speed):
+    s = scenes.small_scene(n=6000, grid_edge=64, seed=seed, v0=(speed, 0.0, 0.0), center=(0.3, 0.5, 0.5))
+    s.dt, s.gravity, s.young = 1e-3, (0.0, 0.0, 0.0), 1.0
+    return s
+
+
+FAST, SLOW = 6.7, 0.1  # 0.43 of a cell a step (3.4 in eight: another order) and 1/156
+
+
+def _steps_to_binning(g, step, most):
+    order = g.storage_order()
+    for k in range(1, most + 1):
+        step()
+        if not np.array_equal(g.storage_order(), order):
+            return k
+    return most + 1
+
+
+@gpu
+@pytest.mark.parametrize("others", [0, 2])
+def test_a_batch_after_an_upload_of_faster_snow(ctx, others):
+    """A slow batch re-bins every 32 steps; with fast snow, every eight unless particles
+    are seen to leave their tiles: the ninth step is the first to bin."""
+    from snow_gb300 import api
+    slow, fast = _scene(631, SLOW), _scene(632, FAST)
+    sims = [api.SimScene(ctx, slow).upload().init() for _ in range(1 + others)]
+    b = api.Batch(ctx, sims)
+    dts = [slow.dt] * len(sims)
+    b.step(17, dt=dts)  # a look at the counters, and a step
+    g = sims[0]
+    g.upload(fast.x, fast.v, fast.m).init()
+    assert _steps_to_binning(g, lambda: b.step(1, dt=dts), 20) <= 9
+    for g in sims:
+        g.check()
+    b.close()
+
+
+@gpu
+def test_a_scene_with_a_chosen_interval_after_an_upload_of_slower_snow(ctx):
+    """Fast snow brings the interval down from the chosen one, slow snow starts at it:
+    64 steps take 7 binnings (after 8, 16, .. 56)."""
+    from snow_gb300 import api
+    slow, fast = _scene(633, SLOW), _scene(634, FAST)
+    g = api.SimScene(ctx, fast, sort_interval=8).upload().init().step(fast.dt, 30)
+    assert g.phase_times(reset=True)["binnings"] > 10
+    g.upload(slow.x, slow.v, slow.m).init().step(slow.dt, 64).check()
+    assert g.phase_times()["binnings"] == 7

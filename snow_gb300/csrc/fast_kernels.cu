@@ -57,6 +57,7 @@ __device__ __forceinline__ void form_prefixes(const SceneDev* __restrict__ scene
       na = *(volatile int*)&S.counters[CNT_SLOTS];
       S.counters[CNT_ACTIVE] = na;
       S.counters[CNT_SLOTS] = 0;
+      S.counters[CNT_OVERFLOW] = max(0, na - S.pool_cap);
       na = min(na, S.pool_cap);
     }
     int ei = ni, ea = na;
@@ -94,7 +95,6 @@ __device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool 
   const int lane = threadIdx.x & 31;
   if (rigid) advance_colliders(S, lane);
   if (lane == 0) {
-    S.counters[CNT_OVERFLOW] = 0;
     S.counters[CNT_WORK] = 0;
     if (!binned) S.counters[CNT_BINNED] = 0;
     // the magnitudes of the particles the pending P2G scattered become the
@@ -194,12 +194,10 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(const SceneDev* __r
       if (flag[k]) {
         S.blk_flag[b] = 0;
         now = slot++;
-        if (now >= S.pool_cap) {
-          atomicAdd(&S.counters[CNT_OVERFLOW], 1);
-          now = -1;
-        } else {
+        if (now >= S.pool_cap)
+          now = -1;  // (counted by form_prefixes)
+        else
           S.active[now] = b;
-        }
       }
       if (now != old[k]) S.blk_slot[b] = now;
       if (now < 0 && old[k] >= 0) clear_block(S, b);

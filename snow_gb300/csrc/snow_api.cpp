@@ -72,6 +72,7 @@ struct snow_scene {
   // fast mode
   SceneDev sd{};
   SceneDev* sd_dev = nullptr;
+  bool sd_stale = true;  // sd_dev is older than sd (or was never written)
   BinScratch bin{};
   FastTuning tune{};
   int key_bits = 0;
@@ -310,10 +311,14 @@ snow_status push_sd(snow_scene* s) {
   snow_ctx* ctx = s->ctx;
   CK(cudaMemcpyAsync(s->sd_dev, &s->sd, sizeof(SceneDev), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  s->sd_stale = false;
   s->version++;
   drop_graphs(s);
   return SNOW_OK;
 }
+// Before a kernel reads the descriptor: a scene that was uploaded but not yet set
+// up has a newer one on the host.
+snow_status current_sd(snow_scene* s) { return s->sd_stale ? push_sd(s) : SNOW_OK; }
 
 // ---- fast-mode buffers ----------------------------------------------------
 snow_status fast_alloc_particles(snow_scene* s, size_t cap) {
@@ -490,9 +495,9 @@ void fast_enqueue_step(snow_scene* s, bool bin, bool follows, cudaStream_t st, b
 snow_status set_dt(snow_scene* s, float dt) {
   if (s->sd.dt != dt) {
     s->sd.dt = dt;
-    return push_sd(s);
+    s->sd_stale = true;
   }
-  return SNOW_OK;
+  return current_sd(s);
 }
 
 // Checks a copy of the device-side counters for the errors counted there.
@@ -674,6 +679,7 @@ snow_status ref_alloc(snow_scene* s, size_t cap) {
 snow_status ensure_capacity(snow_scene* s, size_t n) {
   if (n == 0) return fail(s->ctx, SNOW_EINVAL, "no particles");
   if (n > 0x7fffffffull) return fail(s->ctx, SNOW_EINVAL, "too many particles");
+  s->sd_stale = true;  // n, and maybe the buffers
   if (s->cap == 0) {
     s->cap = n;
     return s->mode == SNOW_MODE_FAST ? fast_alloc_particles(s, n) : ref_alloc(s, n);
@@ -1317,6 +1323,7 @@ snow_status snow_scene_download(snow_scene* s, float* x, float* v, float* FE, fl
   // written in upload order by the unpack kernel: arrays in page-locked memory
   // in place, the others to a staging buffer and from there by one copy each
   if (!x && !v && !FE && !Jp && !volume) return SNOW_OK;
+  if (snow_status r = current_sd(s)) return r;
   float* out[5] = {x, v, FE, Jp, volume};
   const size_t width[5] = {3, 3, 9, 1, 1};
   float* dev[5] = {};
@@ -1389,6 +1396,7 @@ snow_status snow_scene_download_grid(snow_scene* s, float* mass, float* momentum
     }
     return SNOW_OK;
   }
+  if (snow_status r = current_sd(s)) return r;
   float *dm = nullptr, *dp = nullptr, *df = nullptr, *dv = nullptr;
   std::vector<std::pair<void*, size_t>> tmp;
   size_t tb = 0;
@@ -1423,10 +1431,12 @@ snow_status snow_scene_download_colliders(snow_scene* s, snow_collider* out) {
 
 static snow_status stats_enqueue(snow_scene* s, int k) {
   snow_ctx* ctx = s->ctx;
-  if (s->mode == SNOW_MODE_REFERENCE)
+  if (s->mode == SNOW_MODE_REFERENCE) {
     ref_stats(ref_args(s), ctx->d_stats + k, ctx->d_hstats + k, ctx->stream);
-  else
+  } else {
+    if (snow_status r = current_sd(s)) return r;
     fast_stats(s->sd_dev, (int)s->n, ctx->d_stats + k, ctx->d_hstats + k, ctx->stream);
+  }
   CK(cudaGetLastError());
   return SNOW_OK;
 }
@@ -1486,6 +1496,7 @@ snow_status snow_scene_cell_keys(snow_scene* s, uint32_t* keys, uint32_t* perm) 
   if (!s || !keys) return SNOW_EINVAL;
   snow_ctx* ctx = s->ctx;
   if (s->mode != SNOW_MODE_FAST) return fail(ctx, SNOW_EUNSUPPORTED, "binning runs in SNOW_MODE_FAST");
+  if (snow_status r = current_sd(s)) return r;
   const size_t n = s->n;
   cudaStream_t st = ctx->stream;
   // keys of the current positions, then placed at each particle's upload
@@ -1652,6 +1663,7 @@ snow_status batch_refresh(snow_batch* b, const double* dt) {
   for (int i = 0; i < n; i++) {
     snow_scene* s = b->scenes[i];
     CK(cudaMemcpyAsync(s->sd_dev, &s->sd, sizeof(SceneDev), cudaMemcpyHostToDevice, ctx->stream));
+    s->sd_stale = false;
     drop_graphs(s);
     s->version++;
   }
@@ -1823,9 +1835,9 @@ snow_status snow_scene_set_tuning(snow_scene* s, const snow_tuning* t) {
   s->clean_checks = 0;
   if (s->sd.items_max != t->items_max) {
     s->sd.items_max = t->items_max;
-    snow_status r = push_sd(s);
-    if (r) return r;
+    s->sd_stale = true;
   }
+  if (snow_status r = current_sd(s)) return r;
   // the next step re-bins with the new work split
   if (s->p2g_ready) s->steps_since_sort = s->bin_interval;
   if (split_changed) drop_graphs(s);

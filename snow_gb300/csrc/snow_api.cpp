@@ -1856,8 +1856,11 @@ snow_status snow_batch_set_tuning(snow_batch* b, const snow_tuning* t) {
     s->tune.items_chosen = true;
     s->tune.ctas_per_sm = t->ctas_per_sm;
     s->bin_interval = t->sort_interval;
-    s->sd.items_max = t->items_max;
-    s->version++;  // the batch's next step copies the descriptors
+    if (s->sd.items_max != t->items_max) {
+      s->sd.items_max = t->items_max;
+      s->sd_stale = true;  // copied by the next step, the batch's or the scene's own
+    }
+    s->version++;
     drop_graphs(s);
   }
   for (auto& g : b->graphs) cudaGraphExecDestroy(g.second);

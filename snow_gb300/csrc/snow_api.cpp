@@ -681,8 +681,15 @@ snow_status ensure_capacity(snow_scene* s, size_t n) {
   if (n > 0x7fffffffull) return fail(s->ctx, SNOW_EINVAL, "too many particles");
   s->sd_stale = true;  // n, and maybe the buffers
   if (s->cap == 0) {
-    s->cap = n;
-    return s->mode == SNOW_MODE_FAST ? fast_alloc_particles(s, n) : ref_alloc(s, n);
+    const size_t held = s->allocs.size();
+    const snow_status st = s->mode == SNOW_MODE_FAST ? fast_alloc_particles(s, n) : ref_alloc(s, n);
+    if (st == SNOW_OK) {
+      s->cap = n;
+    } else {  // nothing half allocated stays: the next upload tries again
+      while (s->allocs.size() > held) dfree_one(s->ctx, s, s->allocs.back().first);
+      s->ra.gv = nullptr;
+    }
+    return st;
   }
   if (n > s->cap) return fail(s->ctx, SNOW_EINVAL, "more particles than the scene's capacity");
   return SNOW_OK;

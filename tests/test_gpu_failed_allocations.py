@@ -58,3 +58,25 @@ def test_an_upload_without_room_can_be_repeated(mode, fails):
     got = g.upload().init().step(s.dt, 3).check().download()
     assert all(np.array_equal(got[k], want[k]) for k in KEYS)
     ctx.close()
+
+
+@gpu
+def test_an_init_without_room_can_be_repeated():
+    from snow_gb300 import api, native as N
+    created, uploaded, ready, want = _sizes(N.MODE_FAST)
+    s = _scene()
+    big = scenes.small_scene(n=200, grid_edge=64, seed=652)
+    probe = api.Context(0)
+    keep = api.SimScene(probe, big)
+    held = probe.bytes_in_use
+    keep.close(), probe.close()
+    stage = 4 * 7 * s.n + 1024
+    assert ready - uploaded > stage
+    ctx = api.Context(0, hbm_budget=held + uploaded + stage)
+    other, g = api.SimScene(ctx, big), api.SimScene(ctx, s).upload()
+    for _ in range(2):
+        _refused(g.init)
+    other.close()
+    got = g.init().step(s.dt, 3).check().download()
+    assert all(np.array_equal(got[k], want[k]) for k in KEYS)
+    ctx.close()

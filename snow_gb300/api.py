@@ -143,16 +143,16 @@ class SimScene:
         m = np.ascontiguousarray(s.m if m is None else m, np.float32)
         fe = None if FE is None else np.ascontiguousarray(FE, np.float32)
         fp = None if FP is None else np.ascontiguousarray(FP, np.float32)
+        self.ctx.check(self.L.snow_scene_upload(self.h, N.ptr(x), N.ptr(v), N.ptr(m), N.ptr(fe), N.ptr(fp), len(x)))
         self.n = len(x)
-        self.ctx.check(self.L.snow_scene_upload(self.h, N.ptr(x), N.ptr(v), N.ptr(m), N.ptr(fe), N.ptr(fp), self.n))
         return self
 
     def upload_std140(self, pxm, pv, pfe, pfp):
         a = [np.ascontiguousarray(pxm, np.float32), np.ascontiguousarray(pv, np.int32),
              np.ascontiguousarray(pfe, np.float32), np.ascontiguousarray(pfp, np.float32)]
-        self.n = len(a[0])
         self.ctx.check(self.L.snow_scene_upload_std140(self.h, N.ptr(a[0]), N.ptr(a[1], C.c_int32), N.ptr(a[2]),
-                                                       N.ptr(a[3]), self.n))
+                                                       N.ptr(a[3]), len(a[0])))
+        self.n = len(a[0])
         return self
 
     def set_volume(self, volume):

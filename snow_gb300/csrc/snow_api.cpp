@@ -944,10 +944,13 @@ snow_status snow_scene_upload(snow_scene* s, const float* x, const float* v, con
   snow_ctx* ctx = s->ctx;
   snow_status st = ensure_capacity(s, n);
   if (st) return st;
-  s->n = n;
-  s->initialized = false;
-  s->volume_given = false;
+  auto changes = [&] {  // (what fails before it leaves the scene as it was)
+    s->n = n;
+    s->initialized = false;
+    s->volume_given = false;
+  };
   if (s->mode == SNOW_MODE_REFERENCE) {
+    changes();
     // ParticleSystem::initSSBO: pxm = (x, m), pv = (v * 1e8, 0), FE / FP mat4
     std::vector<float4> pxm(n), pfe(4 * n), pfp(4 * n);
     std::vector<int4> pv(n), zero(n);
@@ -977,7 +980,6 @@ snow_status snow_scene_upload(snow_scene* s, const float* x, const float* v, con
   }
   // the pack kernel reads the caller's arrays where they lie when they are
   // pinned; pageable ones are first copied as they are to a staging buffer
-  s->sd.n = (int)n;
   if (n > 0) {
     const float* in[5] = {x, v, m, FE, FP};
     const size_t width[5] = {3, 3, 1, 9, 9};
@@ -993,6 +995,8 @@ snow_status snow_scene_upload(snow_scene* s, const float* x, const float* v, con
     float* stage = nullptr;
     st = dalloc(ctx, tmp, tmp_bytes, words * sizeof(float), (void**)&stage);
     if (st) return st;
+    changes();
+    s->sd.n = (int)n;
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < 5 && e == cudaSuccess; k++) {
       if (!in[k] || dev[k]) continue;

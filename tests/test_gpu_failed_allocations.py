@@ -61,6 +61,30 @@ def test_an_upload_without_room_can_be_repeated(mode, fails):
 
 
 @gpu
+def test_a_second_upload_without_room_leaves_the_state():
+    """Pageable arrays go through a staging buffer; page-locked ones need none."""
+    import torch
+
+    from snow_gb300 import api, native as N
+    created, uploaded, ready, _ = _sizes(N.MODE_FAST)
+    s = _scene()
+    assert ready - uploaded > 4 * 7 * s.n  # the first upload's staging buffer
+    fe = np.tile(np.eye(3, dtype=np.float32), (s.n, 1, 1)).reshape(-1, 9)
+    out = []
+    for budget in (0, ready + 100):
+        ctx = api.Context(0, hbm_budget=budget)
+        g = api.SimScene(ctx, s).upload().init().step(s.dt, 3)
+        if budget:
+            _refused(lambda: g.upload(FE=fe, FP=fe))
+        g.step(s.dt, 3).check()
+        x = torch.empty((s.n, 3), dtype=torch.float32, pin_memory=True).numpy()
+        assert g.L.snow_scene_download(g.h, N.ptr(x), None, None, None, None, None) == N.SNOW_OK
+        out.append(x.copy())
+        ctx.close()
+    assert np.array_equal(*out)
+
+
+@gpu
 def test_an_init_without_room_can_be_repeated():
     from snow_gb300 import api, native as N
     created, uploaded, ready, want = _sizes(N.MODE_FAST)

@@ -588,6 +588,12 @@ template <int FIELDS> struct StageShape {
 constexpr int kStageFloats = kTile * StageShape<kOutFields>::plane;
 static_assert(kTile * StageShape<kImpFields>::plane <= kStageFloats, "the solve's rows fit the same buffer");
 
+// The shares that a cell's particles are summed in: one up to kShareWhole, beyond
+// it one for each kShare, so that an item whose particles lie in a few cells keeps
+// all half-warps at work.
+constexpr int kShareWhole = 32, kShare = 16;
+constexpr int kShares = kCells + kItemMax / kShare + kItemMax / kShareWhole;
+
 struct ItemShared {
   __align__(16) float stage[kStageFloats];             // G2P: the grid values of the tile's nodes
   // the item's particles: its stretch of each stream (fc from an even particle on)
@@ -601,6 +607,7 @@ struct ItemShared {
   int cstart[kCells + 1];            // first pd slot of each tile cell
   int ccount[kCells];                // particles per tile cell (zero between items)
   short cells[kCells];               // occupied tile cells
+  int shares[kShares + 1];           // ... crowded ones once for each share, with its first pd slot above
   int4 item_q[2];                    // this and the next work item of the CTA
   int scene_q[2];                    // ... and their scenes
   int index_q[2];                    // ... and their indices (total: no item)
@@ -615,6 +622,7 @@ struct ItemShared {
   int unit_pairs;                    // 1: the others two items at a time
   float run_bound;                   // sum of the contribution bounds of the particles in the tile's sums
   float item_bound;                  // ... and of this item's particles headed for the tile
+  int crowded;                       // a cell holds more of the item's particles than kShareWhole
   int wide;                          // some of the item's particles go through wide_scatter
   int abort;                         // 1 + parity of a wait for grid rows that ran out, else 0
   int pabort;                        // ... for particles
@@ -773,7 +781,7 @@ __device__ __forceinline__ void tile_init(ItemShared& sh) {
     mbar_init(&sh.pbar, 1);
     sh.abort = sh.pabort = 0;
     sh.run_bound = sh.item_bound = 0.0f;
-    sh.wide = 0;
+    sh.wide = sh.crowded = 0;
   }
   __syncthreads();
 }
@@ -1283,6 +1291,7 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
     if (inside && fast && finite_w) {
       st.cell = lx + kCellsPerAxis * ly + kCellsPerAxis * kCellsPerAxis * lz;
       st.rank = atomicAdd(&sh.ccount[st.cell], 1);
+      if (st.rank == kShareWhole) sh.crowded = 1;
       tile_bound = bound;
     } else {
       // the particle drifted out of its home block's tile since the last
@@ -1332,11 +1341,103 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
   }
 }
 
+// Sums the shares [k0, k1) of the half-warp's slice into the tile. Cells of a
+// slice often follow each other along x: the row's sums then slide one node
+// instead of being flushed, so only the node that leaves the window goes to the
+// shared tile. share(k, ci, j0, j1): the k-th share's cell and pd slots.
+template <int KIND, class Share>
+__device__ __forceinline__ void sum_shares(ItemShared& sh, int k0, int k1, Share share) {
+  constexpr int NF = P2gFields<KIND>::nf;
+  constexpr bool fix = KIND != kP2gForce;
+  const int l16 = threadIdx.x & 15, b = l16 & 3, c = l16 >> 2;
+  int cur = -1;
+  unsigned acc[4][kAccFields];
+  f32x2 facc[4][3];
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+#pragma unroll
+    for (int f = 0; f < kAccFields; f++) acc[a][f] = 0u;
+#pragma unroll
+    for (int f = 0; f < 3; f++) facc[a][f] = 0ull;
+  }
+  unsigned np = 0;
+  for (int k = k0; k < k1; k++) {
+    int ci, j0, j1;
+    share(k, ci, j0, j1);
+    if (cur >= 0) {
+      const int row = cell_row_node(cur, b, c);
+      const unsigned base_bits = np * (unsigned)kMagicBits;
+      if (ci == cur + 1 && ci % kCellsPerAxis != 0) {
+        // only node 0 leaves the window: flush it, slide the rest
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+          if (fix) {
+            atomicAdd(&sh.tilei[f * kTile3 + row], (int)(acc[0][f] - base_bits));
+            acc[0][f] = acc[1][f];
+            acc[1][f] = acc[2][f];
+            acc[2][f] = acc[3][f];
+            acc[3][f] = base_bits;
+          } else {
+            atomicAdd(&sh.tile[f * kTile3 + row], sum2(facc[0][f]));
+            facc[0][f] = facc[1][f];
+            facc[1][f] = facc[2][f];
+            facc[2][f] = facc[3][f];
+            facc[3][f] = 0ull;
+          }
+        }
+      } else if (fix) {
+        row_flush_fix<NF>(sh, row, acc, base_bits);
+      } else {
+        row_flush(sh, row, facc);
+      }
+    }
+    cell_sums<KIND>(sh, j0, j1, b, c, acc, facc, np);
+    cur = ci;
+  }
+  if (cur >= 0) {
+    if (fix)
+      row_flush_fix<NF>(sh, cell_row_node(cur, b, c), acc, np * (unsigned)kMagicBits);
+    else
+      row_flush(sh, cell_row_node(cur, b, c), facc);
+  }
+}
+
+// An item with a cell of more than kShareWhole particles: its cells in shares (which
+// start at a record's first particle), listed by every warp for itself. With whole
+// cells an item of snow pressed to 300 particles a cell kept one half-warp of sixteen
+// at work, on a chain of 128 pairs: 880 us a step of 1M such particles, 480 in shares.
+template <int KIND>
+__device__ __noinline__ void sum_crowded(ItemShared& sh) {
+  const int lane = threadIdx.x & 31;
+  int n = 0;
+  for (int c0 = 0; c0 < kCells; c0 += 32) {
+    const int ci = min(c0 + lane, kCells - 1), first = sh.cstart[ci];
+    const int count = c0 + lane < kCells ? sh.cstart[ci + 1] - first : 0;
+    const int parts = count > kShareWhole ? (count + kShare - 1) / kShare : (count > 0 ? 1 : 0);
+    int incl = parts;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    for (int q = 0; q < parts; q++)
+      sh.shares[n + incl - parts + q] = ci | (q ? (first + count * q / parts) & ~1 : first) << 16;
+    n += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) sh.shares[n] = sh.cstart[kCells] << 16;
+  __syncwarp();
+  const int hw = threadIdx.x >> 4, nhw = blockDim.x >> 4;
+  sum_shares<KIND>(sh, (n * hw) / nhw, (n * (hw + 1)) / nhw, [&](int k, int& ci, int& j0, int& j1) {
+    ci = sh.shares[k] & 0xffff;
+    j0 = sh.shares[k] >> 16;
+    j1 = sh.shares[k + 1] >> 16;
+  });
+}
+
 template <int KIND, bool RUN = false, bool WIDE = false>
 __device__ __forceinline__ void p2g_sum(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, const P2GStored& st,
                                         const AxisW& w) {
   constexpr int nf = P2gFields<KIND>::nf;
-  constexpr bool fix = KIND != kP2gForce;
   const int lane = threadIdx.x & 31;
   const int my_cell = st.cell;
   if (WIDE && sh.wide) wide_sums(sh, S, bx, by, bz, st, w);  // uniform across the CTA
@@ -1367,7 +1468,7 @@ __device__ __forceinline__ void p2g_sum(ItemShared& sh, const SceneDev& S, int b
       const int v = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += v;
     }
-    ncells = __shfl_sync(0xffffffffu, incl, 31) >> 16;
+    ncells = sh.crowded ? -1 : __shfl_sync(0xffffffffu, incl, 31) >> 16;  // uniform across the CTA
     int at = (incl - sum) & 0xffff;
     occ = (incl - sum) >> 16;
 #pragma unroll
@@ -1405,70 +1506,22 @@ __device__ __forceinline__ void p2g_sum(ItemShared& sh, const SceneDev& S, int b
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kCells; i += blockDim.x) sh.ccount[i] = 0;  // every warp has scanned them
+  if (threadIdx.x == 0) sh.crowded = 0;
   if (RUN && threadIdx.x == 0) {  // every thread has read both bounds
     sh.run_bound += sh.item_bound;
     sh.item_bound = 0.0f;
   }
-  {
-    // half-warp h takes a contiguous slice of the occupied-cell list (the
-    // two halves of a warp get neighbouring slices, whose particle counts
-    // are alike). Cells of a slice often follow each other along x: the
-    // row's sums then slide one node instead of being flushed, so only the
-    // node that leaves the window goes to the shared tile.
-    constexpr int NF = nf;
-    const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
-    const int b = l16 & 3, c = l16 >> 2;
-    const int nhw = blockDim.x >> 4;
-    const int k0 = (ncells * hw) / nhw, k1 = (ncells * (hw + 1)) / nhw;
-    int cur = -1;
-    unsigned acc[4][kAccFields];
-    f32x2 facc[4][3];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-#pragma unroll
-      for (int f = 0; f < kAccFields; f++) acc[a][f] = 0u;
-#pragma unroll
-      for (int f = 0; f < 3; f++) facc[a][f] = 0ull;
-    }
-    unsigned np = 0;
-    for (int k = k0; k < k1; k++) {
-      const int ci = sh.cells[k];
-      if (cur >= 0) {
-        const int row = cell_row_node(cur, b, c);
-        const unsigned base_bits = np * (unsigned)kMagicBits;
-        if (ci == cur + 1 && ci % kCellsPerAxis != 0) {
-          // only node 0 leaves the window: flush it, slide the rest
-#pragma unroll
-          for (int f = 0; f < NF; f++) {
-            if (fix) {
-              atomicAdd(&sh.tilei[f * kTile3 + row], (int)(acc[0][f] - base_bits));
-              acc[0][f] = acc[1][f];
-              acc[1][f] = acc[2][f];
-              acc[2][f] = acc[3][f];
-              acc[3][f] = base_bits;
-            } else {
-              atomicAdd(&sh.tile[f * kTile3 + row], sum2(facc[0][f]));
-              facc[0][f] = facc[1][f];
-              facc[1][f] = facc[2][f];
-              facc[2][f] = facc[3][f];
-              facc[3][f] = 0ull;
-            }
-          }
-        } else if (fix) {
-          row_flush_fix<NF>(sh, row, acc, base_bits);
-        } else {
-          row_flush(sh, row, facc);
-        }
-      }
-      cell_sums<KIND>(sh, sh.cstart[ci], sh.cstart[ci + 1], b, c, acc, facc, np);
-      cur = ci;
-    }
-    if (cur >= 0) {
-      if (fix)
-        row_flush_fix<NF>(sh, cell_row_node(cur, b, c), acc, np * (unsigned)kMagicBits);
-      else
-        row_flush(sh, cell_row_node(cur, b, c), facc);
-    }
+  if (ncells < 0) {
+    sum_crowded<KIND>(sh);
+  } else {
+    // half-warp h takes a contiguous slice of the list (the two halves of a warp get
+    // neighbouring slices, whose particle counts are alike)
+    const int hw = threadIdx.x >> 4, nhw = blockDim.x >> 4;
+    sum_shares<KIND>(sh, (ncells * hw) / nhw, (ncells * (hw + 1)) / nhw, [&](int k, int& ci, int& j0, int& j1) {
+      ci = sh.cells[k];
+      j0 = sh.cstart[ci];
+      j1 = sh.cstart[ci + 1];
+    });
   }
   __syncthreads();
 }

@@ -619,7 +619,7 @@ struct ItemShared {
   int next_issue;                    // ... or starts a run whose grid rows the last warp copies
   int unit_left;                     // items of the unit in hand after the one looked up last
   int unit_tail;                     // runs from this item on are handed out item by item
-  int unit_pairs;                    // 1: the others two items at a time
+  int unit_most;                     // the others as many items at a time (a power of two)
   float run_bound;                   // sum of the contribution bounds of the particles in the tile's sums
   float item_bound;                  // ... and of this item's particles headed for the tile
   int crowded;                       // a cell holds more of the item's particles than kShareWhole

@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kItemMax) k_g2p_advance(const SceneDev* __rest
 // re-binned some scene; such a scene's particles are read from its binned
 // copies (CNT_BINNED) and, like every scene's, written to its streams. WIDE: with
 // the sums of kCellWide particles (in shared memory; else by atomics on acc).
-constexpr int kSingleRounds = 3, kPairRounds = 5;
+constexpr int kSingleRounds = 3, kUnitShare = 4;
 template <bool BINNED, bool WIDE>
 __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* __restrict__ scenes,
                                                        const int* item_prefix, int nscenes) {
@@ -548,14 +548,16 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   tile_init(sh);
   chain_wait();
   const int total = item_prefix[nscenes];
-  // A unit is a run; in the last round of the CTAs (runs that start in the
-  // last gridDim.x items), and in launches of up to three rounds, a single item; and in
-  // launches of up to five rounds, before the last, two of a run's items. A run
-  // costs one copy of the grid rows and one flush, but the CTA that takes it last
-  // works on alone: with whole runs to the end 50 steps of 1M particles took 15.46
-  // ms, with single items in the last round 15.08, in the last two or four 15.13
-  // and 15.21; 16M the same. 32 steps of 262k particles (4.6 rounds): 3.97 ms
-  // all single, 3.85 now; 20 steps of 300k (4.8): 3.16, now 3.12, with whole runs 3.41.
+  // A unit is a run, or unit_most of its items at a time; in the last round of the CTAs
+  // (runs that start in the last gridDim.x items), and in launches of up to three
+  // rounds, a single item. A run costs one copy of the grid rows and one flush, but the
+  // CTA that takes it last works on alone: with whole runs to the end 50 steps of 1M
+  // particles took 15.46 ms, with single items in the last round 15.08, in the last two
+  // or four 15.13 and 15.21; 16M the same. 32 steps of 262k particles (4.6 rounds): 3.97
+  // ms all single, 3.85 in pairs; 20 steps of 300k (4.8): 3.16, 3.12, with whole runs
+  // 3.41. unit_most is about a quarter of a CTA's items, and at least two, because snow
+  // pressed together lies in fewer runs than there are CTAs: 1M particles at 300 to a
+  // cell, 218 runs of up to 31 items, 480 us a step in whole runs, 232 in units of up to four.
   // The counter instead of equal shares of consecutive items: the items differ
   // (surface blocks hold few particles, compressed snow costs more), 24 steps of a
   // 1.5M-particle block on a sphere 12.0 to 11.0 ms, 50 of 1M particles 17.2 to 16.3.
@@ -564,9 +566,9 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   auto unit_at = [&](int u, int s, const int4& it) {
     const int at = it.w > 0 ? 0 : -it.w;  // its place in its run
     if (u - at >= sh.unit_tail) return 1;
-    if (at == 0) return sh.unit_pairs ? min(2, it.w) : it.w;
-    if (sh.unit_pairs && (at & 1) == 0) return min(2, scenes[s].items[u - at - item_prefix[s]].w - at);
-    return 0;
+    const int most = sh.unit_most;
+    if ((at & (most - 1)) != 0) return 0;
+    return min(most, (at == 0 ? it.w : scenes[s].items[u - at - item_prefix[s]].w) - at);
   };
   // the first item of the unit that starts at item u or at one handed out after
   // it, and the unit's length
@@ -588,7 +590,7 @@ __global__ void __launch_bounds__(kItemMax, kItemCtas) k_g2p2g(const SceneDev* _
   if (lastw && lane == 0) {
     const int round = (int)gridDim.x;
     sh.unit_tail = total <= kSingleRounds * round ? 0 : total - round;
-    sh.unit_pairs = total <= kPairRounds * round ? 1 : 0;
+    sh.unit_most = 1 << max(1, __clz(round) - __clz(total / kUnitShare | 1));
     int s0 = 0, len = 1;
     int4 it0 = make_int4(0, 0, 0, 0);
     sh.index_q[0] = next_unit((int)blockIdx.x, s0, it0, len);

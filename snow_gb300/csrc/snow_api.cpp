@@ -543,7 +543,11 @@ int safe_interval(const snow_scene* s, float dt) {
 // there is no wait for the queued steps), adapts the re-binning interval to
 // the share of particle-steps that left their work item's tile since then (above
 // 1/256: as short as the speeds ask; below 1/4096 clean_needed times in a row:
-// doubled, up to the tuned one), and copies the counters again for the next one.
+// doubled) and keeps it within the tuned one, or within what the speeds allow now and
+// kCheckSteps (fewer only where particles do leave: a few fast ones are no reason).
+// Snow in free flight leaves its tiles all at once: 64 steps of 1M particles took 21.3
+// ms instead of 16.7 where the interval was doubled beyond what the speeds allow.
+// Copies the counters again for the next look.
 snow_status fast_check_async(snow_scene* s) {
   snow_ctx* ctx = s->ctx;
   if (s->cnt_pending) {
@@ -561,9 +565,11 @@ snow_status fast_check_async(snow_scene* s) {
       s->bin_interval = s->tune.chosen || safe >= s->bin_interval ? 1 : safe;
       s->clean_checks = 0;
     } else if (delta <= work / 4096.0 && ++s->clean_checks >= s->clean_needed) {
-      s->bin_interval = std::min(s->tune.sort_interval, 2 * s->bin_interval);
+      s->bin_interval *= 2;
       s->clean_checks = 0;
     }
+    const int most = s->tune.chosen ? s->tune.sort_interval : std::max(safe_interval(s, s->last_dt), kCheckSteps);
+    s->bin_interval = std::min(s->bin_interval, most);
     snow_status r = check_counters(s, h);
     if (r) return r;
   }

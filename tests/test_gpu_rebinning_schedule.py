@@ -62,3 +62,20 @@ def test_a_scene_with_a_chosen_interval_after_an_upload_of_slower_snow(ctx):
     assert g.phase_times(reset=True)["binnings"] > 10
     g.upload(slow.x, slow.v, slow.m).init().step(slow.dt, 64).check()
     assert g.phase_times()["binnings"] == 7
+
+
+@gpu
+def test_the_interval_stays_within_what_the_speeds_allow(ctx):
+    """Snow in free flight at a twentieth of a cell a step may go 0.8 / 0.05 = 16 steps
+    between binnings, however long all goes well."""
+    from snow_gb300 import api
+    s = _scene(635, 0.05 * 15.625)  # 0.05 of h = 1/64 m in 1 ms
+    g = api.SimScene(ctx, s).upload().init()
+    binned = [0]
+    for k in range(256):
+        before = g.phase_times()["binnings"]
+        if g.step(s.dt, 1).phase_times()["binnings"] > before:
+            binned.append(k)
+    assert len(binned) > 10 and np.diff(binned).max() <= 16
+    g.check()
+    g.close()

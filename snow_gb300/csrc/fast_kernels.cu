@@ -862,7 +862,8 @@ __global__ void __launch_bounds__(kIoTile) k_pack(const float* __restrict__ x, c
 // link (190 GB/s, what a DMA reaches), so that pinned arrays are written in
 // place: 374 us for 1M particles instead of 107 for unpacking to a staging
 // buffer and 386 for five copies; a viewer's frame of 4k particles 79 to 60 us.
-__global__ void __launch_bounds__(256) k_invert(const SceneDev* __restrict__ sd, size_t n, uint32_t* __restrict__ slot) {
+__global__ void __launch_bounds__(256) k_invert(const SceneDev* __restrict__ sd, size_t n, uint32_t* slot) {
+  chain_next();
   const SceneDev& S = *sd;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const size_t j = S.pid[i];
@@ -874,8 +875,9 @@ __device__ __forceinline__ void io_write(float* dst, const float* src, int n) {
   for (int k = threadIdx.x; k < n; k += kIoTile) __stcs(dst + k, src[k]);
 }
 __global__ void __launch_bounds__(kIoTile) k_unpack(const SceneDev* __restrict__ sd, size_t n,
-                                                    const uint32_t* __restrict__ slot, float* x, float* v, float* FE,
+                                                    const uint32_t* slot, float* x, float* v, float* FE,
                                                     float* Jp, float* volume) {
+  chain_wait();
   const SceneDev& S = *sd;
   __shared__ float sx[3 * kIoTile], sv[3 * kIoTile], se[9 * kIoTile], sj[kIoTile], so[kIoTile];
   for (size_t j0 = blockIdx.x * (size_t)kIoTile; j0 < n; j0 += (size_t)gridDim.x * kIoTile) {
@@ -1070,7 +1072,9 @@ void fast_unpack(const SceneDev* sd_dev, size_t n, uint32_t* slot, float* x, flo
   if (n == 0) return;
   const size_t g = std::min((n + kIoTile - 1) / kIoTile, (size_t)num_sms() * 8);
   k_invert<<<(int)g, 256, 0, st>>>(sd_dev, n, slot);
-  k_unpack<<<(int)g, kIoTile, 0, st>>>(sd_dev, n, slot, x, v, FE, Jp, volume);
+  // (chained: the positions of 4k particles to pageable memory took 26.5 us with one
+  // kernel, 30.8 with two, 24.6 now)
+  launch_after(true, k_unpack, (int)g, kIoTile, 0, st, sd_dev, n, slot, x, v, FE, Jp, volume);
 }
 
 void fast_download_grid(const SceneDev* sd_dev, float* mass, float* mom, float* force, float* vstar,

@@ -1255,6 +1255,18 @@ __device__ __forceinline__ void wide_sums(ItemShared& sh, const SceneDev& S, int
   __syncthreads();
 }
 
+// Whether a binning would bring a particle at this base cell into its item's tile:
+// not one well outside the grid, which is binned to the border.
+__device__ __forceinline__ bool binning_helps(const SceneDev& S, const int base[3]) {
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int home = min(max(base[k], 0), S.dim[k] - 1) & ~3;
+    in = in && base[k] >= home - 1 && base[k] <= home + kCellsPerAxis - 2;
+  }
+  return in;
+}
+
 template <int KIND, bool RUN = false, bool WIDE = false>
 __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int bx, int by, int bz, bool have,
                                           const P2GParticle& q, const AxisW& w, const int base[3], const FixScale& sc,
@@ -1296,7 +1308,7 @@ __device__ __forceinline__ void p2g_count(ItemShared& sh, const SceneDev& S, int
     } else {
       // the particle drifted out of its home block's tile since the last
       // binning, outgrew the fast path's range or is not finite
-      if (!inside) atomicAdd(&S.counters[CNT_FALLBACK], 1);
+      if (!inside && binning_helps(S, base)) atomicAdd(&S.counters[CNT_FALLBACK], 1);
       far = fast && finite_w ? kFarFast : kFarWide;
       if (KIND != kP2gForce && far == kFarWide) atomicAdd(&S.fix->wide, 1u);
       if (KIND == kP2gForce && !q.force) far = kFarNone;

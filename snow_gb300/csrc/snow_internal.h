@@ -80,7 +80,7 @@ enum {
   CNT_ITEMS = 2,      // P2G work items since the last binning
   CNT_NONFINITE = 3,  // particles with a non-finite field (cumulative)
   CNT_HOME = 4,       // unused
-  CNT_FALLBACK = 5,   // particles that left their P2G tile (diagnostic, cumulative)
+  CNT_FALLBACK = 5,   // particles that left their P2G tile and that a binning would help (cumulative)
   CNT_TIMEOUT = 6,    // bounded waits that ran out (cumulative)
   CNT_DONE = 7,       // CTAs of the compaction finished (the last forms the prefixes)
   CNT_BINNED = 8,     // 1: this step's binning left the particles in the binned copies

@@ -79,3 +79,17 @@ def test_the_interval_stays_within_what_the_speeds_allow(ctx):
     assert len(binned) > 10 and np.diff(binned).max() <= 16
     g.check()
     g.close()
+
+
+@gpu
+@pytest.mark.parametrize("beyond", [0.3, 3.0])
+def test_particles_outside_the_grid_are_no_reason_to_bin(ctx, beyond):
+    """A third of the particles lie beyond the grid's end, in no tile wherever they are
+    binned to: slow snow still takes 32 steps between binnings (after the first eight)."""
+    from snow_gb300 import api
+    s = _scene(636, SLOW)
+    s.colliders = []
+    s.x[::3, 0] += np.float32(0.7 + beyond)
+    g = api.SimScene(ctx, s).upload().init().step(s.dt, 128).check()
+    assert g.phase_times()["binnings"] <= 128 // 32
+    g.close()

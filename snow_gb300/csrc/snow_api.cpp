@@ -86,6 +86,7 @@ struct snow_scene {
   int bin_interval = 8;
   int clean_checks = 0;
   int clean_needed = 8;
+  bool old_interval = false;  // the last snapshot counts steps at a longer interval
   int steps_since_check = 0;
   float vmax = 0.0f;         // largest particle speed at the last look (init, checks)
   float interval_dt = -1.0f;  // time step bin_interval was chosen for
@@ -559,10 +560,13 @@ snow_status fast_check_async(snow_scene* s) {
     const long long delta = fb - s->fallbacks_seen;
     s->fallbacks_seen = fb;
     const double work = (double)s->steps_at_snapshot * (double)std::max<size_t>(s->n, 1);
-    if (s->steps_at_snapshot > 0 && delta > work / 256.0) {
+    const int before = s->bin_interval;
+    if (s->old_interval) {
+      s->old_interval = false;  // the snapshot was taken as the interval changed: of steps before
+    } else if (s->steps_at_snapshot > 0 && delta > work / 256.0) {
       const int safe = safe_interval(s, s->last_dt);
-      s->clean_needed = std::min(1024, 4 * s->clean_needed);
       s->bin_interval = s->tune.chosen || safe >= s->bin_interval ? 1 : safe;
+      if (s->bin_interval == 1) s->clean_needed = std::min(1024, 4 * s->clean_needed);
       s->clean_checks = 0;
     } else if (delta <= work / 4096.0 && ++s->clean_checks >= s->clean_needed) {
       s->bin_interval *= 2;
@@ -570,6 +574,7 @@ snow_status fast_check_async(snow_scene* s) {
     }
     const int most = s->tune.chosen ? s->tune.sort_interval : std::max(safe_interval(s, s->last_dt), kCheckSteps);
     s->bin_interval = std::min(s->bin_interval, most);
+    s->old_interval = s->old_interval || s->bin_interval < before;
     snow_status r = check_counters(s, h);
     if (r) return r;
   }
@@ -636,6 +641,7 @@ snow_status fast_init(snow_scene* s) {
   s->bin_interval = s->tune.sort_interval;
   s->clean_checks = 0;
   s->clean_needed = 8;
+  s->old_interval = false;
   s->steps_since_check = 0;
   s->steps_since_sort = 0;
   s->set_ups++;

@@ -93,3 +93,20 @@ def test_particles_outside_the_grid_are_no_reason_to_bin(ctx, beyond):
     g = api.SimScene(ctx, s).upload().init().step(s.dt, 128).check()
     assert g.phase_times()["binnings"] <= 128 // 32
     g.close()
+
+
+@gpu
+def test_an_interval_shortened_once_is_not_shortened_twice(ctx):
+    """A snowball that falls at 0.30 to 0.33 of a cell a step, hits the ground and
+    slides: two to three steps between binnings while it falls. That particles left
+    their tiles is counted in one more look after the interval was shortened for it,
+    which is no reason to bin every step for the next hundred."""
+    from snow_gb300 import api
+    s = scenes.small_scene(n=60_000, grid_edge=64, seed=3, v0=(2.0, -4.0, 1.0), young=2e4)
+    s.dt = 1e-3
+    g = api.SimScene(ctx, s).upload().init().step(s.dt, 72)
+    g.phase_times(reset=True)
+    assert g.step(s.dt, 64).phase_times(reset=True)["binnings"] <= 32
+    g.step(s.dt, 64).phase_times(reset=True)
+    assert g.step(s.dt, 64).check().phase_times()["binnings"] <= 16  # 0.08 of a cell: seven
+    g.close()

@@ -616,15 +616,22 @@ snow_status fast_init(snow_scene* s) {
     s->p2g_ready = false;
   }
   if ((r = fast_single_prefix(s))) return r;
+  if ((r = push_sd(s))) return r;
+  fast_bin(s, st, false);
+  fast_enqueue_p2g(s, true, st);  // gMassCompute
   // The output pool has a slot for every grid block: however far the
   // particles spread, the compaction of a step finds a slot for each block
   // that received sums (the footprint bound always counted the pool at this
   // size). Only the active blocks' slots are written or read in a step.
-  // (Before any sums are formed: they would outlive an allocation that fails.)
-  if (s->sd.pool_cap != s->sd.nblocks && (r = fast_alloc_pool(s, s->sd.nblocks))) return r;
-  if ((r = push_sd(s))) return r;
-  fast_bin(s, st, false);
-  fast_enqueue_p2g(s, true, st);  // gMassCompute
+  // (Allocated while these run.)
+  if (s->sd.pool_cap != s->sd.nblocks) {
+    if ((r = fast_alloc_pool(s, s->sd.nblocks))) {  // the masses go with it
+      CK(cudaMemsetAsync(s->sd.acc, 0, (size_t)s->sd.nblocks * kAccBlockWords * sizeof(unsigned long long), st));
+      CK(cudaMemsetAsync(s->sd.blk_flag, 0, (size_t)s->sd.nblocks * sizeof(int), st));
+      return r;
+    }
+    if ((r = push_sd(s))) return r;
+  }
   fast_enqueue_compact(s, st);
   if (!s->volume_given) fast_volume(s->sd_dev, s->work.items, (int)s->n, st);  // pVolumeCompute
   fast_enqueue_grid(s, true, false, st);                         // clear acc

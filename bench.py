@@ -46,8 +46,8 @@ BYTES_GRID = (0, 40)
 # work split named in TRAFFIC_SOURCE, keyed by (particles, grid edge); other
 # workloads report null: DRAM bytes (read + write) per launch, and warp
 # instructions per launch for the issue roofline.
-TRAFFIC_MEASURED = {(1 << 20, 256): 142.7e6}
-INSTRUCTIONS_MEASURED = {(1 << 20, 256): 143.4e6}
+TRAFFIC_MEASURED = {(1 << 20, 256): 143.0e6}
+INSTRUCTIONS_MEASURED = {(1 << 20, 256): 142.1e6}
 TRAFFIC_SOURCE = ("not counted in this run: separate ncu --set full captures of one k_g2p2g launch of this "
                   "workload (256 particles per item, 2 CTAs per SM, sort interval 8)")
 # warp-instruction issue peak: 152 SMs x 4 schedulers x 2.07 GHz

@@ -2,7 +2,7 @@
 // (fast_kernels.cu: the explicit step; implicit.cu: the semi-implicit
 // velocity solve): B-spline weights, colliders, the P2G quantities of a
 // particle, the shared memory of a work item with its bulk copies (TMA) of
-// pool blocks, the G2P gather, the particle advance and the P2G tile pass.
+// grid rows and particles, the G2P gather, the particle advance and the P2G tile pass.
 #pragma once
 #include "snow_internal.h"
 #include "snow_math.cuh"
@@ -462,19 +462,6 @@ __device__ __forceinline__ int fix_force(float wxa, float gxa, const RowFactors&
   return __float_as_int(__fmaf_rn(gxa, f.kk[r], __fmaf_rn(wxa, f.hh[r], kMagic)));
 }
 
-// Scatter of the 64 stencil nodes of a warp's particles that do not go to the
-// tile straight into acc (global atomics), one particle at a time with two nodes
-// per lane, whose words lie in whole sectors. FAR_FAST: the particle lies outside
-// its work item's tile; its contributions are rounded exactly as the tile path
-// rounds them. FAR_WIDE: it outgrew the fast path's range; each contribution is
-// rounded exactly to int64. K u (kP2gForce): float sums into the
-// low 4 bytes of acc's force words (free between the grid update and the next
-// P2G; the solve's node passes read and clear them), in active blocks alone.
-// A thread per particle took the 448 atomics of each in turn, those of a cell's
-// particles to the same words, and rounded the wide ones in double precision: 8
-// steps of half a cell without a binning (300k particles) took 0.69 ms each, now
-// 0.36; a step whose 131k particles are all wide 1.44, now 0.85.
-//
 // round(a b + h) to an integer, ties to even, with one rounding, in integer
 // arithmetic (a 24 x 24 bit product and a shift): this GPU's double precision is
 // 64 times slower than its single. 0 for what is not finite or reaches 4e18.
@@ -516,6 +503,18 @@ __device__ __forceinline__ long long round_bounded(float a, float b, long long h
   return h + ((t + (1ll << (s - 1)) - 1 + odd) >> s);
 }
 
+// Scatter of the 64 stencil nodes of a warp's particles that do not go to the
+// tile straight into acc (global atomics), one particle at a time with two nodes
+// per lane, whose words lie in whole sectors. FAR_FAST: the particle lies outside
+// its work item's tile; its contributions are rounded exactly as the tile path
+// rounds them. FAR_WIDE: it outgrew the fast path's range or is not finite; each
+// contribution is rounded exactly to int64. K u (kP2gForce): float sums into the
+// low 4 bytes of acc's force words (free between the grid update and the next
+// P2G; the solve's node passes read and clear them), in active blocks alone.
+// A thread per particle took the 448 atomics of each in turn, those of a cell's
+// particles to the same words, and rounded the wide ones in double precision: 8
+// steps of half a cell without a binning (300k particles) took 0.69 ms each, now
+// 0.36; a step whose 131k particles are all wide 1.44, now 0.85.
 enum { kFarNone = 0, kFarFast = 1, kFarWide = 2, kFarTile = 3 };
 struct FarParticle {
   float wx[4], gx[4], wy[4], gy[4], wz[4], gz[4];

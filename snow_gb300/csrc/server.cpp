@@ -254,8 +254,8 @@ void run(snow_server* srv) {
   snow_ctx_destroy(ctx);
 }
 
-// The scene's bound plus its entries in the batch tables (a scene descriptor
-// and four prefix words), rounded up.
+// The scene's bound plus its entries in the batch tables (a scene descriptor,
+// five prefix words and the item counts of the binning's sizes), rounded up.
 size_t footprint_of(const snow_params& p, size_t n) {
   const size_t f = snow_scene_footprint(&p, n);
   return f ? f + 4096 : 0;

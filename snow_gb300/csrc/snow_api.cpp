@@ -880,7 +880,7 @@ size_t snow_scene_footprint(const snow_params* p, size_t n) {
   // An upper bound: particle streams (xm, vv, fa, fb, vq: 16 B, fc: 8 B, pid: 4 B)
   // + binning scratch (2 key + 2 value words, 5 x 16 B + 8 B + 4 B permutation
   // targets, radix histograms) + work items (16 B each) + per block the dense
-  // fixed-point P2G sums (320 64-bit words), flags, slot and bin tables (5 ints) + the output
+  // fixed-point P2G sums (448 64-bit words), flags, slot and bin tables (5 ints) + the output
   // pool at its largest (every block: 384 floats + 1 int) + the upload's
   // staging copy of the caller's arrays (x, v, m, F_E, F_P: 100 B).
   const double tiles = (double)radix_tiles(n);

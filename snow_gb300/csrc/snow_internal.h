@@ -172,7 +172,7 @@ struct SceneDev {
   // blocked grid
   int* blk_slot;    // nblocks: pool slot of the block this step, -1 if inactive
   int* blk_flag;    // nblocks: block received P2G sums since the last compaction
-  unsigned long long* acc;  // nblocks x 320 words: the fixed-point P2G sums, word-major per block (dense)
+  unsigned long long* acc;  // nblocks x 448 words: the fixed-point P2G sums, word-major per block (dense)
   FixState* fix;            // their scales and the magnitudes the next scales are chosen from
   int* active;      // pool_cap: block id of each slot
   // grid-update output, dense over the nodes of the blocked grid (4 bdim per
@@ -307,8 +307,11 @@ void fast_implicit_setup();
 // wait); the scenes' descriptors are written by copies, which nothing is chained to.
 // It takes launches and the kernels' set-up out of a short step: one step of 4k
 // particles with its download 56 to 54 us, 100 steps of 32k 3.70 to 3.64 ms, 20
-// steps of 300k with a binning in most 3.20 to 3.16, 50 of 1M 15.58 to 15.46. A
-// long one loses (12 steps of 16M particles 63.1 to 63.4 ms): hence the limit.
+// steps of 300k with a binning in most 3.20 to 3.16. The gain ends near the limit, and
+// longer steps lose (plain to chained, as many steps as take about 15 ms): 524k
+// particles 8.97 to 8.91 ms, 1M 16.42 to 16.37, 1.5M 15.25 both, 2M 15.07 to 15.12, 4M
+// 14.70 to 14.76, 8M 14.45 both, 16M 28.73 to 28.81; batches of 1.6M, 4M and 8M
+// particles in all the same either way.
 constexpr long long kChainParticles = 1 << 20;
 template <typename... P, typename... A>
 inline void launch_after(bool chained, void (*k)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {

@@ -28,7 +28,9 @@
 
 #include "../../include/snow_mpm.h"
 
-void scene_will_batch(snow_scene* s);  // snow_api.cpp
+// snow_api.cpp
+void scene_will_batch(snow_scene* s);
+snow_status batch_step_each(snow_batch* b, const double* dt, int n_steps, snow_status* each);
 
 namespace {
 
@@ -211,13 +213,14 @@ void run(snow_server* srv) {
       k = std::min(k, j->left);
       dts.push_back(j->dt);
     }
-    snow_status s = snow_batch_step(batch, dts.data(), k);
-    if (s == SNOW_OK) s = snow_ctx_synchronize(ctx);
+    std::vector<snow_status> each(running.size(), SNOW_OK);
+    const snow_status s = batch_step_each(batch, dts.data(), k, each.data());
     bool retired = false;
-    for (Job* j : running) {
-      j->left -= (s == SNOW_OK) ? k : j->left;
+    for (size_t i = 0; i < running.size(); i++) {
+      Job* j = running[i];
+      snow_status js = s == SNOW_OK ? each[i] : s;  // a job's own condition ends that job alone
+      j->left -= js == SNOW_OK ? k : j->left;
       if (j->left > 0) continue;
-      snow_status js = s;
       if (js == SNOW_OK) js = snow_scene_stats(j->scene, &j->result.stats);
       if (js == SNOW_OK && j->result.stats.nonfinite) js = SNOW_ENUMERIC;
       if (js == SNOW_OK && j->keep) {

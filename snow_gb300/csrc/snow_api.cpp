@@ -138,8 +138,9 @@ struct snow_batch {
   bool counted = false;  // in its scenes' `batches`
   size_t bytes = 0;
   std::vector<std::pair<void*, size_t>> allocs;
+  bool quiet = false;  // conditions of a scene do not end the batch's steps (batch_step_each)
   // every scene's counters, written by a kernel into mapped pinned memory at
-  // one checking point and read at the next
+  // one checking point and read at the next; then those batch_step_each reads
   int* h_cnt = nullptr;
   int* d_hcnt = nullptr;
   cudaEvent_t cnt_ev = nullptr;
@@ -1629,7 +1630,7 @@ snow_status snow_batch_create(snow_ctx* ctx, snow_scene* const* scenes, int n, s
     snow_batch_destroy(b);
     return st;
   }
-  if (cudaHostAlloc(&b->h_cnt, sizeof(int) * kCounterStride * n, cudaHostAllocMapped) != cudaSuccess ||
+  if (cudaHostAlloc(&b->h_cnt, sizeof(int) * kCounterStride * 2 * n, cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer((void**)&b->d_hcnt, b->h_cnt, 0) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->cnt_ev, cudaEventDisableTiming) != cudaSuccess) {
     st = cuda_fail(ctx, cudaGetLastError(), "batch counter snapshot");
@@ -1799,7 +1800,7 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
         for (size_t k = 0; k < b->scenes.size(); k++) {
           const int* h = b->h_cnt + k * kCounterStride;
           r = check_counters(b->scenes[k], h);
-          if (r) return r;
+          if (r && !b->quiet) return r;
           b->scenes[k]->vmax = fix_vmax(h);
           fb += (unsigned)h[CNT_FALLBACK];
           parts += (double)b->scenes[k]->n;
@@ -1839,6 +1840,26 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
   CK(cudaGetLastError());
   return SNOW_OK;
 }
+
+}  // extern "C"
+
+// For the server: steps that a scene's own condition (particles that are not
+// finite, a wait that ran out) does not end for the others, waited for; each[i]:
+// the i-th scene's.
+snow_status batch_step_each(snow_batch* b, const double* dt, int n_steps, snow_status* each) {
+  snow_ctx* ctx = b->ctx;
+  const size_t n = b->scenes.size();
+  b->quiet = true;
+  snow_status r = snow_batch_step(b, dt, n_steps);
+  b->quiet = false;
+  if (r) return r;
+  fast_gather_counters(b->d_scenes, (int)n, b->d_hcnt + n * kCounterStride, ctx->stream);
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (size_t i = 0; i < n; i++) each[i] = check_counters(b->scenes[i], b->h_cnt + (n + i) * kCounterStride);
+  return SNOW_OK;
+}
+
+extern "C" {
 
 static bool valid_tuning(const snow_tuning* t) {
   return t && t->sort_interval >= 1 && t->sort_interval <= 64 && t->items_max >= kMinItemMax && t->items_max <= 256 &&

@@ -616,6 +616,7 @@ snow_status fast_init(snow_scene* s) {
     fast_enqueue_grid(s, true, false, st);
     s->p2g_ready = false;
   }
+  CK(cudaMemsetAsync(s->sd.counters + CNT_NONFINITE, 0, sizeof(int), st));  // those of the state before
   if ((r = fast_single_prefix(s))) return r;
   if ((r = push_sd(s))) return r;
   fast_bin(s, st, false);

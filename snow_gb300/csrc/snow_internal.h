@@ -78,7 +78,7 @@ enum {
   CNT_ACTIVE = 0,     // active grid blocks this step
   CNT_OVERFLOW = 1,   // blocks that found no slot in the pool
   CNT_ITEMS = 2,      // P2G work items since the last binning
-  CNT_NONFINITE = 3,  // particles with a non-finite field (cumulative)
+  CNT_NONFINITE = 3,  // particles with a non-finite field (cumulative since the set-up)
   CNT_HOME = 4,       // unused
   CNT_FALLBACK = 5,   // particles that left their P2G tile and that a binning would help (cumulative)
   CNT_TIMEOUT = 6,    // bounded waits that ran out (cumulative)

@@ -60,3 +60,24 @@ def test_a_solve_after_steps_that_skipped_it(ctx):
     assert g.solver_report()["iterations"] == 0
     again = g.upload(v=v).init().step(s.dt, 1).solver_report()
     assert again["iterations"] == new["iterations"]
+
+
+@gpu
+@pytest.mark.parametrize("batched", [False, True])
+def test_a_condition_of_the_state_before_is_not_reported(ctx, batched):
+    from snow_gb300 import api, native as N
+    s = _scene(625)
+    v = s.v.copy()
+    v[3] = np.nan
+    g = api.SimScene(ctx, s).upload(v=v).init().step(s.dt, 4)
+    with pytest.raises(N.SnowError) as e:
+        g.check()
+    assert e.value.status == N.SNOW_ENUMERIC
+    g.upload().init()
+    if batched:
+        b = api.Batch(ctx, [g])
+        b.step(40, dt=[s.dt])
+    else:
+        g.step(s.dt, 40)
+    want = api.SimScene(ctx, s).upload().init().step(s.dt, 40).check().download()
+    assert _same(g.check().download(), want)

@@ -1767,6 +1767,8 @@ snow_status snow_batch_step(snow_batch* b, const double* dt, int n_steps) {
   if (dt)
     for (size_t i = 0; i < b->scenes.size(); i++)
       if (!(dt[i] >= 0.0) || !std::isfinite(dt[i])) return fail(ctx, SNOW_EINVAL, "snow_batch_step: bad dt");
+  for (snow_scene* s : b->scenes)
+    if (!s->initialized) return fail(ctx, SNOW_ESTATE, "snow_batch_step: a scene was uploaded and not set up again");
   cudaStream_t st = ctx->stream;
   for (size_t i = 0; i < b->scenes.size(); i++) {
     snow_scene* s = b->scenes[i];

@@ -1,5 +1,5 @@
 """Calls that need no set-up work on a scene that has none: the device's copy of the
-scene's description is there whenever a kernel reads it."""
+scene's description is there whenever a kernel reads it. Steps are refused."""
 import numpy as np
 import pytest
 
@@ -56,3 +56,23 @@ def test_colliders_of_an_uploaded_scene_can_be_advanced(ctx, dt):
     g.dispatch(N.K_RIGID_ADVANCE, dt)
     assert abs(g.colliders()[-1][1] - (0.1 + dt)) < 1e-7
     g.close()
+
+
+@gpu
+def test_a_batch_does_not_step_a_scene_that_is_not_set_up(ctx):
+    from snow_gb300 import api, native as N
+    scs = [scenes.small_scene(n=900, grid_edge=16, seed=644 + i) for i in range(2)]
+    sims = [api.SimScene(ctx, s).upload().init() for s in scs]
+    b = api.Batch(ctx, sims)
+    dts = [s.dt for s in scs]
+    b.step(2, dt=dts)
+    sims[1].upload()
+    with pytest.raises(N.SnowError) as e:
+        b.step(1, dt=dts)
+    assert e.value.status == N.SNOW_ESTATE
+    sims[1].init()
+    b.step(2, dt=dts)
+    want = api.SimScene(ctx, scs[1]).upload().init().step(dts[1], 2).download()
+    got = sims[1].check().download()
+    assert all(np.array_equal(want[k], got[k]) for k in ("x", "v", "FE", "Jp"))
+    b.close()

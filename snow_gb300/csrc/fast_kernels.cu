@@ -91,7 +91,7 @@ __device__ __forceinline__ void advance_colliders(const SceneDev& S, int lane) {
 // The start of a step for scene S, by one warp: counters reset, the magnitudes
 // moved on and the scales of this step's P2G formed from them, colliders
 // advanced, the solve's scalars cleared.
-__device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool binned) {
+__device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool binned, bool set_up) {
   const int lane = threadIdx.x & 31;
   if (rigid) advance_colliders(S, lane);
   if (lane == 0) {
@@ -114,6 +114,7 @@ __device__ __forceinline__ void begin_scene(const SceneDev& S, bool rigid, bool 
     for (int i = lane; i < (int)(offsetof(CrScalars, skipping) / sizeof(int)); i += 32) c[i] = 0;
     if (lane == 0) {  // a step within kCrSkipSteps of a start below kCrSkipFactor * tol skips the solve
       CrScalars& cs = *S.crs;
+      if (set_up) cs.skip_left = 0;
       cs.skipping = cs.skip_left > 0 ? 1 : 0;
       if (cs.skip_left > 0) cs.skip_left--;
     }
@@ -157,14 +158,14 @@ __device__ __noinline__ void clear_block(const SceneDev& S, int b) {
 constexpr int kCompactThreads = 256;
 __global__ void __launch_bounds__(kCompactThreads) k_compact(const SceneDev* __restrict__ scenes, const int* quad_prefix,
                                                              int nscenes, long long total, int* items_prefix,
-                                                             int* active_prefix, int rigid, int binned) {
+                                                             int* active_prefix, int rigid, int binned, int set_up) {
   constexpr int kWarps = kCompactThreads / 32;
   const int begin_ctas = (nscenes + kWarps - 1) / kWarps;
   chain_next();
   chain_wait();
   if ((int)blockIdx.x < begin_ctas) {
     const int s = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
-    if (s < nscenes) begin_scene(scenes[s], rigid != 0, binned != 0);
+    if (s < nscenes) begin_scene(scenes[s], rigid != 0, binned != 0, set_up != 0);
     return;
   }
   const long long u = ((long long)blockIdx.x - begin_ctas) * kCompactThreads + threadIdx.x;
@@ -1006,11 +1007,11 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
   k_gather_counters<<<(n + 255) / 256, 256, 0, st>>>(scenes, nscenes, out);
 }
 
-void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st) {
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st, bool set_up) {
   const long long g = std::max(1ll, (w.total_quads + kCompactThreads - 1) / kCompactThreads);
   const int begin_ctas = (w.nscenes + kCompactThreads / 32 - 1) / (kCompactThreads / 32);
   launch_after(chained, k_compact, (int)g + begin_ctas, kCompactThreads, 0, st, w.scenes, w.quads, w.nscenes,
-               w.total_quads, w.items, w.active, rigid ? 1 : 0, binned ? 1 : 0);
+               w.total_quads, w.items, w.active, rigid ? 1 : 0, binned ? 1 : 0, set_up ? 1 : 0);
 }
 
 void fast_p2g(const SceneDev* scenes, const SceneDev& sd_host, const int* item_prefix, int nscenes, int grid_ctas,

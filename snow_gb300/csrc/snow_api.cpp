@@ -605,18 +605,13 @@ snow_status fast_init(snow_scene* s) {
   cudaStream_t st = ctx->stream;
   snow_status r;
   s->sd.n = (int)s->n;
-  if (s->sd.crs) {
-    fast_implicit_setup();
-    // the state before may have left steps to skip
-    CK(cudaMemsetAsync(s->sd.crs, 0, sizeof(CrScalars), st));
-  }
+  if (s->sd.crs) fast_implicit_setup();
   if (s->p2g_ready) {
     // the sums of the state before lie in acc, to which the masses would be added
     fast_enqueue_compact(s, st);
     fast_enqueue_grid(s, true, false, st);
     s->p2g_ready = false;
   }
-  CK(cudaMemsetAsync(s->sd.counters + CNT_NONFINITE, 0, sizeof(int), st));  // those of the state before
   if ((r = fast_single_prefix(s))) return r;
   if ((r = push_sd(s))) return r;
   fast_bin(s, st, false);
@@ -634,7 +629,7 @@ snow_status fast_init(snow_scene* s) {
     }
     if ((r = push_sd(s))) return r;
   }
-  fast_enqueue_compact(s, st);
+  fast_compact(s->work, false, false, false, st, true);
   if (!s->volume_given) fast_volume(s->sd_dev, s->work.items, (int)s->n, st);  // pVolumeCompute
   fast_enqueue_grid(s, true, false, st);                         // clear acc
   fast_enqueue_p2g(s, false, st);                                // P2G of step 1
@@ -644,6 +639,8 @@ snow_status fast_init(snow_scene* s) {
   CK(cudaMemcpyAsync(s->h_cnt, s->sd.counters, kCounterStride * sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   s->cnt_pending = false;
+  if (s->h_cnt[CNT_NONFINITE] != 0)  // (a set-up advances nothing: those of the state before)
+    CK(cudaMemsetAsync(s->sd.counters + CNT_NONFINITE, 0, sizeof(int), st));
   s->fallbacks_seen = (long long)(unsigned)s->h_cnt[CNT_FALLBACK];
   s->vmax = fix_vmax(s->h_cnt);
   s->interval_dt = -1.0f;

@@ -264,8 +264,9 @@ void fast_gather_counters(const SceneDev* scenes, int nscenes, int* out, cudaStr
 // Flags -> active list and slots; its first CTAs start the step of every scene
 // (counters, scales of the step's P2G; rigid: the colliders), and the CTA that takes
 // its slots last forms the item and active-block prefixes. binned: the step's binning
-// ran before and left the particles in the binned copies.
-void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st);
+// ran before and left the particles in the binned copies. set_up: of a new state, for
+// which no solve may be skipped on account of the last.
+void fast_compact(const WorkSpace& w, bool rigid, bool binned, bool chained, cudaStream_t st, bool set_up = false);
 // P2G of the stored particle state (set-up, per-kernel dispatches), after a
 // pass over the particles that measures the magnitudes its fixed-point
 // scales are chosen from.
